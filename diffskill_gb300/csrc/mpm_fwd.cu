@@ -30,6 +30,14 @@ Consts<T> make_consts(const LaunchCtx& L) {
   c.x_lo = T(p.lower_bound * p.dx);
   c.x_hi = T(1.0 - 3 * p.dx);
   c.status = L.status;
+  c.m64.dt = double(c.dt);
+  c.m64.lam = double(c.lam);
+  c.m64.ks = double(c.ks);
+  c.m64.p_mass = double(c.p_mass);
+  c.m64.mu2 = 2.0 * double(c.mu);
+  c.m64.mu2ks = c.m64.mu2 * c.m64.ks;
+  c.m64.lamks = c.m64.lam * c.m64.ks;
+  c.m64.ysm = double(c.yield_stress) / c.m64.mu2;
   return c;
 }
 template Consts<float> make_consts<float>(const LaunchCtx&);

@@ -36,8 +36,20 @@ struct alignas(4 * sizeof(T)) Node {
   T x, y, z, w;
 };
 
+// material constants of the particle math in the precision S; FP64 with the
+// products the kernels would otherwise form once per thread on the FP64 pipe
+template <typename S>
+struct MatConsts;
+template <>
+struct MatConsts<double> {
+  double dt, lam, ks, p_mass;
+  double mu2, mu2ks, lamks;  // 2 mu, 2 mu ks, lam ks
+  double ysm;                // yield_stress / (2 mu)
+};
+
 template <typename T>
 struct Consts {
+  MatConsts<double> m64;  // of the constants below, rounded to T first
   int n_grid;
   int n_scenes;
   int64_t n_particles;
@@ -341,26 +353,15 @@ struct P2G {
   S sm1[3];  // s - 1 (FP32: from the shifted SVD, exact as s -> 1)
   S sigc[3], ehat[3], nrm, dg, k, e[3];
   bool yield;
-  S newF[9], J, R[9];
+  S J;
   S em1[3];  // singular values of newF minus 1 (e - 1 when yielding, else s - 1)
-  S A[9];    // newF - R (FP32: U diag(e - 1) V^T, no cancellation)
 };
-template <typename S>
-struct MatConsts {
-  S dt, mu, lam, ys, ks, p_mass;
+template <>
+struct MatConsts<float> {
+  float dt, mu, lam, ys, ks, p_mass;
 };
-// affine = ks (2 mu A newF^T + lam J (J - 1) I) + p_mass C (mpm_simulator.py:213-215)
-template <typename S>
-MPM_DI void p2g_affine(const MatConsts<S>& m, const P2G<S>& P, S Jm1, const S* C, S* affine) {
-  S st[9];
-  mmT(P.A, P.newF, st);
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    S v = S(2) * m.mu * st[i];
-    if (i % 4 == 0) v += m.lam * P.J * Jm1;
-    affine[i] = m.ks * v + m.p_mass * C[i];
-  }
-}
+MPM_DI float two_mu(const MatConsts<float>& m) { return 2.f * m.mu; }
+MPM_DI double two_mu(const MatConsts<double>& m) { return m.mu2; }
 // FP32 p2g math in terms of the displacement D = F_tmp - I.  The stress
 // 2 mu (newF - R) newF^T + lam J (J - 1) I is a difference of numbers near 1
 // (newF, R, J) when it is evaluated as written; in FP32 that cancellation
@@ -396,7 +397,7 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
     eps[i] = above ? log1p_strain(P.sm1[i]) : logf(0.05f);
   }
   const float esum = eps[0] + eps[1] + eps[2];
-  const float mean = fast_div(esum, 3.f);
+  const float mean = third(esum);
 #pragma unroll
   for (int i = 0; i < 3; ++i) P.ehat[i] = eps[i] - mean;
   P.nrm = sqrtf(dot3(P.ehat, P.ehat) + 1e-8f);
@@ -468,61 +469,99 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
     }
   }
 }
-// affine (the APIC matrix with the stress) and, when new_F is given, the
-// updated F; P keeps what the adjoint needs
-template <typename S>
-MPM_DI void p2g_particle(const MatConsts<S>& m, const S* C, const S* F, P2G<S>& P, S* affine, S* new_F) {
-  if constexpr (sizeof(S) == 4) {
-    p2g_particle_f32(m, C, F, P, affine, new_F);
-  } else {
-    // FP64: the reference's order of operations
-    S IC[9], Ftmp[9];
+// FP64 p2g math (mpm_simulator.py:122-129, 166-225) from the left SVD of
+// F_tmp (svd3_left64): (newF - R) newF^T = U diag((e - 1) e) U^T, and the
+// yielding newF = U diag(e) V^T = F_tmp + U diag(e / s - 1) U^T F_tmp, so the
+// forward pass needs no V.  The adjoint's recompute (WithV, new_F null) does.
+template <bool WithV>
+MPM_DI void p2g_particle_f64(const MatConsts<double>& m, const double* C, const double* F, P2G<double>& P,
+                             double* affine, double* new_F) {
+  double IC[9], Ftmp[9], is[3];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) IC[i] = m.dt * C[i] + ((i % 4 == 0) ? S(1) : S(0));
-    mm(IC, F, Ftmp);
-    svd3(Ftmp, P.U, P.s, P.V);
-    S eps[3];
+  for (int i = 0; i < 9; ++i) IC[i] = m.dt * C[i] + ((i % 4 == 0) ? 1.0 : 0.0);
+  mm(IC, F, Ftmp);
+  const bool plain = svd3_left64<WithV>(Ftmp, P.U, P.s, is, P.V);
+  double eps[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      P.sm1[i] = P.s[i] - S(1);
-      P.sigc[i] = (S(0.05) < P.s[i]) ? P.s[i] : S(0.05);
-      eps[i] = mlog(P.sigc[i]);
+  for (int i = 0; i < 3; ++i) {
+    P.sm1[i] = P.s[i] - 1.0;
+    P.sigc[i] = (0.05 < P.s[i]) ? P.s[i] : 0.05;
+    eps[i] = mlog(P.sigc[i]);
+  }
+  const double mean = third(eps[0] + eps[1] + eps[2]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) P.ehat[i] = eps[i] - mean;
+  P.nrm = msqrt(dot3(P.ehat, P.ehat) + 1e-8);
+  P.dg = P.nrm - m.ysm;
+  P.yield = P.dg > 0.0;
+  P.k = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) P.e[i] = P.s[i];
+  if (P.yield) {
+    P.k = fast_div(P.dg, P.nrm);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) P.e[i] = mexp(eps[i] - P.k * P.ehat[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) P.em1[i] = P.e[i] - 1.0;
+  P.J = P.e[0] * P.e[1] * P.e[2];
+  double h[3], UH[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) h[i] = m.mu2ks * P.em1[i] * P.e[i];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) UH[r * 3 + i] = P.U[r * 3 + i] * h[i];
+  const double lj = m.lamks * P.J * (P.J - 1.0);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = i; j < 3; ++j) {
+      double st = UH[i * 3] * P.U[j * 3] + UH[i * 3 + 1] * P.U[j * 3 + 1] + UH[i * 3 + 2] * P.U[j * 3 + 2];
+      if (i == j) st += lj;
+      affine[i * 3 + j] = st + m.p_mass * C[i * 3 + j];
+      if (j != i) affine[j * 3 + i] = st + m.p_mass * C[j * 3 + i];
     }
-    S mean = fast_div(eps[0] + eps[1] + eps[2], S(3));
+  if (new_F) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) P.ehat[i] = eps[i] - mean;
-    P.nrm = msqrt(dot3(P.ehat, P.ehat) + S(1e-8));
-    P.dg = P.nrm - fast_div(m.ys, S(2) * m.mu);
-    P.yield = P.dg > S(0);
+    for (int i = 0; i < 9; ++i) new_F[i] = Ftmp[i];
     if (P.yield) {
-      P.k = fast_div(P.dg, P.nrm);
+      double UW[9];
+      if (plain) {
 #pragma unroll
-      for (int i = 0; i < 3; ++i) P.e[i] = mexp(eps[i] - P.k * P.ehat[i]);
-      S UD[9];
+        for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+          for (int i = 0; i < 3; ++i) UW[r * 3 + i] = P.U[r * 3 + i] * P.e[i];
+        mmT(UW, P.V, new_F);
+      } else {
+        double W[9];  // U diag(e / s - 1) U^T, symmetric
 #pragma unroll
-        for (int cc = 0; cc < 3; ++cc) UD[r * 3 + cc] = P.U[r * 3 + cc] * P.e[cc];
-      mmT(UD, P.V, P.newF);
-    } else {
-      P.k = S(0);
+        for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int i = 0; i < 3; ++i) P.e[i] = S(1);
+          for (int i = 0; i < 3; ++i) UW[r * 3 + i] = P.U[r * 3 + i] * fma(P.e[i], is[i], -1.0);
 #pragma unroll
-      for (int i = 0; i < 9; ++i) P.newF[i] = Ftmp[i];
-    }
-    P.J = det3(P.newF);
-    mmT(P.U, P.V, P.R);
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int i = 0; i < 9; ++i) P.A[i] = P.newF[i] - P.R[i];
+          for (int j = i; j < 3; ++j)
+            W[i * 3 + j] = W[j * 3 + i] =
+                UW[i * 3] * P.U[j * 3] + UW[i * 3 + 1] * P.U[j * 3 + 1] + UW[i * 3 + 2] * P.U[j * 3 + 2];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) P.em1[i] = (P.yield ? P.e[i] : P.s[i]) - S(1);
-    p2g_affine(m, P, P.J - S(1), C, affine);
-    if (new_F) {
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int i = 0; i < 9; ++i) new_F[i] = P.newF[i];
+          for (int j = 0; j < 3; ++j)
+            new_F[i * 3 + j] += W[i * 3] * Ftmp[j] + W[i * 3 + 1] * Ftmp[3 + j] + W[i * 3 + 2] * Ftmp[6 + j];
+      }
     }
   }
+}
+// affine (the APIC matrix with the stress) and, when new_F is given, the
+// updated F; P keeps what the adjoint needs (WithV: the adjoint's recompute)
+template <bool WithV, typename S>
+MPM_DI void p2g_particle(const MatConsts<S>& m, const S* C, const S* F, P2G<S>& P, S* affine, S* new_F) {
+  if constexpr (sizeof(S) == 4)
+    p2g_particle_f32(m, C, F, P, affine, new_F);
+  else
+    p2g_particle_f64<WithV>(m, C, F, P, affine, new_F);
 }
 // gradient of the singular values through the return map (yield branch of
 // compute_von_mises, mpm_simulator.py:166-180), from the diagonal of
@@ -540,7 +579,7 @@ MPM_DI void return_map_sigma_grad(const P2G<S>& P, const S* MN, S* gs) {
   S g_nrm = -fast_div(g_k * P.dg, P.nrm * P.nrm) + fast_div(g_k, P.nrm);
 #pragma unroll
   for (int i = 0; i < 3; ++i) g_ehat[i] += fast_div(g_nrm * P.ehat[i], P.nrm);
-  S sh = fast_div(g_ehat[0] + g_ehat[1] + g_ehat[2], S(3));
+  S sh = third(g_ehat[0] + g_ehat[1] + g_ehat[2]);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     g_eps[i] += g_ehat[i] - sh;
@@ -548,133 +587,75 @@ MPM_DI void return_map_sigma_grad(const P2G<S>& P, const S* MN, S* gs) {
   }
 }
 
-// FP32 adjoint of p2g_particle_f32 in the SVD basis.  With G = U^T g_raw U
+// Adjoint of p2g_particle in the SVD basis.  With G = U^T g_raw U
 // (g_raw = ks g_affine), e' = 1 + em1 the singular values of newF, and the
 // stress's matrices written in the bases U, V:
 //   U^T (g_raw newF) V   = G diag(e')        (the adjoint of A = newF - R)
 //   U^T (g_raw^T A) V    = G^T diag(e' - 1)  (through the right factor newF^T)
-//   U^T cof(newF) V      = J diag(1 / e')    (d det / d newF)
+//   U^T cof(newF) V      = J diag(1 / e')    (d det / d newF; det_grad)
 // M_R = U^T g_R V = -2 mu G diag(e') and M_N = U^T g_newF V need no newF, A
 // or cofactor matrix.  The SVD part is svd3_bwd_factored_basis; the elastic
 // branch's direct newF = F_tmp term joins it in the same basis, so one
 // transform U Y V^T gives the gradient of F_tmp.
-MPM_DI void p2g_particle_vjp_f32(const MatConsts<float>& m, const float* C, const float* F, const P2G<float>& P,
-                                 const float* g_affine, const float* g_newF_in, float* g_C, float* g_F) {
-  float G[9], t9[9], MR[9], MN[9];
+// g d det(newF) / d e'_i
+MPM_DI float det_grad(const P2G<float>& P, float g, int i) { return fast_div(g * P.J, 1.f + P.em1[i]); }
+MPM_DI double det_grad(const P2G<double>& P, double g, int i) { return g * (P.e[(i + 1) % 3] * P.e[(i + 2) % 3]); }
+template <typename S>
+MPM_DI void p2g_particle_vjp(const MatConsts<S>& m, const S* C, const S* F, const P2G<S>& P, const S* g_affine,
+                             const S* g_newF_in, S* g_C, S* g_F) {
+  S G[9], t9[9], MR[9], MN[9];
   {
-    float g_raw[9];
+    S g_raw[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) g_raw[i] = m.ks * g_affine[i];
     mTm(P.U, g_raw, t9);
     mm(t9, P.U, G);
   }
-  const float g_J = m.lam * (2.f * P.J - 1.f) * (G[0] + G[4] + G[8]);  // tr g_raw = tr G
+  const S g_J = m.lam * (S(2) * P.J - S(1)) * (G[0] + G[4] + G[8]);  // tr g_raw = tr G
   mTm(P.U, g_newF_in, t9);
   mm(t9, P.V, MN);
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const float ej = 1.f + P.em1[j];
-      const float a = 2.f * m.mu * G[i * 3 + j] * ej;
+      const S ej = S(1) + P.em1[j];
+      const S a = two_mu(m) * G[i * 3 + j] * ej;
       MR[i * 3 + j] = -a;
-      MN[i * 3 + j] += a + 2.f * m.mu * G[j * 3 + i] * P.em1[j] + (i == j ? fast_div(g_J * P.J, ej) : 0.f);
+      MN[i * 3 + j] += a + two_mu(m) * G[j * 3 + i] * P.em1[j] + (i == j ? det_grad(P, g_J, i) : S(0));
     }
-  float gs[3] = {0.f, 0.f, 0.f}, Y[9];
+  S gs[3] = {S(0), S(0), S(0)}, Y[9];
   if (P.yield) return_map_sigma_grad(P, MN, gs);
-  svd3_bwd_factored_basis(P.s, P.sm1, MR, MN, P.e, P.em1, 1.f - P.k, P.yield, gs, Y);
+  svd3_bwd_factored_basis(P.s, P.sm1, MR, MN, P.e, P.em1, S(1) - P.k, P.yield, gs, Y);
   if (!P.yield) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) Y[i] += MN[i];  // newF = F_tmp
   }
-  float g_Ftmp[9];
+  S g_Ftmp[9];
   mm(P.U, Y, t9);
   mmT(t9, P.V, g_Ftmp);
   mmT(g_Ftmp, F, t9);  // Ftmp = (I + dt C) F
 #pragma unroll
   for (int i = 0; i < 9; ++i) g_C[i] = m.p_mass * g_affine[i] + m.dt * t9[i];
-  float IC[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) IC[i] = m.dt * C[i] + ((i % 4 == 0) ? 1.f : 0.f);
-  mTm(IC, g_Ftmp, g_F);
-}
-
-// FP64 adjoint of p2g_particle: the reference's order of operations, with
-// backward_svd as the reference writes it; g_C, g_F are written
-MPM_DI void p2g_particle_vjp_f64(const MatConsts<double>& m, const double* C, const double* F, const P2G<double>& P,
-                                 const double* g_affine, const double* g_newF_in, double* g_C, double* g_F) {
-  using S = double;
-  S g_raw[9], tmp[9], g_newF[9], g_R[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    g_raw[i] = m.ks * g_affine[i];
-    g_C[i] = m.p_mass * g_affine[i];
-  }
-  mm(g_raw, P.newF, tmp);  // d/dA of tr(g^T A newF^T)
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    g_R[i] = S(-2) * m.mu * tmp[i];
-    g_newF[i] = S(2) * m.mu * tmp[i] + g_newF_in[i];
-  }
-  mTm(g_raw, P.A, tmp);  // d/dnewF of the right factor
-  S g_J = m.lam * (S(2) * P.J - S(1)) * (g_raw[0] + g_raw[4] + g_raw[8]);
-  S cf[9];
-  cof3(P.newF, cf);
-#pragma unroll
-  for (int i = 0; i < 9; ++i) g_newF[i] += S(2) * m.mu * tmp[i] + g_J * cf[i];
-  S gs[3] = {S(0), S(0), S(0)}, g_Ftmp[9], gA[9];
-  S gU[9], gV[9];
-  mm(g_R, P.V, gU);  // R = U V^T
-  mTm(g_R, P.U, gV);
-  if (P.yield) {
-    S GV[9], GtU[9], UtGV[9];
-    mm(g_newF, P.V, GV);
-    mTm(g_newF, P.U, GtU);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int cc = 0; cc < 3; ++cc) {
-        gU[r * 3 + cc] += GV[r * 3 + cc] * P.e[cc];
-        gV[r * 3 + cc] += GtU[r * 3 + cc] * P.e[cc];
-      }
-    mTm(P.U, GV, UtGV);
-    return_map_sigma_grad(P, UtGV, gs);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) g_Ftmp[i] = S(0);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 9; ++i) g_Ftmp[i] = g_newF[i];
-  }
-  svd3_bwd(P.U, P.s, P.V, gU, gs, gV, gA);
-#pragma unroll
-  for (int i = 0; i < 9; ++i) g_Ftmp[i] += gA[i];
-  mmT(g_Ftmp, F, tmp);  // Ftmp = (I + dt C) F
-#pragma unroll
-  for (int i = 0; i < 9; ++i) g_C[i] += m.dt * tmp[i];
   S IC[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) IC[i] = m.dt * C[i] + ((i % 4 == 0) ? S(1) : S(0));
   mTm(IC, g_Ftmp, g_F);
 }
-MPM_DI void p2g_particle_vjp(const MatConsts<float>& m, const float* C, const float* F, const P2G<float>& P,
-                             const float* g_affine, const float* g_newF_in, float* g_C, float* g_F) {
-  p2g_particle_vjp_f32(m, C, F, P, g_affine, g_newF_in, g_C, g_F);
-}
-MPM_DI void p2g_particle_vjp(const MatConsts<double>& m, const double* C, const double* F, const P2G<double>& P,
-                             const double* g_affine, const double* g_newF_in, double* g_C, double* g_F) {
-  p2g_particle_vjp_f64(m, C, F, P, g_affine, g_newF_in, g_C, g_F);
-}
 
 template <typename T, typename S>
 MPM_DI MatConsts<S> mat_consts(const Consts<T>& c) {
-  MatConsts<S> m;
-  m.dt = S(c.dt);
-  m.mu = S(c.mu);
-  m.lam = S(c.lam);
-  m.ys = S(c.yield_stress);
-  m.ks = S(c.ks);
-  m.p_mass = S(c.p_mass);
-  return m;
+  if constexpr (sizeof(S) == 8) {
+    return c.m64;
+  } else {
+    MatConsts<S> m;
+    m.dt = S(c.dt);
+    m.mu = S(c.mu);
+    m.lam = S(c.lam);
+    m.ys = S(c.yield_stress);
+    m.ks = S(c.ks);
+    m.p_mass = S(c.p_mass);
+    return m;
+  }
 }
 
 // flags[scene*NB3 + block] = 1 for the blocks of the stencil at `base` (a lane
@@ -739,8 +720,8 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
     load_row_cg(st, c.ld, p, 3, 3, v);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      C[k] = S(__ldcg(st + (int64_t)(6 + k) * c.ld + p));
-      F[k] = S(__ldcg(st + (int64_t)(15 + k) * c.ld + p));
+      C[k] = to_prec<S>(__ldcg(st + (int64_t)(6 + k) * c.ld + p));
+      F[k] = to_prec<S>(__ldcg(st + (int64_t)(15 + k) * c.ld + p));
     }
     const int sc = __ldcg(pscene + p);  // issued with the state rows
     ok = make_stencil(c, x, s);
@@ -748,17 +729,17 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
     P2G<S> P;
     S aff[9];
     S nF[9];
-    p2g_particle(m, C, F, P, aff, st_out ? nF : (S*)nullptr);
+    p2g_particle<false>(m, C, F, P, aff, st_out ? nF : (S*)nullptr);
     if (st_out) {
 #pragma unroll
-      for (int k = 0; k < 9; ++k) st_out[(int64_t)(15 + k) * c.ld + p] = T(nF[k]);
+      for (int k = 0; k < 9; ++k) st_out[(int64_t)(15 + k) * c.ld + p] = to_prec<T>(nF[k]);
     }
     if (!ok) atomicOr(c.status, MPM_STATUS_OUT_OF_GRID);
     if (!finite(P.J)) atomicOr(c.status, MPM_STATUS_NONFINITE);
     if (ok) {
       scene = sc;
 #pragma unroll
-      for (int k = 0; k < 9; ++k) affine[k] = T(aff[k]) * c.dx;
+      for (int k = 0; k < 9; ++k) affine[k] = to_prec<T>(aff[k]) * c.dx;
 #pragma unroll
       for (int k = 0; k < 3; ++k)
         pm[k] = c.p_mass * v[k] - (affine[3 * k] * s.fx[0] + affine[3 * k + 1] * s.fx[1] + affine[3 * k + 2] * s.fx[2]);
@@ -1447,8 +1428,8 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : ((sizeof(T) == 4 && sizeof(
   load_row_cg(st, c.ld, p, 3, 3, v);
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    C[k] = S(__ldcg(st + (int64_t)(6 + k) * c.ld + p));
-    F[k] = S(__ldcg(st + (int64_t)(15 + k) * c.ld + p));
+    C[k] = to_prec<S>(__ldcg(st + (int64_t)(6 + k) * c.ld + p));
+    F[k] = to_prec<S>(__ldcg(st + (int64_t)(15 + k) * c.ld + p));
   }
   const int scene = __ldcg(pscene + p);  // issued with the state rows
   Stencil<T> s;
@@ -1456,10 +1437,10 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : ((sizeof(T) == 4 && sizeof(
   MatConsts<S> m = mat_consts<T, S>(c);
   P2G<S> P;
   S aff[9];
-  p2g_particle(m, C, F, P, aff, (S*)nullptr);
+  p2g_particle<true>(m, C, F, P, aff, (S*)nullptr);
   T affine[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) affine[k] = T(aff[k]);
+  for (int k = 0; k < 9; ++k) affine[k] = to_prec<T>(aff[k]);
   T gx[3], gv[3] = {T(0), T(0), T(0)};
   load_row_cg(g0, c.ld, p, 0, 3, gx);
   S g_aff[9];
@@ -1540,18 +1521,18 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : ((sizeof(T) == 4 && sizeof(
       gx[d] += c.inv_dx * gfx[d];
     }
 #pragma unroll
-    for (int k = 0; k < 9; ++k) g_aff[k] = S(ga[k]);
+    for (int k = 0; k < 9; ++k) g_aff[k] = to_prec<S>(ga[k]);
   }
   S gF1[9], gC[9], gF[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) gF1[k] = S(g1[(int64_t)(15 + k) * c.ld + p]);
+  for (int k = 0; k < 9; ++k) gF1[k] = to_prec<S>(g1[(int64_t)(15 + k) * c.ld + p]);
   p2g_particle_vjp(m, C, F, P, g_aff, gF1, gC, gF);
   store_row(g0, c.ld, p, 0, 3, gx);
   store_row(g0, c.ld, p, 3, 3, gv);
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    g0[(int64_t)(6 + k) * c.ld + p] = T(gC[k]);
-    g0[(int64_t)(15 + k) * c.ld + p] = T(gF[k]);
+    g0[(int64_t)(6 + k) * c.ld + p] = to_prec<T>(gC[k]);
+    g0[(int64_t)(15 + k) * c.ld + p] = to_prec<T>(gF[k]);
   }
 }
 

@@ -5,6 +5,8 @@
 // sorted by eigenvalue, then U from Gram-Schmidt on B = A V.  Output follows
 // the convention of ti.svd used by plb/engine/mpm_simulator.py:127-129:
 // A = U diag(s) V^T, det U = det V = +1, s0 >= s1 >= |s2|, s2 may be negative.
+// FP32 takes the shifted form (svd3_shifted), FP64 an FP32 decomposition that
+// is refined in FP64 (svd3_left64).
 //
 // Backward: backward_svd of plb/engine/mpm_simulator.py:137-156 with the
 // +-1e-6 clamp of clamp() (184-192) on s_j^2 - s_i^2.
@@ -43,19 +45,94 @@ MPM_DI void rot_tc(float theta, float& t, float& c) {
   c = rsqrtf(fmaf(t, t, 1.0f));
 }
 
-// a / b; FP32 by the approximate reciprocal (|b| < 2^126 here).  Used for the
-// Jacobi angle, and for the SVD backward's 1 / (s_j^2 - s_i^2), whose divisor
+// a / b; FP32 by the approximate reciprocal (|b| < 2^126 here), FP64 by rcp64
+// (1e-30 < |b| < 1e30).  Used for the return map, for the Jacobi angle
+// (angle_div: FP64 divides as such there), and for the SVD backward's 1 / (s_j^2 - s_i^2), whose divisor
 // is clamped to |b| >= 1e-6.  The substep kernels are built with -ftz=true, so
 // a subnormal s_pq compares equal to 0 and is never a divisor.
-MPM_DI double fast_div(double a, double b) { return a / b; }
+MPM_DI double fast_div(double a, double b);  // below
 MPM_DI float fast_div(float a, float b) { return __fdividef(a, b); }
+MPM_DI double angle_div(double a, double b) { return a / b; }  // any quotient
+MPM_DI float angle_div(float a, float b) { return __fdividef(a, b); }
+
+// FP64 arithmetic from FP32 starting values.  GB300 issues one FP64
+// instruction per SM every 16 cycles or more (measured: 19 cycles of the SM per
+// FP64 instruction of a warp in p2g, against a quarter of a cycle for an FP32
+// one), so what can start from an FP32 value does: the reciprocal, the inverse
+// square root and the singular vectors below.
+//
+// cut_f32 drops the low mantissa bits of x (0 outside FP32's normal range, NaN
+// and infinity included); widen is exact for a normal or zero x.  Both are
+// integer operations: the conversion instructions occupy the FP64 pipe.
+MPM_DI float cut_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mag = hi & 0x7fffffffu;
+  const unsigned b = __funnelshift_l(lo, mag, 3) - (896u << 23);  // exponent bias 1023 -> 127
+  const bool in = mag - (897u << 20) < (254u << 20);              // exponents 1 .. 254 of FP32
+  return __uint_as_float((hi & 0x80000000u) | (in ? b & 0x7fffffffu : 0u));
+}
+MPM_DI double widen(float x) {
+  const unsigned b = __float_as_uint(x), mag = b & 0x7fffffffu;
+  const unsigned hi = mag >= (1u << 23) ? (mag >> 3) + (896u << 20) : 0u;
+  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(b << 29));
+}
+// float <-> double as the conversion instructions of a -ftz build give them
+// (subnormals to zero, infinities and NaN kept, nearest-even), in integer
+// operations: for the FP64 particle math on FP32 state
+MPM_DI double exact_f64(float x) {
+  const unsigned b = __float_as_uint(x), mag = b & 0x7fffffffu;
+  const unsigned bias = mag >= 0x7f800000u ? 1792u << 20 : 896u << 20;  // infinity, NaN: exponent 2047
+  const unsigned hi = mag >= (1u << 23) ? (mag >> 3) + bias : 0u;
+  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(mag >= (1u << 23) ? b << 29 : 0u));
+}
+MPM_DI float round_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mag = hi & 0x7fffffffu, sign = hi & 0x80000000u;
+  unsigned b = __funnelshift_l(lo, mag, 3) - (896u << 23);
+  const unsigned rest = lo & 0x1fffffffu;
+  b += (rest > 0x10000000u || (rest == 0x10000000u && (b & 1u))) ? 1u : 0u;
+  const bool normal = mag - (897u << 20) < (254u << 20);
+  const bool nan = mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0u);
+  const unsigned big = nan ? 0x7fffffffu : 0x7f800000u;
+  // an exponent of 0 (2^-127 .. 2^-126) may still round up to 2^-126
+  const bool edge = (mag >> 20) == 896u && b >= (1u << 23) && b < (1u << 24);
+  const unsigned r = normal ? b & 0x7fffffffu : (mag >= (1151u << 20) ? big : (edge ? b : 0u));
+  return __uint_as_float(sign | r);
+}
+// x in the precision T
+template <typename T, typename X>
+MPM_DI T to_prec(X x) {
+  if constexpr (sizeof(T) == sizeof(X))
+    return x;
+  else if constexpr (sizeof(T) == 8)
+    return exact_f64(x);
+  else
+    return round_f32(x);
+}
+// 1 / x for 1e-30 < |x| < 1e30: with y0 = 1/x (1 + e), |e| < 1e-6, from FP32,
+// 1/x = y0 (1 + e + e^2) up to e^3 (Newton's iteration and its next term)
+MPM_DI double rcp64(double x) {
+  const double y = widen(__fdividef(1.f, cut_f32(x)));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+MPM_DI double fast_div(double a, double b) { return a * rcp64(b); }
+// 1 / sqrt(x) and sqrt(x) for 1e-30 < x < 1e30: y0 from FP32, e = 1 - x y0^2,
+// 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3 e^2 / 8) up to 5 e^3 / 16
+MPM_DI double rsqrt64(double x) {
+  const double y = widen(rsqrtf(cut_f32(x)));
+  const double e = fma(-x, y * y, 1.0);
+  return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+MPM_DI float third(float x) { return fast_div(x, 3.f); }
+MPM_DI double third(double x) { return x * (1.0 / 3.0); }
 
 // one Jacobi rotation zeroing s_pq of the symmetric matrix held as
 // (s_pp, s_qq, s_pq, s_rp, s_rq); V columns p, q rotated alongside
 template <typename T>
 MPM_DI void jacobi_rot(T& app, T& aqq, T& apq, T& arp, T& arq, T* V, int p, int q) {
   if (apq == T(0)) return;
-  T theta = fast_div(aqq - app, T(2) * apq);
+  T theta = angle_div(aqq - app, T(2) * apq);
   T t, c;
   rot_tc(theta, t, c);
   T s = t * c;
@@ -253,35 +330,200 @@ MPM_DI void svd3_shifted(const float* D, float* U, float* s, float* sm1, float* 
   }
 }
 
+// Two parts of svd3_left64 that few particles reach, out of line so that the
+// kernels do not carry their registers: Jacobi sweeps in FP64 on a matrix whose
+// eigenvalues nearly coincide (S = s00, s11, s22, s01, s02, s12 and U, both
+// updated), and the plain SVD of a matrix that is inverted, nearly singular or
+// not finite.
+__device__ __noinline__ inline void jacobi64_finish(double* S, double* U) {
+  double a00 = S[0], a11 = S[1], a22 = S[2], a01 = S[3], a02 = S[4], a12 = S[5];
+  for (int sweep = 0; sweep < SvdIters<double>::max_sweeps; ++sweep) {
+    const double off = a01 * a01 + a02 * a02 + a12 * a12;
+    const double dg = a00 * a00 + a11 * a11 + a22 * a22;
+    if (off <= SvdIters<double>::tol * dg) break;
+    jacobi_rot(a00, a11, a01, a02, a12, U, 0, 1);
+    jacobi_rot(a00, a22, a02, a01, a12, U, 0, 2);
+    jacobi_rot(a11, a22, a12, a01, a02, U, 1, 2);
+  }
+  S[0] = a00;
+  S[1] = a11;
+  S[2] = a22;
+}
+__device__ __noinline__ inline void svd3_plain64(const double* A, double* U, double* s, double* V) {
+  svd3(A, U, s, V);
+}
+
+// FP64 SVD A = U diag(s) V^T from the left: U and s^2 are the eigenvectors and
+// eigenvalues of A A^T, V = A^T U diag(1/s).  Unlike svd3 the values are in no
+// particular order (nothing here depends on it), unless `plain` is returned:
+// then the matrix was inverted, nearly singular (s < 0.2) or not finite, and
+// U, s, V and `is` come from svd3, s[2] perhaps negative.  V is written when
+// plain or WithV; is = 1/s when not plain.
+//
+// An FP64 Jacobi rotation costs about 68 FP64 instructions, and svd3 takes
+// four to five sweeps of three: about 900 of the 1,245 FP64 instructions that
+// p2g spent on a particle.  Here the sweeps run in FP32 on the shifted matrix
+// A A^T - I (relative to the strain, as svd3_shifted), and FP64 only refines:
+// - U is orthonormalised by Gram-Schmidt (a unit vector's norm is 1 + O(1e-6),
+//   so 1/|u| is a two-term series);
+// - S = U^T A A^T U is then diagonal but for E of about 1e-6 of the strain;
+//   Q = exp(X) with the antisymmetric X = X1 + X2 of second-order perturbation
+//   theory, X1_pq = E_pq / (S_qq - S_pp), X2_pq = 1/2 [E, X1]_pq / (S_qq - S_pp),
+//   diagonalises it to E X^2, far below FP64's rounding of S for |X| <= 2e-4;
+// - a pair with a larger X (eigenvalues nearly equal, but not within rounding)
+//   takes FP64 sweeps instead (jacobi64_finish).
+// About 180 FP64 instructions.  p2g of 0.76M particles (FP32 state, FP64 SVD):
+// SVD64_P2G; its adjoint: SVD64_ADJ.
+template <bool WithV>
+MPM_DI bool svd3_left64(const double* A, double* U, double* s, double* is, double* V) {
+  double S[6];  // 00, 11, 22, 01, 02, 12
+  {
+    const double* a = A;
+    S[0] = dot3(a, a);
+    S[1] = dot3(a + 3, a + 3);
+    S[2] = dot3(a + 6, a + 6);
+    S[3] = dot3(a, a + 3);
+    S[4] = dot3(a, a + 6);
+    S[5] = dot3(a + 3, a + 6);
+  }
+  {
+    float W[9];
+    float a00 = cut_f32(S[0] - 1.0), a11 = cut_f32(S[1] - 1.0), a22 = cut_f32(S[2] - 1.0);
+    float a01 = cut_f32(S[3]), a02 = cut_f32(S[4]), a12 = cut_f32(S[5]);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) W[k] = (k % 4 == 0) ? 1.f : 0.f;
+    for (int sweep = 0; sweep < SvdIters<float>::max_sweeps; ++sweep) {
+      const float off = a01 * a01 + a02 * a02 + a12 * a12;
+      const float dg = a00 * a00 + a11 * a11 + a22 * a22;
+      if (off <= kShiftedTol * dg + 1e-30f) break;
+      jacobi_rot(a00, a11, a01, a02, a12, W, 0, 1);
+      jacobi_rot(a00, a22, a02, a01, a12, W, 0, 2);
+      jacobi_rot(a11, a22, a12, a01, a02, W, 1, 2);
+    }
+    double u0[3], u1[3], u2[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      u0[r] = widen(W[r * 3]);
+      u1[r] = widen(W[r * 3 + 1]);
+    }
+    double e = 1.0 - dot3(u0, u0);
+    double f = fma(e, fma(e, 0.375, 0.5), 1.0);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) u0[r] *= f;
+    const double d = dot3(u0, u1);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) u1[r] = fma(-d, u0[r], u1[r]);
+    e = 1.0 - dot3(u1, u1);
+    f = fma(e, fma(e, 0.375, 0.5), 1.0);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) u1[r] *= f;
+    cross3(u0, u1, u2);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      U[r * 3] = u0[r];
+      U[r * 3 + 1] = u1[r];
+      U[r * 3 + 2] = u2[r];
+    }
+  }
+  {
+    double B[9];
+    mTm(A, U, B);  // columns b_i = A^T u_i
+    const double b0[3] = {B[0], B[3], B[6]}, b1[3] = {B[1], B[4], B[7]}, b2[3] = {B[2], B[5], B[8]};
+    S[0] = dot3(b0, b0);
+    S[1] = dot3(b1, b1);
+    S[2] = dot3(b2, b2);
+    S[3] = dot3(b0, b1);
+    S[4] = dot3(b0, b2);
+    S[5] = dot3(b1, b2);
+  }
+  const float round = 4e-17f * (cut_f32(S[0]) + cut_f32(S[1]) + cut_f32(S[2]));
+  float x32[3], r32[3], e32[3];
+  double x[3];
+  bool far = false;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {  // pairs (0, 1), (0, 2), (1, 2)
+    const double gap = S[q == 0 ? 1 : 2] - S[q == 2 ? 1 : 0], E = S[3 + q];
+    e32[q] = cut_f32(E);
+    const float g = cut_f32(gap);
+    const bool none = fabsf(e32[q]) <= round;
+    far = far || !(none || fabsf(e32[q]) <= 2e-4f * fabsf(g));
+    r32[q] = none || g == 0.f ? 0.f : __fdividef(1.f, g);
+    const double r = widen(r32[q]);
+    x[q] = E * r;
+    x[q] = fma(fma(-x[q], gap, E), r, x[q]);
+    x32[q] = e32[q] * r32[q];
+  }
+  if (far) {
+    double Sl[6], Ul[9];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) Sl[k] = S[k];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Ul[k] = U[k];
+    jacobi64_finish(Sl, Ul);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) S[k] = Sl[k];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) U[k] = Ul[k];
+  } else {
+    x[0] += widen(0.5f * r32[0] * (-e32[1] * x32[2] - x32[1] * e32[2]));
+    x[1] += widen(0.5f * r32[1] * (e32[0] * x32[2] - x32[0] * e32[2]));
+    x[2] += widen(0.5f * r32[2] * (e32[0] * x32[1] + x32[0] * e32[1]));
+    S[0] -= fma(S[3], x[0], S[4] * x[1]);
+    S[1] += fma(S[3], x[0], -S[5] * x[2]);
+    S[2] += fma(S[4], x[1], S[5] * x[2]);
+    const double a = x[0], b = x[1], c = x[2];
+    const double ha = 0.5 * a, hb = 0.5 * b, hc = 0.5 * c;
+    double Q[9], T1[9];  // I + X + X^2 / 2
+    Q[0] = 1.0 - fma(ha, a, hb * b);
+    Q[1] = fma(-hb, c, a);
+    Q[2] = fma(ha, c, b);
+    Q[3] = fma(-hb, c, -a);
+    Q[4] = 1.0 - fma(ha, a, hc * c);
+    Q[5] = fma(-ha, b, c);
+    Q[6] = fma(ha, c, -b);
+    Q[7] = fma(-ha, b, -c);
+    Q[8] = 1.0 - fma(hb, b, hc * c);
+    mm(U, Q, T1);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) U[k] = T1[k];
+  }
+  const bool plain = !(S[0] > 0.04 && S[1] > 0.04 && S[2] > 0.04 && S[0] < 1e6 && S[1] < 1e6 && S[2] < 1e6 &&
+                       det3(A) > 0.0);
+  if (plain) {
+    double Al[9], Ul[9], sl[3], Vl[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Al[k] = A[k];
+    svd3_plain64(Al, Ul, sl, Vl);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      U[k] = Ul[k];
+      V[k] = Vl[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      s[k] = sl[k];
+      is[k] = 0.0;
+    }
+    return true;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    is[k] = rsqrt64(S[k]);
+    s[k] = S[k] * is[k];
+  }
+  if constexpr (WithV) {
+    mTm(A, U, V);
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) V[r * 3 + k] *= is[k];
+  }
+  return false;
+}
+
 template <typename T>
 MPM_DI T svd_clamp(T a) {
   return a >= T(0) ? (a > T(1e-6) ? a : T(1e-6)) : (a < T(-1e-6) ? a : T(-1e-6));
-}
-
-// gA = U [ (F o (U^T gU - gU^T U)) S + S (F o (V^T gV - gV^T V)) + diag(gs) ] V^T
-template <typename T>
-MPM_DI void svd3_bwd(const T* U, const T* s, const T* V, const T* gU, const T* gs, const T* gV, T* gA) {
-  T ss[3] = {s[0] * s[0], s[1] * s[1], s[2] * s[2]};
-  T UtgU[9], VtgV[9];
-  mTm(U, gU, UtgU);
-  mTm(V, gV, VtgV);
-  T X[9];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      if (i == j) {
-        X[i * 3 + j] = gs[i];
-      } else {
-        T Fij = fast_div(T(1), svd_clamp(ss[j] - ss[i]));
-        T au = UtgU[i * 3 + j] - UtgU[j * 3 + i];  // (U^T gU - gU^T U)_ij
-        T av = VtgV[i * 3 + j] - VtgV[j * 3 + i];
-        X[i * 3 + j] = Fij * (au * s[j] + s[i] * av);
-      }
-    }
-  T T1[9];
-  mm(U, X, T1);
-  mmT(T1, V, gA);
 }
 
 // Divided difference D = (e_j - e_i) / (s_j - s_i) of the return map's new
@@ -307,9 +549,25 @@ MPM_DI float ret_map_dd(float si, float sj, float ds, float ei, float em1i, floa
   }
   return ds != 0.f ? (em1j - em1i) / ds : 0.f;
 }
+// FP64: the series below |u| < 2^-10 (L / u to u^5, E1 to z^5; truncation below
+// 2e-19), above it the quotient keeps 1e-13
+MPM_DI double ret_map_dd(double si, double sj, double ds, double ei, double em1i, double em1j, double a) {
+  if (si > 0.05 && sj > 0.05) {
+    const double ri = rcp64(si), u = ds * ri;
+    if (fabs(u) < 0.0009765625) {
+      const double lg =
+          fma(u, fma(u, fma(u, fma(u, fma(u, -1.0 / 6.0, 0.2), -0.25), 1.0 / 3.0), -0.5), 1.0);
+      const double z = a * u * lg;
+      const double e1 =
+          fma(z, fma(z, fma(z, fma(z, fma(z, 1.0 / 720.0, 1.0 / 120.0), 1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0);
+      return ei * a * ri * e1 * lg;
+    }
+  }
+  return ds != 0.0 ? (em1j - em1i) / ds : 0.0;
+}
 
 // backward_svd (mpm_simulator.py:137-156, clamp 184-192) of the two functions
-// p2g takes of the trial F's SVD, in a form without cancellation (FP32):
+// p2g takes of the trial F's SVD, in a form without cancellation:
 // the rotation R = U V^T (gradient gR) and, when the return map yields,
 // newF = U diag(e) V^T (gradient gN).  Then gU = gR V + gN V diag(e),
 // gV = gR^T U + gN^T U diag(e), and with M_R = U^T gR V, M_N = U^T gN V the
@@ -326,22 +584,23 @@ MPM_DI float ret_map_dd(float si, float sj, float ds, float ei, float em1i, floa
 // such cancellation.  The diagonal X_ii = gs_i (sigma_term) is unchanged.
 // Returns X, the gradient of the SVD's input in the bases U, V (gA =
 // U X V^T).  M_N, e and e - 1 (em1) are read only when `yield`.
-MPM_DI void svd3_bwd_factored_basis(const float* s, const float* sm1, const float* MR, const float* MN,
-                                    const float* e, const float* em1, float a, bool yield, const float* gs, float* X) {
+template <typename T>
+MPM_DI void svd3_bwd_factored_basis(const T* s, const T* sm1, const T* MR, const T* MN, const T* e, const T* em1, T a,
+                                    bool yield, const T* gs, T* X) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) X[i * 4] = gs[i];
   // each unordered pair (i, j) once: D and the clamped factor are symmetric in i, j
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     const int i = q == 2 ? 1 : 0, j = q == 0 ? 1 : 2;
-    const float ds = sm1[j] - sm1[i], sm = s[j] + s[i];  // s_j - s_i from s - 1: exact as s_j -> s_i
-    const float f = fast_div(ds, svd_clamp(ds * sm));    // ds / clamp(s_j^2 - s_i^2); swapping i, j keeps it
-    float Kij = MR[i * 3 + j] - MR[j * 3 + i];
-    float Kji = -Kij;
+    const T ds = sm1[j] - sm1[i], sm = s[j] + s[i];  // s_j - s_i from s - 1: exact as s_j -> s_i
+    const T f = fast_div(ds, svd_clamp(ds * sm));    // ds / clamp(s_j^2 - s_i^2); swapping i, j keeps it
+    T Kij = MR[i * 3 + j] - MR[j * 3 + i];
+    T Kji = -Kij;
     if (yield) {
-      const float D = ret_map_dd(s[i], s[j], ds, e[i], em1[i], em1[j], a);
-      const float se = e[i] + e[j];
-      const float p = 0.5f * (D * sm + se), m = 0.5f * (D * sm - se);
+      const T D = ret_map_dd(s[i], s[j], ds, e[i], em1[i], em1[j], a);
+      const T se = e[i] + e[j];
+      const T p = T(0.5) * (D * sm + se), m = T(0.5) * (D * sm - se);
       Kij += MN[i * 3 + j] * p + MN[j * 3 + i] * m;
       Kji += MN[j * 3 + i] * p + MN[i * 3 + j] * m;
     }
