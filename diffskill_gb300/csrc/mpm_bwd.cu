@@ -25,7 +25,8 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
   Node<T>* g_gin = (Node<T>*)L.grid_c;
   Node<T>* g_gout = (Node<T>*)L.grid_d;
   const int* counter = reinterpret_cast<const int*>(L.blockbuf);
-  const unsigned pb = blocks_for(c.n_particles, 128);
+  constexpr int bs_t = kParticleThreads<T>, bs_s = kParticleThreads<S>;
+  const unsigned pb_t = blocks_for(c.n_particles, bs_t), pb_s = blocks_for(c.n_particles, bs_s);
   const unsigned gb = grid_blocks_launch(L, (int64_t)c.n_scenes * c.NB3);
   const Tool<T>* tools_t = (const Tool<T>*)L.tools_t;
   const T* poses_t = (const T*)L.poses_t;
@@ -38,8 +39,8 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
     if (c.n_particles > 0) {
       // with a grid store the recompute usually exits at once: a grid of one
       // wave of CTAs that stride over the particles
-      const unsigned cap = (unsigned)(L.sm_count * 6);
-      MPM_LAUNCH_PDL(L, MPM_K_P2G_RECOMP, (k_p2g<T, S, true>), store && pb > cap ? cap : pb, 128, c, st0,
+      const unsigned cap = (unsigned)(L.sm_count * (bs_s == 32 ? 16 : 6));
+      MPM_LAUNCH_PDL(L, MPM_K_P2G_RECOMP, (k_p2g<T, S, true>), store && pb_s > cap ? cap : pb_s, bs_s, c, st0,
                      (T*)nullptr, L.pscene, gin, saved);
     }
     MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, gb, 64, c, L.active, counter, gin, gout, tools_t, poses_t,
@@ -54,9 +55,9 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
 #define MPM_G2P_ADJ(K)                                                                                 \
   do {                                                                                                 \
     if (plain)                                                                                         \
-      MPM_LAUNCH(L, MPM_K_G2P_ADJ, K, pb, 128, c, st0, st1, g1, g0, L.pscene, gout, g_gout);           \
+      MPM_LAUNCH(L, MPM_K_G2P_ADJ, K, pb_t, bs_t, c, st0, st1, g1, g0, L.pscene, gout, g_gout);        \
     else                                                                                               \
-      MPM_LAUNCH_PDL(L, MPM_K_G2P_ADJ, K, pb, 128, c, st0, st1, g1, g0, L.pscene, gout, g_gout);       \
+      MPM_LAUNCH_PDL(L, MPM_K_G2P_ADJ, K, pb_t, bs_t, c, st0, st1, g1, g0, L.pscene, gout, g_gout);    \
   } while (0)
     if constexpr (sizeof(T) == 4) {
       if (v == 5)
@@ -96,14 +97,14 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
     const int v = L.tune.p2g_adj_ctas;
     if constexpr (sizeof(T) == 4 && sizeof(S) == 4) {
       if (v == 4)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 4>), pb, 128, c, st0, g1, g0, L.pscene, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 4>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
       else if (v == 6)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 6>), pb, 128, c, st0, g1, g0, L.pscene, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 6>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb, 128, c, st0, g1, g0, L.pscene, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb, 128, c, st0, g1, g0, L.pscene, g_gin);
+      MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
     }
   }
   return cudaGetLastError();

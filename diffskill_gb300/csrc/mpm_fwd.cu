@@ -1,5 +1,7 @@
 // Forward launchers: substep (p2g -> grid_op -> g2p), density grid, density
 // L1 loss and the soft tool-contact distance, for the three precision modes.
+#include <type_traits>
+
 #include "mpm_kernels.cuh"
 #include "mpm_launch.h"
 
@@ -30,14 +32,20 @@ Consts<T> make_consts(const LaunchCtx& L) {
   c.x_lo = T(p.lower_bound * p.dx);
   c.x_hi = T(1.0 - 3 * p.dx);
   c.status = L.status;
-  c.m64.dt = double(c.dt);
-  c.m64.lam = double(c.lam);
-  c.m64.ks = double(c.ks);
-  c.m64.p_mass = double(c.p_mass);
-  c.m64.mu2 = 2.0 * double(c.mu);
-  c.m64.mu2ks = c.m64.mu2 * c.m64.ks;
-  c.m64.lamks = c.m64.lam * c.m64.ks;
-  c.m64.ysm = double(c.yield_stress) / c.m64.mu2;
+  auto fill = [&](auto& m) {
+    using S = std::decay_t<decltype(m.dt)>;
+    const double mu2 = 2.0 * double(c.mu);
+    m.dt = S(c.dt);
+    m.lam = S(c.lam);
+    m.ks = S(c.ks);
+    m.p_mass = S(c.p_mass);
+    m.mu2 = S(mu2);
+    m.mu2ks = S(mu2 * double(c.ks));
+    m.lamks = S(double(c.lam) * double(c.ks));
+    m.ysm = S(double(c.yield_stress) / mu2);
+  };
+  fill(c.m32);
+  fill(c.m64);
   return c;
 }
 template Consts<float> make_consts<float>(const LaunchCtx&);
@@ -120,40 +128,42 @@ cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const d
                                     pose_f, pose_f1, premarked);
   if (e != cudaSuccess) return e;
   if (c.n_particles > 0) {
-    const unsigned pb = blocks_for(c.n_particles, 128);
+    constexpr int bs = kParticleThreads<S>;
+    const unsigned pb = blocks_for(c.n_particles, bs);
     const int64_t* none = nullptr;
     // FP32: the CTAs-per-SM variant the tuning selects
     const int v = L.tune.p2g_ctas;
     if constexpr (sizeof(T) == 4 && sizeof(S) == 4) {
       if (v == 6)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 6>), pb, 128, c, st0, st1, L.pscene, gin, none);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 6>), pb, bs, c, st0, st1, L.pscene, gin, none);
       else if (v == 8)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 8>), pb, 128, c, st0, st1, L.pscene, gin, none);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 8>), pb, bs, c, st0, st1, L.pscene, gin, none);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, 128, c, st0, st1, L.pscene, gin, none);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, gin, none);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, 128, c, st0, st1, L.pscene, gin, none);
+      MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, gin, none);
     }
   }
   MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, grid_blocks_launch(L, (int64_t)c.n_scenes * c.NB3), 64, c, L.active,
              counter, gin, gout, (const Tool<T>*)L.tools_t, (const T*)L.poses_t, L.tool_off,
              store ? *store : MpmGridStore{}, store ? slot : -1, (const int64_t*)nullptr);
   if (c.n_particles > 0) {
-    const unsigned pb = blocks_for(c.n_particles, 128);
+    constexpr int bs = kParticleThreads<T>;
+    const unsigned pb = blocks_for(c.n_particles, bs);
     unsigned char* mark = mark_next ? L.blockbuf + 16 : (unsigned char*)nullptr;
     int* header = reinterpret_cast<int*>(L.blockbuf);
     const int v = L.tune.g2p_ctas;
     if constexpr (sizeof(T) == 4) {
       if (v == 10)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 10>), pb, 128, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 10>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
       else if (v == 12)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 12>), pb, 128, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 12>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, 128, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, 128, c, st0, st1, L.pscene, gout, mark, header);
+      MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
     }
   }
   return cudaGetLastError();

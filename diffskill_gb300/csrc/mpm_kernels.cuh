@@ -36,20 +36,19 @@ struct alignas(4 * sizeof(T)) Node {
   T x, y, z, w;
 };
 
-// material constants of the particle math in the precision S; FP64 with the
-// products the kernels would otherwise form once per thread on the FP64 pipe
+// material constants of the particle math in the precision S, with the
+// products that every thread would otherwise form (on the FP64 pipe, in FP64)
 template <typename S>
-struct MatConsts;
-template <>
-struct MatConsts<double> {
-  double dt, lam, ks, p_mass;
-  double mu2, mu2ks, lamks;  // 2 mu, 2 mu ks, lam ks
-  double ysm;                // yield_stress / (2 mu)
+struct MatConsts {
+  S dt, lam, ks, p_mass;
+  S mu2, mu2ks, lamks;  // 2 mu, 2 mu ks, lam ks
+  S ysm;                // yield_stress / (2 mu)
 };
 
 template <typename T>
 struct Consts {
-  MatConsts<double> m64;  // of the constants below, rounded to T first
+  MatConsts<float> m32;   // of the constants below
+  MatConsts<double> m64;  // the same, rounded to T first
   int n_grid;
   int n_scenes;
   int64_t n_particles;
@@ -66,23 +65,13 @@ struct Consts {
   unsigned int* status;
 };
 
-MPM_DI void atomic_add_node(Node<float>* n, float a, float b, float c, float d) {
-  atomicAdd(reinterpret_cast<float4*>(n), make_float4(a, b, c, d));
-}
-MPM_DI void atomic_add_node(Node<double>* n, double a, double b, double c, double d) {
-  atomicAdd(&n->x, a);
-  atomicAdd(&n->y, b);
-  atomicAdd(&n->z, c);
-  atomicAdd(&n->w, d);
-}
-MPM_DI void atomic_add_node3(Node<float>* n, float a, float b, float c) {
-  atomicAdd(reinterpret_cast<float4*>(n), make_float4(a, b, c, 0.f));
-}
-MPM_DI void atomic_add_node3(Node<double>* n, double a, double b, double c) {
-  atomicAdd(&n->x, a);
-  atomicAdd(&n->y, b);
-  atomicAdd(&n->z, c);
-}
+// Threads per CTA of a particle kernel whose arithmetic is in S.  FP32: 128.
+// FP64: one warp.  The FP64 pipe is shared by an SM and bounds these kernels,
+// so what counts is how evenly the warps spread over the SMs: 10,000 particles
+// are 79 CTAs of 128 threads, four warps on each of 79 SMs and none on the other
+// 73, but 313 CTAs of one warp, two or three on every SM.
+template <typename S>
+constexpr int kParticleThreads = sizeof(S) == 8 ? 32 : 128;
 
 // L2 prefetch of the line holding p (no register, no wait)
 MPM_DI void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -162,38 +151,10 @@ MPM_DI int block_node(const Consts<T>& c, int64_t gb, int l, int* I) {
   return scene;
 }
 
-// Warp-level segmented reduction of the scatter.  Particles are sorted by
-// base cell, so lanes with equal key (scene, base cell) are contiguous and
-// scatter into the same 27 nodes: an inclusive segmented scan leaves each
-// segment's sum in its last lane, which alone issues the atomic.  Lanes with a
-// unique key (out of range, out of grid) form single-lane segments.
-struct WarpSeg {
-  int start;  // first lane of this lane's segment
-  bool tail;  // this lane ends its segment
-  int steps;  // doubling steps that cover the longest segment (warp-uniform)
-};
-MPM_DI WarpSeg warp_segments(long long key) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const long long prev = __shfl_up_sync(full, key, 1);
-  const bool head = lane == 0 || prev != key;
-  const unsigned heads = __ballot_sync(full, head);
-  WarpSeg g;
-  g.start = 31 - __clz(heads & (full >> (31 - lane)));
-  g.tail = lane == 31 || ((heads >> (lane + 1)) & 1u);
-  const unsigned run = __reduce_max_sync(full, (unsigned)(lane - g.start + 1));
-  g.steps = run <= 1 ? 0 : 32 - __clz(run - 1);
-  return g;
-}
-template <typename T>
-MPM_DI T seg_scan(T v, const WarpSeg& g) {
-  const int lane = threadIdx.x & 31;
-  for (int i = 0, d = 1; i < g.steps; ++i, d <<= 1) {
-    const T t = __shfl_up_sync(0xffffffffu, v, d);
-    if (lane - d >= g.start) v += t;
-  }
-  return v;
-}
+// Segmented reduction of the scatter.  Particles are sorted by base cell, so
+// lanes with equal key (scene, base cell) are contiguous and scatter into the
+// same 27 nodes; each run of equal keys is summed before it goes to memory.
+// Lanes with a unique key (out of range, out of grid) form runs of one.
 // Segment ends of a warp for the slab scatter: bit r of `tails` is set when
 // lane r ends its run of equal keys, bit r of `emit` when that run is in the
 // grid (out-of-grid lanes carry unique keys, so they are runs of one).
@@ -206,7 +167,7 @@ MPM_DI void warp_tails(long long key, bool ok, unsigned& tails, unsigned& emit) 
   emit = __ballot_sync(full, tail && ok);
 }
 
-// FP32 slab scatter.  The 27-node stencil is scattered one ox slab (9 nodes)
+// Slab scatter.  The 27-node stencil is scattered one ox slab (9 nodes)
 // at a time: every lane writes its 9 node values into row `lane` of v, then
 // lanes 0..26 read the table by columns, lane = g + 3 j summing column j over
 // rows [11 g, 11 g + 11).  Each run of equal keys closed inside a row group
@@ -218,9 +179,22 @@ MPM_DI void warp_tails(long long key, bool ok, unsigned& tails, unsigned& emit) 
 // 9 l + n) and the loads (slot 99 g + 9 i + j, i.e. 3 g + i + j mod 8 with
 // lane = g + 3 j) fall in distinct 16-byte bank groups within each quarter
 // warp.
-struct SlabStage {
+// FP64: a node's four values are two double2, each in a table of its own with
+// the same stride.  The shuffle scan that FP64 took before cost 4 x 5 additions
+// per node and lane; summed by columns it is 33 rows x 4 per slab and lane
+// (SCAN64).
+template <typename T>
+struct SlabStage;
+template <>
+struct SlabStage<float> {
   float4 v[33][9];  // row 32: read, never used (the open run of group 2 after row 31)
   Node<float>* base[32];  // grid of the row's scene + ax[ox] of the row's base cell
+  int ay[32][3], az[32][3];
+};
+template <>
+struct SlabStage<double> {
+  double2 v[33][9], u[33][9];  // (x, y) and (z, w)
+  Node<double>* base[32];
   int ay[32][3], az[32][3];
 };
 // Packed FP32 pairs (add/mul/fma .f32x2): one instruction for two lanes of
@@ -256,12 +230,12 @@ MPM_DI float4 f4_shfl_up(const float4& a, int d) {
   return make_float4(__shfl_up_sync(0xffffffffu, a.x, d), __shfl_up_sync(0xffffffffu, a.y, d),
                      __shfl_up_sync(0xffffffffu, a.z, d), __shfl_up_sync(0xffffffffu, a.w, d));
 }
-MPM_DI void slab_emit(const SlabStage& sb, int r, int oy, int oz, const float4& a) {
+MPM_DI void slab_emit(const SlabStage<float>& sb, int r, int oy, int oz, const float4& a) {
   atomicAdd(reinterpret_cast<float4*>(sb.base[r] + sb.ay[r][oy] + sb.az[r][oz]), a);
 }
 // call between two __syncwarp()s, after all lanes wrote their row of sb.v
 template <bool Packed = false>
-MPM_DI void slab_reduce(const SlabStage& sb, unsigned tails, unsigned emit) {
+MPM_DI void slab_reduce(const SlabStage<float>& sb, unsigned tails, unsigned emit) {
   const int lane = threadIdx.x & 31;
   // lanes 27..31 (g = 3) read lane 24's cells (a broadcast) and emit nothing
   const int g = lane < 27 ? lane % 3 : 3;
@@ -292,6 +266,64 @@ MPM_DI void slab_reduce(const SlabStage& sb, unsigned tails, unsigned emit) {
   if (g >= 1 && g < 3 && head_row >= 0) {
     f4_add(head, g == 1 ? c1 : c2);
     if ((emit >> head_row) & 1u) slab_emit(sb, head_row, oy, oz, head);
+  }
+}
+// The same for FP64.  W: the fourth value is summed too, and multiplied by wm
+// when it is added to the grid (p2g: the weights' sum times the particle mass).
+template <bool W>
+MPM_DI void slab_reduce64(const SlabStage<double>& sb, unsigned tails, unsigned emit, double wm) {
+  const int lane = threadIdx.x & 31;
+  const int g = lane < 27 ? lane % 3 : 3;
+  const int j = lane < 27 ? lane / 3 : 8;
+  const int oy = j / 3, oz = j - 3 * (j / 3);
+  const int r0 = 11 * (g < 3 ? g : 0);
+  const unsigned mine = g < 3 ? tails >> r0 : 0u;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0}, head[4] = {0.0, 0.0, 0.0, 0.0};
+  int head_row = -1;
+  auto put = [&](int r, const double* a) {
+    if (!((emit >> r) & 1u)) return;
+    Node<double>* n = sb.base[r] + sb.ay[r][oy] + sb.az[r][oz];
+    atomicAdd(&n->x, a[0]);
+    atomicAdd(&n->y, a[1]);
+    atomicAdd(&n->z, a[2]);
+    if (W) atomicAdd(&n->w, wm * a[3]);
+  };
+#pragma unroll 1
+  for (int i = 0; i < 11; ++i) {
+    const double2 lo = sb.v[r0 + i][j], hi = sb.u[r0 + i][j];
+    acc[0] += lo.x;
+    acc[1] += lo.y;
+    acc[2] += hi.x;
+    if (W) acc[3] += hi.y;
+    if ((mine >> i) & 1u) {
+      if (g > 0 && head_row < 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) head[k] = acc[k];
+        head_row = r0 + i;
+      } else {
+        put(r0 + i, acc);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[k] = 0.0;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < (W ? 4 : 3); ++k) {
+    const double c1 = __shfl_up_sync(0xffffffffu, acc[k], 1);
+    const double fwd = acc[k] + ((g == 1 && head_row < 0) ? c1 : 0.0);
+    const double c2 = __shfl_up_sync(0xffffffffu, fwd, 1);
+    head[k] += g == 1 ? c1 : c2;
+  }
+  if (g >= 1 && g < 3 && head_row >= 0) put(head_row, head);
+}
+// the slab's rows start at the grid of the lane's scene
+template <typename T>
+MPM_DI void slab_addresses(SlabStage<T>& sb, const StencilAddr& A) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    sb.ay[lane][k] = A.ay[k];
+    sb.az[lane][k] = A.az[k];
   }
 }
 
@@ -350,18 +382,13 @@ MPM_DI void store_row(T* __restrict__ st, int64_t ld, int64_t p, int r0, int n, 
 template <typename S>
 struct P2G {
   S U[9], s[3], V[9];
+  S is[3];   // 1 / s (FP64 only)
   S sm1[3];  // s - 1 (FP32: from the shifted SVD, exact as s -> 1)
-  S sigc[3], ehat[3], nrm, dg, k, e[3];
+  S sigc[3], ehat[3], nrm, inrm, dg, k, e[3];  // inrm = 1 / nrm (FP64 only)
   bool yield;
   S J;
   S em1[3];  // singular values of newF minus 1 (e - 1 when yielding, else s - 1)
 };
-template <>
-struct MatConsts<float> {
-  float dt, mu, lam, ys, ks, p_mass;
-};
-MPM_DI float two_mu(const MatConsts<float>& m) { return 2.f * m.mu; }
-MPM_DI double two_mu(const MatConsts<double>& m) { return m.mu2; }
 // FP32 p2g math in terms of the displacement D = F_tmp - I.  The stress
 // 2 mu (newF - R) newF^T + lam J (J - 1) I is a difference of numbers near 1
 // (newF, R, J) when it is evaluated as written; in FP32 that cancellation
@@ -401,7 +428,7 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
 #pragma unroll
   for (int i = 0; i < 3; ++i) P.ehat[i] = eps[i] - mean;
   P.nrm = sqrtf(dot3(P.ehat, P.ehat) + 1e-8f);
-  P.dg = P.nrm - fast_div(m.ys, 2.f * m.mu);
+  P.dg = P.nrm - m.ysm;
   P.yield = P.dg > 0.f;
   float* em1 = P.em1;
   float pc[3];  // e - s, the return map's change of the singular values
@@ -441,17 +468,17 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
   // (newF - R) newF^T = U diag(e - 1) V^T V diag(e) U^T = U diag((e - 1) e) U^T
   float h[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) h[i] = em1[i] * (1.f + em1[i]);
-  const float lj = m.lam * P.J * Jm1;
+  for (int i = 0; i < 3; ++i) h[i] = m.mu2ks * em1[i] * (1.f + em1[i]);
+  const float lj = m.lamks * P.J * Jm1;
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = i; j < 3; ++j) {
       float st = P.U[i * 3] * P.U[j * 3] * h[0] + P.U[i * 3 + 1] * P.U[j * 3 + 1] * h[1] +
                  P.U[i * 3 + 2] * P.U[j * 3 + 2] * h[2];
-      st = 2.f * m.mu * st + (i == j ? lj : 0.f);
-      affine[i * 3 + j] = m.ks * st + m.p_mass * C[i * 3 + j];
-      if (j != i) affine[j * 3 + i] = m.ks * st + m.p_mass * C[j * 3 + i];
+      if (i == j) st += lj;
+      affine[i * 3 + j] = st + m.p_mass * C[i * 3 + j];
+      if (j != i) affine[j * 3 + i] = st + m.p_mass * C[j * 3 + i];
     }
   if (new_F) {
     if (P.yield) {
@@ -476,34 +503,39 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
 template <bool WithV>
 MPM_DI void p2g_particle_f64(const MatConsts<double>& m, const double* C, const double* F, P2G<double>& P,
                              double* affine, double* new_F) {
-  double IC[9], Ftmp[9], is[3];
+  double IC[9], Ftmp[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) IC[i] = m.dt * C[i] + ((i % 4 == 0) ? 1.0 : 0.0);
   mm(IC, F, Ftmp);
-  const bool plain = svd3_left64<WithV>(Ftmp, P.U, P.s, is, P.V);
+  const bool plain = svd3_left64<WithV>(Ftmp, P.U, P.s, P.is, P.V);
   double eps[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     P.sm1[i] = P.s[i] - 1.0;
-    P.sigc[i] = (0.05 < P.s[i]) ? P.s[i] : 0.05;
-    eps[i] = mlog(P.sigc[i]);
+    eps[i] = 0.05 < P.s[i] ? log_strain64(P.s[i], P.sm1[i]) : log(0.05);
   }
   const double mean = third(eps[0] + eps[1] + eps[2]);
 #pragma unroll
   for (int i = 0; i < 3; ++i) P.ehat[i] = eps[i] - mean;
-  P.nrm = msqrt(dot3(P.ehat, P.ehat) + 1e-8);
+  const double n2 = dot3(P.ehat, P.ehat) + 1e-8;
+  P.inrm = rsqrt64(n2);
+  P.nrm = n2 * P.inrm;
   P.dg = P.nrm - m.ysm;
   P.yield = P.dg > 0.0;
   P.k = 0.0;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) P.e[i] = P.s[i];
-  if (P.yield) {
-    P.k = fast_div(P.dg, P.nrm);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) P.e[i] = mexp(eps[i] - P.k * P.ehat[i]);
+  for (int i = 0; i < 3; ++i) {
+    P.em1[i] = P.sm1[i];
+    P.e[i] = P.s[i];
   }
+  if (P.yield) {
+    P.k = P.dg * P.inrm;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) P.em1[i] = P.e[i] - 1.0;
+    for (int i = 0; i < 3; ++i) {
+      P.em1[i] = expm1_strain64(fma(-P.k, P.ehat[i], eps[i]));
+      P.e[i] = 1.0 + P.em1[i];
+    }
+  }
   P.J = P.e[0] * P.e[1] * P.e[2];
   double h[3], UH[9];
 #pragma unroll
@@ -538,7 +570,7 @@ MPM_DI void p2g_particle_f64(const MatConsts<double>& m, const double* C, const 
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
-          for (int i = 0; i < 3; ++i) UW[r * 3 + i] = P.U[r * 3 + i] * fma(P.e[i], is[i], -1.0);
+          for (int i = 0; i < 3; ++i) UW[r * 3 + i] = P.U[r * 3 + i] * fma(P.e[i], P.is[i], -1.0);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -576,14 +608,24 @@ MPM_DI void return_map_sigma_grad(const P2G<S>& P, const S* MN, S* gs) {
     g_k -= g_eps2[i] * P.ehat[i];
     g_ehat[i] = -P.k * g_eps2[i];
   }
-  S g_nrm = -fast_div(g_k * P.dg, P.nrm * P.nrm) + fast_div(g_k, P.nrm);
+  S g_nrm;
+  if constexpr (sizeof(S) == 8) {
+    g_nrm = g_k * P.inrm * (S(1) - P.k);  // k = dg / nrm
 #pragma unroll
-  for (int i = 0; i < 3; ++i) g_ehat[i] += fast_div(g_nrm * P.ehat[i], P.nrm);
+    for (int i = 0; i < 3; ++i) g_ehat[i] += g_nrm * P.ehat[i] * P.inrm;
+  } else {
+    g_nrm = -fast_div(g_k * P.dg, P.nrm * P.nrm) + fast_div(g_k, P.nrm);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) g_ehat[i] += fast_div(g_nrm * P.ehat[i], P.nrm);
+  }
   S sh = third(g_ehat[0] + g_ehat[1] + g_ehat[2]);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     g_eps[i] += g_ehat[i] - sh;
-    gs[i] = (S(0.05) < P.s[i]) ? fast_div(g_eps[i], P.sigc[i]) : S(0);
+    if constexpr (sizeof(S) == 8)
+      gs[i] = (S(0.05) < P.s[i]) ? g_eps[i] * P.is[i] : S(0);
+    else
+      gs[i] = (S(0.05) < P.s[i]) ? fast_div(g_eps[i], P.sigc[i]) : S(0);
   }
 }
 
@@ -603,29 +645,25 @@ MPM_DI double det_grad(const P2G<double>& P, double g, int i) { return g * (P.e[
 template <typename S>
 MPM_DI void p2g_particle_vjp(const MatConsts<S>& m, const S* C, const S* F, const P2G<S>& P, const S* g_affine,
                              const S* g_newF_in, S* g_C, S* g_F) {
-  S G[9], t9[9], MR[9], MN[9];
-  {
-    S g_raw[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) g_raw[i] = m.ks * g_affine[i];
-    mTm(P.U, g_raw, t9);
-    mm(t9, P.U, G);
-  }
-  const S g_J = m.lam * (S(2) * P.J - S(1)) * (G[0] + G[4] + G[8]);  // tr g_raw = tr G
+  S G[9], t9[9], MR[9], MN[9];  // here G = U^T g_affine U: ks is in the constants
+  mTm(P.U, g_affine, t9);
+  mm(t9, P.U, G);
+  const S g_J = m.lamks * (S(2) * P.J - S(1)) * (G[0] + G[4] + G[8]);  // tr g_affine = tr G
   mTm(P.U, g_newF_in, t9);
   mm(t9, P.V, MN);
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+  for (int j = 0; j < 3; ++j) {
+    const S cm = m.mu2ks * P.em1[j], ce = m.mu2ks + cm;  // times e' - 1 and e'
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const S ej = S(1) + P.em1[j];
-      const S a = two_mu(m) * G[i * 3 + j] * ej;
+    for (int i = 0; i < 3; ++i) {
+      const S a = ce * G[i * 3 + j];
       MR[i * 3 + j] = -a;
-      MN[i * 3 + j] += a + two_mu(m) * G[j * 3 + i] * P.em1[j] + (i == j ? det_grad(P, g_J, i) : S(0));
+      MN[i * 3 + j] += a + cm * G[j * 3 + i] + (i == j ? det_grad(P, g_J, i) : S(0));
     }
+  }
   S gs[3] = {S(0), S(0), S(0)}, Y[9];
   if (P.yield) return_map_sigma_grad(P, MN, gs);
-  svd3_bwd_factored_basis(P.s, P.sm1, MR, MN, P.e, P.em1, S(1) - P.k, P.yield, gs, Y);
+  svd3_bwd_factored_basis(P.s, P.is, P.sm1, MR, MN, P.e, P.em1, S(1) - P.k, P.yield, gs, Y);
   if (!P.yield) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) Y[i] += MN[i];  // newF = F_tmp
@@ -643,19 +681,11 @@ MPM_DI void p2g_particle_vjp(const MatConsts<S>& m, const S* C, const S* F, cons
 }
 
 template <typename T, typename S>
-MPM_DI MatConsts<S> mat_consts(const Consts<T>& c) {
-  if constexpr (sizeof(S) == 8) {
+MPM_DI const MatConsts<S>& mat_consts(const Consts<T>& c) {
+  if constexpr (sizeof(S) == 8)
     return c.m64;
-  } else {
-    MatConsts<S> m;
-    m.dt = S(c.dt);
-    m.mu = S(c.mu);
-    m.lam = S(c.lam);
-    m.ys = S(c.yield_stress);
-    m.ks = S(c.ks);
-    m.p_mass = S(c.p_mass);
-    return m;
-  }
+  else
+    return c.m32;
 }
 
 // flags[scene*NB3 + block] = 1 for the blocks of the stencil at `base` (a lane
@@ -698,7 +728,7 @@ MPM_DI void mark_stencil_blocks(const Consts<T>& c, bool ok, const int* base, in
 // ---------------------------------------------------------------------------
 // forward kernels
 // ---------------------------------------------------------------------------
-// one 128-particle chunk of p2g (all 128 threads of the block take part)
+// one chunk of p2g, a particle per thread (all threads of the block take part)
 template <typename T, typename S>
 MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restrict__ st_out,
                       const int* __restrict__ pscene, Node<T>* __restrict__ grid, int64_t p) {
@@ -725,7 +755,7 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
     }
     const int sc = __ldcg(pscene + p);  // issued with the state rows
     ok = make_stencil(c, x, s);
-    MatConsts<S> m = mat_consts<T, S>(c);
+    const MatConsts<S>& m = mat_consts<T, S>(c);
     P2G<S> P;
     S aff[9];
     S nF[9];
@@ -750,26 +780,15 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
   const long long key = ok ? cell_key(c, scene, s) : -1 - (long long)(threadIdx.x & 31);
   Node<T>* g = grid + (int64_t)scene * c.G;
   const StencilAddr A = stencil_addr(c, s);
-  constexpr bool slab = sizeof(T) == 4;
   const int lane = threadIdx.x & 31;
-  WarpSeg seg{};
-  unsigned tails = 0, emit = 0;
-  SlabStage* sb = nullptr;
-  if constexpr (slab) {
-    __shared__ SlabStage stage[4];  // one per warp of the 128-thread block
-    sb = &stage[threadIdx.x >> 5];
-    warp_tails(key, ok, tails, emit);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      sb->ay[lane][k] = A.ay[k];
-      sb->az[lane][k] = A.az[k];
-    }
-  } else {
-    seg = warp_segments(key);
-  }
+  unsigned tails, emit;
+  __shared__ SlabStage<T> stage[kParticleThreads<S> / 32];  // one per warp
+  SlabStage<T>* sb = &stage[threadIdx.x >> 5];
+  warp_tails(key, ok, tails, emit);
+  slab_addresses(*sb, A);
   pdl_wait();  // the grid blocks are zeroed by the compaction before
   pdl_trigger();
-  if constexpr (slab) {
+  if constexpr (sizeof(T) == 4) {
     // FP32: the node value wgt (m v + A dp, m) in packed pairs: (x, y) and
     // (z, m), stepped across the stencil by the columns of A (and 0 for m)
     float2 cxA = make_float2(pm[0], pm[1]), cxB = make_float2(pm[2], c.p_mass);
@@ -813,18 +832,12 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
 #pragma unroll
       for (int oy = 0; oy < 3; ++oy) {
         T cz[3] = {cy[0], cy[1], cy[2]};
+        const T wxy = wx * s.w[oy][1];
 #pragma unroll
         for (int oz = 0; oz < 3; ++oz) {
-          const T wgt = wx * s.w[oy][1] * s.w[oz][2];
-          T mv[4];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) mv[k] = wgt * cz[k];
-          mv[3] = wgt * c.p_mass;
-          if (seg.steps) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) mv[k] = seg_scan(mv[k], seg);
-          }
-          if (ok && seg.tail) atomic_add_node(g + ax + A.ay[oy] + A.az[oz], mv[0], mv[1], mv[2], mv[3]);
+          const T wgt = wxy * s.w[oz][2];
+          sb->v[lane][oy * 3 + oz] = make_double2(wgt * cz[0], wgt * cz[1]);
+          sb->u[lane][oy * 3 + oz] = make_double2(wgt * cz[2], wgt);
 #pragma unroll
           for (int k = 0; k < 3; ++k) cz[k] += affine[3 * k + 2];
         }
@@ -833,6 +846,10 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k) cx[k] += affine[3 * k];
+      sb->base[lane] = g + ax;
+      __syncwarp();
+      slab_reduce64<true>(*sb, tails, emit, c.p_mass);
+      __syncwarp();
     }
   }
 }
@@ -842,7 +859,7 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
 // Strided: the CTAs stride over the particle chunks (the adjoint's recompute,
 // which exits at once when the grid store holds the substep)
 template <typename T, typename S, bool Strided = false, int MB = 0>
-__global__ void __launch_bounds__(128, MB > 0 ? MB : ((sizeof(T) == 4 && sizeof(S) == 4) ? 7 : 4)) k_p2g(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
+__global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 7 : 16)) k_p2g(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
                                              const int* __restrict__ pscene, Node<T>* __restrict__ grid,
                                              const int64_t* __restrict__ saved) {
   if (saved && __ldcg(saved) >= 0) {  // the grid of this substep was restored from the grid store
@@ -923,8 +940,8 @@ MPM_DI void walls(const Consts<T>& c, const int* I, T* v, WallTape<T>* tp) {
       } else if (c.ground_friction < T(10)) {
         T lin = v[1] + T(1e-30);
         T vit[3] = {v[0] - T(I[0]) * T(1e-30), v[1] - lin - T(I[1]) * T(1e-30), v[2] - T(I[2]) * T(1e-30)};
-        T lit = msqrt(dot3(vit, vit) + T(1e-8));
-        T a = T(1) + c.ground_friction * lin / lit;
+        T lit = len8(vit);
+        T a = T(1) + quot(c.ground_friction * lin, lit);
         T fac = (T(0) < a) ? a : T(0);
 #pragma unroll
         for (int k = 0; k < 3; ++k) v[k] = fac * (vit[k] + T(I[k]) * T(1e-30));
@@ -950,8 +967,8 @@ MPM_DI void walls_vjp(const Consts<T>& c, const int* I, const WallTape<T>& tp, T
       const T* v = tp.v_pre[d];
       T lin = v[1] + T(1e-30);
       T vit[3] = {v[0] - T(I[0]) * T(1e-30), v[1] - lin - T(I[1]) * T(1e-30), v[2] - T(I[2]) * T(1e-30)};
-      T lit = msqrt(dot3(vit, vit) + T(1e-8));
-      T a = T(1) + c.ground_friction * lin / lit;
+      T lit = len8(vit);
+      T a = T(1) + quot(c.ground_friction * lin, lit);
       T fac = (T(0) < a) ? a : T(0);
       const T go[3] = {g[0], T(0), g[2]};
       const T w[3] = {vit[0] + T(I[0]) * T(1e-30), vit[1] + T(I[1]) * T(1e-30), vit[2] + T(I[2]) * T(1e-30)};
@@ -959,11 +976,11 @@ MPM_DI void walls_vjp(const Consts<T>& c, const int* I, const WallTape<T>& tp, T
       T g_vit[3] = {fac * go[0], fac * go[1], fac * go[2]};
       T g_lin = T(0), g_lit = T(0);
       if (T(0) < a) {
-        g_lin = g_fac * c.ground_friction / lit;
-        g_lit = -g_fac * c.ground_friction * lin / (lit * lit);
+        g_lin = quot(g_fac * c.ground_friction, lit);
+        g_lit = quot(-g_fac * c.ground_friction * lin, lit * lit);
       }
 #pragma unroll
-      for (int k = 0; k < 3; ++k) g_vit[k] += g_lit * vit[k] / lit;
+      for (int k = 0; k < 3; ++k) g_vit[k] += quot(g_lit * vit[k], lit);
       g_lin -= g_vit[1];
       g[0] = g_vit[0];
       g[1] = g_vit[1] + g_lin;
@@ -973,6 +990,10 @@ MPM_DI void walls_vjp(const Consts<T>& c, const int* I, const WallTape<T>& tp, T
     }
   }
 }
+
+// 1 / m of a node with mass (m > 1e-12)
+MPM_DI float node_rcp(float m) { return 1.f / m; }
+MPM_DI double node_rcp(double m) { return rcp64(m); }
 
 // grid_op over the active blocks: one 64-thread CTA per block, grid-stride.
 // store_slot >= 0: list block b of grid_in and of grid_out are also copied to
@@ -1008,7 +1029,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<
     }
     Node<T> out = {T(0), T(0), T(0), in.w};
     if (in.w > T(1e-12)) {
-      T inv = T(1) / in.w;
+      T inv = node_rcp(in.w);
       T v[3] = {inv * in.x + c.gdt[0], inv * in.y + c.gdt[1], inv * in.z + c.gdt[2]};
       const T p[3] = {T(I[0]) * c.dx, T(I[1]) * c.dx, T(I[2]) * c.dx};
       for (int t = 0; t < sh.n; ++t) tool_collide(sh.tool[t], sh.p0(t), sh.p1(t), p, c.dt, v);
@@ -1088,7 +1109,7 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
 // At least MB CTAs of 128 threads per SM (MpmTuning.g2p_ctas; 0 = 8 in FP32:
 // at most 64 registers)
 template <typename T, int MB = 0>
-__global__ void __launch_bounds__(128, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k_g2p(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
+__global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k_g2p(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
                                              const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
                                              unsigned char* __restrict__ mark, int* __restrict__ header) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1120,7 +1141,7 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k
 // small spill; measured 20 % faster than the unconstrained 108 registers);
 // MB > 0: MB CTAs per SM (MpmTuning.g2p_adj_ctas)
 template <typename T, int MB = 0>
-__global__ void __launch_bounds__(128, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 2)) k_g2p_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ st1,
+__global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 8)) k_g2p_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ st1,
                                                  const T* __restrict__ g1, T* __restrict__ g0,
                                                  const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
                                                  Node<T>* __restrict__ g_grid) {
@@ -1189,23 +1210,12 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 2)) k
     }
   }
   const long long key = ok ? cell_key(c, scene, s) : -1 - (long long)(threadIdx.x & 31);
-  constexpr bool slab = sizeof(T) == 4;
   const int lane = threadIdx.x & 31;
-  WarpSeg seg{};
-  unsigned tails = 0, emit = 0;
-  SlabStage* sb = nullptr;
-  if constexpr (slab) {
-    __shared__ SlabStage stage[4];  // one per warp of the 128-thread block
-    sb = &stage[threadIdx.x >> 5];
-    warp_tails(key, ok, tails, emit);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      sb->ay[lane][k] = A.ay[k];
-      sb->az[lane][k] = A.az[k];
-    }
-  } else {
-    seg = warp_segments(key);
-  }
+  unsigned tails, emit;
+  __shared__ SlabStage<T> stage[kParticleThreads<T> / 32];  // one per warp
+  SlabStage<T>* sb = &stage[threadIdx.x >> 5];
+  warp_tails(key, ok, tails, emit);
+  slab_addresses(*sb, A);
   const T k4 = T(4) * c.inv_dx;
   T gw[3][3];
 #pragma unroll
@@ -1266,15 +1276,11 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 2)) k
 #pragma unroll
       for (int oz = 0; oz < 3; ++oz) {
         const T wgt = wx * s.w[oy][1] * s.w[oz][2];
-        T sc3[3] = {wgt * uz[0], wgt * uz[1], wgt * uz[2]};
-        if constexpr (slab) {
-          sb->v[lane][oy * 3 + oz] = make_float4(sc3[0], sc3[1], sc3[2], 0.f);
+        if constexpr (sizeof(T) == 4) {
+          sb->v[lane][oy * 3 + oz] = make_float4(wgt * uz[0], wgt * uz[1], wgt * uz[2], 0.f);
         } else {
-          if (seg.steps) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) sc3[k] = seg_scan(sc3[k], seg);
-          }
-          if (ok && seg.tail) atomic_add_node3(gg + ax + A.ay[oy] + A.az[oz], sc3[0], sc3[1], sc3[2]);
+          sb->v[lane][oy * 3 + oz] = make_double2(wgt * uz[0], wgt * uz[1]);
+          sb->u[lane][oy * 3 + oz] = make_double2(wgt * uz[2], 0.0);
         }
 #pragma unroll
         for (int i = 0; i < 3; ++i) uz[i] += gC[3 * i + 2];
@@ -1284,12 +1290,13 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 2)) k
     }
 #pragma unroll
     for (int i = 0; i < 3; ++i) ux[i] += gC[3 * i];
-    if constexpr (slab) {
-      sb->base[lane] = gg + ax;
-      __syncwarp();
+    sb->base[lane] = gg + ax;
+    __syncwarp();
+    if constexpr (sizeof(T) == 4)
       slab_reduce(*sb, tails, emit);
-      __syncwarp();
-    }
+    else
+      slab_reduce64<false>(*sb, tails, emit, 1.0);
+    __syncwarp();
   }
   if (ok) {
 #pragma unroll
@@ -1367,32 +1374,33 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
     T vt[MAX_TOOLS_PER_SCENE + 1][3];
     WallTape<T> wt;
     T g[3] = {go.x, go.y, go.z};
-    const T inv = active_node ? T(1) / in.w : T(0);
+    const T inv = active_node ? node_rcp(in.w) : T(0);
+    unsigned hits = 0u;  // bit t: tool t is in contact with this node
     if (active_node) {
       T v[3] = {inv * in.x + c.gdt[0], inv * in.y + c.gdt[1], inv * in.z + c.gdt[2]};
       for (int t = 0; t < sh.n; ++t) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) vt[t][k] = v[k];
-        tool_collide(sh.tool[t], sh.p0(t), sh.p1(t), p, c.dt, v);
+        if (tool_collide(sh.tool[t], sh.p0(t), sh.p1(t), p, c.dt, v)) hits |= 1u << t;
       }
       walls(c, I, v, &wt);
       walls_vjp(c, I, wt, g);
     }
     const int t0 = tool_off[scene];
     for (int t = sh.n - 1; t >= 0; --t) {
+      const bool hit = (hits >> t) & 1u;  // without contact g passes unchanged
+      if (!__any_sync(0xffffffffu, hit)) continue;
       PoseGrad<T> g0, g1;
       g0.zero();
       g1.zero();
-      if (active_node) tool_collide_vjp(sh.tool[t], sh.p0(t), sh.p1(t), p, c.dt, vt[t], g, g0, g1);
-      if (__any_sync(0xffffffffu, active_node)) {
-        double* d0 = g_pose_f + 8 * (t0 + t);
-        double* d1 = g_pose_f1 + 8 * (t0 + t);
-        T v16[16] = {g0.pos[0], g0.pos[1], g0.pos[2], g0.rot[0], g0.rot[1], g0.rot[2], g0.rot[3], g0.gap,
-                     g1.pos[0], g1.pos[1], g1.pos[2], g1.rot[0], g1.rot[1], g1.rot[2], g1.rot[3], g1.gap};
-        int k;
-        const T v = warp_reduce_scatter16(v16, k);
-        if ((threadIdx.x & 1) == 0 && v != T(0)) atomicAdd((k < 8 ? d0 + k : d1 + (k - 8)), double(v));
-      }
+      if (hit) tool_collide_vjp(sh.tool[t], sh.p0(t), sh.p1(t), p, c.dt, vt[t], g, g0, g1);
+      double* d0 = g_pose_f + 8 * (t0 + t);
+      double* d1 = g_pose_f1 + 8 * (t0 + t);
+      T v16[16] = {g0.pos[0], g0.pos[1], g0.pos[2], g0.rot[0], g0.rot[1], g0.rot[2], g0.rot[3], g0.gap,
+                   g1.pos[0], g1.pos[1], g1.pos[2], g1.rot[0], g1.rot[1], g1.rot[2], g1.rot[3], g1.gap};
+      int k;
+      const T v = warp_reduce_scatter16(v16, k);
+      if ((threadIdx.x & 1) == 0 && v != T(0)) atomicAdd((k < 8 ? d0 + k : d1 + (k - 8)), double(v));
     }
     Node<T> res = {T(0), T(0), T(0), T(0)};
     if (active_node) {
@@ -1411,7 +1419,7 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
 // small spill), measured 3 % faster than 4 CTAs at 128 registers; MB > 0: MB
 // CTAs per SM (MpmTuning.p2g_adj_ctas)
 template <typename T, typename S, int MB = 0>
-__global__ void __launch_bounds__(128, MB > 0 ? MB : ((sizeof(T) == 4 && sizeof(S) == 4) ? 5 : 2)) k_p2g_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ g1,
+__global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 5 : 8)) k_p2g_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ g1,
                                                  T* __restrict__ g0, const int* __restrict__ pscene,
                                                  const Node<T>* __restrict__ g_in) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1434,7 +1442,7 @@ __global__ void __launch_bounds__(128, MB > 0 ? MB : ((sizeof(T) == 4 && sizeof(
   const int scene = __ldcg(pscene + p);  // issued with the state rows
   Stencil<T> s;
   bool ok = make_stencil(c, x, s);
-  MatConsts<S> m = mat_consts<T, S>(c);
+  const MatConsts<S>& m = mat_consts<T, S>(c);
   P2G<S> P;
   S aff[9];
   p2g_particle<true>(m, C, F, P, aff, (S*)nullptr);

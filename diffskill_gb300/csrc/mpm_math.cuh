@@ -118,22 +118,109 @@ MPM_DI void cof3(const T* A, T* Cf) {
   Cf[8] = A[0] * A[4] - A[1] * A[3];
 }
 
+// FP64 arithmetic from FP32 starting values.  GB300 issues one FP64
+// instruction per SM every 16 cycles or more (measured: 19 cycles of the SM per
+// FP64 instruction of a warp in p2g, against a quarter of a cycle for an FP32
+// one), so what can start from an FP32 value does: the reciprocal, the inverse
+// square root and the singular vectors (mpm_svd.cuh).
+//
+// cut_f32 drops the low mantissa bits of x (0 outside FP32's normal range, NaN
+// and infinity included); widen is exact for a normal or zero x.  Both are
+// integer operations: the conversion instructions occupy the FP64 pipe.
+MPM_DI float cut_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mag = hi & 0x7fffffffu;
+  const unsigned b = __funnelshift_l(lo, mag, 3) - (896u << 23);  // exponent bias 1023 -> 127
+  const bool in = mag - (897u << 20) < (254u << 20);              // exponents 1 .. 254 of FP32
+  return __uint_as_float((hi & 0x80000000u) | (in ? b & 0x7fffffffu : 0u));
+}
+MPM_DI double widen(float x) {
+  const unsigned b = __float_as_uint(x), mag = b & 0x7fffffffu;
+  const unsigned hi = mag >= (1u << 23) ? (mag >> 3) + (896u << 20) : 0u;
+  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(b << 29));
+}
+// float <-> double as the conversion instructions of a -ftz build give them
+// (subnormals to zero, infinities and NaN kept, nearest-even), in integer
+// operations: for the FP64 particle math on FP32 state
+MPM_DI double exact_f64(float x) {
+  const unsigned b = __float_as_uint(x), mag = b & 0x7fffffffu;
+  const unsigned bias = mag >= 0x7f800000u ? 1792u << 20 : 896u << 20;  // infinity, NaN: exponent 2047
+  const unsigned hi = mag >= (1u << 23) ? (mag >> 3) + bias : 0u;
+  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(mag >= (1u << 23) ? b << 29 : 0u));
+}
+MPM_DI float round_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mag = hi & 0x7fffffffu, sign = hi & 0x80000000u;
+  unsigned b = __funnelshift_l(lo, mag, 3) - (896u << 23);
+  const unsigned rest = lo & 0x1fffffffu;
+  b += (rest > 0x10000000u || (rest == 0x10000000u && (b & 1u))) ? 1u : 0u;
+  const bool normal = mag - (897u << 20) < (254u << 20);
+  const bool nan = mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0u);
+  const unsigned big = nan ? 0x7fffffffu : 0x7f800000u;
+  // an exponent of 0 (2^-127 .. 2^-126) may still round up to 2^-126
+  const bool edge = (mag >> 20) == 896u && b >= (1u << 23) && b < (1u << 24);
+  const unsigned r = normal ? b & 0x7fffffffu : (mag >= (1151u << 20) ? big : (edge ? b : 0u));
+  return __uint_as_float(sign | r);
+}
+// x in the precision T
+template <typename T, typename X>
+MPM_DI T to_prec(X x) {
+  if constexpr (sizeof(T) == sizeof(X))
+    return x;
+  else if constexpr (sizeof(T) == 8)
+    return exact_f64(x);
+  else
+    return round_f32(x);
+}
+// 1 / x for 1e-30 < |x| < 1e30: with y0 = 1/x (1 + e), |e| < 1e-6, from FP32,
+// 1/x = y0 (1 + e + e^2) up to e^3 (Newton's iteration and its next term)
+MPM_DI double rcp64(double x) {
+  const double y = widen(__fdividef(1.f, cut_f32(x)));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+// 1 / sqrt(x) and sqrt(x) for 1e-30 < x < 1e30: y0 from FP32, e = 1 - x y0^2,
+// 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3 e^2 / 8) up to 5 e^3 / 16
+MPM_DI double rsqrt64(double x) {
+  const double y = widen(rsqrtf(cut_f32(x)));
+  const double e = fma(-x, y * y, 1.0);
+  return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+
 // length() with the eps of plb/engine/primitive/primitives.py:13-15
 template <typename T>
 MPM_DI T len14(const T* a) {
-  return msqrt(dot3(a, a) + T(1e-14));
+  const T d = dot3(a, a) + T(1e-14);
+  if constexpr (sizeof(T) == 8)
+    return d * rsqrt64(d);
+  else
+    return msqrt(d);
+}
+// its reciprocal
+template <typename T>
+MPM_DI T inv_len14(const T* a) {
+  if constexpr (sizeof(T) == 8)
+    return rsqrt64(dot3(a, a) + T(1e-14));
+  else
+    return T(1) / len14(a);
 }
 // length() with the eps of plb/engine/primitive/utils.py:4-6
 template <typename T>
 MPM_DI T len8(const T* a) {
-  return msqrt(dot3(a, a) + T(1e-8));
+  const T d = dot3(a, a) + T(1e-8);
+  if constexpr (sizeof(T) == 8)
+    return d * rsqrt64(d);
+  else
+    return msqrt(d);
 }
+// a / b for 1e-30 < |b| < 1e30
+MPM_DI float quot(float a, float b) { return a / b; }
+MPM_DI double quot(double a, double b) { return a * rcp64(b); }
 // d(u/len14(u))^T g
 template <typename T>
 MPM_DI void unit14_vjp(const T* u, const T* g, T* gu) {
-  T L = len14(u);
   T ug = dot3(u, g);
-  T iL = T(1) / L;
+  T iL = inv_len14(u);
   T c = ug * iL * iL * iL;
 #pragma unroll
   for (int k = 0; k < 3; ++k) gu[k] = g[k] * iL - u[k] * c;

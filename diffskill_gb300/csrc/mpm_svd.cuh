@@ -50,79 +50,39 @@ MPM_DI void rot_tc(float theta, float& t, float& c) {
 // (angle_div: FP64 divides as such there), and for the SVD backward's 1 / (s_j^2 - s_i^2), whose divisor
 // is clamped to |b| >= 1e-6.  The substep kernels are built with -ftz=true, so
 // a subnormal s_pq compares equal to 0 and is never a divisor.
-MPM_DI double fast_div(double a, double b);  // below
+MPM_DI double fast_div(double a, double b) { return a * rcp64(b); }
 MPM_DI float fast_div(float a, float b) { return __fdividef(a, b); }
 MPM_DI double angle_div(double a, double b) { return a / b; }  // any quotient
 MPM_DI float angle_div(float a, float b) { return __fdividef(a, b); }
 
-// FP64 arithmetic from FP32 starting values.  GB300 issues one FP64
-// instruction per SM every 16 cycles or more (measured: 19 cycles of the SM per
-// FP64 instruction of a warp in p2g, against a quarter of a cycle for an FP32
-// one), so what can start from an FP32 value does: the reciprocal, the inverse
-// square root and the singular vectors below.
-//
-// cut_f32 drops the low mantissa bits of x (0 outside FP32's normal range, NaN
-// and infinity included); widen is exact for a normal or zero x.  Both are
-// integer operations: the conversion instructions occupy the FP64 pipe.
-MPM_DI float cut_f32(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const unsigned mag = hi & 0x7fffffffu;
-  const unsigned b = __funnelshift_l(lo, mag, 3) - (896u << 23);  // exponent bias 1023 -> 127
-  const bool in = mag - (897u << 20) < (254u << 20);              // exponents 1 .. 254 of FP32
-  return __uint_as_float((hi & 0x80000000u) | (in ? b & 0x7fffffffu : 0u));
+// log(s) of a singular value from sm1 = s - 1: 2 atanh(z) with
+// z = (s - 1) / (s + 1), by the series of atanh to z^13 for |s - 1| < 1/8
+// (|z| < 1/15: truncation below 3e-18 of the result)
+MPM_DI double log_strain64(double s, double sm1) {
+  if (fabs(sm1) < 0.125) {
+    const double z = 2.0 * sm1 * rcp64(s + 1.0);  // 2 z
+    const double w = 0.25 * z * z;
+    const double p = fma(w, fma(w, fma(w, fma(w, fma(w, 1.0 / 13.0, 1.0 / 11.0), 1.0 / 9.0), 1.0 / 7.0), 1.0 / 5.0),
+                         1.0 / 3.0);
+    return fma(z * w, p, z);
+  }
+  return log(s);
 }
-MPM_DI double widen(float x) {
-  const unsigned b = __float_as_uint(x), mag = b & 0x7fffffffu;
-  const unsigned hi = mag >= (1u << 23) ? (mag >> 3) + (896u << 20) : 0u;
-  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(b << 29));
-}
-// float <-> double as the conversion instructions of a -ftz build give them
-// (subnormals to zero, infinities and NaN kept, nearest-even), in integer
-// operations: for the FP64 particle math on FP32 state
-MPM_DI double exact_f64(float x) {
-  const unsigned b = __float_as_uint(x), mag = b & 0x7fffffffu;
-  const unsigned bias = mag >= 0x7f800000u ? 1792u << 20 : 896u << 20;  // infinity, NaN: exponent 2047
-  const unsigned hi = mag >= (1u << 23) ? (mag >> 3) + bias : 0u;
-  return __hiloint2double((int)((b & 0x80000000u) | hi), (int)(mag >= (1u << 23) ? b << 29 : 0u));
-}
-MPM_DI float round_f32(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const unsigned mag = hi & 0x7fffffffu, sign = hi & 0x80000000u;
-  unsigned b = __funnelshift_l(lo, mag, 3) - (896u << 23);
-  const unsigned rest = lo & 0x1fffffffu;
-  b += (rest > 0x10000000u || (rest == 0x10000000u && (b & 1u))) ? 1u : 0u;
-  const bool normal = mag - (897u << 20) < (254u << 20);
-  const bool nan = mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0u);
-  const unsigned big = nan ? 0x7fffffffu : 0x7f800000u;
-  // an exponent of 0 (2^-127 .. 2^-126) may still round up to 2^-126
-  const bool edge = (mag >> 20) == 896u && b >= (1u << 23) && b < (1u << 24);
-  const unsigned r = normal ? b & 0x7fffffffu : (mag >= (1151u << 20) ? big : (edge ? b : 0u));
-  return __uint_as_float(sign | r);
-}
-// x in the precision T
-template <typename T, typename X>
-MPM_DI T to_prec(X x) {
-  if constexpr (sizeof(T) == sizeof(X))
-    return x;
-  else if constexpr (sizeof(T) == 8)
-    return exact_f64(x);
-  else
-    return round_f32(x);
-}
-// 1 / x for 1e-30 < |x| < 1e30: with y0 = 1/x (1 + e), |e| < 1e-6, from FP32,
-// 1/x = y0 (1 + e + e^2) up to e^3 (Newton's iteration and its next term)
-MPM_DI double rcp64(double x) {
-  const double y = widen(__fdividef(1.f, cut_f32(x)));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-MPM_DI double fast_div(double a, double b) { return a * rcp64(b); }
-// 1 / sqrt(x) and sqrt(x) for 1e-30 < x < 1e30: y0 from FP32, e = 1 - x y0^2,
-// 1/sqrt(x) = y0 (1 - e)^(-1/2) = y0 (1 + e/2 + 3 e^2 / 8) up to 5 e^3 / 16
-MPM_DI double rsqrt64(double x) {
-  const double y = widen(rsqrtf(cut_f32(x)));
-  const double e = fma(-x, y * y, 1.0);
-  return fma(y, e * fma(e, 0.375, 0.5), y);
+// exp(x) - 1 by its Taylor series to x^11 for |x| < 1/8 (truncation below 2e-20)
+MPM_DI double expm1_strain64(double x) {
+  if (fabs(x) < 0.125) {
+    double p = fma(x, 1.0 / 39916800.0, 1.0 / 3628800.0);
+    p = fma(x, p, 1.0 / 362880.0);
+    p = fma(x, p, 1.0 / 40320.0);
+    p = fma(x, p, 1.0 / 5040.0);
+    p = fma(x, p, 1.0 / 720.0);
+    p = fma(x, p, 1.0 / 120.0);
+    p = fma(x, p, 1.0 / 24.0);
+    p = fma(x, p, 1.0 / 6.0);
+    p = fma(x, p, 0.5);
+    return fma(x * x, p, x);
+  }
+  return expm1(x);
 }
 MPM_DI float third(float x) { return fast_div(x, 3.f); }
 MPM_DI double third(double x) { return x * (1.0 / 3.0); }
@@ -358,7 +318,7 @@ __device__ __noinline__ inline void svd3_plain64(const double* A, double* U, dou
 // particular order (nothing here depends on it), unless `plain` is returned:
 // then the matrix was inverted, nearly singular (s < 0.2) or not finite, and
 // U, s, V and `is` come from svd3, s[2] perhaps negative.  V is written when
-// plain or WithV; is = 1/s when not plain.
+// plain or WithV; is = 1/s (plain: 0 for s at or below the return map's 0.05).
 //
 // An FP64 Jacobi rotation costs about 68 FP64 instructions, and svd3 takes
 // four to five sweeps of three: about 900 of the 1,245 FP64 instructions that
@@ -373,7 +333,8 @@ __device__ __noinline__ inline void svd3_plain64(const double* A, double* U, dou
 // - a pair with a larger X (eigenvalues nearly equal, but not within rounding)
 //   takes FP64 sweeps instead (jacobi64_finish).
 // About 180 FP64 instructions.  p2g of 0.76M particles (FP32 state, FP64 SVD):
-// SVD64_P2G; its adjoint: SVD64_ADJ.
+// 1469 -> 547 us; its
+// adjoint: 2096 -> 1087 us.
 template <bool WithV>
 MPM_DI bool svd3_left64(const double* A, double* U, double* s, double* is, double* V) {
   double S[6];  // 00, 11, 22, 01, 02, 12
@@ -502,7 +463,7 @@ MPM_DI bool svd3_left64(const double* A, double* U, double* s, double* is, doubl
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       s[k] = sl[k];
-      is[k] = 0.0;
+      is[k] = 0.05 < sl[k] ? rcp64(sl[k]) : 0.0;
     }
     return true;
   }
@@ -537,7 +498,7 @@ MPM_DI T svd_clamp(T a) {
 // of s and the plain quotient is exact enough, as it is when a singular value
 // sits at the return map's 0.05 floor.  ds = s_j - s_i and e_j - e_i are
 // formed from s - 1 and e - 1.
-MPM_DI float ret_map_dd(float si, float sj, float ds, float ei, float em1i, float em1j, float a) {
+MPM_DI float ret_map_dd(float si, float, float sj, float ds, float ei, float em1i, float em1j, float a) {
   if (si > 0.05f && sj > 0.05f) {
     const float u = ds / si;
     if (fabsf(u) < 0.015625f) {
@@ -551,9 +512,9 @@ MPM_DI float ret_map_dd(float si, float sj, float ds, float ei, float em1i, floa
 }
 // FP64: the series below |u| < 2^-10 (L / u to u^5, E1 to z^5; truncation below
 // 2e-19), above it the quotient keeps 1e-13
-MPM_DI double ret_map_dd(double si, double sj, double ds, double ei, double em1i, double em1j, double a) {
+MPM_DI double ret_map_dd(double si, double ri, double sj, double ds, double ei, double em1i, double em1j, double a) {
   if (si > 0.05 && sj > 0.05) {
-    const double ri = rcp64(si), u = ds * ri;
+    const double u = ds * ri;
     if (fabs(u) < 0.0009765625) {
       const double lg =
           fma(u, fma(u, fma(u, fma(u, fma(u, -1.0 / 6.0, 0.2), -0.25), 1.0 / 3.0), -0.5), 1.0);
@@ -563,7 +524,7 @@ MPM_DI double ret_map_dd(double si, double sj, double ds, double ei, double em1i
       return ei * a * ri * e1 * lg;
     }
   }
-  return ds != 0.0 ? (em1j - em1i) / ds : 0.0;
+  return fabs(ds) > 1e-30 ? fast_div(em1j - em1i, ds) : 0.0;
 }
 
 // backward_svd (mpm_simulator.py:137-156, clamp 184-192) of the two functions
@@ -577,7 +538,7 @@ MPM_DI double ret_map_dd(double si, double sj, double ds, double ei, double em1i
 //   X_ij = K_ij (s_j - s_i) / clamp((s_j - s_i)(s_j + s_i)),
 //   K_ij = (M_R,ij - M_R,ji) + 1/2 [M_N,ij (D S + E) + M_N,ji (D S - E)]
 // with S = s_i + s_j, E = e_i + e_j and D the divided difference of e
-// (ret_map_dd); s_j - s_i is taken from sm1 = s - 1.  The reference's numerator is a difference of terms of size
+// (ret_map_dd; is = 1/s, read in FP64 only); s_j - s_i is taken from sm1 = s - 1.  The reference's numerator is a difference of terms of size
 // |g| that leaves a value of size |g| (s_j - s_i), so in FP32 its rounding
 // error is amplified by 1 / (s_j^2 - s_i^2), up to 1e6 at the clamp, whenever
 // two singular values nearly coincide (near-isotropic deformation); K has no
@@ -585,8 +546,8 @@ MPM_DI double ret_map_dd(double si, double sj, double ds, double ei, double em1i
 // Returns X, the gradient of the SVD's input in the bases U, V (gA =
 // U X V^T).  M_N, e and e - 1 (em1) are read only when `yield`.
 template <typename T>
-MPM_DI void svd3_bwd_factored_basis(const T* s, const T* sm1, const T* MR, const T* MN, const T* e, const T* em1, T a,
-                                    bool yield, const T* gs, T* X) {
+MPM_DI void svd3_bwd_factored_basis(const T* s, const T* is, const T* sm1, const T* MR, const T* MN, const T* e,
+                                    const T* em1, T a, bool yield, const T* gs, T* X) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) X[i * 4] = gs[i];
   // each unordered pair (i, j) once: D and the clamped factor are symmetric in i, j
@@ -598,7 +559,7 @@ MPM_DI void svd3_bwd_factored_basis(const T* s, const T* sm1, const T* MR, const
     T Kij = MR[i * 3 + j] - MR[j * 3 + i];
     T Kji = -Kij;
     if (yield) {
-      const T D = ret_map_dd(s[i], s[j], ds, e[i], em1[i], em1[j], a);
+      const T D = ret_map_dd(s[i], is[i], s[j], ds, e[i], em1[i], em1[j], a);
       const T se = e[i] + e[j];
       const T p = T(0.5) * (D * sm + se), m = T(0.5) * (D * sm - se);
       Kij += MN[i * 3 + j] * p + MN[j * 3 + i] * m;

@@ -362,7 +362,7 @@ MPM_DI void box_sdf_grad(const T* size, const T* q, T g, T* gq) {
     qq[k] = mabs(q[k]) - size[k];
     mq[k] = (T(0) < qq[k]) ? qq[k] : T(0);
   }
-  T iL = T(1) / len14(mq);
+  T iL = inv_len14(mq);
   T gqq[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) gqq[k] = (T(0) < qq[k]) ? g * mq[k] * iL : T(0);
@@ -424,7 +424,7 @@ MPM_DI void local_sdf_grad(const Tool<T>& t, const T* q, T gap, T g, T* gq, T* g
   if (capsule_shape(t.type)) {
     T p2[3], dp;
     capsule_p2(t, q, p2, &dp);
-    T iL = g / len14(p2);
+    T iL = quot(g, len14(p2));
     gq[0] += p2[0] * iL;
     gq[1] += p2[1] * iL * dp;
     gq[2] += p2[2] * iL;
@@ -483,7 +483,7 @@ MPM_DI void local_normal(const Tool<T>& t, const T* q, T gap, T* n, T* r_out = n
   } else {
     fd_normal_raw(t, q, r);
   }
-  T iL = T(1) / len14(r);
+  T iL = inv_len14(r);
 #pragma unroll
   for (int k = 0; k < 3; ++k) n[k] = r[k] * iL;
   if (r_out) {
@@ -557,7 +557,7 @@ MPM_DI void shape_sdf_vjp(const Tool<T>& t, const T* pos, const T* rot, T gap, c
                           T* grot, T* ggap) {
   if (t.type == TOOL_SPHERE) {
     const T d[3] = {p[0] - pos[0], p[1] - pos[1], p[2] - pos[2]};
-    T c = g / len14(d);
+    T c = quot(g, len14(d));
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       if (gp) gp[k] += c * d[k];
@@ -576,7 +576,7 @@ MPM_DI void shape_normal(const Tool<T>& t, const T* pos, const T* rot, T gap, co
                          T* r_out = nullptr) {
   if (t.type == TOOL_SPHERE) {
     const T d[3] = {p[0] - pos[0], p[1] - pos[1], p[2] - pos[2]};
-    T iL = T(1) / len14(d);
+    T iL = inv_len14(d);
 #pragma unroll
     for (int k = 0; k < 3; ++k) n[k] = d[k] * iL;
     return;
@@ -607,7 +607,7 @@ MPM_DI void shape_normal_vjp(const Tool<T>& t, const T* pos, const T* rot, T gap
   if (r_in && !dual_shape(t.type)) {  // the normal from r exactly as local_normal forms it
 #pragma unroll
     for (int k = 0; k < 3; ++k) r[k] = r_in[k];
-    T iL = T(1) / len14(r);
+    T iL = inv_len14(r);
 #pragma unroll
     for (int k = 0; k < 3; ++k) nl[k] = r[k] * iL;
   } else {
@@ -624,7 +624,7 @@ MPM_DI void collider_v(const T* pos0, const T* rot0, const T* pos1, const T* rot
   T rel[3], nw[3];
   inv_trans(p, pos0, rot0, rel);
   qrot(rot1, rel, nw);
-  T idt = T(1) / dt;
+  T idt = quot(T(1), dt);
 #pragma unroll
   for (int k = 0; k < 3; ++k) cv[k] = (nw[k] + pos1[k] - p[k]) * idt;
 }
@@ -633,7 +633,7 @@ MPM_DI void collider_v_vjp(const T* pos0, const T* rot0, const T* pos1, const T*
                            T* gpos0, T* grot0, T* gpos1, T* grot1) {
   T rel[3];
   inv_trans(p, pos0, rot0, rel);
-  T idt = T(1) / dt;
+  T idt = quot(T(1), dt);
   const T gnw[3] = {g[0] * idt, g[1] * idt, g[2] * idt};
 #pragma unroll
   for (int k = 0; k < 3; ++k) gpos1[k] += gnw[k];
@@ -642,16 +642,60 @@ MPM_DI void collider_v_vjp(const T* pos0, const T* rot0, const T* pos1, const T*
   inv_trans_vjp(p, pos0, rot0, grel, (T*)nullptr, gpos0, grot0);
 }
 
+// |vt| > 1e-30 (the friction response's guard)
+MPM_DI bool moving(const float* vt) { return msqrt(dot3(vt, vt)) > 1e-30f; }
+MPM_DI bool moving(const double* vt) { return dot3(vt, vt) > 1e-60; }
+
+// Whether p is certainly out of the contact range of a shape, FP64 only: the
+// FP32 SDF, less a margin far above its rounding error, gives an influence
+// exp(-dist softness) below exp(-3) < 0.1 and dist > 0.  Most grid nodes are far
+// from every tool, and the FP64 SDF, square roots and exponential of a node cost
+// some 100 FP64 instructions per tool (16 cycles of the SM each).
+template <typename T>
+MPM_DI bool out_of_range(const Tool<T>& t, const T* pos, const T* rot, T gap, const T* p) {
+  if constexpr (sizeof(T) == 8) {
+    Tool<float> f;
+    f.type = t.type;
+    f.radius = cut_f32(t.radius);
+    f.cap_h = cut_f32(t.cap_h);
+    f.cap_r = cut_f32(t.cap_r);
+    float d[3], r[4];
+    const float origin[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      f.size[k] = cut_f32(t.size[k]);
+      d[k] = cut_f32(p[k] - pos[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      f.prism_h[k] = cut_f32(t.prism_h[k]);
+      f.torus[k] = cut_f32(t.torus[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      f.prot_inv[k] = cut_f32(t.prot_inv[k]);
+      r[k] = cut_f32(rot[k]);
+    }
+    const float margin = 1e-4f + 1e-5f * (fabsf(d[0]) + fabsf(d[1]) + fabsf(d[2]));
+    const float dist = shape_sdf(f, origin, r, cut_f32(gap), d) - margin;
+    const float soft = cut_f32(t.softness);
+    return dist > 0.f && (soft <= 0.f || dist * soft > 3.f);
+  } else {
+    return false;
+  }
+}
+
 // Primitive.collide (primive_base.py:96-120).  Returns whether the contact
 // branch ran; vout = vin otherwise.
 template <typename T>
 MPM_DI bool collide_fwd(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, const T* pos1, const T* rot1,
                         const T* p, T dt, const T* vin, T* vout) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) vout[k] = vin[k];
+  if (out_of_range(t, pos0, rot0, gap0, p)) return false;
   T dist = shape_sdf(t, pos0, rot0, gap0, p);
   T e = mexp_fast(-dist * t.softness);
   T infl = (e < T(1)) ? e : T(1);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) vout[k] = vin[k];
   if (!((t.softness > T(0) && infl > T(0.1)) || dist <= T(0))) return false;
   T D[3], cv[3], iv[3], vt[3];
   shape_normal(t, pos0, rot0, gap0, p, D);
@@ -665,10 +709,10 @@ MPM_DI bool collide_fwd(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, 
   T vtn = len8(vt);
   T a = vtn + nc * t.friction;
   T m = (a < T(0)) ? T(0) : a;
-  T flag = (nc < T(0) && msqrt(dot3(vt, vt)) > T(1e-30)) ? T(1) : T(0);
+  T flag = (nc < T(0) && moving(vt)) ? T(1) : T(0);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    T vtf = vt[k] / vtn * m;
+    T vtf = quot(vt[k], vtn) * m;
     T vt2 = vtf * flag + vt[k] * (T(1) - flag);
     vout[k] = cv[k] + iv[k] * (T(1) - infl) + vt2 * infl;
   }
@@ -678,6 +722,11 @@ template <typename T>
 MPM_DI void collide_vjp(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, const T* pos1, const T* rot1,
                         const T* p, T dt, const T* vin, const T* gout, T* gvin, T* gpos0, T* grot0, T* ggap0,
                         T* gpos1, T* grot1) {
+  if (out_of_range(t, pos0, rot0, gap0, p)) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) gvin[k] = gout[k];
+    return;
+  }
   T dist = shape_sdf(t, pos0, rot0, gap0, p);
   T e = mexp_fast(-dist * t.softness);
   T infl = (e < T(1)) ? e : T(1);
@@ -698,11 +747,11 @@ MPM_DI void collide_vjp(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, 
   T vtn = len8(vt);
   T a = vtn + nc * t.friction;
   T m = (a < T(0)) ? T(0) : a;
-  T flag = (nc < T(0) && msqrt(dot3(vt, vt)) > T(1e-30)) ? T(1) : T(0);
+  T flag = (nc < T(0) && moving(vt)) ? T(1) : T(0);
   T g_cv[3], g_iv[3], g_vt[3], g_vtf[3], g_infl = T(0);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    T vtf = vt[k] / vtn * m;
+    T vtf = quot(vt[k], vtn) * m;
     T vt2 = vtf * flag + vt[k] * (T(1) - flag);
     g_cv[k] = gout[k];
     g_iv[k] = gout[k] * (T(1) - infl);
@@ -711,15 +760,15 @@ MPM_DI void collide_vjp(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, 
     g_vt[k] = gout[k] * infl * (T(1) - flag);
   }
   T gvtf_vt = dot3(g_vtf, vt);
-  T g_vtn = -gvtf_vt * m / (vtn * vtn);
-  T g_m = gvtf_vt / vtn;
+  T g_vtn = quot(-gvtf_vt * m, vtn * vtn);
+  T g_m = quot(gvtf_vt, vtn);
   T g_nc = T(0);
   if (!(a < T(0))) {
     g_vtn += g_m;
     g_nc += g_m * t.friction;
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) g_vt[k] += g_vtf[k] * m / vtn + g_vtn * vt[k] / vtn;
+  for (int k = 0; k < 3; ++k) g_vt[k] += quot(g_vtf[k] * m, vtn) + quot(g_vtn * vt[k], vtn);
   T g_D[3] = {T(0), T(0), T(0)};
 #pragma unroll
   for (int k = 0; k < 3; ++k) g_iv[k] += g_vt[k];
