@@ -17,6 +17,7 @@ MPM_OK = 0
 STATUS_OUT_OF_GRID = 1
 STATUS_NONFINITE = 2
 STATUS_RENDER_BOX = 4
+STATUS_TIMEOUT = 8
 
 _c_p = ctypes.c_void_p
 _i32 = ctypes.c_int32

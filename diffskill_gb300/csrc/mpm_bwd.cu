@@ -120,35 +120,47 @@ __global__ void __launch_bounds__(128) k_contact_adj(Consts<T> c, const T* __res
                                                      const double* __restrict__ sums,
                                                      const double* __restrict__ g_min, T* __restrict__ gst,
                                                      double* __restrict__ g_pose) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= c.n_particles) return;
-  int sc = pscene[p];
-  T x[3];
-  load_row(st, c.ld, p, 0, 3, x);
+  __shared__ StagedTools<T> sh;
+  stage_tools(sh, pscene, (int64_t)blockIdx.x * blockDim.x, tools, tool_off, pose);
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = p < c.n_particles;
+  const int sc = valid ? pscene[p] : -1;
+  const bool per_warp = one_scene(valid, sc);
+  const int scene = per_warp ? __shfl_sync(0xffffffffu, sc, 0) : sc;
+  if (scene < 0) return;
+  T x[3] = {T(0), T(0), T(0)};
+  if (valid) load_row(st, c.ld, p, 0, 3, x);
   T gx[3] = {T(0), T(0), T(0)};
-  for (int t = tool_off[sc]; t < tool_off[sc + 1]; ++t) {
+  for (int t = tool_off[scene]; t < tool_off[scene + 1]; ++t) {
     if (tools[t].action_dim <= 0 || g_min[t] == 0.0) continue;
-    Tool<T> tl;
-    Pose<T> P;
-    to_tool(tools[t], tl);
-    to_pose(pose + 8 * t, P);
-    T sd = tool_sdf(tl, P, x);
-    if (!(T(0) < sd)) continue;
-    double norm = sums[2 * t], md = sums[2 * t + 1] / norm;
-    double d = double(sd), w = 1.0 / (1.0 + d * d * 10000.0);
-    double g_norm = -g_min[t] * md / norm;
-    double g_w = g_min[t] * d / norm + g_norm;
-    double g_d = g_min[t] * w / norm + g_w * (-2e4 * d * w * w);
     PoseGrad<T> gP;
     gP.zero();
-    tool_sdf_vjp(tl, P, x, T(g_d), gx, gP);
-    const T* gv = &gP.pos[0];
-    for (int k = 0; k < 3; ++k) atomicAdd(g_pose + 8 * t + k, double(gv[k]));
-    for (int k = 0; k < 4; ++k) atomicAdd(g_pose + 8 * t + 3 + k, double(gP.rot[k]));
-    atomicAdd(g_pose + 8 * t + 7, double(gP.gap));
+    bool any = false;
+    if (valid) {
+      Tool<T> tl;
+      Pose<T> P;
+      staged_tool(sh, scene, t, tools, pose, tl, P);
+      const T sd = tool_sdf(tl, P, x);
+      if (T(0) < sd) {
+        any = true;
+        const double inorm = 1.0 / sums[2 * t], md = sums[2 * t + 1] * inorm;
+        const double d = to_prec<double>(sd), w = rcp64(1.0 + d * d * 10000.0);
+        const double g_norm = -g_min[t] * md * inorm;
+        const double g_w = g_min[t] * d * inorm + g_norm;
+        const double g_d = g_min[t] * w * inorm + g_w * (-2e4 * d * w * w);
+        tool_sdf_vjp(tl, P, x, to_prec<T>(g_d), gx, gP);
+      }
+    }
+    if (per_warp ? __any_sync(0xffffffffu, any) : any) {
+      double v[8];
+      pose_values(gP, v);
+      add8(g_pose + 8 * t, v, per_warp);
+    }
   }
+  if (valid) {
 #pragma unroll
-  for (int d = 0; d < 3; ++d) gst[(int64_t)d * c.ld + p] += gx[d];
+    for (int d = 0; d < 3; ++d) gst[(int64_t)d * c.ld + p] += gx[d];
+  }
 }
 
 template <typename T>
@@ -172,48 +184,56 @@ __global__ void __launch_bounds__(128) k_tool_distance_adj(Consts<T> c, const T*
                                                            const double* __restrict__ pose,
                                                            const T* __restrict__ g_out, T* __restrict__ gst,
                                                            double* __restrict__ g_pose) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= c.n_particles) return;
-  int sc = pscene[p];
-  T x[3];
-  load_row(st, c.ld, p, 0, 3, x);
+  __shared__ StagedTools<T> sh;
+  stage_tools(sh, pscene, (int64_t)blockIdx.x * blockDim.x, tools, tool_off, pose);
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = p < c.n_particles;
+  const int sc = valid ? pscene[p] : -1;
+  const bool per_warp = one_scene(valid, sc);
+  const int scene = per_warp ? __shfl_sync(0xffffffffu, sc, 0) : sc;
+  if (scene < 0) return;
+  T x[3] = {T(0), T(0), T(0)};
+  if (valid) load_row(st, c.ld, p, 0, 3, x);
   T gx[3] = {T(0), T(0), T(0)};
-  for (int t = tool_off[sc]; t < tool_off[sc + 1]; ++t) {
-    Tool<T> tl;
-    Pose<T> P;
-    to_tool(tools[t], tl);
-    to_pose(pose + 8 * t, P);
+  for (int t = tool_off[scene]; t < tool_off[scene + 1]; ++t) {
     const int col = col_off[t];
     PoseGrad<T> gP;
     gP.zero();
     bool any = false;
-    if (fingered(tl.type)) {
+    if (valid) {
+      Tool<T> tl;
+      Pose<T> P;
+      staged_tool(sh, scene, t, tools, pose, tl, P);
+      if (fingered(tl.type)) {
 #pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        T g = g_out[(int64_t)(col + side) * c.ld + p];
-        if (g == T(0)) continue;
-        any = true;
-        T flag = side == 0 ? T(-1) : T(1);
-        T fp[3], gf[3] = {T(0), T(0), T(0)};
-        finger_pos(P, flag, fp);
-        shape_sdf_vjp(tl, fp, P.rot, T(0), x, g, gx, gf, gP.rot, (T*)nullptr);
-        finger_pos_vjp(P, flag, gf, gP);
-      }
-    } else {
-      T g = g_out[(int64_t)col * c.ld + p];
-      if (g != T(0)) {
-        any = true;
-        tool_sdf_vjp(tl, P, x, g, gx, gP);
+        for (int side = 0; side < 2; ++side) {
+          T g = g_out[(int64_t)(col + side) * c.ld + p];
+          if (g == T(0)) continue;
+          any = true;
+          T flag = side == 0 ? T(-1) : T(1);
+          T fp[3], gf[3] = {T(0), T(0), T(0)};
+          finger_pos(P, flag, fp);
+          shape_sdf_vjp(tl, fp, P.rot, T(0), x, g, gx, gf, gP.rot, (T*)nullptr);
+          finger_pos_vjp(P, flag, gf, gP);
+        }
+      } else {
+        T g = g_out[(int64_t)col * c.ld + p];
+        if (g != T(0)) {
+          any = true;
+          tool_sdf_vjp(tl, P, x, g, gx, gP);
+        }
       }
     }
-    if (any) {
-      for (int k = 0; k < 3; ++k) atomicAdd(g_pose + 8 * t + k, double(gP.pos[k]));
-      for (int k = 0; k < 4; ++k) atomicAdd(g_pose + 8 * t + 3 + k, double(gP.rot[k]));
-      atomicAdd(g_pose + 8 * t + 7, double(gP.gap));
+    if (per_warp ? __any_sync(0xffffffffu, any) : any) {
+      double v[8];
+      pose_values(gP, v);
+      add8(g_pose + 8 * t, v, per_warp);
     }
   }
+  if (valid) {
 #pragma unroll
-  for (int d = 0; d < 3; ++d) gst[(int64_t)d * c.ld + p] += gx[d];
+    for (int d = 0; d < 3; ++d) gst[(int64_t)d * c.ld + p] += gx[d];
+  }
 }
 
 template <typename T>

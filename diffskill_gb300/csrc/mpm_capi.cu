@@ -29,7 +29,8 @@ struct MpmHandle {
   const void* premarked = nullptr;  // frame whose block flags the last forward g2p set
   std::vector<MpmToolDesc> h_tools;
   unsigned int* d_status = nullptr;
-  int* d_flags = nullptr;  // convergence flags of mpm_target_sdf
+  int* d_flags = nullptr;  // convergence flags and barrier counter of mpm_target_sdf
+  unsigned char* d_tile_flags = nullptr;  // its changed tiles
   int* d_pair_off = nullptr;  // [n_scenes + 1] first collision pair of each scene
   int n_pairs = 0;            // tool-tool collision pairs over all scenes
   int max_scene_pairs = 0;    // most pairs of one scene
@@ -196,6 +197,7 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
   ok = ok && cudaMalloc(&h->d_tool_off, toff.size() * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_status, sizeof(unsigned int)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_flags, 4 * sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc(&h->d_tile_flags, mpm::target_sdf_flag_bytes(p.n_scenes, p.n_grid)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_pair_off, toff.size() * sizeof(int)) == cudaSuccess;
   for (int i = 0; i < 4 && ok; ++i) ok = cudaMalloc(&h->grid[i], gbytes) == cudaSuccess;
   const int64_t nb = p.n_grid / 4;
@@ -241,6 +243,7 @@ int mpm_destroy(MpmHandle* h) {
   cudaFree(h->d_tools);
   cudaFree(h->d_status);
   cudaFree(h->d_flags);
+  cudaFree(h->d_tile_flags);
   cudaFree(h->d_pair_off);
   cudaFree(h->d_coll_pts);
   for (int i = 0; i < 4; ++i) cudaFree(h->grid[i]);
@@ -726,9 +729,9 @@ int mpm_target_sdf(MpmHandle* h, const void* target_density, void* target_sdf, v
   MPM_TRY(check_aligned(h, work, "work"));
   mpm::LaunchCtx L = ctx(h, stream);
   cudaError_t e = h->p.precision == MPM_PREC_FP64
-                      ? mpm::launch_target_sdf<double>(L, h->d_flags, (const double*)target_density,
+                      ? mpm::launch_target_sdf<double>(L, h->d_flags, h->d_tile_flags, (const double*)target_density,
                                                        (double*)target_sdf, (double*)nearest, (double*)work, n_iters)
-                      : mpm::launch_target_sdf<float>(L, h->d_flags, (const float*)target_density,
+                      : mpm::launch_target_sdf<float>(L, h->d_flags, h->d_tile_flags, (const float*)target_density,
                                                       (float*)target_sdf, (float*)nearest, (float*)work, n_iters);
   return e == cudaSuccess ? MPM_OK : cuda_fail(h, e, "mpm_target_sdf");
 }

@@ -205,22 +205,38 @@ __global__ void __launch_bounds__(128) k_contact_sums(Consts<T> c, const T* __re
                                                       const MpmToolDesc* __restrict__ tools,
                                                       const int* __restrict__ tool_off,
                                                       const double* __restrict__ pose, double* __restrict__ sums) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= c.n_particles) return;
-  int sc = pscene[p];
-  T x[3];
-  load_row(st, c.ld, p, 0, 3, x);
-  for (int t = tool_off[sc]; t < tool_off[sc + 1]; ++t) {
+  __shared__ StagedTools<T> sh;
+  stage_tools(sh, pscene, (int64_t)blockIdx.x * blockDim.x, tools, tool_off, pose);
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = p < c.n_particles;
+  const int sc = valid ? pscene[p] : -1;
+  const bool per_warp = one_scene(valid, sc);
+  const int scene = per_warp ? __shfl_sync(0xffffffffu, sc, 0) : sc;  // -1: a warp past the end
+  if (scene < 0) return;
+  T x[3] = {T(0), T(0), T(0)};
+  if (valid) load_row(st, c.ld, p, 0, 3, x);
+  for (int t = tool_off[scene]; t < tool_off[scene + 1]; ++t) {
     if (tools[t].action_dim <= 0) continue;
-    Tool<T> tl;
-    Pose<T> P;
-    to_tool(tools[t], tl);
-    to_pose(pose + 8 * t, P);
-    T sd = tool_sdf(tl, P, x);
-    double d = (T(0) < sd) ? double(sd) : 0.0;
-    double w = 1.0 / (1.0 + d * d * 10000.0);
+    double w = 0.0, dw = 0.0;
+    if (valid) {
+      Tool<T> tl;
+      Pose<T> P;
+      staged_tool(sh, scene, t, tools, pose, tl, P);
+      const T sd = tool_sdf(tl, P, x);
+      const double d = (T(0) < sd) ? to_prec<double>(sd) : 0.0;
+      w = rcp64(1.0 + d * d * 10000.0);
+      dw = d * w;
+    }
+    if (per_warp) {  // once per warp: a tool's two sums are one address each
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        w += __shfl_xor_sync(0xffffffffu, w, o);
+        dw += __shfl_xor_sync(0xffffffffu, dw, o);
+      }
+      if ((threadIdx.x & 31) != 0) continue;
+    }
     atomicAdd(sums + 2 * t, w);
-    atomicAdd(sums + 2 * t + 1, d * w);
+    atomicAdd(sums + 2 * t + 1, dw);
   }
 }
 __global__ void k_contact_finish(int n_tools, const double* __restrict__ sums, double* __restrict__ min_dist) {

@@ -1671,6 +1671,93 @@ __global__ void __launch_bounds__(256) k_compact_clear(unsigned char* __restrict
 }
 
 // ---------------------------------------------------------------------------
+// per-particle tool terms (contact losses, tool distances)
+// ---------------------------------------------------------------------------
+// The tools of the scene of a CTA's first particle in the compute precision,
+// converted once per CTA: a thread that converts a descriptor and a pose itself
+// takes some 35 FP64 conversions per tool, on the pipe that issues one
+// instruction every 16 cycles.  A particle of another scene (a CTA that
+// straddles scenes) still converts its own.
+template <typename T>
+struct StagedTools {
+  int scene, t0, n;
+  Tool<T> tool[MAX_TOOLS_PER_SCENE];
+  Pose<T> pose[MAX_TOOLS_PER_SCENE];
+};
+// all threads of the CTA; `first`: the CTA's first particle (in range)
+template <typename T>
+MPM_DI void stage_tools(StagedTools<T>& sh, const int* __restrict__ pscene, int64_t first,
+                        const MpmToolDesc* __restrict__ tools, const int* __restrict__ tool_off,
+                        const double* __restrict__ pose) {
+  const int sc = pscene[first];
+  const int t0 = tool_off[sc], n = tool_off[sc + 1] - t0;
+  if (threadIdx.x == 0) {
+    sh.scene = sc;
+    sh.t0 = t0;
+    sh.n = n;
+  }
+  if ((int)threadIdx.x < n) {
+    to_tool(tools[t0 + threadIdx.x], sh.tool[threadIdx.x]);
+    to_pose(pose + 8 * (t0 + threadIdx.x), sh.pose[threadIdx.x]);
+  }
+  __syncthreads();
+}
+template <typename T>
+MPM_DI void staged_tool(const StagedTools<T>& sh, int scene, int t, const MpmToolDesc* __restrict__ tools,
+                        const double* __restrict__ pose, Tool<T>& tl, Pose<T>& P) {
+  if (scene == sh.scene) {
+    tl = sh.tool[t - sh.t0];
+    P = sh.pose[t - sh.t0];
+  } else {
+    to_tool(tools[t], tl);
+    to_pose(pose + 8 * t, P);
+  }
+}
+// whether the valid lanes of a warp are of one scene (then the scene of lane 0,
+// which is valid whenever any lane is): their sums go to memory once per warp
+MPM_DI bool one_scene(bool valid, int scene) {
+  const int s0 = __shfl_sync(0xffffffffu, scene, 0);
+  return __all_sync(0xffffffffu, !valid || scene == s0);
+}
+// Adds 8 values of every lane to dst[0..7] in FP64: per warp (all 32 lanes, one
+// atomic per value; reduce-scatter, 9 additions per lane) or per lane.  One
+// atomic per particle and value made these kernels wait on the 8 addresses of a
+// tool (30,000 particles: tool distance adjoint 261 us per call).
+MPM_DI void add8(double* dst, double (&v)[8], bool per_warp) {
+  if (!per_warp) {
+    for (int k = 0; k < 8; ++k)
+      if (v[k] != 0.0) atomicAdd(dst + k, v[k]);
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double send = h4 ? v[i] : v[i + 4];
+    v[i] = (h4 ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double send = h3 ? v[i] : v[i + 2];
+    v[i] = (h3 ? v[i + 2] : v[i]) + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  const double send = h2 ? v[0] : v[1];
+  double s = (h2 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, send, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  const int k = (h4 ? 4 : 0) + (h3 ? 2 : 0) + (h2 ? 1 : 0);
+  if ((lane & 3) == 0 && s != 0.0) atomicAdd(dst + k, s);
+}
+template <typename T>
+MPM_DI void pose_values(const PoseGrad<T>& g, double (&v)[8]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v[k] = to_prec<double>(g.pos[k]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[3 + k] = to_prec<double>(g.rot[k]);
+  v[7] = to_prec<double>(g.gap);
+}
+
+// ---------------------------------------------------------------------------
 // density grid and losses
 // ---------------------------------------------------------------------------
 template <typename T>

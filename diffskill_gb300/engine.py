@@ -336,6 +336,8 @@ class MpmEngine:
             raise FloatingPointError("MPM substep produced a NaN/Inf (device status word)")
         if st & _lib.STATUS_OUT_OF_GRID:
             raise _lib.MpmError("a particle stencil left the grid; its scatter was skipped")
+        if st & _lib.STATUS_TIMEOUT:
+            raise _lib.MpmError("a wait between the target-SDF iterations ran out; the result is incomplete")
 
     @property
     def launches(self) -> int:

@@ -65,6 +65,7 @@ extern "C" {
 #define MPM_STATUS_OUT_OF_GRID 1u /* a particle stencil left the grid; it was skipped */
 #define MPM_STATUS_NONFINITE 2u   /* a NaN/Inf velocity or deformation was produced */
 #define MPM_STATUS_RENDER_BOX 4u  /* mpm_render_bake: the particles' box exceeds the render volume */
+#define MPM_STATUS_TIMEOUT 8u     /* mpm_target_sdf: a wait between its iterations ran out; its outputs are incomplete */
 
 /* Simulator constants: MPMSimulator.__init__ (mpm_simulator.py:8-67). */
 typedef struct MpmParams {
@@ -294,8 +295,8 @@ int mpm_soft_contact_bwd(MpmHandle* h, const void* state, const double* pose, co
  * else inf.  target_density: real[n_scenes][n_grid^3]; target_sdf:
  * real[n_scenes][n_grid^3] and nearest: real[n_scenes][n_grid^3][3] written
  * (nearest = 0 where sdf stays inf); work: real[n_scenes][n_grid^3][4]
- * scratch.  Launches after the first iteration that changes no node return
- * at once (every later iteration would reproduce it). */
+ * scratch.  The iterations run in one cooperative launch, which ends after the
+ * first iteration that changes no node (every later one would reproduce it). */
 int mpm_target_sdf(MpmHandle* h, const void* target_density, void* target_sdf, void* nearest, void* work,
                    int32_t n_iters, void* stream);
 
