@@ -29,8 +29,8 @@ struct MpmHandle {
   const void* premarked = nullptr;  // frame whose block flags the last forward g2p set
   std::vector<MpmToolDesc> h_tools;
   unsigned int* d_status = nullptr;
-  int* d_flags = nullptr;  // convergence flags and barrier counter of mpm_target_sdf
-  unsigned char* d_tile_flags = nullptr;  // its changed tiles
+  int* d_flags = nullptr;  // convergence flags and counters of mpm_target_sdf
+  unsigned* d_tile_flags = nullptr;  // its changed nodes
   int* d_pair_off = nullptr;  // [n_scenes + 1] first collision pair of each scene
   int n_pairs = 0;            // tool-tool collision pairs over all scenes
   int max_scene_pairs = 0;    // most pairs of one scene
@@ -196,7 +196,7 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
   ok = ok && cudaMalloc(&h->d_pscene, std::max<size_t>(1, ps.size()) * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_tool_off, toff.size() * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_status, sizeof(unsigned int)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_flags, 4 * sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc(&h->d_flags, mpm::kTargetSdfFlags * sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_tile_flags, mpm::target_sdf_flag_bytes(p.n_scenes, p.n_grid)) == cudaSuccess;
   ok = ok && cudaMalloc(&h->d_pair_off, toff.size() * sizeof(int)) == cudaSuccess;
   for (int i = 0; i < 4 && ok; ++i) ok = cudaMalloc(&h->grid[i], gbytes) == cudaSuccess;

@@ -182,7 +182,7 @@ MPM_DI void warp_tails(long long key, bool ok, unsigned& tails, unsigned& emit) 
 // FP64: a node's four values are two double2, each in a table of its own with
 // the same stride.  The shuffle scan that FP64 took before cost 4 x 5 additions
 // per node and lane; summed by columns it is 33 rows x 4 per slab and lane
-// (SCAN64).
+// (37,001 particles: p2g 115 -> 68 us, g2p.grad 81 -> 59 us).
 template <typename T>
 struct SlabStage;
 template <>

@@ -175,10 +175,11 @@ cudaError_t launch_tools_action(const LaunchCtx& L, int n_tools, const int* pair
 cudaError_t launch_tools_action_bwd(const LaunchCtx& L, int n_tools, const int* pair_off, int n_pairs,
                                     const double* coll_pts, const double* vel, const double* pose, const double* coll,
                                     double* g_pose, double* g_action, int n_sub);
-// flags: 4 ints; changed: target_sdf_flag_bytes (both scratch of the handle)
+// flags: kTargetSdfFlags ints; changed: target_sdf_flag_bytes (both scratch of the handle)
+constexpr int kTargetSdfFlags = 192;
 size_t target_sdf_flag_bytes(int n_scenes, int n_grid);
 template <typename T>
-cudaError_t launch_target_sdf(const LaunchCtx& L, int* flags, unsigned char* changed, const T* dens, T* sdf, T* near,
+cudaError_t launch_target_sdf(const LaunchCtx& L, int* flags, unsigned* changed, const T* dens, T* sdf, T* near,
                               T* work, int n_iters);
 template <typename T>
 cudaError_t launch_sdf_loss(const LaunchCtx& L, const T* gm, const T* sdf, double weight, double* loss, T* ggm);

@@ -32,35 +32,53 @@ MPM_DI double add_rn(double a, double b) { return __dadd_rn(a, b); }
 // point.  Any other node takes, over the offsets (-3..2)^3 \ {0} in the
 // reference's ndrange order, the first strict minimum of
 // sqrt(|grid_pos - nearest_copy[v]|^2 + 1e-8) among in-grid neighbours with
-// sdf_copy[v] < 1000, else sdf 1000.  A CTA computes 8^3 tiles of one scene
-// from a 13^3 shared-memory copy of the nearest points around each.  The copy
-// holds a NaN for a neighbour with sdf_copy >= 1000, whose squared distance then
-// compares below nothing; a candidate is one 16-byte load in FP32.
+// sdf_copy[v] < 1000, else sdf 1000.  A CTA of 128 threads computes patches of
+// 4 x 4 x 8 nodes of one scene from a 9 x 9 x 13 shared-memory copy of the
+// nearest points around each.  The copy holds a NaN for a neighbour with
+// sdf_copy >= 1000, whose squared distance then compares below nothing; a
+// candidate is one 16-byte load in FP32.
 //
-// The square root is taken only for candidates whose squared distance is
-// below the best one so far: sqrt(dd + 1e-8) is monotone in dd, so a
-// candidate with dd >= best_dd cannot have a strictly smaller distance and
-// skipping it leaves the reference's result unchanged.
+// A candidate replaces the best one iff its rounded distance is smaller.  With
+// e = dd + 1e-8, e below the best one's by more than 8 ulp is certainly smaller
+// after the square root, and e not below it never is, so the loop compares e and
+// keeps the position of the best, without a branch or a square root per
+// candidate.  In between (neither on a grid of a power of two, where all dd are
+// exact and 1e-5 apart) the node is redone candidate by candidate.  With a branch
+// at each candidate whose dd was below the best one's, some lane of a warp took
+// it nearly every time: 60 us for a patch, however few were active.
 //
 // The iterations are separated by a grid barrier of a cooperative launch (all
 // CTAs are resident; the wait is bounded, and gives up with
 // MPM_STATUS_TIMEOUT).  Two facts leave work out without changing a value:
-// - an iteration whose tile and 26 neighbouring tiles did not change in the one
-//   before reproduces the tile's values, which both buffers already hold, so
-//   the tile is skipped (changed[t & 1][tile], one byte each);
+// - a warp (one plane of a patch) none of whose nodes' 6^3 neighbourhoods changed
+//   in the iteration before reproduces its values, which both buffers already
+//   hold, so it is skipped, and its patch if all four warps are
+//   (changed[t & 1][patch][warp], one bit per node).  The front and what still
+//   moves behind it are about a quarter of the warps;
 // - once an iteration changes nothing anywhere, neither does any later one
 //   (any[3]: iteration t sets any[t % 3], CTA 0 clears any[(t + 1) % 3]).
-// 64^3, 128 iterations: 128 launches of one iteration each took 1,205 us, of
-// which those after convergence about 2.5 us each; now TSDF_NOW.
-constexpr int TS_TILE = 8;
-constexpr int TS_SPAN = TS_TILE + 5;  // halo of 3 below and 2 above
-constexpr int TS_N = TS_SPAN * TS_SPAN * TS_SPAN;
+// What is left sits in a shell that no fixed assignment spreads evenly (with one
+// 8^3 tile per CTA an iteration took 50 us, the time of the SM with the most
+// active tiles), so the CTAs take the next patch from a counter (next[3], cleared
+// like any[3]).  64^3, 128 iterations: 128 launches of one iteration each took
+// 1,205 us; now 430.
+constexpr int TS_THREADS = 128;
+constexpr int TS_A = 4, TS_B = 4, TS_C = 8;             // nodes of a patch
+constexpr int TS_HA = 9, TS_HB = 9, TS_HC = 13;         // with the halo of 3 below and 2 above
+constexpr int TS_N = TS_HA * TS_HB * TS_HC;
 constexpr double TS_INF = 1000.0;
 
 template <typename T>
 struct alignas(4 * sizeof(T)) Near {
   T x, y, z, w;
 };
+
+// squared distance of p and a nearest point, each operation rounded on its own
+template <typename T>
+MPM_DI T near_dd(const T* p, const Near<T>& q) {
+  const T d0 = p[0] - q.x, d1 = p[1] - q.y, d2 = p[2] - q.z;
+  return add_rn(add_rn(mul_rn(d0, d0), mul_rn(d1, d1)), mul_rn(d2, d2));
+}
 
 // arrival counter of the grid barrier: barrier k is passed once it reaches
 // gridDim.x * (k + 1).  False when the wait ran out.
@@ -73,12 +91,12 @@ MPM_DI bool grid_barrier(unsigned* bar, unsigned target, unsigned* status) {
     ok = 0;
     for (int poll = 0; poll < (1 << 22); ++poll) {
       unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
       if (v >= target) {
         ok = 1;
         break;
       }
-      __nanosleep(64);
+      __nanosleep(100);
     }
     if (!ok) atomicOr(status, MPM_STATUS_TIMEOUT);
     __threadfence();
@@ -88,65 +106,90 @@ MPM_DI bool grid_barrier(unsigned* bar, unsigned target, unsigned* status) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(512) k_target_sdf(int n, int64_t G, int tiles, int64_t n_tiles,
-                                                    const T* __restrict__ dens, T* sdf, T* near, T* w_sdf, T* w_near,
-                                                    double dx, int n_iters, int* any, unsigned* bar,
-                                                    unsigned char* changed, unsigned* status) {
-  extern __shared__ __align__(32) unsigned char ts_smem[];
-  Near<T>* s_near = reinterpret_cast<Near<T>*>(ts_smem);
-  const int t3 = tiles * tiles * tiles;
+__global__ void __launch_bounds__(TS_THREADS, sizeof(T) == 4 ? 4 : 1) k_target_sdf(int n, int64_t G, int n_scenes, const T* __restrict__ dens,
+                                                           T* sdf, T* near, T* w_sdf, T* w_near, double dx, int n_iters,
+                                                           int* any, int* next, unsigned* bar, unsigned* changed,
+                                                           unsigned* status) {
+  __shared__ Near<T> s_near[TS_N];
+  __shared__ int s_patch;
+  const int na = (n + TS_A - 1) / TS_A, nb = (n + TS_B - 1) / TS_B, nc = (n + TS_C - 1) / TS_C;
+  const int per_scene = na * nb * nc, n_patches = n_scenes * per_scene;
   const T inf = T(TS_INF);
   const T none = T(NAN);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int l0 = warp, l1 = lane >> 3, l2 = lane & 7;
   for (int iter = 0; iter < n_iters; ++iter) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) any[(iter + 1) % 3] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      any[(iter + 1) % 3] = 0;
+      next[(iter + 1) % 3] = 0;
+    }
     // the last iteration writes the caller's arrays
     const bool to_out = ((n_iters - 1 - iter) & 1) == 0;
     const T* sdf_c = to_out ? w_sdf : sdf;
     const T* near_c = to_out ? w_near : near;
     T* sdf_o = to_out ? sdf : w_sdf;
     T* near_o = to_out ? near : w_near;
-    const unsigned char* before = changed + (int64_t)((iter + 1) & 1) * n_tiles;
-    unsigned char* now = changed + (int64_t)(iter & 1) * n_tiles;
-    for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-      const int scene = (int)(tile / t3);
-      const int tb = (int)(tile - (int64_t)scene * t3);
-      const int ta = tb / (tiles * tiles), tm = (tb / tiles) % tiles, tc = tb % tiles;
+    const unsigned* before = changed + (int64_t)((iter + 1) & 1) * n_patches * 4;
+    unsigned* now = changed + (int64_t)(iter & 1) * n_patches * 4;
+    while (true) {
+      // taken only now: a CTA that held its next patch while it worked on one
+      // would make the iteration wait for both
+      if (threadIdx.x == 0) s_patch = atomicAdd(next + iter % 3, 1);
+      __syncthreads();
+      const int patch = s_patch;
+      if (patch >= n_patches) break;
+      const int scene = patch / per_scene, q0 = patch - scene * per_scene;
+      const int pa = q0 / (nb * nc), pb = (q0 / nc) % nb, pc = q0 % nc;
+      bool work = true;
       if (iter > 0) {
-        int c = 0;
-        if (threadIdx.x < 27) {
-          const int i = ta + (int)threadIdx.x / 9 - 1, j = tm + ((int)threadIdx.x / 3) % 3 - 1,
-                    k = tc + (int)threadIdx.x % 3 - 1;
-          if (i >= 0 && i < tiles && j >= 0 && j < tiles && k >= 0 && k < tiles)
-            c = __ldcg(before + (int64_t)scene * t3 + (i * tiles + j) * tiles + k);
+        // the words of planes l0 - 3 .. l0 + 2 in the patches one before, here
+        // and one after along the other axes, less the nodes more than 3 before
+        // or 2 after this warp's
+        unsigned c = 0u;
+        for (int w = lane; w < 54; w += 32) {
+          const int plane = pa * TS_A + l0 - 3 + w / 9, db = (w / 3) % 3 - 1, dc = w % 3 - 1;
+          const int j = pb + db, k = pc + dc;
+          if (plane < 0 || plane >= na * TS_A || j < 0 || j >= nb || k < 0 || k >= nc) continue;
+          const unsigned rows = db < 0 ? 0xffffff00u : (db > 0 ? 0x0000ffffu : 0xffffffffu);
+          const unsigned cols = dc < 0 ? 0xe0e0e0e0u : (dc > 0 ? 0x03030303u : 0xffffffffu);
+          const int at = scene * per_scene + ((plane >> 2) * nb + j) * nc + k;
+          c |= __ldcg(before + (int64_t)at * 4 + (plane & 3)) & rows & cols;
         }
-        if (!__syncthreads_or(c)) {
-          if (threadIdx.x == 0) now[tile] = 0;
+        work = __any_sync(0xffffffffu, c != 0u);
+        if (!__syncthreads_or(work)) {  // (every thread has read s_patch)
+          if (threadIdx.x < 4) now[(int64_t)patch * 4 + threadIdx.x] = 0u;
           continue;
         }
       }
-      const int o0 = ta * TS_TILE, o1 = tm * TS_TILE, o2 = tc * TS_TILE;
+      const int o0 = pa * TS_A, o1 = pb * TS_B, o2 = pc * TS_C;
       const int64_t base = (int64_t)scene * G;
       if (iter > 0) {
-        for (int s = threadIdx.x; s < TS_N; s += blockDim.x) {
-          const int a = o0 - 3 + s / (TS_SPAN * TS_SPAN), b = o1 - 3 + (s / TS_SPAN) % TS_SPAN,
-                    c = o2 - 3 + s % TS_SPAN;
-          Near<T> q = {none, none, none, T(0)};
-          if (a >= 0 && a < n && b >= 0 && b < n && c >= 0 && c < n) {
+        // all of a thread's loads are issued together
+        constexpr int kRounds = (TS_N + TS_THREADS - 1) / TS_THREADS;
+        T v[kRounds], q[kRounds][3];
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+          const int s = threadIdx.x + TS_THREADS * r;
+          const int a = o0 - 3 + s / (TS_HB * TS_HC), b = o1 - 3 + (s / TS_HC) % TS_HB, c = o2 - 3 + s % TS_HC;
+          v[r] = inf;
+          if (s < TS_N && a >= 0 && a < n && b >= 0 && b < n && c >= 0 && c < n) {
             const int64_t id = base + ((int64_t)a * n + b) * n + c;
-            if (__ldcg(sdf_c + id) < inf) {
-              q.x = __ldcg(near_c + 3 * id);
-              q.y = __ldcg(near_c + 3 * id + 1);
-              q.z = __ldcg(near_c + 3 * id + 2);
-            }
+            v[r] = __ldcg(sdf_c + id);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) q[r][k] = __ldcg(near_c + 3 * id + k);
           }
-          s_near[s] = q;
+        }
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+          const int s = threadIdx.x + TS_THREADS * r;
+          if (s < TS_N)
+            s_near[s] = v[r] < inf ? Near<T>{q[r][0], q[r][1], q[r][2], T(0)} : Near<T>{none, none, none, T(0)};
         }
         __syncthreads();
       }
-      const int l0 = threadIdx.x / 64, l1 = (threadIdx.x / 8) % 8, l2 = threadIdx.x % 8;
       const int i0 = o0 + l0, i1 = o1 + l1, i2 = o2 + l2;
       bool diff = false;
-      if (i0 < n && i1 < n && i2 < n) {
+      if (work && i0 < n && i1 < n && i2 < n) {
         const int64_t id = base + ((int64_t)i0 * n + i1) * n + i2;
         const T gp[3] = {T(double(i0) * dx), T(double(i1) * dx), T(double(i2) * dx)};
         T best = inf, bn[3] = {T(0), T(0), T(0)};
@@ -156,28 +199,69 @@ __global__ void __launch_bounds__(512) k_target_sdf(int n, int64_t G, int tiles,
           bn[1] = gp[1];
           bn[2] = gp[2];
         } else if (iter > 0) {
-          T bdd = T(1e30);
-          for (int a = 0; a < 6; ++a)
-            for (int b = 0; b < 6; ++b) {
-              const Near<T>* row = s_near + ((l0 + a) * TS_SPAN + (l1 + b)) * TS_SPAN + l2;
+          const T keep = T(1) - (sizeof(T) == 4 ? T(4.76837158e-7) : T(1.7763568394002505e-15));  // 1 - 8 ulp
+          // three chains over two planes of neighbours each, joined in order: a
+          // single chain leaves the few warps of an SM waiting on it
+          constexpr int kChains = 3;
+          T e_best[kChains], lim[kChains];
+          int pos[kChains];
+          bool unsure = false;
 #pragma unroll
-              for (int c = 0; c < 6; ++c) {
-                if (c == 3 && a == 3 && b == 3) continue;
-                const Near<T> q = row[c];
-                const T d0 = gp[0] - q.x, d1 = gp[1] - q.y, d2 = gp[2] - q.z;
-                const T dd = add_rn(add_rn(mul_rn(d0, d0), mul_rn(d1, d1)), mul_rn(d2, d2));
-                if (dd < bdd) {
-                  const T dist = sqrt(add_rn(dd, T(1e-8)));
-                  if (dist < best) {
-                    best = dist;
-                    bdd = dd;
-                    bn[0] = q.x;
-                    bn[1] = q.y;
-                    bn[2] = q.z;
-                  }
+          for (int h = 0; h < kChains; ++h) {
+            e_best[h] = T(TS_INF * TS_INF);
+            lim[h] = e_best[h] * keep;
+            pos[h] = -1;
+          }
+#pragma unroll 1
+          for (int a = 0; a < 2; ++a)
+#pragma unroll 1
+            for (int b = 0; b < 6; ++b)
+#pragma unroll
+              for (int c = 0; c < 6; ++c)
+#pragma unroll
+                for (int h = 0; h < kChains; ++h) {
+                  if (h == 1 && c == 3 && a == 1 && b == 3) continue;  // the node itself
+                  const int s = ((l0 + 2 * h + a) * TS_HB + (l1 + b)) * TS_HC + l2 + c;
+                  const T e = add_rn(near_dd(gp, s_near[s]), T(1e-8));
+                  const bool less = e < e_best[h], win = e < lim[h];
+                  unsure = unsure || (less && !win);
+                  e_best[h] = win ? e : e_best[h];
+                  pos[h] = win ? s : pos[h];
+                  lim[h] = win ? e * keep : lim[h];
+                }
+          int at = pos[0];
+#pragma unroll
+          for (int h = 1; h < kChains; ++h) {
+            const bool less = e_best[h] < e_best[0], win = e_best[h] < lim[0];
+            unsure = unsure || (less && !win);
+            e_best[0] = win ? e_best[h] : e_best[0];
+            lim[0] = win ? lim[h] : lim[0];
+            at = win ? pos[h] : at;
+          }
+          if (unsure) {
+            at = -1;
+            T bdd = T(1e30);
+            for (int k = 0; k < 216; ++k) {
+              if (k == 3 * 36 + 3 * 6 + 3) continue;
+              const int s = ((l0 + k / 36) * TS_HB + (l1 + (k / 6) % 6)) * TS_HC + l2 + k % 6;
+              const T dd = near_dd(gp, s_near[s]);
+              if (dd < bdd) {
+                const T dist = sqrt(add_rn(dd, T(1e-8)));
+                if (dist < best) {
+                  best = dist;
+                  bdd = dd;
+                  at = s;
                 }
               }
             }
+          }
+          if (at >= 0) {
+            const Near<T> q = s_near[at];
+            best = sqrt(add_rn(near_dd(gp, q), T(1e-8)));
+            bn[0] = q.x;
+            bn[1] = q.y;
+            bn[2] = q.z;
+          }
         }
         if (iter == 0) {  // both buffers hold iteration 0
           diff = best < inf;
@@ -193,11 +277,12 @@ __global__ void __launch_bounds__(512) k_target_sdf(int n, int64_t G, int tiles,
           near_o[3 * id + 2] = bn[2];
         }
       }
-      const int moved = __syncthreads_or(diff);  // also: the tile's shared copy may be overwritten
-      if (threadIdx.x == 0) {
-        now[tile] = moved ? 1 : 0;
-        if (moved) any[iter % 3] = 1;
+      const unsigned bits = __ballot_sync(0xffffffffu, diff);
+      if (lane == 0) {
+        now[(int64_t)patch * 4 + warp] = bits;
+        if (bits) any[iter % 3] = 1;
       }
+      __syncthreads();  // s_patch and s_near are free
     }
     if (!grid_barrier(bar, gridDim.x * (unsigned)(iter + 1), status)) return;
     if (__ldcg(any + iter % 3) == 0) return;  // uniform over the grid
@@ -205,36 +290,35 @@ __global__ void __launch_bounds__(512) k_target_sdf(int n, int64_t G, int tiles,
 }
 
 size_t target_sdf_flag_bytes(int n_scenes, int n_grid) {
-  const int64_t tiles = (n_grid + TS_TILE - 1) / TS_TILE;
-  return (size_t)(2 * n_scenes * tiles * tiles * tiles);
+  auto up = [](int a, int b) { return (int64_t)((a + b - 1) / b); };
+  return (size_t)(2 * n_scenes * up(n_grid, TS_A) * up(n_grid, TS_B) * up(n_grid, TS_C)) * 4 * sizeof(unsigned);
 }
 
 template <typename T>
-cudaError_t launch_target_sdf(const LaunchCtx& L, int* flags, unsigned char* changed, const T* dens, T* sdf, T* near,
+cudaError_t launch_target_sdf(const LaunchCtx& L, int* flags, unsigned* changed, const T* dens, T* sdf, T* near,
                               T* work, int n_iters) {
-  int n = L.p->n_grid;
-  const int S = L.p->n_scenes;
+  int n = L.p->n_grid, S = L.p->n_scenes;
   if (n_iters <= 0 || S <= 0) return cudaSuccess;
-  int tiles = (n + TS_TILE - 1) / TS_TILE;
-  const size_t smem = (size_t)TS_N * sizeof(Near<T>);
-  cudaError_t e = cudaFuncSetAttribute(k_target_sdf<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_target_sdf<T>, 512, smem);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_target_sdf<T>, TS_THREADS, 0);
   if (e != cudaSuccess) return e;
-  int64_t n_tiles = (int64_t)S * tiles * tiles * tiles, G = L.G;
+  // few enough CTAs that each takes several patches, enough to hide a patch's loads
+  if (per_sm > 4) per_sm = 4;
+  const int64_t patches = (int64_t)(target_sdf_flag_bytes(S, n) / (8 * sizeof(unsigned)));
   const int64_t resident = (int64_t)per_sm * L.sm_count;
-  const unsigned grid = (unsigned)(n_tiles < resident ? n_tiles : resident);
-  MPM_MEMSET(L, flags, 4 * sizeof(int));
-  int* any = flags;
-  unsigned* bar = reinterpret_cast<unsigned*>(flags + 3);
+  const unsigned grid = (unsigned)(patches < resident ? patches : resident);
+  // each on lines of its own: the waiting CTAs poll bar
+  MPM_MEMSET(L, flags, kTargetSdfFlags * sizeof(int));
+  int *any = flags, *next = flags + 64;
+  unsigned* bar = reinterpret_cast<unsigned*>(flags + 128);
+  int64_t G = L.G;
   T* w_near = work + (int64_t)S * G;
   double dx = L.p->dx;
   unsigned* status = L.status;
-  void* args[] = {&n,      &G,  &tiles,   &n_tiles, (void*)&dens, &sdf,     &near,  &work,
-                  &w_near, &dx, &n_iters, &any,     &bar,         &changed, &status};
+  void* args[] = {&n,  &G,       &S,   (void*)&dens, &sdf, &near,    &work,  &w_near,
+                  &dx, &n_iters, &any, &next,        &bar, &changed, &status};
   const int slot = prof_begin(L.prof, L.stream);
-  e = cudaLaunchCooperativeKernel((const void*)k_target_sdf<T>, dim3(grid), dim3(512), args, smem, L.stream);
+  e = cudaLaunchCooperativeKernel((const void*)k_target_sdf<T>, dim3(grid), dim3(TS_THREADS), args, 0, L.stream);
   prof_end(L.prof, slot, MPM_K_OTHER, L.stream);
   ++*L.launches;
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -249,7 +333,7 @@ cudaError_t launch_target_sdf(const LaunchCtx& L, int* flags, unsigned char* cha
 // A node where both factors are zero adds nothing, and most of a grid is empty:
 // a warp whose 32 nodes are all empty skips the FP64 additions (an SM issues one
 // every 16 cycles).  With one CTA per scene and no such test the FP64 pipe of a
-// single SM did all the work: 64^3 IoU 525 us, SDF loss 151 us (LOSS_NOW).
+// single SM did all the work: 64^3 IoU 525 us, SDF loss 151 us now 24 and 15.
 // ---------------------------------------------------------------------------
 constexpr int RED_THREADS = 512;
 // 16 CTAs per scene while they are few (a non-portable size), else 8
@@ -535,7 +619,7 @@ cudaError_t launch_contact_min_bwd(const LaunchCtx& L, int n_tools, const T* st,
 }
 
 #define MPM_INST_LOSS(T)                                                                                       \
-  template cudaError_t launch_target_sdf<T>(const LaunchCtx&, int*, unsigned char*, const T*, T*, T*, T*, int); \
+  template cudaError_t launch_target_sdf<T>(const LaunchCtx&, int*, unsigned*, const T*, T*, T*, T*, int); \
   template cudaError_t launch_sdf_loss<T>(const LaunchCtx&, const T*, const T*, double, double*, T*);          \
   template cudaError_t launch_iou<T>(const LaunchCtx&, const T*, const T*, double*);                          \
   template cudaError_t launch_contact_min<T>(const LaunchCtx&, int, const T*, const double*, double*, int64_t*); \
