@@ -151,91 +151,144 @@ MPM_DI int block_node(const Consts<T>& c, int64_t gb, int l, int* I) {
   return scene;
 }
 
-// Segmented reduction of the scatter.  Particles are sorted by base cell, so
-// lanes with equal key (scene, base cell) are contiguous and scatter into the
-// same 27 nodes; each run of equal keys is summed before it goes to memory.
-// Lanes with a unique key (out of range, out of grid) form runs of one.
-// Segment ends of a warp for the slab scatter: bit r of `tails` is set when
-// lane r ends its run of equal keys, bit r of `emit` when that run is in the
-// grid (out-of-grid lanes carry unique keys, so they are runs of one).
-MPM_DI void warp_tails(long long key, bool ok, unsigned& tails, unsigned& emit) {
+// Scatter rows of a warp.  Particles of one grid cell scatter into the same 27
+// nodes, so a warp sums them before it goes to memory.  The particles were sorted
+// by cell some substeps ago; since then some have moved to a neighbouring cell and
+// sit between particles of their old one (after 25 substeps a warp of 32 holds 7
+// runs of equal cells but 4 different cells, after 50 substeps 14 and 5).  So the
+// warp's lanes are put in order again: lane l's row is its place when the lanes
+// are grouped by key, groups in the order of their first lanes.  Bit r of `tails`
+// is set when row r ends its group, bit r of `emit` when that group is in the grid
+// (lanes out of the grid carry unique keys).
+struct WarpRows {
+  int row;
+  unsigned tails, emit;
+};
+MPM_DI WarpRows warp_rows(long long key, bool ok) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const long long next = __shfl_down_sync(full, key, 1);
-  const bool tail = lane == 31 || next != key;
-  tails = __ballot_sync(full, tail);
-  emit = __ballot_sync(full, tail && ok);
+  const unsigned below = (1u << lane) - 1u;
+  const unsigned peers = __match_any_sync(full, key);
+  const int size = __popc(peers), first = __ffs(peers) - 1;
+  // rows before each lane's group, if the lane is its first: an exclusive scan
+  int before = lane == first ? size : 0;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int t = __shfl_up_sync(full, before, d);
+    if (lane >= d) before += t;
+  }
+  const int end = __shfl_sync(full, before, first);  // rows up to and with this lane's group
+  WarpRows w;
+  w.row = end - size + __popc(peers & below);
+  const unsigned last = 1u << (end - 1);
+  w.tails = __reduce_or_sync(full, last);
+  w.emit = __reduce_or_sync(full, ok ? last : 0u);
+  return w;
 }
 
-// Slab scatter.  The 27-node stencil is scattered one ox slab (9 nodes)
-// at a time: every lane writes its 9 node values into row `lane` of v, then
-// lanes 0..26 read the table by columns, lane = g + 3 j summing column j over
-// rows [11 g, 11 g + 11).  Each run of equal keys closed inside a row group
-// issues one red.global.add.v4.f32 per node; the run still open at the end of
-// a group is carried into the next group by two shuffles.  This replaces a
-// shuffle scan of 4 values x 27 nodes x up to 5 steps per lane with 27
-// shared-memory stores, 11 loads per slab and 8 shuffles per slab, and keeps
-// one atomic per (run, node).  Row stride 9 x 16 B: the stores (lane l, slot
-// 9 l + n) and the loads (slot 99 g + 9 i + j, i.e. 3 g + i + j mod 8 with
-// lane = g + 3 j) fall in distinct 16-byte bank groups within each quarter
-// warp.
-// FP64: a node's four values are two double2, each in a table of its own with
-// the same stride.  The shuffle scan that FP64 took before cost 4 x 5 additions
-// per node and lane; summed by columns it is 33 rows x 4 per slab and lane
-// (37,001 particles: p2g 115 -> 68 us, g2p.grad 81 -> 59 us).
-template <typename T>
-struct SlabStage;
-template <>
-struct SlabStage<float> {
-  float4 v[33][9];  // row 32: read, never used (the open run of group 2 after row 31)
-  Node<float>* base[32];  // grid of the row's scene + ax[ox] of the row's base cell
-  int ay[32][3], az[32][3];
-};
-template <>
-struct SlabStage<double> {
-  double2 v[33][9], u[33][9];  // (x, y) and (z, w)
-  Node<double>* base[32];
-  int ay[32][3], az[32][3];
+// FP32 row scatter.  Every lane writes what its particle contributes to a node,
+// wgt(o) (u + G o) and wgt(o), as the 12 values of u and G's columns, the 9
+// products wy wz and the 3 wx; then 27 lanes, one per node o, walk the 32 rows: a
+// row is three broadcast 16-byte loads, two weights and nine fused multiply-adds
+// (three of them packed pairs) in registers, and a group's end is the same row for
+// all lanes, so its sum leaves by one 27-lane red.global.add.v4.f32 without
+// divergence.  Before, every lane stored its 27 node values one slab of 9 at a
+// time and 27 lanes = 9 nodes x 3 row groups read them back, which closed each
+// run three times per substep and diverged over the row groups (ROWSCATTER).
+struct RowStage {
+  float4 q0[32];       // u.x, u.y, G00, G10
+  float4 q1[32];       // G01, G11, G02, G12
+  float4 q2[32];       // u.z, G20, G21, G22
+  float wyz[32][9];
+  float wx[32][4];
+  Node<float>* base[32];  // grid of the row's scene
+  int off[32][12];        // ax[3], ay[3], az[3] of the row's stencil
 };
 // Packed FP32 pairs (add/mul/fma .f32x2): one instruction for two lanes of
 // arithmetic, each rounded as the scalar operation would be
 MPM_DI unsigned long long f2_bits(float2 a) { return *reinterpret_cast<unsigned long long*>(&a); }
 MPM_DI float2 f2_of(unsigned long long b) { return *reinterpret_cast<float2*>(&b); }
-MPM_DI float2 add2(float2 a, float2 b) {
+MPM_DI float2 fma2(float2 a, float2 b, float2 c) {
   unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
   return f2_of(d);
 }
-MPM_DI float2 mul2(float2 a, float2 b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2_bits(a)), "l"(f2_bits(b)));
-  return f2_of(d);
+// row r of the stage: the lane's particle (u, G row-major)
+MPM_DI void row_put(RowStage& sb, int r, const float* u, const float* G, const Stencil<float>& s, const StencilAddr& A,
+                    Node<float>* grid) {
+  sb.q0[r] = make_float4(u[0], u[1], G[0], G[3]);
+  sb.q1[r] = make_float4(G[1], G[4], G[2], G[5]);
+  sb.q2[r] = make_float4(u[2], G[6], G[7], G[8]);
+#pragma unroll
+  for (int oy = 0; oy < 3; ++oy)
+#pragma unroll
+    for (int oz = 0; oz < 3; ++oz) sb.wyz[r][oy * 3 + oz] = s.w[oy][1] * s.w[oz][2];
+  *reinterpret_cast<float4*>(sb.wx[r]) = make_float4(s.w[0][0], s.w[1][0], s.w[2][0], 0.f);
+  sb.base[r] = grid;
+  int4* off = reinterpret_cast<int4*>(sb.off[r]);
+  off[0] = make_int4(A.ax[0], A.ax[1], A.ax[2], A.ay[0]);
+  off[1] = make_int4(A.ay[1], A.ay[2], A.az[0], A.az[1]);
+  off[2] = make_int4(A.az[2], 0, 0, 0);
 }
-// a += b, in two packed pair additions or four scalar ones (measured: the
-// packed form helps p2g and slows g2p.grad, whose fourth lane is zero)
-template <bool Packed = false>
-MPM_DI void f4_add(float4& a, const float4& b) {
-  if constexpr (Packed) {
-    const float2 lo = add2(make_float2(a.x, a.y), make_float2(b.x, b.y));
-    const float2 hi = add2(make_float2(a.z, a.w), make_float2(b.z, b.w));
-    a = make_float4(lo.x, lo.y, hi.x, hi.y);
-  } else {
-    a.x += b.x;
-    a.y += b.y;
-    a.z += b.z;
-    a.w += b.w;
+// after a __syncwarp() that follows row_put by all lanes.  W: the fourth value of
+// a node gets the weights' sum times wm (else 0).
+template <bool W>
+MPM_DI void row_scatter(const RowStage& sb, unsigned tails, unsigned emit, float wm) {
+  const int lane = threadIdx.x & 31;
+  const int node = lane < 27 ? lane : 26;  // lanes 27..31 shadow lane 26 and emit nothing
+  const int ox = node / 9, j = node - 9 * ox, oy = j / 3, oz = j - 3 * oy;
+  const float fx = (float)ox, fy = (float)oy, fz = (float)oz;
+  const float2 fx2 = make_float2(fx, fx), fy2 = make_float2(fy, fy), fz2 = make_float2(fz, fz);
+  float2 xy = make_float2(0.f, 0.f), zw = xy;
+#pragma unroll 4
+  for (int r = 0; r < 32; ++r) {
+    const float4 q0 = sb.q0[r], q1 = sb.q1[r], q2 = sb.q2[r];
+    const float wgt = sb.wx[r][ox] * sb.wyz[r][j];
+    const float2 w2 = make_float2(wgt, wgt);
+    float2 v = fma2(fx2, make_float2(q0.z, q0.w), make_float2(q0.x, q0.y));
+    v = fma2(fy2, make_float2(q1.x, q1.y), v);
+    v = fma2(fz2, make_float2(q1.z, q1.w), v);
+    const float z = fmaf(fz, q2.w, fmaf(fy, q2.z, fmaf(fx, q2.y, q2.x)));
+    xy = fma2(w2, v, xy);
+    zw = fma2(w2, make_float2(z, W ? 1.f : 0.f), zw);
+    if ((tails >> r) & 1u) {  // the same row for the whole warp
+      if (((emit >> r) & 1u) && lane < 27)
+        atomicAdd(reinterpret_cast<float4*>(sb.base[r] + (sb.off[r][ox] + sb.off[r][3 + oy] + sb.off[r][6 + oz])),
+                  make_float4(xy.x, xy.y, zw.x, W ? wm * zw.y : 0.f));
+      xy = zw = make_float2(0.f, 0.f);
+    }
   }
 }
-MPM_DI float4 f4_shfl_up(const float4& a, int d) {
-  return make_float4(__shfl_up_sync(0xffffffffu, a.x, d), __shfl_up_sync(0xffffffffu, a.y, d),
-                     __shfl_up_sync(0xffffffffu, a.z, d), __shfl_up_sync(0xffffffffu, a.w, d));
+
+// FP64 slab scatter.  The 27-node stencil is scattered one ox slab (9 nodes) at a
+// time: every lane writes its 9 node values into its row of v and u, then lanes
+// 0..26 read the table by columns, lane = g + 3 j summing column j over rows
+// [11 g, 11 g + 11).  Each run of equal keys closed inside a row group issues its
+// atomics; the run still open at the end of a group is carried into the next by
+// two shuffles.  A node's four values are two double2, each in a table of its own
+// with row stride 9 x 16 B: stores and loads fall in distinct 16-byte bank groups
+// within each quarter warp.  (The FP32 row scatter would take 13 FP64 operations
+// per row and lane, 416 per warp, against some 360 here.)  The shuffle scan that
+// FP64 took before cost 4 x 5 additions per node and lane; summed by columns it is
+// 33 rows x 4 per slab and lane (37,001 particles: p2g 115 -> 68 us, g2p.grad
+// 81 -> 59 us).
+struct SlabStage {
+  double2 v[33][9], u[33][9];  // (x, y) and (z, w); row 32: read, never used
+  Node<double>* base[32];      // grid of the row's scene + ax[ox] of the row's base cell
+  int ay[32][3], az[32][3];
+};
+MPM_DI void slab_addresses(SlabStage& sb, int row, const StencilAddr& A) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    sb.ay[row][k] = A.ay[k];
+    sb.az[row][k] = A.az[k];
+  }
 }
-MPM_DI void slab_emit(const SlabStage<float>& sb, int r, int oy, int oz, const float4& a) {
-  atomicAdd(reinterpret_cast<float4*>(sb.base[r] + sb.ay[r][oy] + sb.az[r][oz]), a);
-}
-// call between two __syncwarp()s, after all lanes wrote their row of sb.v
-template <bool Packed = false>
-MPM_DI void slab_reduce(const SlabStage<float>& sb, unsigned tails, unsigned emit) {
+// Called between two __syncwarp()s, after all lanes wrote their row of sb.v and
+// sb.u.  W: the fourth value is summed too, and multiplied by wm when it is added
+// to the grid (p2g: the weights' sum times the particle mass).
+template <bool W>
+MPM_DI void slab_reduce64(const SlabStage& sb, unsigned tails, unsigned emit, double wm) {
   const int lane = threadIdx.x & 31;
   // lanes 27..31 (g = 3) read lane 24's cells (a broadcast) and emit nothing
   const int g = lane < 27 ? lane % 3 : 3;
@@ -243,41 +296,6 @@ MPM_DI void slab_reduce(const SlabStage<float>& sb, unsigned tails, unsigned emi
   const int oy = j / 3, oz = j - 3 * (j / 3);
   const int r0 = 11 * (g < 3 ? g : 0);
   const unsigned mine = g < 3 ? tails >> r0 : 0u;  // group 2: bit 10 (row 32) is 0
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), head = acc;
-  int head_row = -1;
-#pragma unroll
-  for (int i = 0; i < 11; ++i) {
-    f4_add<Packed>(acc, sb.v[r0 + i][j]);
-    if ((mine >> i) & 1u) {
-      if (g > 0 && head_row < 0) {
-        head = acc;  // closes a run that may have started in the group before
-        head_row = r0 + i;
-      } else if ((emit >> (r0 + i)) & 1u) {
-        slab_emit(sb, r0 + i, oy, oz, acc);
-      }
-      acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  // acc = the open run at the group's end; group 2 always closes (row 31)
-  const float4 c1 = f4_shfl_up(acc, 1);  // group 1: open run of group 0
-  float4 fwd = acc;
-  if (g == 1 && head_row < 0) f4_add(fwd, c1);  // group 1 without a tail passes the run on
-  const float4 c2 = f4_shfl_up(fwd, 1);          // group 2: open run of groups 0..1
-  if (g >= 1 && g < 3 && head_row >= 0) {
-    f4_add(head, g == 1 ? c1 : c2);
-    if ((emit >> head_row) & 1u) slab_emit(sb, head_row, oy, oz, head);
-  }
-}
-// The same for FP64.  W: the fourth value is summed too, and multiplied by wm
-// when it is added to the grid (p2g: the weights' sum times the particle mass).
-template <bool W>
-MPM_DI void slab_reduce64(const SlabStage<double>& sb, unsigned tails, unsigned emit, double wm) {
-  const int lane = threadIdx.x & 31;
-  const int g = lane < 27 ? lane % 3 : 3;
-  const int j = lane < 27 ? lane / 3 : 8;
-  const int oy = j / 3, oz = j - 3 * (j / 3);
-  const int r0 = 11 * (g < 3 ? g : 0);
-  const unsigned mine = g < 3 ? tails >> r0 : 0u;
   double acc[4] = {0.0, 0.0, 0.0, 0.0}, head[4] = {0.0, 0.0, 0.0, 0.0};
   int head_row = -1;
   auto put = [&](int r, const double* a) {
@@ -307,6 +325,7 @@ MPM_DI void slab_reduce64(const SlabStage<double>& sb, unsigned tails, unsigned 
       for (int k = 0; k < 4; ++k) acc[k] = 0.0;
     }
   }
+  // acc = the open run at the group's end; group 2 always closes (row 31)
 #pragma unroll
   for (int k = 0; k < (W ? 4 : 3); ++k) {
     const double c1 = __shfl_up_sync(0xffffffffu, acc[k], 1);
@@ -316,16 +335,17 @@ MPM_DI void slab_reduce64(const SlabStage<double>& sb, unsigned tails, unsigned 
   }
   if (g >= 1 && g < 3 && head_row >= 0) put(head_row, head);
 }
-// the slab's rows start at the grid of the lane's scene
+
 template <typename T>
-MPM_DI void slab_addresses(SlabStage<T>& sb, const StencilAddr& A) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    sb.ay[lane][k] = A.ay[k];
-    sb.az[lane][k] = A.az[k];
-  }
-}
+struct ScatterStage;
+template <>
+struct ScatterStage<float> {
+  using type = RowStage;
+};
+template <>
+struct ScatterStage<double> {
+  using type = SlabStage;
+};
 
 template <typename T>
 MPM_DI void zero_stencil(Stencil<T>& s) {
@@ -382,7 +402,7 @@ MPM_DI void store_row(T* __restrict__ st, int64_t ld, int64_t p, int r0, int n, 
 template <typename S>
 struct P2G {
   S U[9], s[3], V[9];
-  S is[3];   // 1 / s (FP64 only)
+  S is[3];   // 1 / s (0: the SVD was plain, see svd3_left32 and svd3_left64)
   S sm1[3];  // s - 1 (FP32: from the shifted SVD, exact as s -> 1)
   S sigc[3], ehat[3], nrm, inrm, dg, k, e[3];  // inrm = 1 / nrm (FP64 only)
   bool yield;
@@ -396,7 +416,7 @@ struct P2G {
 // (1e-4 at a strain of 1e-3), which then drives the trajectory apart from the
 // FP64 one.  Here every small quantity is formed directly: D = G + dt C (I + G)
 // with G = F - I (exact for F_ii in [0.5, 2]); the SVD of I + D from the
-// shifted matrix (svd3_shifted) with s - 1; log(s) = log1p(s - 1); the
+// shifted matrix (svd3_left32) with s - 1; log(s) = log1p(s - 1); the
 // projected singular values e - 1 = expm1(eps'); newF - R = U diag(e - 1) V^T;
 // J - 1 = det(I + D) - 1 = tr D + (tr(D)^2 - tr(D^2)) / 2 + det D (elastic) or
 // expm1(sum eps) (yield: the von Mises map keeps the volume).  The stored F
@@ -407,6 +427,7 @@ struct P2G {
 // 122-129, 166-225).  The stress takes the SVD basis,
 // (newF - R) newF^T = U diag((e - 1) e) U^T; new_F (may be null: the
 // adjoint's recompute) receives the updated F.
+template <bool WithV>
 MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const float* F, P2G<float>& P,
                              float* affine, float* new_F) {
   float G[9], CG[9], D[9];
@@ -415,7 +436,17 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
   mm(C, G, CG);
 #pragma unroll
   for (int i = 0; i < 9; ++i) D[i] = G[i] + m.dt * (C[i] + CG[i]);
-  svd3_shifted(D, P.U, P.s, P.sm1, P.V);
+  // J - 1 = det(I + D) - 1 by its invariants
+  float Jm1 = D[0] + D[4] + D[8];
+  {
+    float D2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) D2 += D[i * 3 + j] * D[j * 3 + i];
+    Jm1 += 0.5f * (Jm1 * Jm1 - D2) + det3(D);
+  }
+  const bool plain = svd3_left32<WithV>(D, 1.f + Jm1, P.U, P.s, P.sm1, P.is, P.V);
   float eps[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -450,20 +481,9 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
       pc[i] = 0.f;
     }
   }
-  // J - 1: det(I + D) - 1 by its invariants; the return map keeps the volume,
-  // unless a singular value sits at the 0.05 floor (then J = prod sigc)
-  float Jm1;
-  if (P.yield && !(0.05f < P.s[0] && 0.05f < P.s[1] && 0.05f < P.s[2])) {
-    Jm1 = expm1f(esum);
-  } else {
-    const float tr = D[0] + D[4] + D[8];
-    float D2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) D2 += D[i * 3 + j] * D[j * 3 + i];
-    Jm1 = tr + 0.5f * (tr * tr - D2) + det3(D);
-  }
+  // the return map keeps the volume, unless a singular value sits at the 0.05
+  // floor (then J = prod sigc)
+  if (P.yield && !(0.05f < P.s[0] && 0.05f < P.s[1] && 0.05f < P.s[2])) Jm1 = expm1f(esum);
   P.J = 1.f + Jm1;
   // (newF - R) newF^T = U diag(e - 1) V^T V diag(e) U^T = U diag((e - 1) e) U^T
   float h[3];
@@ -483,11 +503,28 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
   if (new_F) {
     if (P.yield) {
       float UP[9], corr[9];
+      if (plain) {
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+        for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int cc = 0; cc < 3; ++cc) UP[r * 3 + cc] = P.U[r * 3 + cc] * pc[cc];
-      mmT(UP, P.V, corr);
+          for (int cc = 0; cc < 3; ++cc) UP[r * 3 + cc] = P.U[r * 3 + cc] * pc[cc];
+        mmT(UP, P.V, corr);
+      } else {  // U diag(pc) V^T = W (I + D), W = U diag(pc / s) U^T
+        float W[9];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+          for (int cc = 0; cc < 3; ++cc) UP[r * 3 + cc] = P.U[r * 3 + cc] * (pc[cc] * P.is[cc]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = i; j < 3; ++j)
+            W[i * 3 + j] = W[j * 3 + i] =
+                UP[i * 3] * P.U[j * 3] + UP[i * 3 + 1] * P.U[j * 3 + 1] + UP[i * 3 + 2] * P.U[j * 3 + 2];
+        mm(W, D, corr);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) corr[i] += W[i];
+      }
 #pragma unroll
       for (int i = 0; i < 9; ++i) new_F[i] = (D[i] + corr[i]) + ((i % 4 == 0) ? 1.f : 0.f);
     } else {
@@ -591,7 +628,7 @@ MPM_DI void p2g_particle_f64(const MatConsts<double>& m, const double* C, const 
 template <bool WithV, typename S>
 MPM_DI void p2g_particle(const MatConsts<S>& m, const S* C, const S* F, P2G<S>& P, S* affine, S* new_F) {
   if constexpr (sizeof(S) == 4)
-    p2g_particle_f32(m, C, F, P, affine, new_F);
+    p2g_particle_f32<WithV>(m, C, F, P, affine, new_F);
   else
     p2g_particle_f64<WithV>(m, C, F, P, affine, new_F);
 }
@@ -780,49 +817,20 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
   const long long key = ok ? cell_key(c, scene, s) : -1 - (long long)(threadIdx.x & 31);
   Node<T>* g = grid + (int64_t)scene * c.G;
   const StencilAddr A = stencil_addr(c, s);
-  const int lane = threadIdx.x & 31;
-  unsigned tails, emit;
-  __shared__ SlabStage<T> stage[kParticleThreads<S> / 32];  // one per warp
-  SlabStage<T>* sb = &stage[threadIdx.x >> 5];
-  warp_tails(key, ok, tails, emit);
-  slab_addresses(*sb, A);
-  pdl_wait();  // the grid blocks are zeroed by the compaction before
-  pdl_trigger();
+  __shared__ typename ScatterStage<T>::type stage[kParticleThreads<S> / 32];  // one per warp
+  auto* sb = &stage[threadIdx.x >> 5];
+  const WarpRows rows = warp_rows(key, ok);
   if constexpr (sizeof(T) == 4) {
-    // FP32: the node value wgt (m v + A dp, m) in packed pairs: (x, y) and
-    // (z, m), stepped across the stencil by the columns of A (and 0 for m)
-    float2 cxA = make_float2(pm[0], pm[1]), cxB = make_float2(pm[2], c.p_mass);
-    const float2 a0A = make_float2(affine[0], affine[3]), a0B = make_float2(affine[6], 0.f);
-    const float2 a1A = make_float2(affine[1], affine[4]), a1B = make_float2(affine[7], 0.f);
-    const float2 a2A = make_float2(affine[2], affine[5]), a2B = make_float2(affine[8], 0.f);
-#pragma unroll 1
-    for (int ox = 0; ox < 3; ++ox) {
-      const float wx = sel3(s.w[0][0], s.w[1][0], s.w[2][0], ox);
-      const int ax = sel3(A.ax[0], A.ax[1], A.ax[2], ox);
-      float2 cyA = cxA, cyB = cxB;
-#pragma unroll
-      for (int oy = 0; oy < 3; ++oy) {
-        float2 czA = cyA, czB = cyB;
-#pragma unroll
-        for (int oz = 0; oz < 3; ++oz) {
-          const float wgt = wx * s.w[oy][1] * s.w[oz][2];
-          const float2 w2 = make_float2(wgt, wgt);
-          const float2 lo = mul2(w2, czA), hi = mul2(w2, czB);
-          sb->v[lane][oy * 3 + oz] = make_float4(lo.x, lo.y, hi.x, hi.y);
-          czA = add2(czA, a2A);
-          czB = add2(czB, a2B);
-        }
-        cyA = add2(cyA, a1A);
-        cyB = add2(cyB, a1B);
-      }
-      cxA = add2(cxA, a0A);
-      cxB = add2(cxB, a0B);
-      sb->base[lane] = g + ax;
-      __syncwarp();
-      slab_reduce<true>(*sb, tails, emit);
-      __syncwarp();
-    }
+    __syncwarp();  // a strided caller's previous chunk has been read
+    row_put(*sb, rows.row, pm, affine, s, A, g);
+    __syncwarp();
+    pdl_wait();  // the grid blocks are zeroed by the compaction before
+    pdl_trigger();
+    row_scatter<true>(*sb, rows.tails, rows.emit, c.p_mass);
   } else {
+    slab_addresses(*sb, rows.row, A);
+    pdl_wait();
+    pdl_trigger();
     T cx[3] = {pm[0], pm[1], pm[2]};
 #pragma unroll 1
     for (int ox = 0; ox < 3; ++ox) {
@@ -836,8 +844,8 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
 #pragma unroll
         for (int oz = 0; oz < 3; ++oz) {
           const T wgt = wxy * s.w[oz][2];
-          sb->v[lane][oy * 3 + oz] = make_double2(wgt * cz[0], wgt * cz[1]);
-          sb->u[lane][oy * 3 + oz] = make_double2(wgt * cz[2], wgt);
+          sb->v[rows.row][oy * 3 + oz] = make_double2(wgt * cz[0], wgt * cz[1]);
+          sb->u[rows.row][oy * 3 + oz] = make_double2(wgt * cz[2], wgt);
 #pragma unroll
           for (int k = 0; k < 3; ++k) cz[k] += affine[3 * k + 2];
         }
@@ -846,9 +854,9 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k) cx[k] += affine[3 * k];
-      sb->base[lane] = g + ax;
+      sb->base[rows.row] = g + ax;
       __syncwarp();
-      slab_reduce64<true>(*sb, tails, emit, c.p_mass);
+      slab_reduce64<true>(*sb, rows.tails, rows.emit, c.p_mass);
       __syncwarp();
     }
   }
@@ -1210,12 +1218,9 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
     }
   }
   const long long key = ok ? cell_key(c, scene, s) : -1 - (long long)(threadIdx.x & 31);
-  const int lane = threadIdx.x & 31;
-  unsigned tails, emit;
-  __shared__ SlabStage<T> stage[kParticleThreads<T> / 32];  // one per warp
-  SlabStage<T>* sb = &stage[threadIdx.x >> 5];
-  warp_tails(key, ok, tails, emit);
-  slab_addresses(*sb, A);
+  __shared__ typename ScatterStage<T>::type stage[kParticleThreads<T> / 32];  // one per warp
+  auto* sb = &stage[threadIdx.x >> 5];
+  const WarpRows rows = warp_rows(key, ok);
   const T k4 = T(4) * c.inv_dx;
   T gw[3][3];
 #pragma unroll
@@ -1265,38 +1270,39 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
       for (int i = 0; i < 3; ++i) vx[i] += gC[3 * i];
     }
   }
+  if constexpr (sizeof(T) == 4) {
+    row_put(*sb, rows.row, ux, gC, s, A, gg);
+    __syncwarp();
+    row_scatter<false>(*sb, rows.tails, rows.emit, 0.f);
+  } else {
+    slab_addresses(*sb, rows.row, A);
 #pragma unroll 1
-  for (int ox = 0; ox < 3; ++ox) {
-    const T wx = sel3(s.w[0][0], s.w[1][0], s.w[2][0], ox);
-    const int ax = sel3(A.ax[0], A.ax[1], A.ax[2], ox);
-    T uy[3] = {ux[0], ux[1], ux[2]};
+    for (int ox = 0; ox < 3; ++ox) {
+      const T wx = sel3(s.w[0][0], s.w[1][0], s.w[2][0], ox);
+      const int ax = sel3(A.ax[0], A.ax[1], A.ax[2], ox);
+      T uy[3] = {ux[0], ux[1], ux[2]};
 #pragma unroll
-    for (int oy = 0; oy < 3; ++oy) {
-      T uz[3] = {uy[0], uy[1], uy[2]};
+      for (int oy = 0; oy < 3; ++oy) {
+        T uz[3] = {uy[0], uy[1], uy[2]};
+        const T wxy = wx * s.w[oy][1];
 #pragma unroll
-      for (int oz = 0; oz < 3; ++oz) {
-        const T wgt = wx * s.w[oy][1] * s.w[oz][2];
-        if constexpr (sizeof(T) == 4) {
-          sb->v[lane][oy * 3 + oz] = make_float4(wgt * uz[0], wgt * uz[1], wgt * uz[2], 0.f);
-        } else {
-          sb->v[lane][oy * 3 + oz] = make_double2(wgt * uz[0], wgt * uz[1]);
-          sb->u[lane][oy * 3 + oz] = make_double2(wgt * uz[2], 0.0);
+        for (int oz = 0; oz < 3; ++oz) {
+          const T wgt = wxy * s.w[oz][2];
+          sb->v[rows.row][oy * 3 + oz] = make_double2(wgt * uz[0], wgt * uz[1]);
+          sb->u[rows.row][oy * 3 + oz] = make_double2(wgt * uz[2], 0.0);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) uz[i] += gC[3 * i + 2];
         }
 #pragma unroll
-        for (int i = 0; i < 3; ++i) uz[i] += gC[3 * i + 2];
+        for (int i = 0; i < 3; ++i) uy[i] += gC[3 * i + 1];
       }
 #pragma unroll
-      for (int i = 0; i < 3; ++i) uy[i] += gC[3 * i + 1];
+      for (int i = 0; i < 3; ++i) ux[i] += gC[3 * i];
+      sb->base[rows.row] = gg + ax;
+      __syncwarp();
+      slab_reduce64<false>(*sb, rows.tails, rows.emit, 1.0);
+      __syncwarp();
     }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) ux[i] += gC[3 * i];
-    sb->base[lane] = gg + ax;
-    __syncwarp();
-    if constexpr (sizeof(T) == 4)
-      slab_reduce(*sb, tails, emit);
-    else
-      slab_reduce64<false>(*sb, tails, emit, 1.0);
-    __syncwarp();
   }
   if (ok) {
 #pragma unroll

@@ -290,6 +290,84 @@ MPM_DI void svd3_shifted(const float* D, float* U, float* s, float* sm1, float* 
   }
 }
 
+// The plain shifted SVD, out of line: for the few matrices that svd3_left32
+// leaves to it.
+__device__ __noinline__ inline void svd3_plain32(const float* D, float* U, float* s, float* sm1, float* V) {
+  svd3_shifted(D, U, s, sm1, V);
+}
+// FP32 SVD of A = I + D = U diag(s) V^T from the left: the Jacobi rotations of
+// svd3_shifted on A A^T - I = D + D^T + D D^T give U and s^2 - 1 at once, so the
+// forward pass, which needs no V, has neither svd3_shifted's product A V nor its
+// Gram-Schmidt, and V = A^T U diag(1/s) takes their place in the adjoint.  The
+// values are in no particular order (nothing depends on it).  A rotation scales
+// its two columns by sqrt(c^2 + s^2) = 1 + O(1e-7), so each column is normalised
+// once at the end by 3/2 - |u|^2 / 2.  detA = det(I + D).  Returns true (plain) for an inverted or
+// nearly singular matrix (s < 0.2): then U, s, sm1, V come from svd3_shifted
+// and is = 0.  V is written when plain or WithV; is = 1/s.
+template <bool WithV>
+MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* sm1, float* is, float* V) {
+  float ev[3];
+  {
+    float a00 = 2.f * D[0] + dot3(D, D), a11 = 2.f * D[4] + dot3(D + 3, D + 3), a22 = 2.f * D[8] + dot3(D + 6, D + 6);
+    float a01 = D[1] + D[3] + dot3(D, D + 3), a02 = D[2] + D[6] + dot3(D, D + 6), a12 = D[5] + D[7] + dot3(D + 3, D + 6);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) U[k] = (k % 4 == 0) ? 1.f : 0.f;
+    for (int sweep = 0; sweep < SvdIters<float>::max_sweeps; ++sweep) {
+      const float off = a01 * a01 + a02 * a02 + a12 * a12;
+      const float dg = a00 * a00 + a11 * a11 + a22 * a22;
+      // relative to the matrix; the absolute floor stops sweeps on rounding noise (rigid rotations)
+      if (off <= kShiftedTol * dg + 1e-30f) break;
+      jacobi_rot(a00, a11, a01, a02, a12, U, 0, 1);
+      jacobi_rot(a00, a22, a02, a01, a12, U, 0, 2);
+      jacobi_rot(a11, a22, a12, a01, a02, U, 1, 2);
+    }
+    ev[0] = a00;
+    ev[1] = a11;
+    ev[2] = a22;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float f = 1.5f - 0.5f * (U[k] * U[k] + U[3 + k] * U[3 + k] + U[6 + k] * U[6 + k]);
+    U[k] *= f;
+    U[3 + k] *= f;
+    U[6 + k] *= f;
+  }
+  const bool plain = !(fminf(fminf(ev[0], ev[1]), ev[2]) > -0.96f && detA > 0.f);
+  if (plain) {
+    float Dl[9], Ul[9], sl[3], ml[3], Vl[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Dl[k] = D[k];
+    svd3_plain32(Dl, Ul, sl, ml, Vl);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      U[k] = Ul[k];
+      V[k] = Vl[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      s[k] = sl[k];
+      sm1[k] = ml[k];
+      is[k] = 0.f;
+    }
+    return true;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float q = 1.f + ev[k];
+    is[k] = rsqrtf(q);
+    s[k] = q * is[k];
+    sm1[k] = fast_div(ev[k], 1.f + s[k]);  // (s^2 - 1) / (s + 1)
+  }
+  if constexpr (WithV) {
+    mTm(D, U, V);
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) V[r * 3 + k] = (V[r * 3 + k] + U[r * 3 + k]) * is[k];
+  }
+  return false;
+}
+
 // Two parts of svd3_left64 that few particles reach, out of line so that the
 // kernels do not carry their registers: Jacobi sweeps in FP64 on a matrix whose
 // eigenvalues nearly coincide (S = s00, s11, s22, s01, s02, s12 and U, both
