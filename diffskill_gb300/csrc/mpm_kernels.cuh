@@ -116,6 +116,13 @@ MPM_DI T dweight(const Stencil<T>& s, int k, int d) {
   return k == 0 ? -(T(1.5) - f) : (k == 1 ? T(-2) * (f - T(1)) : (f - T(0.5)));
 }
 template <typename T>
+MPM_DI void stencil_derivatives(const Stencil<T>& s, T (&dw)[3][3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) dw[k][d] = dweight(s, k, d);
+}
+template <typename T>
 MPM_DI int64_t node_of(const Consts<T>& c, const Stencil<T>& s, int ox, int oy, int oz) {
   return ((int64_t)(s.base[0] + ox) * c.n_grid + (s.base[1] + oy)) * c.n_grid + (s.base[2] + oz);
 }
@@ -1052,6 +1059,19 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<
   }
 }
 
+// sums over a stencil's line along z: l0 = sum_o w n(o), l1 = sum_o o w n(o)
+template <typename T>
+MPM_DI void line_sums(const Stencil<T>& s, const Node<T>& n0, const Node<T>& n1, const Node<T>& n2, T* l0, T* l1) {
+  const T w0 = s.w[0][2], w1 = s.w[1][2], w2 = s.w[2][2];
+  const T a0[3] = {n0.x, n0.y, n0.z}, a1[3] = {n1.x, n1.y, n1.z}, a2[3] = {n2.x, n2.y, n2.z};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const T t1 = w1 * a1[i], t2 = w2 * a2[i];
+    l0[i] = w0 * a0[i] + t1 + t2;
+    l1[i] = T(2) * t2 + t1;
+  }
+}
+
 // g2p of particle p (mpm_simulator.py:265-284): writes rows 0..14 of st_out
 // and xn; returns false (the state copied unchanged) for a particle whose
 // stencil left the grid
@@ -1069,32 +1089,38 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
   const Node<T>* g = grid + (int64_t)scene * c.G;
   const StencilAddr A = stencil_addr(c, s);
   pdl_wait();  // the grid is grid_op's output
-  // C = k4 sum_o wgt v(o) (o - fx)^T = k4 (m1 - nv fx^T) with m1 = sum_o wgt v(o) o^T:
-  // the offsets o are 0, 1, 2, so m1 takes only additions
+  // C = k4 sum_o wgt v(o) (o - fx)^T = k4 (m1 - nv fx^T) with m1 = sum_o wgt v(o) o^T,
+  // summed axis by axis (line_sums): per component 24 operations on each of the 9
+  // lines along z and 12 on each plane, where a sum over nodes took 12 per node
   T nv[3] = {T(0), T(0), T(0)}, m1[9], nC[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) m1[k] = T(0);
   const T k4 = T(4) * c.inv_dx;
 #pragma unroll
-  for (int ox = 0; ox < 3; ++ox)
+  for (int k = 0; k < 9; ++k) m1[k] = T(0);
 #pragma unroll
-    for (int oy = 0; oy < 3; ++oy)
+  for (int ox = 0; ox < 3; ++ox) {
+    T p0[3] = {T(0), T(0), T(0)}, py[3] = {T(0), T(0), T(0)}, pz[3] = {T(0), T(0), T(0)};
 #pragma unroll
-      for (int oz = 0; oz < 3; ++oz) {
-        T wgt = s.w[ox][0] * s.w[oy][1] * s.w[oz][2];
-        Node<T> gv = g[A.at(ox, oy, oz)];
-        const T q[3] = {wgt * gv.x, wgt * gv.y, wgt * gv.z};
-        const int o[3] = {ox, oy, oz};
+    for (int oy = 0; oy < 3; ++oy) {
+      const Node<T> n0 = g[A.at(ox, oy, 0)], n1 = g[A.at(ox, oy, 1)], n2 = g[A.at(ox, oy, 2)];
+      T l0[3], l1[3];
+      line_sums(s, n0, n1, n2, l0, l1);
+      const T wy = s.w[oy][1];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          nv[i] += q[i];
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            if (o[j] == 1) m1[i * 3 + j] += q[i];
-            if (o[j] == 2) m1[i * 3 + j] += T(2) * q[i];
-          }
-        }
+      for (int i = 0; i < 3; ++i) {
+        p0[i] += wy * l0[i];
+        pz[i] += wy * l1[i];
+        if (oy > 0) py[i] += T(oy) * wy * l0[i];
       }
+    }
+    const T wx = s.w[ox][0];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      nv[i] += wx * p0[i];
+      if (ox > 0) m1[i * 3] += T(ox) * wx * p0[i];
+      m1[i * 3 + 1] += wx * py[i];
+      m1[i * 3 + 2] += wx * pz[i];
+    }
+  }
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -1222,11 +1248,6 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
   auto* sb = &stage[threadIdx.x >> 5];
   const WarpRows rows = warp_rows(key, ok);
   const T k4 = T(4) * c.inv_dx;
-  T gw[3][3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) gw[a][b] = T(0);
   // the x-derivative through dp = o - fx of sum_o wgt gv(o) . (k4 gC dp) is
   // -k4 gC^T sum_o wgt gv(o) = -k4 gC^T new_v
   T gfx[3];
@@ -1241,34 +1262,48 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
     for (int j = 0; j < 3; ++j) gC[3 * i + j] *= k4;
     ux[i] = gnv[i] - (gC[3 * i] * s.fx[0] + gC[3 * i + 1] * s.fx[1] + gC[3 * i + 2] * s.fx[2]);
   }
-  // weight adjoints g_wgt(o) = gv(o) . u(o): the 27 gathers of the grid
-  // velocity in one unrolled loop (their loads issue together), before the
-  // scatter, which then touches no global memory but its atomics
+  // weight adjoints h(o) = gv(o) . u(o), summed axis by axis against the weights
+  // and their derivatives; the 27 gathers of the grid velocity come in one
+  // unrolled loop before the scatter, which then touches no global memory but
+  // its atomics
   if (ok) {
+    T dw[3][3];
+    stencil_derivatives(s, dw);
+    T sx = T(0), sy = T(0), sz = T(0);
     T vx[3] = {ux[0], ux[1], ux[2]};
 #pragma unroll
     for (int ox = 0; ox < 3; ++ox) {
+      T p0 = T(0), p1 = T(0), pz = T(0);
       T vy[3] = {vx[0], vx[1], vx[2]};
 #pragma unroll
       for (int oy = 0; oy < 3; ++oy) {
         T vz[3] = {vy[0], vy[1], vy[2]};
+        T l0 = T(0), lz = T(0);
 #pragma unroll
         for (int oz = 0; oz < 3; ++oz) {
           const Node<T> n = g[A.at(ox, oy, oz)];
           const T gv[3] = {n.x, n.y, n.z};
-          const T g_wgt = dot3(gv, vz);
-          gw[ox][0] += g_wgt * s.w[oy][1] * s.w[oz][2];
-          gw[oy][1] += g_wgt * s.w[ox][0] * s.w[oz][2];
-          gw[oz][2] += g_wgt * s.w[ox][0] * s.w[oy][1];
+          const T h = dot3(gv, vz);
+          l0 += s.w[oz][2] * h;
+          lz += dw[oz][2] * h;
 #pragma unroll
           for (int i = 0; i < 3; ++i) vz[i] += gC[3 * i + 2];
         }
+        p0 += s.w[oy][1] * l0;
+        p1 += dw[oy][1] * l0;
+        pz += s.w[oy][1] * lz;
 #pragma unroll
         for (int i = 0; i < 3; ++i) vy[i] += gC[3 * i + 1];
       }
+      sx += dw[ox][0] * p0;
+      sy += s.w[ox][0] * p1;
+      sz += s.w[ox][0] * pz;
 #pragma unroll
       for (int i = 0; i < 3; ++i) vx[i] += gC[3 * i];
     }
+    gfx[0] += sx;
+    gfx[1] += sy;
+    gfx[2] += sz;
   }
   if constexpr (sizeof(T) == 4) {
     row_put(*sb, rows.row, ux, gC, s, A, gg);
@@ -1306,11 +1341,7 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
   }
   if (ok) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) gfx[d] += gw[k][d] * dweight(s, k, d);
-      gx[d] += c.inv_dx * gfx[d];
-    }
+    for (int d = 0; d < 3; ++d) gx[d] += c.inv_dx * gfx[d];
     store_row(g0, c.ld, p, 0, 3, gx);
   }
 }
@@ -1465,19 +1496,17 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
   if (ok) {
     const Node<T>* gg = g_in + (int64_t)scene * c.G;
     const StencilAddr A = stencil_addr(c, s);
-    T ga[9];
+    T ga[9], dw[3][3];
+    stencil_derivatives(s, dw);
 #pragma unroll
     for (int k = 0; k < 9; ++k) ga[k] = T(0);
-    T gw[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int b = 0; b < 3; ++b) gw[a][b] = T(0);
     // q(o) = wgt(o) gn(o) and sq = sum_o q(o): the adjoints of m v (gv = m sq) and of
     // dp = (o - fx) dx through A dp (gfx = -dx A^T sq) need only the sum; the adjoint
-    // of A (ga = sum_o q dp^T) takes sum_o q o^T, additions only as o is 0, 1, 2; the
-    // node value m v + A dp is stepped across the stencil by the columns of dx A
-    T sq[3] = {T(0), T(0), T(0)};
+    // of A (ga = sum_o q dp^T) takes sum_o q o^T, and the weights' adjoints
+    // h(o) = gn(o) . (m v + A dp) + gm(o) m their sums against the weights and their
+    // derivatives.  All are summed axis by axis; the node value m v + A dp is
+    // stepped across the stencil by the columns of dx A
+    T sq[3] = {T(0), T(0), T(0)}, sx = T(0), sy = T(0), sz = T(0);
     T ad[9], cx[3];
 #pragma unroll
     for (int k = 0; k < 9; ++k) ad[k] = affine[k] * c.dx;
@@ -1485,36 +1514,48 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
     for (int k = 0; k < 3; ++k) cx[k] = c.p_mass * v[k] - (ad[3 * k] * s.fx[0] + ad[3 * k + 1] * s.fx[1] + ad[3 * k + 2] * s.fx[2]);
 #pragma unroll
     for (int ox = 0; ox < 3; ++ox) {
+      T p0[3] = {T(0), T(0), T(0)}, py[3] = {T(0), T(0), T(0)}, pz[3] = {T(0), T(0), T(0)};
+      T h0 = T(0), h1 = T(0), hz = T(0);
       T cy[3] = {cx[0], cx[1], cx[2]};
 #pragma unroll
       for (int oy = 0; oy < 3; ++oy) {
         T cz[3] = {cy[0], cy[1], cy[2]};
+        const Node<T> n[3] = {gg[A.at(ox, oy, 0)], gg[A.at(ox, oy, 1)], gg[A.at(ox, oy, 2)]};
+        T l0[3], l1[3], m0 = T(0), mz = T(0);
+        line_sums(s, n[0], n[1], n[2], l0, l1);
 #pragma unroll
         for (int oz = 0; oz < 3; ++oz) {
-          T wgt = s.w[ox][0] * s.w[oy][1] * s.w[oz][2];
-          const int o[3] = {ox, oy, oz};
-          Node<T> n = gg[A.at(ox, oy, oz)];
-          const T gn[3] = {n.x, n.y, n.z};
-          T g_wgt = dot3(gn, cz) + n.w * c.p_mass;
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const T q = wgt * gn[k];
-            sq[k] += q;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              if (o[j] == 1) ga[3 * k + j] += q;
-              if (o[j] == 2) ga[3 * k + j] += T(2) * q;
-            }
-          }
-          gw[ox][0] += g_wgt * s.w[oy][1] * s.w[oz][2];
-          gw[oy][1] += g_wgt * s.w[ox][0] * s.w[oz][2];
-          gw[oz][2] += g_wgt * s.w[ox][0] * s.w[oy][1];
+          const T gn[3] = {n[oz].x, n[oz].y, n[oz].z};
+          const T h = dot3(gn, cz) + n[oz].w * c.p_mass;
+          m0 += s.w[oz][2] * h;
+          mz += dw[oz][2] * h;
 #pragma unroll
           for (int k = 0; k < 3; ++k) cz[k] += ad[3 * k + 2];
         }
+        const T wy = s.w[oy][1];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          p0[k] += wy * l0[k];
+          pz[k] += wy * l1[k];
+          if (oy > 0) py[k] += T(oy) * wy * l0[k];
+        }
+        h0 += wy * m0;
+        h1 += dw[oy][1] * m0;
+        hz += wy * mz;
 #pragma unroll
         for (int k = 0; k < 3; ++k) cy[k] += ad[3 * k + 1];
       }
+      const T wx = s.w[ox][0];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        sq[k] += wx * p0[k];
+        if (ox > 0) ga[3 * k] += T(ox) * wx * p0[k];
+        ga[3 * k + 1] += wx * py[k];
+        ga[3 * k + 2] += wx * pz[k];
+      }
+      sx += dw[ox][0] * h0;
+      sy += wx * h1;
+      sz += wx * hz;
 #pragma unroll
       for (int k = 0; k < 3; ++k) cx[k] += ad[3 * k];
     }
@@ -1523,17 +1564,13 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
     for (int k = 0; k < 3; ++k)
 #pragma unroll
       for (int j = 0; j < 3; ++j) ga[3 * k + j] = c.dx * (ga[3 * k + j] - s.fx[j] * sq[k]);
-    T gfx[3];
+    T gfx[3] = {sx, sy, sz};
 #pragma unroll
-    for (int j = 0; j < 3; ++j) gfx[j] = -(ad[j] * sq[0] + ad[3 + j] * sq[1] + ad[6 + j] * sq[2]);
+    for (int j = 0; j < 3; ++j) gfx[j] -= ad[j] * sq[0] + ad[3 + j] * sq[1] + ad[6 + j] * sq[2];
 #pragma unroll
     for (int k = 0; k < 3; ++k) gv[k] = c.p_mass * sq[k];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) gfx[d] += gw[k][d] * dweight(s, k, d);
-      gx[d] += c.inv_dx * gfx[d];
-    }
+    for (int d = 0; d < 3; ++d) gx[d] += c.inv_dx * gfx[d];
 #pragma unroll
     for (int k = 0; k < 9; ++k) g_aff[k] = to_prec<S>(ga[k]);
   }
