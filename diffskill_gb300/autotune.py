@@ -33,8 +33,8 @@ import numpy as np
 # candidates per launch-shape field, the default first
 CANDIDATES: Dict[str, Sequence[int]] = {
     "p2g_ctas": (7, 6, 8),
-    "g2p_adj_ctas": (6, 5, 7, 8),
-    "p2g_adj_ctas": (5, 4, 6),
+    "g2p_adj_ctas": (8, 5, 6, 7),
+    "p2g_adj_ctas": (4, 5, 6),
     "grid_ctas_per_sm": (16, 8, 32),
     "g2p_ctas": (8, 10, 12),
     "grid_op_adj_ctas": (6, 12, 16),

@@ -64,8 +64,8 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
         MPM_G2P_ADJ((k_g2p_adj<T, 5>));
       else if (v == 7)
         MPM_G2P_ADJ((k_g2p_adj<T, 7>));
-      else if (v == 8)
-        MPM_G2P_ADJ((k_g2p_adj<T, 8>));
+      else if (v == 6)
+        MPM_G2P_ADJ((k_g2p_adj<T, 6>));
       else
         MPM_G2P_ADJ(k_g2p_adj<T>);
     } else {
@@ -96,8 +96,8 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
   if ((phases & BWD_PARTICLES) && c.n_particles > 0) {
     const int v = L.tune.p2g_adj_ctas;
     if constexpr (sizeof(T) == 4 && sizeof(S) == 4) {
-      if (v == 4)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 4>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
+      if (v == 5)
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 5>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
       else if (v == 6)
         MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 6>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
       else

@@ -558,8 +558,8 @@ int mpm_get_tuning(MpmHandle* h, MpmTuning* t) {
   if (!h || !t) return fail(h, MPM_E_INVALID, "mpm_get_tuning: NULL argument");
   *t = h->tune;
   if (!t->p2g_ctas) t->p2g_ctas = 7;
-  if (!t->g2p_adj_ctas) t->g2p_adj_ctas = 6;
-  if (!t->p2g_adj_ctas) t->p2g_adj_ctas = 5;
+  if (!t->g2p_adj_ctas) t->g2p_adj_ctas = 8;
+  if (!t->p2g_adj_ctas) t->p2g_adj_ctas = 4;
   if (!t->grid_ctas_per_sm) t->grid_ctas_per_sm = 16;
   if (!t->g2p_ctas) t->g2p_ctas = 8;
   if (!t->grid_op_adj_ctas) t->grid_op_adj_ctas = 6;

@@ -1171,11 +1171,11 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
 // g2p.grad: writes the x rows of g0 (partial) and scatters into g_grid
 // st1 (frame f+1, may be null): its v rows are the g2p output, so the clamp
 // mask needs no second gather of the grid.
-// FP32: 6 CTAs of 128 threads per SM by default (at most 80 registers, a
-// small spill; measured 20 % faster than the unconstrained 108 registers);
+// FP32: 8 CTAs of 128 threads per SM by default (64 registers, 48 B of spill): it
+// waits on its gathers (1.1M particles: 5, 6, 7, 8 CTAs 95.6, 90.8, 89.3, 86.3 us);
 // MB > 0: MB CTAs per SM (MpmTuning.g2p_adj_ctas)
 template <typename T, int MB = 0>
-__global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 8)) k_g2p_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ st1,
+__global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ st1,
                                                  const T* __restrict__ g1, T* __restrict__ g0,
                                                  const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
                                                  Node<T>* __restrict__ g_grid) {
@@ -1452,11 +1452,11 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
 
 // p2g.grad + svd_grad + compute_F_tmp.grad: gathers g_in; reads the partial
 // x gradient left in g0 by k_g2p_adj and writes all 24 rows of g0.
-// FP32: at most 102 registers by default (5 CTAs of 128 threads per SM; a
-// small spill), measured 3 % faster than 4 CTAs at 128 registers; MB > 0: MB
-// CTAs per SM (MpmTuning.p2g_adj_ctas)
+// FP32: 4 CTAs of 128 threads per SM by default (128 registers, 48 B of spill;
+// 1.1M particles: 4, 5, 6 CTAs 112.7, 118.8, 130.0 us, the latter spilling 160
+// and 430 B); MB > 0: MB CTAs per SM (MpmTuning.p2g_adj_ctas)
 template <typename T, typename S, int MB = 0>
-__global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 5 : 8)) k_p2g_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ g1,
+__global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 4 : 8)) k_p2g_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ g1,
                                                  T* __restrict__ g0, const int* __restrict__ pscene,
                                                  const Node<T>* __restrict__ g_in) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
