@@ -41,7 +41,7 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
       // wave of CTAs that stride over the particles
       const unsigned cap = (unsigned)(L.sm_count * (bs_s == 32 ? 16 : 6));
       MPM_LAUNCH_PDL(L, MPM_K_P2G_RECOMP, (k_p2g<T, S, true>), store && pb_s > cap ? cap : pb_s, bs_s, c, st0,
-                     (T*)nullptr, L.pscene, gin, saved);
+                     (T*)nullptr, L.pscene, L.order, gin, saved);
     }
     MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, gb, 64, c, L.active, counter, gin, gout, tools_t, poses_t,
                    L.tool_off, MpmGridStore{}, -1, saved);
@@ -55,9 +55,9 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
 #define MPM_G2P_ADJ(K)                                                                                 \
   do {                                                                                                 \
     if (plain)                                                                                         \
-      MPM_LAUNCH(L, MPM_K_G2P_ADJ, K, pb_t, bs_t, c, st0, st1, g1, g0, L.pscene, gout, g_gout);        \
+      MPM_LAUNCH(L, MPM_K_G2P_ADJ, K, pb_t, bs_t, c, st0, st1, g1, g0, L.pscene, L.order, L.add, gout, g_gout); \
     else                                                                                               \
-      MPM_LAUNCH_PDL(L, MPM_K_G2P_ADJ, K, pb_t, bs_t, c, st0, st1, g1, g0, L.pscene, gout, g_gout);    \
+      MPM_LAUNCH_PDL(L, MPM_K_G2P_ADJ, K, pb_t, bs_t, c, st0, st1, g1, g0, L.pscene, L.order, L.add, gout, g_gout); \
   } while (0)
     if constexpr (sizeof(T) == 4) {
       if (v == 5)
@@ -97,14 +97,14 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
     const int v = L.tune.p2g_adj_ctas;
     if constexpr (sizeof(T) == 4 && sizeof(S) == 4) {
       if (v == 5)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 5>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 5>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
       else if (v == 6)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 6>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 6>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, g_gin);
+      MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
     }
   }
   return cudaGetLastError();

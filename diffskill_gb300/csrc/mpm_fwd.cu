@@ -135,14 +135,14 @@ cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const d
     const int v = L.tune.p2g_ctas;
     if constexpr (sizeof(T) == 4 && sizeof(S) == 4) {
       if (v == 6)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 6>), pb, bs, c, st0, st1, L.pscene, gin, none);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 6>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
       else if (v == 8)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 8>), pb, bs, c, st0, st1, L.pscene, gin, none);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 8>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, gin, none);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, gin, none);
+      MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
     }
   }
   MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, grid_blocks_launch(L, (int64_t)c.n_scenes * c.NB3), 64, c, L.active,
@@ -156,14 +156,14 @@ cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const d
     const int v = L.tune.g2p_ctas;
     if constexpr (sizeof(T) == 4) {
       if (v == 10)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 10>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 10>), pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
       else if (v == 12)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 12>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 12>), pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+      MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
     }
   }
   return cudaGetLastError();

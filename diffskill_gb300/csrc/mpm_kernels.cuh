@@ -772,11 +772,19 @@ MPM_DI void mark_stencil_blocks(const Consts<T>& c, bool ok, const int* base, in
 // ---------------------------------------------------------------------------
 // forward kernels
 // ---------------------------------------------------------------------------
+// The particle of thread i.  order (may be null): a permutation that sorts the
+// particles by cell, for frames that are kept in the caller's order.  Its loads
+// before a pdl_wait() go to L2 (load_row_cg).
+MPM_DI int64_t particle_of(const int* __restrict__ order, int64_t i, bool valid) {
+  return order && valid ? (int64_t)__ldcg(order + i) : i;
+}
 // one chunk of p2g, a particle per thread (all threads of the block take part)
 template <typename T, typename S>
 MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restrict__ st_out,
-                      const int* __restrict__ pscene, Node<T>* __restrict__ grid, int64_t p) {
-  const bool valid = p < c.n_particles;  // every lane stays for the warp scan
+                      const int* __restrict__ pscene, const int* __restrict__ order, Node<T>* __restrict__ grid,
+                      int64_t i) {
+  const bool valid = i < c.n_particles;  // every lane stays for the warp's scatter
+  const int64_t p = particle_of(order, i, valid);
   Stencil<T> s;
   zero_stencil(s);
   bool ok = false;
@@ -875,17 +883,17 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
 // which exits at once when the grid store holds the substep)
 template <typename T, typename S, bool Strided = false, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 7 : 16)) k_p2g(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
-                                             const int* __restrict__ pscene, Node<T>* __restrict__ grid,
-                                             const int64_t* __restrict__ saved) {
+                                             const int* __restrict__ pscene, const int* __restrict__ order,
+                                             Node<T>* __restrict__ grid, const int64_t* __restrict__ saved) {
   if (saved && __ldcg(saved) >= 0) {  // the grid of this substep was restored from the grid store
     pdl_wait();  // completes only after the kernel before it (dependent launches chain through it)
     return;
   }
   if constexpr (Strided) {
     for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x; p0 < c.n_particles; p0 += (int64_t)gridDim.x * blockDim.x)
-      p2g_chunk<T, S>(c, st, st_out, pscene, grid, p0 + threadIdx.x);
+      p2g_chunk<T, S>(c, st, st_out, pscene, order, grid, p0 + threadIdx.x);
   } else {
-    p2g_chunk<T, S>(c, st, st_out, pscene, grid, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    p2g_chunk<T, S>(c, st, st_out, pscene, order, grid, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
   }
 }
 
@@ -1144,10 +1152,12 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
 // at most 64 registers)
 template <typename T, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k_g2p(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
-                                             const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
-                                             unsigned char* __restrict__ mark, int* __restrict__ header) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = p < c.n_particles;
+                                             const int* __restrict__ pscene, const int* __restrict__ order,
+                                             const Node<T>* __restrict__ grid, unsigned char* __restrict__ mark,
+                                             int* __restrict__ header) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < c.n_particles;
+  const int64_t p = particle_of(order, i, valid);
   const int scene = valid ? __ldcg(pscene + p) : 0;  // issued with x
   T xn[3] = {T(0), T(0), T(0)};
   const bool moved = valid && g2p_particle(c, st, st_out, p, scene, grid, xn);
@@ -1168,7 +1178,8 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
 // ---------------------------------------------------------------------------
 // adjoint kernels
 // ---------------------------------------------------------------------------
-// g2p.grad: writes the x rows of g0 (partial) and scatters into g_grid
+// g2p.grad: writes the x rows of g0 (partial; add: adds to them) and scatters into
+// g_grid
 // st1 (frame f+1, may be null): its v rows are the g2p output, so the clamp
 // mask needs no second gather of the grid.
 // FP32: 8 CTAs of 128 threads per SM by default (64 registers, 48 B of spill): it
@@ -1177,10 +1188,12 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
 template <typename T, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ st1,
                                                  const T* __restrict__ g1, T* __restrict__ g0,
-                                                 const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
+                                                 const int* __restrict__ pscene, const int* __restrict__ order,
+                                                 bool add, const Node<T>* __restrict__ grid,
                                                  Node<T>* __restrict__ g_grid) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = p < c.n_particles;  // every lane stays for the warp scan
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < c.n_particles;  // every lane stays for the warp's scatter
+  const int64_t p = particle_of(order, i, valid);
   Stencil<T> s;
   zero_stencil(s);
   bool ok = false;
@@ -1203,7 +1216,7 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_ad
       zero_stencil(s);
       scene = 0;
       const T z[3] = {T(0), T(0), T(0)};
-      store_row(g0, c.ld, p, 0, 3, z);
+      if (!add) store_row(g0, c.ld, p, 0, 3, z);
     }
   }
   if (!ok) {  // no contribution (and no 0 * inf) from particles outside the grid
@@ -1341,7 +1354,10 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_ad
   }
   if (ok) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) gx[d] += c.inv_dx * gfx[d];
+    for (int d = 0; d < 3; ++d) {
+      gx[d] += c.inv_dx * gfx[d];
+      if (add) gx[d] += g0[(int64_t)d * c.ld + p];
+    }
     store_row(g0, c.ld, p, 0, 3, gx);
   }
 }
@@ -1451,16 +1467,19 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
 }
 
 // p2g.grad + svd_grad + compute_F_tmp.grad: gathers g_in; reads the partial
-// x gradient left in g0 by k_g2p_adj and writes all 24 rows of g0.
+// x gradient left in g0 by k_g2p_adj and writes all 24 rows of g0 (add: adds to
+// rows 3..23; k_g2p_adj already added rows 0..2 to theirs).
 // FP32: 4 CTAs of 128 threads per SM by default (128 registers, 48 B of spill;
 // 1.1M particles: 4, 5, 6 CTAs 112.7, 118.8, 130.0 us, the latter spilling 160
 // and 430 B); MB > 0: MB CTAs per SM (MpmTuning.p2g_adj_ctas)
 template <typename T, typename S, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 4 : 8)) k_p2g_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ g1,
                                                  T* __restrict__ g0, const int* __restrict__ pscene,
+                                                 const int* __restrict__ order, bool add,
                                                  const Node<T>* __restrict__ g_in) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= c.n_particles) return;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c.n_particles) return;
+  const int64_t p = particle_of(order, i, true);
   // the adjoint rows read after the forward recompute and the gather are
   // fetched into L2 now, so those later loads do not wait on DRAM
 #pragma unroll
@@ -1579,11 +1598,17 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
   for (int k = 0; k < 9; ++k) gF1[k] = to_prec<S>(g1[(int64_t)(15 + k) * c.ld + p]);
   p2g_particle_vjp(m, C, F, P, g_aff, gF1, gC, gF);
   store_row(g0, c.ld, p, 0, 3, gx);
-  store_row(g0, c.ld, p, 3, 3, gv);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    T* o = g0 + (int64_t)(3 + k) * c.ld + p;
+    *o = add ? *o + gv[k] : gv[k];
+  }
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    g0[(int64_t)(6 + k) * c.ld + p] = to_prec<T>(gC[k]);
-    g0[(int64_t)(15 + k) * c.ld + p] = to_prec<T>(gF[k]);
+    T *oC = g0 + (int64_t)(6 + k) * c.ld + p, *oF = g0 + (int64_t)(15 + k) * c.ld + p;
+    const T vC = to_prec<T>(gC[k]), vF = to_prec<T>(gF[k]);
+    *oC = add ? *oC + vC : vC;
+    *oF = add ? *oF + vF : vF;
   }
 }
 

@@ -50,6 +50,8 @@ struct LaunchCtx {
   int64_t* launches;           // launch counter
   Profiler* prof;              // may be null
   MpmTuning tune = {0, 0, 0, 0, 0, 0};  // launch shapes (mpm_set_tuning); 0 = default
+  const int* order = nullptr;  // [n_particles] particle of each thread of the particle kernels; null: thread i, particle i
+  bool add = false;            // the adjoint adds to the gradient frame it writes
 };
 
 // launch helper: counts and (optionally) times one kernel launch
@@ -111,6 +113,9 @@ size_t sort_hist_words(int64_t n_particles);
 int sort_key_bits(int n_scenes, int n_grid);
 template <typename T>
 cudaError_t launch_sort_frame(const LaunchCtx& L, const T* src, T* dst, int32_t* perm, const SortScratch& s);
+// the permutation of launch_sort_frame alone
+template <typename T>
+cudaError_t launch_sort_order(const LaunchCtx& L, const T* src, int32_t* perm, const SortScratch& s);
 template <typename T>
 cudaError_t launch_unsort_frame(const LaunchCtx& L, const T* src, T* dst, const int32_t* perm);
 

@@ -222,7 +222,7 @@ int sort_key_bits(int n_scenes, int n_grid) {
 }
 
 template <typename T>
-cudaError_t launch_sort_frame(const LaunchCtx& L, const T* src, T* dst, int32_t* perm, const SortScratch& s) {
+cudaError_t launch_sort_order(const LaunchCtx& L, const T* src, int32_t* perm, const SortScratch& s) {
   const MpmParams& p = *L.p;
   const int64_t n = p.n_particles;
   if (n == 0) return cudaSuccess;
@@ -241,6 +241,16 @@ cudaError_t launch_sort_frame(const LaunchCtx& L, const T* src, T* dst, int32_t*
     MPM_LAUNCH(L, MPM_K_SORT, k_radix_scatter, (unsigned)tiles, kSortThreads, k[a], v[a], k[b], v[b], n, 8 * i,
                (const uint32_t*)s.hist, tiles, (const uint32_t*)totals);
   }
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_sort_frame(const LaunchCtx& L, const T* src, T* dst, int32_t* perm, const SortScratch& s) {
+  const MpmParams& p = *L.p;
+  const int64_t n = p.n_particles;
+  if (n == 0) return cudaSuccess;
+  const cudaError_t e = launch_sort_order(L, src, perm, s);
+  if (e != cudaSuccess) return e;
   MPM_LAUNCH(L, MPM_K_SORT, k_sort_gather<T>, blocks_of(n, 256), 256, src, dst, p.ld, n, (const int32_t*)perm);
   return cudaGetLastError();
 }
@@ -254,6 +264,8 @@ cudaError_t launch_unsort_frame(const LaunchCtx& L, const T* src, T* dst, const 
   return cudaGetLastError();
 }
 
+template cudaError_t launch_sort_order<float>(const LaunchCtx&, const float*, int32_t*, const SortScratch&);
+template cudaError_t launch_sort_order<double>(const LaunchCtx&, const double*, int32_t*, const SortScratch&);
 template cudaError_t launch_sort_frame<float>(const LaunchCtx&, const float*, float*, int32_t*, const SortScratch&);
 template cudaError_t launch_sort_frame<double>(const LaunchCtx&, const double*, double*, int32_t*,
                                                const SortScratch&);

@@ -230,6 +230,22 @@ class MpmEngine:
                                                       ctypes.byref(store.struct), slot, _stream()), self.h,
                        "mpm_substep_bwd_store")
 
+    def substeps(self, frames: torch.Tensor, poses: torch.Tensor, n: int, store: "GridStore" = None,
+                 slot0: int = 0) -> None:
+        """``n`` consecutive substeps on contiguous frames (``frames`` [n + 1, 24, ld],
+        ``poses`` [n + 1, T, 8]), the grids kept in slots slot0 .. slot0 + n - 1."""
+        _lib.check(self.lib.mpm_substeps_fwd(self.h, _ptr(frames), _ptr(poses), n,
+                                             None if store is None else ctypes.byref(store.struct), slot0, _stream()),
+                   self.h, "mpm_substeps_fwd")
+
+    def substeps_bwd(self, frames, g_frames, poses, g_poses, n: int, store: "GridStore" = None,
+                     slot0: int = 0) -> None:
+        """Adjoint of ``substeps``, last to first: each substep adds to the gradient
+        frame below it and to ``g_poses``."""
+        _lib.check(self.lib.mpm_substeps_bwd(self.h, _ptr(frames), _ptr(g_frames), _ptr(poses), _ptr(g_poses), n,
+                                             None if store is None else ctypes.byref(store.struct), slot0, _stream()),
+                   self.h, "mpm_substeps_bwd")
+
     def sort_frame(self, src: torch.Tensor, dst: torch.Tensor, perm: torch.Tensor) -> None:
         """dst = src with its particles sorted by (scene, 4^3 block, cell), stably;
         ``perm`` (int32 [P]) receives the order: dst[:, i] = src[:, perm[i]]."""
@@ -395,6 +411,13 @@ class GridStore:
         """Forget every slot (device-side; capturable)."""
         self.bump.zero_()
         self.slot_start.fill_(-1)
+
+    def forget(self, first: int, last: int) -> None:
+        """Empty slots ``first`` .. ``last`` (clipped to the store): their substeps' frames
+        or poses changed, so their adjoints recompute the grids."""
+        first, last = max(first, 0), min(last, self.slot_start.numel() - 1)
+        if first <= last:
+            self.slot_start[first:last + 1].fill_(-1)
 
     def bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (self.blocks, self.block_ids, self.slot_start,

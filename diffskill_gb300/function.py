@@ -91,9 +91,8 @@ class GradModel:
         n = self.sim.n_particles[None]
         fr = self.sim._frames[f]
         x = fr[0:6, :n].t().float()
-        c = torch.zeros((len(self.primitives), 8), dtype=torch.float32, device=fr.device)
-        for i, p in enumerate(self.primitives):
-            c[i, :p.state_dim] = self.sim._pose[f, i, :p.state_dim].float()
+        T = len(self.primitives)
+        c = torch.where(self.sim._state_mask, self.sim._pose[f], 0.0)[:T].float()
         if self.return_dist:
             d = self._dists(f)[:, :n].t().float()
             x = torch.cat((x, d), 1)
@@ -120,25 +119,24 @@ class GradModel:
             obs_grad = obs_grad[..., :-k]
         obs_grad = obs_grad.reshape(-1, self.dim * 2)
         sim._gframes[f, 0:6, :n].add_(obs_grad.t().to(sim._gframes.dtype))
-        mg = manipulator_grad.reshape(len(self.primitives), 8)
-        for i, p in enumerate(self.primitives):
-            sim._g_pose[f, i, :p.state_dim] += mg[i, :p.state_dim].to(torch.float64)
+        T = len(self.primitives)
+        mg = manipulator_grad.reshape(T, 8).to(sim._g_pose.device, torch.float64)
+        sim._g_pose[f, :T] += torch.where(sim._state_mask[:T], mg, 0.0)
 
     # ------------------------------------------------------------ steps
     def forward_step(self, s: int, a) -> None:
         """function.py:166-175."""
         a = a.reshape(-1).clamp(-1, 1)
         self.primitives.set_action(s, self.substeps, a)
-        for i in range(s * self.substeps, (s + 1) * self.substeps):
-            self.sim.substep(i)
+        self.sim._substeps(s * self.substeps, self.substeps)
 
     def backward_step(self, s: int) -> torch.Tensor:
         """function.py:177-190: adjoint of action s; returns d/d(action s) (flat)."""
-        for i in range((s + 1) * self.substeps - 1, s * self.substeps - 1, -1):
-            self.sim.substep_grad(i)
+        self.sim._substeps_grad(s * self.substeps, self.substeps)
         self.sim._tools_action_bwd(s)
-        grads = [torch.as_tensor(p.get_action_grad(s, 1)[0]) for p in self.primitives if p.action_dim > 0]
-        return torch.cat(grads).to(self.device) if grads else torch.zeros(0, device=self.device)
+        if not any(p.action_dim > 0 for p in self.primitives):
+            return torch.zeros(0, device=self.device)
+        return self.sim._g_act[s].reshape(-1)[self.sim._act_index].to(self.device)
 
     @property
     def forward(self):

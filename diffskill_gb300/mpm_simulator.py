@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from .config import PREC_FP64, SimulatorConfig
-from .engine import MpmEngine
+from .engine import GridStore, MpmEngine
 from .primitives import Primitives
 
 
@@ -85,7 +85,6 @@ class MPMSimulator:
         M = self.max_steps
         self._frames = torch.zeros((M, 24, eng.ld), dtype=eng.dtype, device=eng.device)
         self._gframes = torch.zeros_like(self._frames)
-        self._tmp = eng.new_state()
         self._pose = torch.zeros((M + 1, T, 8), dtype=torch.float64, device=eng.device)
         self._pose[0, :eng.T] = eng.pose0
         self._vel = torch.zeros((M, T, 8), dtype=torch.float64, device=eng.device)
@@ -96,6 +95,21 @@ class MPMSimulator:
         self._coll = eng.new_coll(n_act)  # tool-tool collision records per action
         self.grid_m_t = torch.zeros((1, eng.G), dtype=eng.dtype, device=eng.device)
         self.grid_m_grad_t = torch.zeros_like(self.grid_m_t)
+        # which entries of a tool's pose are its state, and where the flat action's
+        # entries sit in an action's [T, 8] row
+        state = torch.zeros((T, 8), dtype=torch.bool)
+        for i, p in enumerate(self.primitives):
+            state[i, :p.state_dim] = True
+        self._state_mask = state.to(eng.device)
+        dims = self.primitives.action_dims
+        self._act_index = torch.tensor([8 * i + k for i in range(eng.T) for k in range(dims[i + 1] - dims[i])],
+                                       dtype=torch.long, device=eng.device)
+        # the grids of each substep, for its adjoint: slot s belongs to substep(s) as it
+        # last ran, and is emptied whenever frame s or the poses of frames s, s + 1 change
+        free, _ = torch.cuda.mem_get_info(eng.device)
+        block = 2 * 64 * 4 * (8 if eng.dtype == torch.float64 else 4) + 4
+        worst = M * min((eng.n_grid // 4) ** 3, 8 * max(eng.P, 1))
+        self._store = GridStore(eng, M, min(worst, min(1 << 30, free // 16) // block))
         self.cur = 0
 
     def _t64(self, a) -> torch.Tensor:
@@ -110,20 +124,20 @@ class MPMSimulator:
             eng.softness = softness
             from . import _lib
             _lib.check(eng.lib.mpm_set_tools(eng.h, eng._descs, eng.T), eng.h, "mpm_set_tools")
+            self._store.reset()
 
     # ------------------------------------------------------------- tools
     def _set_action(self, s: int, action: np.ndarray, only: Optional[int] = None) -> None:
         eng, n = self._eng, self.substeps
         if (s + 1) * n > self.max_steps - 1:
             raise IndexError(f"action {s} runs past max_steps={self.max_steps}")
-        row = self._act[s].clone()
-        dims = self.primitives.action_dims
-        for i in range(eng.T):
-            if only is not None and i != only:
-                continue
-            d = dims[i + 1] - dims[i]
-            row[i, :d] = self._t64(action[dims[i]:dims[i + 1]])
-        self._act[s].copy_(row)
+        index, dims = self._act_index, self.primitives.action_dims
+        action = torch.as_tensor(action, dtype=torch.float64, device=self.device)
+        if only is not None:
+            part = slice(dims[only], dims[only + 1])
+            index, action = index[part], action[part]
+        self._act[s].view(-1).index_copy_(0, index, action)
+        self._store.forget(s * n, (s + 1) * n)
         if eng.T:
             eng.tools_action(self._act[s], self._vel[s * n], self._pose[s * n],
                              None if self._coll is None else self._coll[s])
@@ -142,13 +156,24 @@ class MPMSimulator:
     # ------------------------------------------------------------ substeps
     def substep(self, s: int) -> None:
         """``substep`` (mpm_simulator.py:307-323)."""
-        self._eng.substep(self._frames[s], self._frames[s + 1], self._pose[s], self._pose[s + 1])
+        self._substeps(s, 1)
+
+    def _substeps(self, first: int, n: int) -> None:
+        """Substeps first .. first + n - 1 in order."""
+        if not 0 <= first <= first + n < self.max_steps:
+            raise IndexError(f"substeps {first} .. {first + n - 1} run past max_steps={self.max_steps}")
+        self._eng.substeps(self._frames[first], self._pose[first], n, self._store, first)
 
     def substep_grad(self, s: int) -> None:
         """``substep_grad`` (mpm_simulator.py:325-345): frame-(s+1) adjoint -> frame s (accumulated)."""
-        self._eng.substep_bwd(self._frames[s], self._gframes[s + 1], self._tmp, self._pose[s], self._pose[s + 1],
-                              self._g_pose[s], self._g_pose[s + 1], st1=self._frames[s + 1])
-        self._gframes[s].add_(self._tmp)
+        self._substeps_grad(s, 1)
+
+    def _substeps_grad(self, first: int, n: int) -> None:
+        """Adjoints of substeps first + n - 1 .. first, last to first."""
+        if not 0 <= first <= first + n < self.max_steps:
+            raise IndexError(f"substeps {first} .. {first + n - 1} run past max_steps={self.max_steps}")
+        self._eng.substeps_bwd(self._frames[first], self._gframes[first], self._pose[first], self._g_pose[first], n,
+                               self._store, first)
 
     def step(self, is_copy: bool, action=None) -> None:
         """``step`` (mpm_simulator.py:440-451)."""
@@ -156,8 +181,7 @@ class MPMSimulator:
         self.cur = start + self.substeps
         if action is not None:
             self.primitives.set_action(start // self.substeps, self.substeps, action)
-        for s in range(start, self.cur):
-            self.substep(s)
+        self._substeps(start, self.substeps)
         if is_copy:
             self.copyframe(self.cur, 0)
             self.cur = 0
@@ -165,6 +189,7 @@ class MPMSimulator:
     def copyframe(self, source: int, target: int) -> None:
         self._frames[target].copy_(self._frames[source])
         self._pose[target].copy_(self._pose[source])
+        self._store.reset()
 
     # ----------------------------------------------------------------- io
     def _rows(self, f: int, r0: int, r1: int) -> np.ndarray:
@@ -196,18 +221,26 @@ class MPMSimulator:
         n = len(state[0])
         if self._eng is None or n != self.n_particles[None]:
             self.initialize(n)
-        fr = torch.zeros((24, n), dtype=torch.float64)
-        fr[0:3] = torch.as_tensor(np.asarray(state[0], dtype=np.float64).T)
-        fr[3:6] = torch.as_tensor(np.asarray(state[1], dtype=np.float64).T)
-        fr[15:24] = torch.as_tensor(np.asarray(state[2], dtype=np.float64).reshape(n, 9).T)
-        fr[6:15] = torch.as_tensor(np.asarray(state[3], dtype=np.float64).reshape(n, 9).T)
-        self._frames[f, :, :n].copy_(fr.to(self.device, self._frames.dtype))
-        for s, p in zip(state[4:], self.primitives):
-            p.set_state(f, s)
+        # the rows are transposed and rounded to the frame's type on the device
+        for rows, a in ((slice(0, 3), state[0]), (slice(3, 6), state[1]), (slice(15, 24), state[2]),
+                        (slice(6, 15), state[3])):
+            self._frames[f, rows, :n].copy_(self._t64(a).reshape(n, -1).t())
+        self._set_poses(f, {i: s for i, s in enumerate(state[4:4 + self.n_primitive])})
 
     def set_primitive_state(self, f: int, state) -> None:
-        for s, p in zip(state[4:], self.primitives):
-            p.set_state(f, s)
+        self._set_poses(f, {i: s for i, s in enumerate(state[4:4 + self.n_primitive])})
+
+    def _set_poses(self, f: int, states: dict) -> None:
+        """Leading pose entries of the tools ``states`` at frame ``f``."""
+        new = np.full((max(self.n_primitive, 1), 8), np.nan)
+        given = np.zeros(new.shape, dtype=bool)
+        for i, s in states.items():
+            s = np.asarray(s, dtype=np.float64).reshape(-1)
+            new[i, :len(s)] = s
+            given[i, :len(s)] = True
+        both = self._t64(np.stack([new, given]))
+        self._pose[f].copy_(torch.where(both[1] != 0, both[0], self._pose[f]))
+        self._store.reset() if f == 0 else self._store.forget(f - 1, f)
 
     def reset(self, x) -> None:
         """``reset`` (402-413): x given, v = 0, F = I, C = 0 at frame 0."""
@@ -215,6 +248,7 @@ class MPMSimulator:
         if self._eng is None or x.shape[0] != self.n_particles[None]:
             self.initialize(x.shape[0])
         self._frames[0].copy_(self._eng.init_state([x]))
+        self._store.reset()
         self.cur = 0
 
     def get_m(self) -> np.ndarray:

@@ -53,10 +53,7 @@ class Primitive:
         return self.sim._pose[f, self.index, :self.state_dim].float()
 
     def set_state(self, f: int, state) -> None:
-        state = np.asarray(state, dtype=np.float64).reshape(-1)
-        cur = self.sim._pose[f, self.index].cpu().numpy()
-        cur[:len(state)] = state
-        self.sim._pose[f, self.index] = self.sim._t64(cur)
+        self.sim._set_poses(f, {self.index: state})
 
     # -- actions (primive_base.py:241-282) --------------------------------------
     def set_action(self, s: int, n_substeps: int, action) -> None:
@@ -127,14 +124,14 @@ class Primitives:
     def set_action(self, s: int, n_substeps: int, action, only: Optional[int] = None) -> None:
         """Clip to [-1, 1] and run set_velocity + kinematics for action ``s`` (primitives.py:863-867)."""
         if isinstance(action, np.ndarray) or not hasattr(action, "detach"):
-            action = np.asarray(action, dtype=np.float64).reshape(-1)
-        else:
-            action = action.detach().double().reshape(-1).cpu().numpy()
+            action = np.clip(np.asarray(action, dtype=np.float64).reshape(-1), -1, 1)
+        else:  # stays where it is: a device action costs no wait for the device
+            action = action.detach().double().reshape(-1).clamp(-1, 1)
         if len(action) != self.action_dim:
             raise ValueError(f"action has {len(action)} entries, expected {self.action_dim}")
         if n_substeps != self.sim.substeps:
             raise ValueError("n_substeps must equal the simulator's substeps")
-        self.sim._set_action(s, np.clip(action, -1, 1), only=only)
+        self.sim._set_action(s, action, only=only)
 
     def get_grad(self, n: int) -> np.ndarray:
         grads = [g for g in (p.get_action_grad(0, n) for p in self.primitives) if g is not None]

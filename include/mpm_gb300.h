@@ -300,6 +300,22 @@ int mpm_soft_contact_bwd(MpmHandle* h, const void* state, const double* pose, co
 int mpm_target_sdf(MpmHandle* h, const void* target_density, void* target_sdf, void* nearest, void* work,
                    int32_t n_iters, void* stream);
 
+/* n consecutive substeps of a handle whose frames are contiguous: frames is
+ * real[n + 1][24][ld], poses double[n + 1][max(n_tools, 1)][8].  mpm_substeps_fwd equals
+ * n calls of mpm_substep_fwd (mpm_substep_fwd_store into slots slot0 .. slot0 +
+ * n - 1 when store is not NULL) in order, and then marks slot slot0 + n, whose
+ * frame it rewrote, as empty.  mpm_substeps_bwd runs their adjoints from the last
+ * to the first; g_frames is real[n + 1][24][ld], and each substep ADDS to the
+ * gradient frame below it (mpm_substep_bwd overwrites); g_poses accumulates.  A
+ * slot must hold its own substep or be empty (slot_start = -1): then the substep's
+ * grids are recomputed.  Each call may sort the particles by cell once, in scratch
+ * of the handle: the frames stay in the caller's order, and the sums on the grid
+ * are taken in another order than by single substeps. */
+int mpm_substeps_fwd(MpmHandle* h, void* frames, const double* poses, int32_t n, const MpmGridStore* store,
+                     int32_t slot0, void* stream);
+int mpm_substeps_bwd(MpmHandle* h, const void* frames, void* g_frames, const double* poses, double* g_poses, int32_t n,
+                     const MpmGridStore* store, int32_t slot0, void* stream);
+
 /* compute_sdf_loss_kernel (loss.py:178-180) per scene, FP64 sum in a fixed
  * order: loss[s] = weight * sum_I target_sdf * grid_m (double[n_scenes],
  * overwritten).  If g_grid_m is not NULL, weight * target_sdf is ADDED to it,
