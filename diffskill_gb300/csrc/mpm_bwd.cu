@@ -97,14 +97,14 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
     const int v = L.tune.p2g_adj_ctas;
     if constexpr (sizeof(T) == 4 && sizeof(S) == 4) {
       if (v == 5)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 5>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 5>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.add, g_gin);
       else if (v == 6)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 6>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S, 6>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.add, g_gin);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
+        MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.add, g_gin);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.order, L.add, g_gin);
+      MPM_LAUNCH_PDL(L, MPM_K_P2G_ADJ, (k_p2g_adj<T, S>), pb_s, bs_s, c, st0, g1, g0, L.pscene, L.add, g_gin);
     }
   }
   return cudaGetLastError();

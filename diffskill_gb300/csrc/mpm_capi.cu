@@ -42,7 +42,8 @@ struct MpmHandle {
   void* d_tools_t = nullptr;  // tools in the compute precision (converted by mpm_set_tools)
   void* d_poses_t = nullptr;  // poses of the current substep in the compute precision
   mpm::SortScratch sort;      // particle re-sort (mpm_sort_frame)
-  int* d_order = nullptr;     // particles by cell for the substeps of one mpm_substeps_fwd / _bwd
+  int* d_order = nullptr;     // particles by cell for the substeps of mpm_substeps_fwd / _bwd
+  bool ordered = false;       // d_order holds a permutation
   // pipelined adjoint (mpm_set_pipelined_adjoint): the grid preparation of an
   // adjoint substep runs on pipe_side beside the previous substep's p2g.grad
   bool pipelined = false;
@@ -614,23 +615,29 @@ int check_sortable(MpmHandle* h, const char* fn) {
 }  // namespace
 
 // Particle order of a run of substeps on frames in the caller's order: by cell at
-// the run's first frame, so that a warp's particles share their nodes.  Unsorted, each of
-// its 32 particles adds to 27 nodes of its own (30,000 particles: p2g 23 us,
-// ORDERED sorted).  The rows are then gathered 4 or 8 bytes at a time, which only
-// pays while the frame stays in L2 (at most 32 MiB), and the sort some 30 us, which
-// takes a few substeps to earn.
-static int run_order(MpmHandle* h, const void* frame, int32_t n, void* stream, const int** order) {
-  *order = nullptr;
+// the run's first frame, so that the particles of a warp of p2g and g2p.grad share
+// nodes.  Unsorted, each of its 32 particles adds to 27 nodes of its own.  The rows
+// are then gathered 4 or 8 bytes at a time, which only pays while the frame stays in
+// L2 (at most 32 MiB), and the sort takes eleven launches, which some thousand
+// particles and a few substeps have to earn.  19 substeps forward / adjoint in the
+// caller's order and by cell, us: FP32 16,000 particles 480 / 665 and 497 / 686,
+// 30,000 624 / 821 and 541 / 787, 100,000 1,670 / 1,439 and 869 / 1,269; FP64 8,000
+// 1,717 / 3,435 and 1,702 / 3,430, 16,000 2,089 / 3,624 and 1,867 / 3,566.  An
+// adjoint run takes the order of the last forward run: any permutation is right,
+// and a particle seldom changes its cell within an action.
+static bool run_ordered(const MpmHandle* h, int32_t n) {
   const size_t bytes = (size_t)24 * (size_t)h->p.ld * real_size(h->p.precision);
-  if (n < 4 || h->p.n_particles < 64 || bytes > ((size_t)32 << 20) ||
-      mpm::sort_key_bits(h->p.n_scenes, h->p.n_grid) > 32)
-    return MPM_OK;
+  const int64_t least = h->p.precision == MPM_PREC_FP64 ? 12000 : 20000;
+  return n >= 4 && h->p.n_particles >= least && bytes <= ((size_t)32 << 20) &&
+         mpm::sort_key_bits(h->p.n_scenes, h->p.n_grid) <= 32;
+}
+static int sort_run(MpmHandle* h, const void* frame, void* stream) {
   mpm::LaunchCtx L = ctx(h, stream);
   const cudaError_t e = h->p.precision == MPM_PREC_FP64
                             ? mpm::launch_sort_order<double>(L, (const double*)frame, h->d_order, h->sort)
                             : mpm::launch_sort_order<float>(L, (const float*)frame, h->d_order, h->sort);
   if (e != cudaSuccess) return cuda_fail(h, e, "particle order");
-  *order = h->d_order;
+  h->ordered = true;
   return MPM_OK;
 }
 
@@ -646,8 +653,8 @@ int mpm_substeps_fwd(MpmHandle* h, void* frames, const double* poses, int32_t n,
     return fail(h, MPM_E_INVALID, "mpm_substeps_fwd: grid store slots out of range");
   const size_t frame = (size_t)24 * (size_t)h->p.ld * real_size(h->p.precision);
   const size_t pose = (size_t)8 * (size_t)(h->n_tools > 0 ? h->n_tools : 1);
-  const int* order = nullptr;
-  MPM_TRY(run_order(h, frames, n, stream, &order));
+  const int* order = run_ordered(h, n) ? h->d_order : nullptr;
+  if (order) MPM_TRY(sort_run(h, frames, stream));
   int rc = MPM_OK;
   for (int32_t i = 0; i < n && rc == MPM_OK; ++i) {
     // each frame goes unmodified from one substep to the next: chained
@@ -679,8 +686,8 @@ int mpm_substeps_bwd(MpmHandle* h, const void* frames, void* g_frames, const dou
     return fail(h, MPM_E_INVALID, "mpm_substeps_bwd: grid store slots out of range");
   const size_t frame = (size_t)24 * (size_t)h->p.ld * real_size(h->p.precision);
   const size_t pose = (size_t)8 * (size_t)(h->n_tools > 0 ? h->n_tools : 1);
-  const int* order = nullptr;
-  MPM_TRY(run_order(h, frames, n, stream, &order));
+  const int* order = run_ordered(h, n) ? h->d_order : nullptr;
+  if (order && !h->ordered) MPM_TRY(sort_run(h, frames, stream));
   // no forward substep in between: each one's grid preparation runs beside the
   // p2g.grad of the one before (mpm_set_pipelined_adjoint)
   const bool pipelined = h->pipelined;

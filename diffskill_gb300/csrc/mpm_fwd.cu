@@ -156,14 +156,14 @@ cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const d
     const int v = L.tune.g2p_ctas;
     if constexpr (sizeof(T) == 4) {
       if (v == 10)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 10>), pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 10>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
       else if (v == 12)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 12>), pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 12>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
+        MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, L.order, gout, mark, header);
+      MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
     }
   }
   return cudaGetLastError();

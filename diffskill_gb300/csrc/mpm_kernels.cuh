@@ -772,9 +772,12 @@ MPM_DI void mark_stencil_blocks(const Consts<T>& c, bool ok, const int* base, in
 // ---------------------------------------------------------------------------
 // forward kernels
 // ---------------------------------------------------------------------------
-// The particle of thread i.  order (may be null): a permutation that sorts the
-// particles by cell, for frames that are kept in the caller's order.  Its loads
-// before a pdl_wait() go to L2 (load_row_cg).
+// The particle of thread i of a scattering kernel.  order (may be null): a
+// permutation that sorts the particles by cell, for frames that are kept in the
+// caller's order; its load before a pdl_wait() goes to L2 (load_row_cg).  The rows
+// are then read one sector per particle, which g2p and p2g.grad, with nothing to
+// scatter, would only lose by (30,000 particles: g2p 8.8 -> 11.5 us, p2g.grad
+// 13.6 -> 35; p2g 24 -> 14, g2p.grad 25 -> 20).
 MPM_DI int64_t particle_of(const int* __restrict__ order, int64_t i, bool valid) {
   return order && valid ? (int64_t)__ldcg(order + i) : i;
 }
@@ -1152,12 +1155,10 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
 // at most 64 registers)
 template <typename T, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k_g2p(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
-                                             const int* __restrict__ pscene, const int* __restrict__ order,
-                                             const Node<T>* __restrict__ grid, unsigned char* __restrict__ mark,
-                                             int* __restrict__ header) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < c.n_particles;
-  const int64_t p = particle_of(order, i, valid);
+                                             const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
+                                             unsigned char* __restrict__ mark, int* __restrict__ header) {
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = p < c.n_particles;
   const int scene = valid ? __ldcg(pscene + p) : 0;  // issued with x
   T xn[3] = {T(0), T(0), T(0)};
   const bool moved = valid && g2p_particle(c, st, st_out, p, scene, grid, xn);
@@ -1474,12 +1475,10 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
 // and 430 B); MB > 0: MB CTAs per SM (MpmTuning.p2g_adj_ctas)
 template <typename T, typename S, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 4 : 8)) k_p2g_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ g1,
-                                                 T* __restrict__ g0, const int* __restrict__ pscene,
-                                                 const int* __restrict__ order, bool add,
+                                                 T* __restrict__ g0, const int* __restrict__ pscene, bool add,
                                                  const Node<T>* __restrict__ g_in) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.n_particles) return;
-  const int64_t p = particle_of(order, i, true);
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= c.n_particles) return;
   // the adjoint rows read after the forward recompute and the gather are
   // fetched into L2 now, so those later loads do not wait on DRAM
 #pragma unroll
@@ -1597,19 +1596,22 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
 #pragma unroll
   for (int k = 0; k < 9; ++k) gF1[k] = to_prec<S>(g1[(int64_t)(15 + k) * c.ld + p]);
   p2g_particle_vjp(m, C, F, P, g_aff, gF1, gC, gF);
-  store_row(g0, c.ld, p, 0, 3, gx);
+  T out[21];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    T* o = g0 + (int64_t)(3 + k) * c.ld + p;
-    *o = add ? *o + gv[k] : gv[k];
-  }
+  for (int k = 0; k < 3; ++k) out[k] = gv[k];
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    T *oC = g0 + (int64_t)(6 + k) * c.ld + p, *oF = g0 + (int64_t)(15 + k) * c.ld + p;
-    const T vC = to_prec<T>(gC[k]), vF = to_prec<T>(gF[k]);
-    *oC = add ? *oC + vC : vC;
-    *oF = add ? *oF + vF : vF;
+    out[3 + k] = to_prec<T>(gC[k]);
+    out[12 + k] = to_prec<T>(gF[k]);
   }
+  if (add) {  // all 21 loads before the first store
+    T old[21];
+    load_row_cg(g0, c.ld, p, 3, 21, old);
+#pragma unroll
+    for (int k = 0; k < 21; ++k) out[k] += old[k];
+  }
+  store_row(g0, c.ld, p, 0, 3, gx);
+  store_row(g0, c.ld, p, 3, 21, out);
 }
 
 // ---------------------------------------------------------------------------
