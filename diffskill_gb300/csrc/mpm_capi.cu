@@ -18,6 +18,7 @@ struct MpmHandle {
   int device = -1;
   int64_t G = 0;
   std::vector<int64_t> offsets;
+  char* arena = nullptr;  // holds the buffers below that mpm_create sets
   int* d_pscene = nullptr;
   int* d_tool_off = nullptr;
   int* d_col_off = nullptr;  // first tool-distance column of each tool
@@ -194,26 +195,38 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
     for (int64_t i = scene_offsets[s]; i < scene_offsets[s + 1]; ++i) ps[i] = s;
   std::vector<int> toff(p.n_scenes + 1, 0);
   const size_t gbytes = (size_t)p.n_scenes * h->G * 4 * real_size(p.precision);
-  bool ok = true;
-  ok = ok && cudaMalloc(&h->d_pscene, std::max<size_t>(1, ps.size()) * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_tool_off, toff.size() * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_status, sizeof(unsigned int)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_flags, mpm::kTargetSdfFlags * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_tile_flags, mpm::target_sdf_flag_bytes(p.n_scenes, p.n_grid)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_pair_off, toff.size() * sizeof(int)) == cudaSuccess;
-  for (int i = 0; i < 4 && ok; ++i) ok = cudaMalloc(&h->grid[i], gbytes) == cudaSuccess;
   const int64_t nb = p.n_grid / 4;
   const int64_t nblocks = (int64_t)p.n_scenes * nb * nb * nb;
-  ok = ok && cudaMalloc(&h->d_blockbuf, mpm::blockbuf_bytes(p.n_scenes, p.n_grid)) == cudaSuccess;
-  // block flags start clean; every compaction clears the flags it reads
-  ok = ok && cudaMemset(h->d_blockbuf, 0, mpm::blockbuf_bytes(p.n_scenes, p.n_grid)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_active, nblocks * sizeof(int)) == cudaSuccess;
   const size_t np = (size_t)std::max<int64_t>(p.n_particles, 1);
-  ok = ok && cudaMalloc(&h->sort.keys_a, np * sizeof(uint32_t)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->sort.keys_b, np * sizeof(uint32_t)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->sort.vals_b, np * sizeof(int32_t)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->d_order, np * sizeof(int)) == cudaSuccess;
-  ok = ok && cudaMalloc(&h->sort.hist, mpm::sort_hist_words(p.n_particles) * sizeof(uint32_t)) == cudaSuccess;
+  // two allocations: the four grids, and an arena of everything else (a cudaMalloc
+  // each made creating a small handle mostly allocation)
+  const size_t bbytes = mpm::blockbuf_bytes(p.n_scenes, p.n_grid);
+  size_t at = 0;
+  std::vector<std::pair<void**, size_t>> parts;
+  auto part = [&](auto** ptr, size_t bytes) {
+    parts.emplace_back((void**)ptr, at);
+    at += (bytes + 255) / 256 * 256;
+  };
+  part(&h->d_pscene, np * sizeof(int));
+  part(&h->d_tool_off, toff.size() * sizeof(int));
+  part(&h->d_status, sizeof(unsigned int));
+  part(&h->d_flags, mpm::kTargetSdfFlags * sizeof(int));
+  part(&h->d_tile_flags, mpm::target_sdf_flag_bytes(p.n_scenes, p.n_grid));
+  part(&h->d_pair_off, toff.size() * sizeof(int));
+  part(&h->d_blockbuf, bbytes);
+  part(&h->d_active, nblocks * sizeof(int));
+  part(&h->sort.keys_a, np * sizeof(uint32_t));
+  part(&h->sort.keys_b, np * sizeof(uint32_t));
+  part(&h->sort.vals_b, np * sizeof(int32_t));
+  part(&h->d_order, np * sizeof(int));
+  part(&h->sort.hist, mpm::sort_hist_words(p.n_particles) * sizeof(uint32_t));
+  bool ok = cudaMalloc(&h->arena, at) == cudaSuccess;
+  for (auto& q : parts) *q.first = ok ? h->arena + q.second : nullptr;
+  char* grids = nullptr;
+  ok = ok && cudaMalloc(&grids, 4 * gbytes) == cudaSuccess;
+  for (int i = 0; i < 4; ++i) h->grid[i] = ok ? grids + (size_t)i * gbytes : nullptr;
+  // block flags start clean; every compaction clears the flags it reads
+  ok = ok && cudaMemset(h->d_blockbuf, 0, bbytes) == cudaSuccess;
   // the pipelined adjoint's internal stream and events (created here, outside any stream capture)
   ok = ok && cudaStreamCreateWithFlags(&h->pipe_side, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&h->pipe_grid_done, cudaEventDisableTiming) == cudaSuccess;
@@ -240,25 +253,13 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
 
 int mpm_destroy(MpmHandle* h) {
   if (!h) return MPM_OK;
-  cudaFree(h->d_pscene);
-  cudaFree(h->d_tool_off);
+  cudaFree(h->arena);
+  cudaFree(h->grid[0]);
   cudaFree(h->d_col_off);
   cudaFree(h->d_tools);
-  cudaFree(h->d_status);
-  cudaFree(h->d_flags);
-  cudaFree(h->d_tile_flags);
-  cudaFree(h->d_pair_off);
   cudaFree(h->d_coll_pts);
-  for (int i = 0; i < 4; ++i) cudaFree(h->grid[i]);
-  cudaFree(h->d_blockbuf);
-  cudaFree(h->d_active);
   cudaFree(h->d_tools_t);
   cudaFree(h->d_poses_t);
-  cudaFree(h->sort.keys_a);
-  cudaFree(h->sort.keys_b);
-  cudaFree(h->sort.vals_b);
-  cudaFree(h->d_order);
-  cudaFree(h->sort.hist);
   if (h->pipe_side) cudaStreamDestroy(h->pipe_side);
   if (h->pipe_grid_done) cudaEventDestroy(h->pipe_grid_done);
   if (h->pipe_prep_done) cudaEventDestroy(h->pipe_prep_done);

@@ -395,7 +395,7 @@ class GridStore:
         self.blocks = torch.empty((max(self.capacity, 1), 2, 64, 4), dtype=eng.dtype, device=dev)
         self.block_ids = torch.empty(max(self.capacity, 1), dtype=torch.int32, device=dev)
         self.slot_start = torch.full((n_slots,), -1, dtype=torch.int64, device=dev)
-        self.slot_count = torch.zeros(n_slots, dtype=torch.int32, device=dev)
+        self.slot_count = torch.empty(n_slots, dtype=torch.int32, device=dev)  # read where slot_start >= 0
         self.bump = torch.zeros(1, dtype=torch.int64, device=dev)
         st = _lib.MpmGridStore()
         st.blocks = self.blocks.data_ptr()

@@ -148,5 +148,4 @@ class Primitives:
 
     def initialize(self) -> None:
         if self.sim is not None:
-            for p in self.primitives:
-                p.set_state(0, p.init_state)
+            self.sim._set_poses(0, {p.index: p.init_state for p in self.primitives})
