@@ -7,11 +7,10 @@ namespace mpm {
 
 template <typename T>
 Consts<T> make_consts(const LaunchCtx& L);  // mpm_fwd.cu
-template <typename T>
-cudaError_t prepare_blocks(const LaunchCtx& L, const Consts<T>& c, const T* st, Node<T>* a, Node<T>* a_out,
-                           Node<T>* b, const MpmGridStore* restore, int restore_slot, const MpmGridStore* reserve,
-                           int reserve_slot, const double* pose_f, const double* pose_f1, bool premarked);
 unsigned grid_blocks_launch(const LaunchCtx& L, int64_t total_blocks);
+int* list_counter(const LaunchCtx& L, bool adjoint);
+template <typename T>
+cudaError_t launch_list_blocks(const LaunchCtx& L, const Consts<T>& c, int* counter, const int64_t* saved);
 
 static inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
@@ -24,27 +23,31 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
   Node<T>* gout = (Node<T>*)L.grid_b;
   Node<T>* g_gin = (Node<T>*)L.grid_c;
   Node<T>* g_gout = (Node<T>*)L.grid_d;
-  const int* counter = reinterpret_cast<const int*>(L.blockbuf);
+  int* counter = list_counter(L, true);
+  const int* active = L.active;
   constexpr int bs_t = kParticleThreads<T>, bs_s = kParticleThreads<S>;
   const unsigned pb_t = blocks_for(c.n_particles, bs_t), pb_s = blocks_for(c.n_particles, bs_s);
   const unsigned gb = grid_blocks_launch(L, (int64_t)c.n_scenes * c.NB3);
   const Tool<T>* tools_t = (const Tool<T>*)L.tools_t;
   const T* poses_t = (const T*)L.poses_t;
   if (phases & BWD_PREPARE) {
-    // recompute the grids of this substep (substep_grad, mpm_simulator.py:327-333)
-    // unless the grid store holds them (then p2g and grid_op return at once)
+    // the grids of this substep come from the grid store, or are recomputed
+    // (substep_grad, mpm_simulator.py:327-333); then p2g and grid_op return at once
     const int64_t* saved = store ? store->slot_start + slot : nullptr;
-    cudaError_t e = prepare_blocks<T>(L, c, st0, gin, gout, g_gout, store, slot, nullptr, -1, pose_f, pose_f1, false);
-    if (e != cudaSuccess) return e;
+    const PoseTableArgs pt{L.n_tools, pose_f, pose_f1, L.poses_t, nullptr};
+    MPM_LAUNCH_PDL(L, MPM_K_CLEAR, k_restore<T>, store ? (unsigned)(L.sm_count * 8) : 1u, 256, counter,
+                   store ? *store : MpmGridStore{}, store ? slot : -1, L.active, gin, gout, g_gout, pt);
     if (c.n_particles > 0) {
       // with a grid store the recompute usually exits at once: a grid of one
       // wave of CTAs that stride over the particles
       const unsigned cap = (unsigned)(L.sm_count * (bs_s == 32 ? 16 : 6));
       MPM_LAUNCH_PDL(L, MPM_K_P2G_RECOMP, (k_p2g<T, S, true>), store && pb_s > cap ? cap : pb_s, bs_s, c, st0,
-                     (T*)nullptr, L.pscene, L.order, gin, saved);
+                     (T*)nullptr, L.pscene, L.order, gin, L.blockbuf + 16, pt, saved);
+      const cudaError_t e = launch_list_blocks<T>(L, c, counter, saved);
+      if (e != cudaSuccess) return e;
     }
-    MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, gb, 64, c, L.active, counter, gin, gout, tools_t, poses_t,
-                   L.tool_off, MpmGridStore{}, -1, saved);
+    MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, gb, 64, c, active, (const int*)counter, gin, gout, g_gout, tools_t,
+                   poses_t, L.tool_off, MpmGridStore{}, -1, saved);
   }
   if ((phases & BWD_GRID) && c.n_particles > 0) {
     // FP32: the CTAs-per-SM variant the tuning selects.  BWD_G2P_PLAIN: the
@@ -79,17 +82,17 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
     const int v = L.tune.grid_op_adj_ctas;
     if constexpr (sizeof(T) == 4) {
       if (v == 12)
-        MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, (k_grid_op_adj<T, 12>), gb, 64, c, L.active, counter, gin, g_gout, g_gin,
+        MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, (k_grid_op_adj<T, 12>), gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin,
                        tools_t, poses_t, L.tool_off, g_pose_f, g_pose_f1);
       else if (v == 16)
-        MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, (k_grid_op_adj<T, 16>), gb, 64, c, L.active, counter, gin, g_gout, g_gin,
+        MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, (k_grid_op_adj<T, 16>), gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin,
                        tools_t, poses_t, L.tool_off, g_pose_f, g_pose_f1);
       else
-        MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, k_grid_op_adj<T>, gb, 64, c, L.active, counter, gin, g_gout, g_gin,
+        MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, k_grid_op_adj<T>, gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin,
                        tools_t, poses_t, L.tool_off, g_pose_f, g_pose_f1);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, k_grid_op_adj<T>, gb, 64, c, L.active, counter, gin, g_gout, g_gin, tools_t,
+      MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, k_grid_op_adj<T>, gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin, tools_t,
                      poses_t, L.tool_off, g_pose_f, g_pose_f1);
     }
   }

@@ -25,9 +25,8 @@ struct MpmHandle {
   int n_cols = 0;
   MpmToolDesc* d_tools = nullptr;
   int n_tools = 0;
-  bool chained = false;           // mpm_set_chained
   MpmTuning tune = {0, 0, 0, 0, 0, 0};  // mpm_set_tuning
-  const void* premarked = nullptr;  // frame whose block flags the last forward g2p set
+  bool dirty = false;  // a launch failed inside a substep: grid a and the block flags may not be zero
   std::vector<MpmToolDesc> h_tools;
   unsigned int* d_status = nullptr;
   int* d_flags = nullptr;  // convergence flags and counters of mpm_target_sdf
@@ -225,8 +224,9 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
   char* grids = nullptr;
   ok = ok && cudaMalloc(&grids, 4 * gbytes) == cudaSuccess;
   for (int i = 0; i < 4; ++i) h->grid[i] = ok ? grids + (size_t)i * gbytes : nullptr;
-  // block flags start clean; every compaction clears the flags it reads
+  // the p2g grid and the block flags start at zero; every substep leaves them so
   ok = ok && cudaMemset(h->d_blockbuf, 0, bbytes) == cudaSuccess;
+  ok = ok && cudaMemset(h->grid[0], 0, gbytes) == cudaSuccess;
   // the pipelined adjoint's internal stream and events (created here, outside any stream capture)
   ok = ok && cudaStreamCreateWithFlags(&h->pipe_side, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&h->pipe_grid_done, cudaEventDisableTiming) == cudaSuccess;
@@ -419,9 +419,28 @@ static int check_store(MpmHandle* h, const MpmGridStore* store, int32_t slot) {
   return check_aligned(h, store->blocks, "store->blocks", store->capacity == 0);
 }
 
+// Between substeps grid a and the block flags are zero; a substep that failed on the
+// way left them unknown, so the next one clears them.
+static int substep_begin(MpmHandle* h, void* stream) {
+  if (h->dirty) {
+    cudaError_t e = cudaMemsetAsync(h->grid[0], 0, (size_t)h->p.n_scenes * h->G * 4 * real_size(h->p.precision),
+                                    (cudaStream_t)stream);
+    if (e == cudaSuccess)
+      e = cudaMemsetAsync(h->d_blockbuf, 0, mpm::blockbuf_bytes(h->p.n_scenes, h->p.n_grid), (cudaStream_t)stream);
+    if (e != cudaSuccess) return cuda_fail(h, e, "clearing the grid");
+  }
+  h->dirty = true;
+  return MPM_OK;
+}
+static int substep_done(MpmHandle* h, cudaError_t e, const char* what) {
+  if (e != cudaSuccess) return cuda_fail(h, e, what);
+  h->dirty = false;
+  return MPM_OK;
+}
+
 static int substep_fwd_impl(MpmHandle* h, const void* state_f, void* state_f1, const double* pose_f,
-                            const double* pose_f1, const MpmGridStore* store, int32_t slot, void* stream, bool pre,
-                            bool next, const int* order = nullptr) {
+                            const double* pose_f1, const MpmGridStore* store, int32_t slot, void* stream,
+                            const int* order = nullptr) {
   if (!h) return fail(nullptr, MPM_E_INVALID, "mpm_substep_fwd: NULL handle");
   MPM_TRY(check_device(h));
   MPM_TRY(check_aligned(h, state_f, "state_f"));
@@ -432,27 +451,23 @@ static int substep_fwd_impl(MpmHandle* h, const void* state_f, void* state_f1, c
   MPM_TRY(check_store(h, store, slot));
   mpm::LaunchCtx L = ctx(h, stream);
   L.order = order;
-  // pre: the previous forward substep's g2p flagged the blocks of this substep's
-  // input frame; next: this one's flags those of its output
-  h->premarked = nullptr;
+  MPM_TRY(substep_begin(h, stream));
   h->pipe_pending = false;  // a forward substep rewrites the grids: no adjoint overlaps it
   cudaError_t e;
   switch (h->p.precision) {
     case MPM_PREC_FP32:
       e = mpm::launch_substep_fwd<float, float>(L, (const float*)state_f, (float*)state_f1, pose_f, pose_f1, store,
-                                                slot, pre, next);
+                                                slot);
       break;
     case MPM_PREC_FP32_SVD64:
       e = mpm::launch_substep_fwd<float, double>(L, (const float*)state_f, (float*)state_f1, pose_f, pose_f1, store,
-                                                 slot, pre, next);
+                                                 slot);
       break;
     default:
       e = mpm::launch_substep_fwd<double, double>(L, (const double*)state_f, (double*)state_f1, pose_f, pose_f1,
-                                                  store, slot, pre, next);
+                                                  store, slot);
   }
-  if (e != cudaSuccess) return cuda_fail(h, e, "mpm_substep_fwd");
-  if (next) h->premarked = state_f1;
-  return MPM_OK;
+  return substep_done(h, e, "mpm_substep_fwd");
 }
 
 static int substep_bwd_impl(MpmHandle* h, const void* state_f, const void* state_f1, const void* g_state_f1,
@@ -476,7 +491,7 @@ static int substep_bwd_impl(MpmHandle* h, const void* state_f, const void* state
   mpm::LaunchCtx L = ctx(h, stream);
   L.order = order;
   L.add = add;
-  h->premarked = nullptr;  // the adjoint's compaction may consume the flags
+  MPM_TRY(substep_begin(h, stream));
   auto run = [&](const mpm::LaunchCtx& C, unsigned phases) -> cudaError_t {
     switch (h->p.precision) {
       case MPM_PREC_FP32:
@@ -523,7 +538,7 @@ static int substep_bwd_impl(MpmHandle* h, const void* state_f, const void* state
     h->pipe_pending = e == cudaSuccess;
     h->pipe_stream = stream;
   }
-  return e == cudaSuccess ? MPM_OK : cuda_fail(h, e, "mpm_substep_bwd");
+  return substep_done(h, e, "mpm_substep_bwd");
 }
 
 int mpm_set_pipelined_adjoint(MpmHandle* h, int32_t on) {
@@ -535,8 +550,7 @@ int mpm_set_pipelined_adjoint(MpmHandle* h, int32_t on) {
 
 int mpm_set_chained(MpmHandle* h, int32_t on) {
   if (!h) return fail(nullptr, MPM_E_INVALID, "mpm_set_chained: NULL handle");
-  h->chained = on != 0;
-  h->premarked = nullptr;
+  (void)on;  // every substep builds its own list
   return MPM_OK;
 }
 
@@ -576,14 +590,12 @@ int mpm_get_tuning(MpmHandle* h, MpmTuning* t) {
 
 int mpm_substep_fwd(MpmHandle* h, const void* state_f, void* state_f1, const double* pose_f, const double* pose_f1,
                     void* stream) {
-  return substep_fwd_impl(h, state_f, state_f1, pose_f, pose_f1, nullptr, -1, stream, h && h->chained && h->premarked == state_f,
-                          h && h->chained);
+  return substep_fwd_impl(h, state_f, state_f1, pose_f, pose_f1, nullptr, -1, stream);
 }
 int mpm_substep_fwd_store(MpmHandle* h, const void* state_f, void* state_f1, const double* pose_f,
                           const double* pose_f1, const MpmGridStore* store, int32_t slot, void* stream) {
   if (!store) return fail(h, MPM_E_INVALID, "mpm_substep_fwd_store: NULL store");
-  return substep_fwd_impl(h, state_f, state_f1, pose_f, pose_f1, store, slot, stream,
-                          h && h->chained && h->premarked == state_f, h && h->chained);
+  return substep_fwd_impl(h, state_f, state_f1, pose_f, pose_f1, store, slot, stream);
 }
 int mpm_substep_bwd(MpmHandle* h, const void* state_f, const void* state_f1, const void* g_state_f1,
                     void* g_state_f, const double* pose_f, const double* pose_f1, double* g_pose_f,
@@ -658,13 +670,10 @@ int mpm_substeps_fwd(MpmHandle* h, void* frames, const double* poses, int32_t n,
   if (order) MPM_TRY(sort_run(h, frames, stream));
   int rc = MPM_OK;
   for (int32_t i = 0; i < n && rc == MPM_OK; ++i) {
-    // each frame goes unmodified from one substep to the next: chained
     char* f = (char*)frames + (size_t)i * frame;
     const double* q = poses ? poses + (size_t)i * pose : nullptr;
-    rc = substep_fwd_impl(h, f, f + frame, q, q ? q + pose : nullptr, store, store ? slot0 + i : -1, stream, i > 0,
-                          i + 1 < n, order);
+    rc = substep_fwd_impl(h, f, f + frame, q, q ? q + pose : nullptr, store, store ? slot0 + i : -1, stream, order);
   }
-  h->premarked = nullptr;
   // the frame after the run changed: what its slot held belongs to another content
   if (rc == MPM_OK && store && (int64_t)slot0 + n < store->n_slots) {
     const cudaError_t e = cudaMemsetAsync(store->slot_start + slot0 + n, 0xff, sizeof(int64_t), (cudaStream_t)stream);
@@ -733,8 +742,6 @@ int mpm_sort_frame(MpmHandle* h, const void* src, void* dst, int32_t* perm, void
                       ? mpm::launch_sort_frame<double>(L, (const double*)src, (double*)dst, perm, h->sort)
                       : mpm::launch_sort_frame<float>(L, (const float*)src, (float*)dst, perm, h->sort);
   if (e != cudaSuccess) return cuda_fail(h, e, "mpm_sort_frame");
-  // same particle set: the block flags a chained forward set for src hold for dst
-  if (h->premarked == src) h->premarked = dst;
   return MPM_OK;
 }
 

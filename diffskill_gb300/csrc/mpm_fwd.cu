@@ -51,52 +51,22 @@ Consts<T> make_consts(const LaunchCtx& L) {
 template Consts<float> make_consts<float>(const LaunchCtx&);
 template Consts<double> make_consts<double>(const LaunchCtx&);
 
-static inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
-
-// Active blocks of frame st: mark, then compact the list and zero the listed
-// blocks of grid a (and b if given).  Leaves the list in L.active and its
-// length at L.blockbuf[0..3] (a ticket counter at [4..7]); the block flags at
-// L.blockbuf + 16 are clean before and after (cleared by the compaction).
-// ``restore`` (may be null): the adjoint's grid store; when its slot holds
-// this substep the list, grid a and grid a_out (the grid_op output) are
-// restored from it and b is zeroed.
-// ``reserve`` (may be null): the forward's grid store; room for the list is
-// reserved in slot ``reserve_slot`` by the compaction's last CTA.
-// The compaction also fills L.poses_t for the poses pose_f, pose_f1.
-// premarked (forward only): the flags and the header were set by the previous
-// substep's g2p, so the marking launch is skipped.
+// The list length has a word of its own for the forward substep (p2g empties it) and
+// for the adjoint (k_restore does): with a pipelined adjoint the next
+// substep's list begins before this one's last kernel ends.
+int* list_counter(const LaunchCtx& L, bool adjoint) { return reinterpret_cast<int*>(L.blockbuf) + (adjoint ? 1 : 0); }
+// flags to list; 2,048 blocks per CTA
 template <typename T>
-cudaError_t prepare_blocks(const LaunchCtx& L, const Consts<T>& c, const T* st, Node<T>* a, Node<T>* a_out,
-                           Node<T>* b, const MpmGridStore* restore, int restore_slot, const MpmGridStore* reserve,
-                           int reserve_slot, const double* pose_f, const double* pose_f1, bool premarked) {
+cudaError_t launch_list_blocks(const LaunchCtx& L, const Consts<T>& c, int* counter, const int64_t* saved) {
   const int64_t total = (int64_t)c.n_scenes * c.NB3;
-  int* counter = reinterpret_cast<int*>(L.blockbuf);
-  unsigned* ticket = reinterpret_cast<unsigned*>(L.blockbuf + 4);
-  unsigned char* flags = L.blockbuf + 16;
-  const int64_t* saved = restore ? restore->slot_start + restore_slot : nullptr;
-  // one thread per particle for the marking; the restore strides over the stored nodes
-  unsigned mb = blocks_for(c.n_particles, 256);
-  const unsigned floor_ctas = (unsigned)(L.sm_count * 8);
-  if (restore && mb < floor_ctas) mb = floor_ctas;
-  if (mb == 0) mb = 1;
-  MpmGridStore rst{};
-  if (restore) rst = *restore;
-  if (!premarked || restore)
-    MPM_LAUNCH_PDL(L, MPM_K_CLEAR, k_mark_or_restore<T>, mb, 256, c, st, L.pscene, flags, counter, rst,
-               restore ? restore_slot : -1, L.active, a, a_out, b);
-  MpmGridStore rs{};
-  if (reserve) rs = *reserve;
-  const PoseTableArgs tt{L.n_tools, pose_f, pose_f1, L.poses_t};
-  MPM_LAUNCH_PDL(L, MPM_K_CLEAR, k_compact_clear<T>, blocks_for(total, 256), 256, flags, total, L.active, counter, ticket,
-             a, b, saved, rs, reserve ? reserve_slot : -1, tt);
-  return cudaGetLastError();
+  MPM_LAUNCH_PDL(L, MPM_K_CLEAR, k_list_blocks<T>, (unsigned)((total + 2047) / 2048), 128, L.blockbuf + 16, total,
+                 L.active, counter, saved);
+  return cudaSuccess;
 }
-template cudaError_t prepare_blocks<float>(const LaunchCtx&, const Consts<float>&, const float*, Node<float>*,
-                                           Node<float>*, Node<float>*, const MpmGridStore*, int,
-                                           const MpmGridStore*, int, const double*, const double*, bool);
-template cudaError_t prepare_blocks<double>(const LaunchCtx&, const Consts<double>&, const double*, Node<double>*,
-                                            Node<double>*, Node<double>*, const MpmGridStore*, int,
-                                            const MpmGridStore*, int, const double*, const double*, bool);
+template cudaError_t launch_list_blocks<float>(const LaunchCtx&, const Consts<float>&, int*, const int64_t*);
+template cudaError_t launch_list_blocks<double>(const LaunchCtx&, const Consts<double>&, int*, const int64_t*);
+
+static inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 size_t tools_t_bytes(int64_t n_tools) { return (size_t)(n_tools > 0 ? n_tools : 1) * sizeof(Tool<double>); }
 size_t poses_t_bytes(int64_t n_tools) { return (size_t)(n_tools > 0 ? n_tools : 1) * 16 * sizeof(double); }
@@ -118,53 +88,60 @@ unsigned grid_blocks_launch(const LaunchCtx& L, int64_t total_blocks) {
 
 template <typename T, typename S>
 cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const double* pose_f,
-                               const double* pose_f1, const MpmGridStore* store, int slot, bool premarked,
-                               bool mark_next) {
+                               const double* pose_f1, const MpmGridStore* store, int slot) {
   Consts<T> c = make_consts<T>(L);
+  if (c.n_particles == 0) return cudaSuccess;  // no mass on the grid, nothing to move
   Node<T>* gin = (Node<T>*)L.grid_a;
   Node<T>* gout = (Node<T>*)L.grid_b;
-  const int* counter = reinterpret_cast<const int*>(L.blockbuf);
-  cudaError_t e = prepare_blocks<T>(L, c, st0, gin, (Node<T>*)nullptr, (Node<T>*)nullptr, nullptr, -1, store, slot,
-                                    pose_f, pose_f1, premarked);
-  if (e != cudaSuccess) return e;
-  if (c.n_particles > 0) {
+  int* counter = list_counter(L, false);
+  unsigned char* flags = L.blockbuf + 16;
+  const int64_t* none = nullptr;
+  const MpmGridStore keep = store ? *store : MpmGridStore{};
+  const int keep_slot = store ? slot : -1;
+  {
     constexpr int bs = kParticleThreads<S>;
     const unsigned pb = blocks_for(c.n_particles, bs);
-    const int64_t* none = nullptr;
+    const PoseTableArgs pt{L.n_tools, pose_f, pose_f1, L.poses_t, counter};
     // FP32: the CTAs-per-SM variant the tuning selects
-    const int v = L.tune.p2g_ctas;
-    if constexpr (sizeof(T) == 4 && sizeof(S) == 4) {
+    const int v = sizeof(S) == 4 ? L.tune.p2g_ctas : 0;
+#define MPM_P2G(KERNEL) \
+  MPM_LAUNCH_PDL(L, MPM_K_P2G, KERNEL, pb, bs, c, st0, st1, L.pscene, L.order, gin, flags, pt, none)
+    if constexpr (sizeof(S) == 4) {
       if (v == 6)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 6>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
+        MPM_P2G((k_p2g<T, S, false, 6>));
       else if (v == 8)
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S, false, 8>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
+        MPM_P2G((k_p2g<T, S, false, 8>));
       else
-        MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
+        MPM_P2G((k_p2g<T, S>));
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_P2G, (k_p2g<T, S>), pb, bs, c, st0, st1, L.pscene, L.order, gin, none);
+      MPM_P2G((k_p2g<T, S>));
     }
+#undef MPM_P2G
   }
-  MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, grid_blocks_launch(L, (int64_t)c.n_scenes * c.NB3), 64, c, L.active,
-             counter, gin, gout, (const Tool<T>*)L.tools_t, (const T*)L.poses_t, L.tool_off,
-             store ? *store : MpmGridStore{}, store ? slot : -1, (const int64_t*)nullptr);
-  if (c.n_particles > 0) {
+  const cudaError_t e = launch_list_blocks<T>(L, c, counter, none);
+  if (e != cudaSuccess) return e;
+  MPM_LAUNCH_PDL(L, MPM_K_GRID_OP, k_grid_op<T>, grid_blocks_launch(L, (int64_t)c.n_scenes * c.NB3), 64, c,
+                 (const int*)L.active, (const int*)counter, gin, gout, (Node<T>*)nullptr, (const Tool<T>*)L.tools_t,
+                 (const T*)L.poses_t, L.tool_off, keep, keep_slot, none);
+  {
     constexpr int bs = kParticleThreads<T>;
     const unsigned pb = blocks_for(c.n_particles, bs);
-    unsigned char* mark = mark_next ? L.blockbuf + 16 : (unsigned char*)nullptr;
-    int* header = reinterpret_cast<int*>(L.blockbuf);
-    const int v = L.tune.g2p_ctas;
+    const int v = sizeof(T) == 4 ? L.tune.g2p_ctas : 0;
+#define MPM_G2P(KERNEL) \
+  MPM_LAUNCH_PDL(L, MPM_K_G2P, KERNEL, pb, bs, c, st0, st1, L.pscene, gout, (const int*)L.active, (const int*)counter, gin, keep, keep_slot)
     if constexpr (sizeof(T) == 4) {
       if (v == 10)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 10>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_G2P((k_g2p<T, 10>));
       else if (v == 12)
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, (k_g2p<T, 12>), pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_G2P((k_g2p<T, 12>));
       else
-        MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+        MPM_G2P(k_g2p<T>);
     } else {
       (void)v;
-      MPM_LAUNCH_PDL(L, MPM_K_G2P, k_g2p<T>, pb, bs, c, st0, st1, L.pscene, gout, mark, header);
+      MPM_G2P(k_g2p<T>);
     }
+#undef MPM_G2P
   }
   return cudaGetLastError();
 }
@@ -306,7 +283,7 @@ template cudaError_t launch_tool_distance<double>(const LaunchCtx&, const int*, 
 
 #define MPM_INST_FWD(T, S)                                                                             \
   template cudaError_t launch_substep_fwd<T, S>(const LaunchCtx&, const T*, T*, const double*, const double*, \
-                                                const MpmGridStore*, int, bool, bool);
+                                                const MpmGridStore*, int);
 MPM_INST_FWD(float, float)
 MPM_INST_FWD(float, double)
 MPM_INST_FWD(double, double)

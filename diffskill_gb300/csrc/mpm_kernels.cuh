@@ -15,13 +15,20 @@
 // Particle state is component-major: row k of a frame is st[k*ld + p].
 //
 // Sparse grid: the scratch grids of a substep are stored block-contiguous
-// (blocks of 4x4x4 nodes, 64 nodes = 1 KiB in FP32 per block).  Each substep
-// marks the blocks that particle stencils touch (k_mark_or_restore), compacts
-// them into a device-side list and clears only those (k_compact_clear), and
-// runs grid_op / grid_op.grad over that list with
-// grid-stride loops (no host round trip; capturable in a CUDA graph).  Nodes
-// outside the list hold no mass, so grid_op leaves them at zero exactly as the
-// dense reference does; g2p and p2g.grad only read nodes inside the list.
+// (blocks of 4x4x4 nodes, 64 nodes = 1 KiB in FP32 per block).  Between substeps
+// the p2g grid is zero everywhere and no block is flagged.  p2g adds to the grid
+// and flags the blocks that particle stencils touch, k_list_blocks turns the flags
+// into a device-side list and clears them, grid_op and grid_op.grad run over that
+// list with grid-stride loops (no host round trip; capturable in a CUDA graph), and
+// a kernel after the p2g grid's last reader zeroes its listed blocks (g2p forward,
+// grid_op.grad itself in the adjoint).  So no pass over the particles only marks
+// blocks and none only clears the grid.  One substep of 64 scenes (1.1M particles,
+// 32 us of compulsory traffic): with the marking in g2p and a compaction that also
+// clears, p2g 82, grid_op 14, g2p 48, clear 8 us; now 85, 14, 39 and 7.  The zeroing
+// is in g2p because that kernel waits for latency and has bandwidth to spare (+2 us);
+// in grid_op, which is bound by bandwidth, it cost 12.  Nodes outside the list hold
+// no mass, so grid_op leaves them at zero exactly as the dense reference does; g2p
+// and p2g.grad only read nodes inside the list.
 #pragma once
 #include "../../include/mpm_gb300.h"
 #include "mpm_math.cuh"
@@ -170,6 +177,7 @@ MPM_DI int block_node(const Consts<T>& c, int64_t gb, int l, int* I) {
 struct WarpRows {
   int row;
   unsigned tails, emit;
+  bool first;  // this lane is the first of its group
 };
 MPM_DI WarpRows warp_rows(long long key, bool ok) {
   const unsigned full = 0xffffffffu;
@@ -190,6 +198,7 @@ MPM_DI WarpRows warp_rows(long long key, bool ok) {
   const unsigned last = 1u << (end - 1);
   w.tails = __reduce_or_sync(full, last);
   w.emit = __reduce_or_sync(full, ok ? last : 0u);
+  w.first = lane == first;
   return w;
 }
 
@@ -201,7 +210,9 @@ MPM_DI WarpRows warp_rows(long long key, bool ok) {
 // all lanes, so its sum leaves by one 27-lane red.global.add.v4.f32 without
 // divergence.  Before, every lane stored its 27 node values one slab of 9 at a
 // time and 27 lanes = 9 nodes x 3 row groups read them back, which closed each
-// run three times per substep and diverged over the row groups (ROWSCATTER).
+// run three times per substep and diverged over the row groups: 2,850 instructions
+// per warp in p2g and 2,288 in g2p.grad, now 2,225 and 1,760 (1.1M particles: p2g 128
+// to 81 us, g2p.grad 136 to 86).
 struct RowStage {
   float4 q0[32];       // u.x, u.y, G00, G10
   float4 q1[32];       // G01, G11, G02, G12
@@ -732,46 +743,45 @@ MPM_DI const MatConsts<S>& mat_consts(const Consts<T>& c) {
     return c.m32;
 }
 
-// flags[scene*NB3 + block] = 1 for the blocks of the stencil at `base` (a lane
-// with ok), called by all 32 lanes of a warp.  In cell order neighbouring
-// particles touch the same blocks, so a lane whose (scene, block range)
-// equals the previous lane's writes nothing: about one flag store per block
-// per warp instead of one per particle.
+// flags[scene*NB3 + block] = 1 for the 1, 2, 4 or 8 blocks of the stencil at base, by
+// one lane per group of equal cells (`mine`).  Plain byte stores: reading the flags
+// and appending the fresh blocks to the list from here made p2g 20 us slower (1.1M
+// particles, 102 against 85 us for the stores and 6 for k_list_blocks).
 template <typename T>
-MPM_DI void mark_stencil_blocks(const Consts<T>& c, bool ok, const int* base, int scene,
-                                unsigned char* __restrict__ flags) {
-  const int lane = threadIdx.x & 31;
-  int lo[3] = {0, 0, 0}, ext[3] = {0, 0, 0};
-  unsigned long long key = ~0ull;
-  if (ok) {
+MPM_DI void flag_blocks(const Consts<T>& c, bool mine, const int* base, int scene, unsigned char* __restrict__ flags) {
+  if (!mine) return;
+  int lo[3], ext[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = base[d] >> 2;
-      ext[d] = ((base[d] + 2) >> 2) - lo[d];  // 0 or 1
-    }
-    // n_grid <= 1024: block coordinates fit 9 bits
-    key = ((unsigned long long)scene << 30) | ((unsigned long long)lo[0] << 21) |
-          ((unsigned long long)lo[1] << 12) | ((unsigned long long)lo[2] << 3) |
-          (unsigned long long)(ext[0] << 2 | ext[1] << 1 | ext[2]);
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = base[d] >> 2;
+    ext[d] = ((base[d] + 2) >> 2) - lo[d];  // 0 or 1
   }
-  const unsigned long long prev = __shfl_up_sync(0xffffffffu, key, 1);
-  if (ok && (lane == 0 || prev != key)) {
-    // the 1, 2, 4 or 8 blocks (lo + {0, ext}) as predicated stores; the
-    // offset within a scene fits 32 bits (nb <= 256)
-    unsigned char* f = flags + (int64_t)scene * c.NB3;
-    const int nb = c.nb;
-    const int i0 = (lo[0] * nb + lo[1]) * nb + lo[2];
+  const int nb = c.nb;
+  unsigned char* f = flags + (int64_t)scene * c.NB3 + ((lo[0] * nb + lo[1]) * nb + lo[2]);
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int di = m >> 2, dj = (m >> 1) & 1, dk = m & 1;
-      if (di <= ext[0] && dj <= ext[1] && dk <= ext[2]) f[i0 + (di * nb + dj) * nb + dk] = 1;
-    }
+  for (int m = 0; m < 8; ++m) {
+    const int di = m >> 2, dj = (m >> 1) & 1, dk = m & 1;
+    if (di <= ext[0] && dj <= ext[1] && dk <= ext[2]) f[(di * nb + dj) * nb + dk] = 1;
   }
 }
 
 // ---------------------------------------------------------------------------
 // forward kernels
 // ---------------------------------------------------------------------------
+struct PoseTableArgs {
+  int n_tools;
+  const double *pose_f, *pose_f1;
+  void* poses;  // T[n_tools * 16]
+  int* counter;  // the list's length, emptied by the forward p2g
+};
+template <typename T>
+MPM_DI void pose_table_fill(const PoseTableArgs& a, int64_t i, int64_t stride) {
+  for (int64_t j = i; j < (int64_t)a.n_tools * 16; j += stride) {
+    const int64_t t = j >> 4;
+    const int k = (int)(j & 15);
+    static_cast<T*>(a.poses)[j] = T(k < 8 ? a.pose_f[8 * t + k] : a.pose_f1[8 * t + k - 8]);
+  }
+}
 // The particle of thread i of a scattering kernel.  order (may be null): a
 // permutation that sorts the particles by cell, for frames that are kept in the
 // caller's order; its load before a pdl_wait() goes to L2 (load_row_cg).  The rows
@@ -785,7 +795,7 @@ MPM_DI int64_t particle_of(const int* __restrict__ order, int64_t i, bool valid)
 template <typename T, typename S>
 MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restrict__ st_out,
                       const int* __restrict__ pscene, const int* __restrict__ order, Node<T>* __restrict__ grid,
-                      int64_t i) {
+                      unsigned char* __restrict__ flags, int64_t i) {
   const bool valid = i < c.n_particles;  // every lane stays for the warp's scatter
   const int64_t p = particle_of(order, i, valid);
   Stencil<T> s;
@@ -838,17 +848,14 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
   __shared__ typename ScatterStage<T>::type stage[kParticleThreads<S> / 32];  // one per warp
   auto* sb = &stage[threadIdx.x >> 5];
   const WarpRows rows = warp_rows(key, ok);
+  flag_blocks(c, ok && rows.first, s.base, scene, flags);
   if constexpr (sizeof(T) == 4) {
     __syncwarp();  // a strided caller's previous chunk has been read
     row_put(*sb, rows.row, pm, affine, s, A, g);
     __syncwarp();
-    pdl_wait();  // the grid blocks are zeroed by the compaction before
-    pdl_trigger();
     row_scatter<true>(*sb, rows.tails, rows.emit, c.p_mass);
   } else {
     slab_addresses(*sb, rows.row, A);
-    pdl_wait();
-    pdl_trigger();
     T cx[3] = {pm[0], pm[1], pm[2]};
 #pragma unroll 1
     for (int ox = 0; ox < 3; ++ox) {
@@ -883,27 +890,32 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
 // spill; measured 6 % faster than 6 CTAs); MB > 0 compiles the kernel for MB
 // CTAs per SM instead (the autotuner's candidates, MpmTuning.p2g_ctas).
 // Strided: the CTAs stride over the particle chunks (the adjoint's recompute,
-// which exits at once when the grid store holds the substep)
+// which exits at once when the grid store holds the substep; its poses were
+// converted by the restore)
 template <typename T, typename S, bool Strided = false, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 7 : 16)) k_p2g(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
                                              const int* __restrict__ pscene, const int* __restrict__ order,
-                                             Node<T>* __restrict__ grid, const int64_t* __restrict__ saved) {
-  if (saved && __ldcg(saved) >= 0) {  // the grid of this substep was restored from the grid store
-    pdl_wait();  // completes only after the kernel before it (dependent launches chain through it)
-    return;
-  }
+                                             Node<T>* __restrict__ grid, unsigned char* __restrict__ flags,
+                                             PoseTableArgs pt,
+                                             const int64_t* __restrict__ saved) {
+  pdl_wait();     // forward: the frame is g2p's output; adjoint: the restore comes before
+  pdl_trigger();
   if constexpr (Strided) {
+    if (saved && *saved >= 0) return;  // the grids of this substep were restored from the grid store
     for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x; p0 < c.n_particles; p0 += (int64_t)gridDim.x * blockDim.x)
-      p2g_chunk<T, S>(c, st, st_out, pscene, order, grid, p0 + threadIdx.x);
+      p2g_chunk<T, S>(c, st, st_out, pscene, order, grid, flags, p0 + threadIdx.x);
   } else {
-    p2g_chunk<T, S>(c, st, st_out, pscene, order, grid, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pose_table_fill<T>(pt, i, (int64_t)gridDim.x * blockDim.x);
+    if (i == 0) *pt.counter = 0;
+    p2g_chunk<T, S>(c, st, st_out, pscene, order, grid, flags, i);
   }
 }
 
 // Tools in the compute precision, for grid_op and grid_op.grad.  The tool
 // fields (primive_base.py:313-329) are converted once when the tools are set
 // (k_tools_convert: tools_t[i] = Tool<T> of descriptor i).  The poses of
-// frames f and f+1 are converted every substep by the block compaction
+// frames f and f+1 are converted every substep by p2g or the adjoint's restore
 // (poses_t[16 i + k]: k < 8 frame f, else frame f+1, one value per thread).
 // Both kernels read them straight from global memory: the lanes of a warp
 // load the same words (a broadcast), with no per-block staging, barrier or
@@ -913,19 +925,6 @@ __global__ void __launch_bounds__(128) k_tools_convert(int n, const MpmToolDesc*
                                                        Tool<T>* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) to_tool(tools[i], out[i]);
-}
-struct PoseTableArgs {
-  int n_tools;
-  const double *pose_f, *pose_f1;
-  void* poses;  // T[n_tools * 16]
-};
-template <typename T>
-MPM_DI void pose_table_fill(const PoseTableArgs& a, int64_t i, int64_t stride) {
-  for (int64_t j = i; j < (int64_t)a.n_tools * 16; j += stride) {
-    const int64_t t = j >> 4;
-    const int k = (int)(j & 15);
-    static_cast<T*>(a.poses)[j] = T(k < 8 ? a.pose_f[8 * t + k] : a.pose_f1[8 * t + k - 8]);
-  }
 }
 // the tools of one scene: tool[t], pose p0(t) at frame f, p1(t) at frame f+1
 template <typename T>
@@ -1017,22 +1016,40 @@ MPM_DI void walls_vjp(const Consts<T>& c, const int* I, const WallTape<T>& tp, T
   }
 }
 
+// Grid store: the forward grids of a substep (the active blocks of the p2g
+// grid and of the grid_op output) are kept so the adjoint substep restores
+// them instead of recomputing p2g and grid_op (copy in k_grid_op, restore in
+// k_restore).  Its free space is a bump counter, which all CTAs of grid_op read to
+// see where the substep's n blocks go (-1: the store is full, the adjoint then
+// recomputes); g2p, after them, moves it on and books the slot.
+MPM_DI int64_t store_room(const MpmGridStore& st, int n) {
+  const int64_t start = *st.bump;
+  return start + n <= st.capacity ? start : -1;
+}
+MPM_DI void store_book(const MpmGridStore& st, int slot, int n) {
+  const int64_t start = store_room(st, n);
+  st.slot_start[slot] = start;
+  st.slot_count[slot] = start >= 0 ? n : 0;
+  if (start >= 0) *st.bump = start + n;
+}
+
 // 1 / m of a node with mass (m > 1e-12)
 MPM_DI float node_rcp(float m) { return 1.f / m; }
 MPM_DI double node_rcp(double m) { return rcp64(m); }
 
 // grid_op over the active blocks: one 64-thread CTA per block, grid-stride.
 // store_slot >= 0: list block b of grid_in and of grid_out are also copied to
-// the grid store at slot_start + b (reserved by the compaction; -1 when the
+// the grid store at its next free block + b (g2p then books them; nothing when the
 // store is full).  saved (may be null; the adjoint's recompute): when it
 // points at a slot start >= 0 both grids were restored from the store and the
 // kernel returns at once.  FP32: at least 16 CTAs per SM (64 registers, a small
 // spill): with the grid-stride width of 16 CTAs per SM all of them are
 // resident at once (measured 9.8 -> 9.2 us on 32 scenes against 80 registers).
+// Adjoint (zero_b given): the block of zero_b (the velocity adjoint) is zeroed.
 template <typename T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<T> c, const int* __restrict__ active,
-                                                const int* __restrict__ n_active,
-                                                const Node<T>* __restrict__ grid_in, Node<T>* __restrict__ grid_out,
+                                                const int* __restrict__ n_active, Node<T>* __restrict__ grid_in,
+                                                Node<T>* __restrict__ grid_out, Node<T>* __restrict__ zero_b,
                                                 const Tool<T>* __restrict__ tools_t, const T* __restrict__ poses_t,
                                                 const int* __restrict__ tool_off, MpmGridStore store,
                                                 int store_slot, const int64_t* __restrict__ saved) {
@@ -1040,7 +1057,8 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<
   pdl_trigger();  // g2p reads its particle rows while the grid is updated
   if (saved && *saved >= 0) return;
   const int na = *n_active;
-  const int64_t start = store_slot >= 0 ? store.slot_start[store_slot] : -1;
+  const int64_t start = store_slot >= 0 ? store_room(store, na) : -1;
+  const Node<T> zero = {T(0), T(0), T(0), T(0)};
   for (int b = blockIdx.x; b < na; b += gridDim.x) {
     const int64_t gb = active[b];
     int I[3];
@@ -1048,6 +1066,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<
     const SceneToolView<T> sh(tools_t, poses_t, tool_off, scene);
     const int64_t idx = gb * 64 + threadIdx.x;
     Node<T> in = grid_in[idx];
+    if (zero_b) zero_b[idx] = zero;
     Node<T>* stored = start >= 0 ? reinterpret_cast<Node<T>*>(store.blocks) + ((start + b) << 7) : nullptr;
     if (stored) {
       stored[threadIdx.x] = in;
@@ -1147,33 +1166,27 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
   store_row(st_out, c.ld, p, 6, 9, nC);
   return true;
 }
-// mark (may be null; chained forward substeps): also flags the blocks the
-// stencils of the new positions touch, for the next substep, whose
-// compaction reads them instead of a marking pass; header[0..1] (list length,
-// reservation ticket) are reset for that substep.
+// Ends the substep's block bookkeeping: the listed blocks of the p2g grid are zeroed,
+// and one thread books what grid_op put into the grid store (store_slot >= 0).  The
+// next p2g empties the list.
 // At least MB CTAs of 128 threads per SM (MpmTuning.g2p_ctas; 0 = 8 in FP32:
 // at most 64 registers)
 template <typename T, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k_g2p(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
                                              const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
-                                             unsigned char* __restrict__ mark, int* __restrict__ header) {
+                                             const int* __restrict__ active, const int* __restrict__ counter,
+                                             Node<T>* __restrict__ grid_in, MpmGridStore store, int store_slot) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < c.n_particles;
   const int scene = valid ? __ldcg(pscene + p) : 0;  // issued with x
-  T xn[3] = {T(0), T(0), T(0)};
-  const bool moved = valid && g2p_particle(c, st, st_out, p, scene, grid, xn);
-  pdl_wait();  // grid_op reads the header reset below (and lanes without a stencil have not waited)
+  T xn[3];
+  if (valid) g2p_particle(c, st, st_out, p, scene, grid, xn);
+  pdl_wait();  // grid_op reads the counter (and lanes without a stencil have not waited)
   pdl_trigger();
-  if (mark) {  // uniform; all lanes take part in the warp's writer election
-    Stencil<T> sn;
-    zero_stencil(sn);
-    const bool ok = moved && make_stencil(c, xn, sn);
-    mark_stencil_blocks(c, ok, sn.base, scene, mark);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      header[0] = 0;
-      header[1] = 0;
-    }
-  }
+  const int na = *counter;
+  if (store_slot >= 0 && blockIdx.x == 0 && threadIdx.x == 0) store_book(store, store_slot, na);
+  for (int64_t i = p; i < (int64_t)na * 64; i += (int64_t)gridDim.x * blockDim.x)
+    grid_in[(int64_t)active[i >> 6] * 64 + (i & 63)] = Node<T>{T(0), T(0), T(0), T(0)};
 }
 
 // ---------------------------------------------------------------------------
@@ -1407,7 +1420,7 @@ MPM_DI T warp_reduce_scatter16(T (&v)[16], int& k) {
 template <typename T, int MB = 0>
 __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_grid_op_adj(Consts<T> c, const int* __restrict__ active,
                                                     const int* __restrict__ n_active,
-                                                    const Node<T>* __restrict__ grid_in,
+                                                    Node<T>* __restrict__ grid_in,
                                                     const Node<T>* __restrict__ g_grid, Node<T>* __restrict__ g_in,
                                                     const Tool<T>* __restrict__ tools_t,
                                                     const T* __restrict__ poses_t, const int* __restrict__ tool_off,
@@ -1422,6 +1435,7 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
     const SceneToolView<T> sh(tools_t, poses_t, tool_off, scene);
     const int64_t idx = gb * 64 + threadIdx.x;
     Node<T> in = grid_in[idx];
+    grid_in[idx] = Node<T>{T(0), T(0), T(0), T(0)};  // its last reader
     Node<T> go = g_grid[idx];
     const bool active_node = in.w > T(1e-12) && (go.x != T(0) || go.y != T(0) || go.z != T(0));
     const T p[3] = {T(I[0]) * c.dx, T(I[1]) * c.dx, T(I[2]) * c.dx};
@@ -1615,129 +1629,73 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
 }
 
 // ---------------------------------------------------------------------------
-// active-block bookkeeping
+// start of an adjoint substep
 // ---------------------------------------------------------------------------
-// Start of a substep's block bookkeeping, one launch:
-// - restore (when the grid store's slot holds this substep): the active list,
-//   its length, grid a (p2g) and grid a_out (grid_op output) come back from
-//   the store, and the same blocks of grid b (may be null) are zeroed;
-// - otherwise: the list length and the reservation ticket are reset, and
-//   flags[scene*NB3 + block] = 1 for every block a particle stencil touches
-//   (mark_stencil_blocks).  The flags are clean on entry (the compaction
-//   clears every flag it reads).
-// Grid-stride over warp-aligned ranges.
+// Converts the substep's tool poses, and when the grid store's slot holds the
+// substep, restores the active list, its length, grid a (p2g) and grid a_out
+// (grid_op output) and zeroes the same blocks of grid b (the velocity adjoint).
+// Otherwise it empties the list, for the p2g that follows.  Grid-stride.
 template <typename T>
-__global__ void __launch_bounds__(256) k_mark_or_restore(Consts<T> c, const T* __restrict__ st,
-                                                         const int* __restrict__ pscene,
-                                                         unsigned char* __restrict__ flags, int* __restrict__ header,
-                                                         MpmGridStore store, int slot, int* __restrict__ active,
-                                                         Node<T>* __restrict__ a, Node<T>* __restrict__ a_out,
-                                                         Node<T>* __restrict__ b) {
+__global__ void __launch_bounds__(256) k_restore(int* __restrict__ counter, MpmGridStore store, int slot,
+                                                 int* __restrict__ active, Node<T>* __restrict__ a,
+                                                 Node<T>* __restrict__ a_out, Node<T>* __restrict__ b,
+                                                 PoseTableArgs pt) {
   pdl_wait();
   pdl_trigger();
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  pose_table_fill<T>(pt, i0, stride);
   const int64_t start = slot >= 0 ? store.slot_start[slot] : -1;
-  if (start >= 0) {
-    const int cnt = store.slot_count[slot];
-    if (blockIdx.x == 0 && threadIdx.x == 0) header[0] = cnt;
-    const Node<T>* src = reinterpret_cast<const Node<T>*>(store.blocks);
-    const Node<T> z = {T(0), T(0), T(0), T(0)};
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)cnt * 64; i += stride) {
-      const int blk = store.block_ids[start + (i >> 6)];
-      if ((i & 63) == 0) active[i >> 6] = blk;
-      const Node<T>* sb = src + ((start + (i >> 6)) << 7) + (i & 63);
-      a[(int64_t)blk * 64 + (i & 63)] = sb[0];
-      if (a_out) a_out[(int64_t)blk * 64 + (i & 63)] = sb[64];
-      if (b) b[(int64_t)blk * 64 + (i & 63)] = z;
-    }
-    return;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    header[0] = 0;  // list length (the compaction's append counter)
-    header[1] = 0;  // reservation ticket
-  }
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p - (threadIdx.x & 31) < c.n_particles;
-       p += stride) {
-    bool ok = false;
-    int scene = 0;
-    Stencil<T> s;
-    zero_stencil(s);
-    if (p < c.n_particles) {
-      T x[3];
-      load_row(st, c.ld, p, 0, 3, x);
-      scene = pscene[p];  // issued with the x loads
-      ok = make_stencil(c, x, s);  // out-of-grid particles are skipped (and flagged) by the scatter
-    }
-    mark_stencil_blocks(c, ok, s.base, scene, flags);
+  const int cnt = start >= 0 ? store.slot_count[slot] : 0;
+  if (i0 == 0) *counter = cnt;
+  const Node<T>* src = reinterpret_cast<const Node<T>*>(store.blocks);
+  const Node<T> z = {T(0), T(0), T(0), T(0)};
+  for (int64_t i = i0; i < (int64_t)cnt * 64; i += stride) {
+    const int blk = store.block_ids[start + (i >> 6)];
+    if ((i & 63) == 0) active[i >> 6] = blk;
+    const Node<T>* sb = src + ((start + (i >> 6)) << 7) + (i & 63);
+    a[(int64_t)blk * 64 + (i & 63)] = sb[0];
+    a_out[(int64_t)blk * 64 + (i & 63)] = sb[64];
+    b[(int64_t)blk * 64 + (i & 63)] = z;
   }
 }
 
-// Grid store: the forward grids of a substep (the active blocks of the p2g
-// grid and of the grid_op output) are kept so the adjoint substep restores
-// them instead of recomputing p2g and grid_op (copy in k_grid_op, restore in
-// k_mark_or_restore).  One thread reserves room for n active blocks
-// of substep `slot` (bump allocator); slot_start = -1 when the store is full
-// (the adjoint then recomputes)
-MPM_DI void store_reserve(const MpmGridStore& st, int slot, int n) {
-  const unsigned long long start = atomicAdd(st.bump, (unsigned long long)n);
-  const bool fits = start + (unsigned long long)n <= (unsigned long long)st.capacity;
-  st.slot_start[slot] = fits ? (int64_t)start : -1;
-  st.slot_count[slot] = fits ? n : 0;
-}
-
-// List of flagged blocks (warp-aggregated append; order is not significant).
-// Every flag read is cleared, so the flags are clean for the next substep.
-// The appending warp zeroes its blocks in grids a and b (either may be null).
-// With reserve_slot >= 0 the last CTA to finish (threadfence + ticket, no
-// waiting) reserves room for the list in the grid store.  The threads also
-// convert the substep's tool poses (pose_table_fill).
+// The list of flagged blocks, in runs of consecutive blocks (the order of the runs is
+// not significant), and the flags cleared: 16 flags per thread.  saved (may be
+// null): nothing to do when the grid store held the substep.
 template <typename T>
-__global__ void __launch_bounds__(256) k_compact_clear(unsigned char* __restrict__ flags, int64_t total,
-                                                       int* __restrict__ active, int* __restrict__ counter,
-                                                       unsigned* __restrict__ ticket, Node<T>* __restrict__ a,
-                                                       Node<T>* __restrict__ b, const int64_t* __restrict__ saved,
-                                                       MpmGridStore store, int reserve_slot, PoseTableArgs pt) {
+__global__ void __launch_bounds__(128) k_list_blocks(unsigned char* __restrict__ flags, int64_t total,
+                                                     int* __restrict__ active, int* __restrict__ counter,
+                                                     const int64_t* __restrict__ saved) {
   pdl_wait();
   pdl_trigger();
+  if (saved && *saved >= 0) return;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  pose_table_fill<T>(pt, i, (int64_t)gridDim.x * blockDim.x);
-  if (saved && *saved >= 0) return;  // list and grid a restored; b zeroed by the restore
-  const bool f = i < total && flags[i] != 0;
-  if (f) flags[i] = 0;
-  unsigned m = __ballot_sync(0xffffffffu, f);
-  const int lane = threadIdx.x & 31;
-  if (m) {
-    const int leader = __ffs(m) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(counter, __popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (f) active[base + __popc(m & ((1u << lane) - 1u))] = (int)i;
-    const int64_t w0 = i - lane;
-    const Node<T> z = {T(0), T(0), T(0), T(0)};
-    while (m) {
-      const int k = __ffs(m) - 1;
-      m &= m - 1;
-      const int64_t node0 = (w0 + k) * 64;
+  const int64_t first = 16 * i;
+  uint4 f = make_uint4(0u, 0u, 0u, 0u);
+  if (first < total) {  // the flag buffer is padded to 16 bytes with zeros
+    uint4* at = reinterpret_cast<uint4*>(flags) + i;
+    f = *at;
+    if (f.x | f.y | f.z | f.w) *at = make_uint4(0u, 0u, 0u, 0u);
+  }
+  const unsigned w[4] = {f.x, f.y, f.z, f.w};  // bytes 0 or 1
+  int mine = 0;
 #pragma unroll
-      for (int l = 0; l < 64; l += 32) {
-        if (a) a[node0 + l + lane] = z;
-        if (b) b[node0 + l + lane] = z;
-      }
-    }
+  for (int k = 0; k < 4; ++k) mine += __popc(w[k]);
+  const int lane = threadIdx.x & 31;
+  int upto = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, upto, d);
+    if (lane >= d) upto += t;
   }
-  if (reserve_slot >= 0) {
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-      __threadfence();
-      store_reserve(store, reserve_slot, atomicAdd(counter, 0));
-    }
-  }
+  const int all = __shfl_sync(0xffffffffu, upto, 31);
+  if (all == 0) return;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(counter, all);
+  at = __shfl_sync(0xffffffffu, at, 0) + upto - mine;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    for (unsigned m = w[k]; m; m &= m - 1u) active[at++] = (int)(first + 4 * k + ((__ffs(m) - 1) >> 3));
 }
 
 // ---------------------------------------------------------------------------

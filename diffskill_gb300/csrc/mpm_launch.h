@@ -37,11 +37,11 @@ struct LaunchCtx {
   const int* tool_off;         // [n_scenes + 1] device
   int n_tools;
   unsigned int* status;        // sticky status word
-  void* grid_a;                // scratch grids, n_scenes*G nodes of 4 reals
+  void* grid_a;                // scratch grids, n_scenes*G nodes of 4 reals; grid_a is zero between substeps
   void* grid_b;                //   (block-contiguous layout, see mpm_kernels.cuh)
   void* grid_c;
   void* grid_d;
-  unsigned char* blockbuf;     // [16-byte counter header][n_scenes * NB3 block flags]
+  unsigned char* blockbuf;     // [16-byte header: list lengths][n_scenes * NB3 block flags], flags zero between substeps
   int* active;                 // [n_scenes * NB3] list of active blocks
   const void* tools_t;         // [n_tools] Tool<T>, converted when the tools are set (convert_tools)
   void* poses_t;               // [n_tools * 16] T: poses of frames f, f+1, converted every substep
@@ -129,18 +129,14 @@ cudaError_t convert_tools(int precision, int n, const MpmToolDesc* tools, void* 
 // bytes of the block-flag buffer (counter header + one flag per block)
 inline size_t blockbuf_bytes(int64_t n_scenes, int n_grid) {
   const int64_t nb = n_grid / 4;
-  return 16 + (size_t)(n_scenes * nb * nb * nb);
+  return 16 + (size_t)(n_scenes * nb * nb * nb + 15) / 16 * 16;  // the flags are read 16 at a time
 }
 
-// premarked: the block flags of st0 were set by the previous substep's g2p
-// (chained substeps), so the marking pass is skipped; mark_next: this
-// substep's g2p flags the blocks of st1 for the next substep
 template <typename T, typename S>
 cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const double* pose_f,
-                               const double* pose_f1, const MpmGridStore* store = nullptr, int slot = -1,
-                               bool premarked = false, bool mark_next = false);
+                               const double* pose_f1, const MpmGridStore* store = nullptr, int slot = -1);
 // The adjoint substep in three phases, which a caller may issue on two
-// streams: BWD_PREPARE (active blocks, pose table, the grids restored from the
+// streams: BWD_PREPARE (pose table, the active blocks and grids restored from the
 // store or recomputed), BWD_GRID (g2p.grad, grid_op.grad) and BWD_PARTICLES
 // (p2g.grad).  BWD_G2P_PLAIN launches g2p.grad without the programmatic
 // dependency on the kernel before it.

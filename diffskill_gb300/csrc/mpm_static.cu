@@ -14,9 +14,10 @@
 // The scratch is the file-scope array g_static_scratch below (20 MiB + 64 KiB).  Every GPU that
 // loads this library holds it until the process exits.  All calls share it
 // and it keeps the last call's contents: the tool table, the scratch status
-// word, the active-block flags and the grid blocks the scatter accumulates
-// into are rewritten or cleared on every call; the scene-index region is
-// zeroed once per device and never written afterwards.  Calls whose
+// word and the velocity grid are rewritten on every call, the active-block flags
+// and the grid the scatter accumulates into are zero between calls (every call
+// leaves them so; a failed one has them cleared by the next); the scene-index
+// region is zeroed once per device and never written afterwards.  Calls whose
 // kernels overlap on the GPU (different streams, or different host threads,
 // on the same device) race on the array; serialise them.
 //
@@ -44,7 +45,7 @@ namespace {
 //   [49152, +8 Tool<double>)    the tools in the compute precision
 //   [kPosesT, +8*16 doubles)     their poses at frames f, f+1 in the compute precision
 //   [kHeader, +kScene)          zero scene index of every particle
-//   [kHeader+kScene, +kGrids)   forward grid (mv, m) then velocity grid
+//   [kHeader+kScene, +kGrids)   forward grid (mv, m) in the first half, velocity grid in the second
 constexpr size_t kBlockBuf = 4096;
 constexpr size_t kActive = 16384;
 constexpr size_t kToolsT = 49152;
@@ -84,11 +85,11 @@ int scratch_base(int dev, unsigned char** out) {
       return set_err(MPM_E_CUDA, std::string("mpm_substep_fwd_static: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
     unsigned char* base = static_cast<unsigned char*>(p);
     e = cudaMemset(base + kHeader, 0, kScene);
-    // block flags start clean; every compaction clears the flags it reads
+    if (e == cudaSuccess) e = cudaMemset(base + kHeader + kScene, 0, kGrids / 2);
     if (e == cudaSuccess) e = cudaMemset(base + kBlockBuf, 0, 16 + kMaxBlocks);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess)
-      return set_err(MPM_E_CUDA, std::string("mpm_substep_fwd_static: clearing the scene index and block flags: ") +
+      return set_err(MPM_E_CUDA, std::string("mpm_substep_fwd_static: clearing the scratch: ") +
                                      cudaGetErrorString(e));
     g_base[dev] = base;
   }
@@ -198,11 +199,11 @@ int mpm_substep_fwd_static(const MpmParams* params, const MpmToolDesc* tools, in
   // the caller's status word when given (sticky: the caller clears it), else
   // the scratch word, which is cleared per call and not reported
   L.status = status ? reinterpret_cast<unsigned int*>(status) : reinterpret_cast<unsigned int*>(base);
-  L.grid_a = base + kHeader + kScene;              // active blocks cleared by the launcher before the scatter
-  L.grid_b = base + kHeader + kScene + grid_bytes;  // fully written by grid_op
+  L.grid_a = base + kHeader + kScene;               // zero between calls
+  L.grid_b = base + kHeader + kScene + kGrids / 2;  // written by grid_op
   L.grid_c = nullptr;
   L.grid_d = nullptr;
-  L.blockbuf = base + kBlockBuf;  // flags cleared once above, then by every compaction
+  L.blockbuf = base + kBlockBuf;  // zero between calls
   L.active = reinterpret_cast<int*>(base + kActive);
   L.tools_t = base + kToolsT;
   L.poses_t = base + kPosesT;
@@ -222,7 +223,11 @@ int mpm_substep_fwd_static(const MpmParams* params, const MpmToolDesc* tools, in
     default:
       e = mpm::launch_substep_fwd<double, double>(L, (const double*)state_f, (double*)state_f1, pose_f, pose_f1);
   }
-  if (e != cudaSuccess) return set_err(MPM_E_CUDA, std::string("mpm_substep_fwd_static: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_base[dev] = nullptr;  // the next call clears the scratch
+    return set_err(MPM_E_CUDA, std::string("mpm_substep_fwd_static: ") + cudaGetErrorString(e));
+  }
   return MPM_OK;
 }
 

@@ -196,10 +196,8 @@ class MpmEngine:
                    "mpm_tools_action_bwd")
 
     def set_chained(self, on: bool) -> None:
-        """Chained forward substeps (``mpm_set_chained``): each forward substep's
-        g2p flags the grid blocks of its output, and the next forward substep on
-        that frame skips its marking pass.  Only frames left unmodified between
-        substeps (up to the per-scene re-sort) may be chained."""
+        """Accepted and without effect (``mpm_set_chained``): no substep has a marking
+        pass to skip."""
         _lib.check(self.lib.mpm_set_chained(self.h, 1 if on else 0), self.h, "mpm_set_chained")
 
     def set_pipelined_adjoint(self, on: bool) -> None:
@@ -589,27 +587,21 @@ class Horizon:
         if store is not None:
             store.reset()
         cur = self.ckpt[0]
-        # each frame goes unmodified (up to the re-sort, a permutation within
-        # scenes) from one substep to the next: chain the substeps
-        eng.set_chained(True)
-        try:
-            for f in range(self.F):
-                if ready and f % n == 0:
-                    main.wait_event(ready[f // n])
-                if (f + 1) % self.k == 0:
-                    nxt = self.ckpt[(f + 1) // self.k]
-                else:
-                    nxt = self.seg[(f + 1) % 2]
-                if self.R and (f + 1) % self.R == 0 and f + 1 < self.F and eng.P:
-                    # a re-sort boundary: the substep writes the scratch frame, which is
-                    # sorted into the frame's place (the permutation kept for the adjoint)
-                    eng.substep(cur, self._tmp, self.pose[f], self.pose[f + 1], store, f)
-                    eng.sort_frame(self._tmp, nxt, self.perms[(f + 1) // self.R - 1])
-                else:
-                    eng.substep(cur, nxt, self.pose[f], self.pose[f + 1], store, f)
-                cur = nxt
-        finally:
-            eng.set_chained(False)
+        for f in range(self.F):
+            if ready and f % n == 0:
+                main.wait_event(ready[f // n])
+            if (f + 1) % self.k == 0:
+                nxt = self.ckpt[(f + 1) // self.k]
+            else:
+                nxt = self.seg[(f + 1) % 2]
+            if self.R and (f + 1) % self.R == 0 and f + 1 < self.F and eng.P:
+                # a re-sort boundary: the substep writes the scratch frame, which is
+                # sorted into the frame's place (the permutation kept for the adjoint)
+                eng.substep(cur, self._tmp, self.pose[f], self.pose[f + 1], store, f)
+                eng.sort_frame(self._tmp, nxt, self.perms[(f + 1) // self.R - 1])
+            else:
+                eng.substep(cur, nxt, self.pose[f], self.pose[f + 1], store, f)
+            cur = nxt
         if ready:
             main.wait_stream(self.side)
 

@@ -204,13 +204,8 @@ int mpm_substep_bwd(MpmHandle* h, const void* state_f, const void* state_f1, con
                     void* g_state_f, const double* pose_f, const double* pose_f1, double* g_pose_f,
                     double* g_pose_f1, void* stream);
 
-/* Chained forward substeps (on = 1; off by default).  While on, each forward
- * substep's g2p also flags the grid blocks of its output frame, and a forward
- * substep whose input frame is the previous forward substep's output skips
- * its own marking pass.  Contract: between two such substeps the frame is
- * not modified, except by a permutation of the particles within their scene
- * columns (the re-sort), which leaves the set of blocks unchanged.  Any
- * adjoint substep ends the chain.  No counterpart in the reference. */
+/* Accepted and without effect: every substep's p2g flags its own grid blocks, so
+ * there is no marking pass to skip between consecutive forward substeps. */
 int mpm_set_chained(MpmHandle* h, int32_t on);
 
 /* Pipelined adjoint substeps (on = 1; off by default).  While on, an
@@ -252,8 +247,7 @@ int mpm_substep_bwd_store(MpmHandle* h, const void* state_f, const void* state_f
  * Particles stay inside their scene, so losses and action gradients do not
  * change.  perm: int32[n_particles] (device, 4-byte aligned) receives the
  * permutation.  src and dst must not overlap.  Needs n_particles < 2^31 and
- * n_scenes * n_grid^3 < 2^32 (MPM_E_INVALID otherwise).  The block flags a
- * chained forward substep set for src are kept for dst.  No allocation;
+ * n_scenes * n_grid^3 < 2^32 (MPM_E_INVALID otherwise).  No allocation;
  * capturable. */
 int mpm_sort_frame(MpmHandle* h, const void* src, void* dst, int32_t* perm, void* stream);
 /* Adjoint of mpm_sort_frame for a frame gradient: g_dst[:, perm[i]] =
