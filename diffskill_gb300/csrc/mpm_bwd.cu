@@ -30,13 +30,14 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
   const unsigned gb = grid_blocks_launch(L, (int64_t)c.n_scenes * c.NB3);
   const Tool<T>* tools_t = (const Tool<T>*)L.tools_t;
   const T* poses_t = (const T*)L.poses_t;
+  const void* kept = store ? store->blocks : nullptr;
+  const int64_t* saved = store ? store->slot_start + slot : nullptr;
   if (phases & BWD_PREPARE) {
     // the grids of this substep come from the grid store, or are recomputed
     // (substep_grad, mpm_simulator.py:327-333); then p2g and grid_op return at once
-    const int64_t* saved = store ? store->slot_start + slot : nullptr;
-    const PoseTableArgs pt{L.n_tools, pose_f, pose_f1, L.poses_t, nullptr};
+    const PoseTableArgs pt{L.n_tools, pose_f, pose_f1, L.poses_t};
     MPM_LAUNCH_PDL(L, MPM_K_CLEAR, k_restore<T>, store ? (unsigned)(L.sm_count * 8) : 1u, 256, counter,
-                   store ? *store : MpmGridStore{}, store ? slot : -1, L.active, gin, gout, g_gout, pt);
+                   store ? *store : MpmGridStore{}, store ? slot : -1, L.active, gout, g_gout, pt);
     if (c.n_particles > 0) {
       // with a grid store the recompute usually exits at once: a grid of one
       // wave of CTAs that stride over the particles
@@ -83,17 +84,17 @@ cudaError_t launch_substep_bwd(const LaunchCtx& L, const T* st0, const T* st1, c
     if constexpr (sizeof(T) == 4) {
       if (v == 12)
         MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, (k_grid_op_adj<T, 12>), gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin,
-                       tools_t, poses_t, L.tool_off, g_pose_f, g_pose_f1);
+                       tools_t, poses_t, L.tool_off, kept, saved, g_pose_f, g_pose_f1);
       else if (v == 16)
         MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, (k_grid_op_adj<T, 16>), gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin,
-                       tools_t, poses_t, L.tool_off, g_pose_f, g_pose_f1);
+                       tools_t, poses_t, L.tool_off, kept, saved, g_pose_f, g_pose_f1);
       else
         MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, k_grid_op_adj<T>, gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin,
-                       tools_t, poses_t, L.tool_off, g_pose_f, g_pose_f1);
+                       tools_t, poses_t, L.tool_off, kept, saved, g_pose_f, g_pose_f1);
     } else {
       (void)v;
       MPM_LAUNCH_PDL(L, MPM_K_GRID_OP_ADJ, k_grid_op_adj<T>, gb, 64, c, active, (const int*)counter, gin, g_gout, g_gin, tools_t,
-                     poses_t, L.tool_off, g_pose_f, g_pose_f1);
+                     poses_t, L.tool_off, kept, saved, g_pose_f, g_pose_f1);
     }
   }
   if ((phases & BWD_PARTICLES) && c.n_particles > 0) {

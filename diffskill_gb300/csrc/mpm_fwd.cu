@@ -51,7 +51,7 @@ Consts<T> make_consts(const LaunchCtx& L) {
 template Consts<float> make_consts<float>(const LaunchCtx&);
 template Consts<double> make_consts<double>(const LaunchCtx&);
 
-// The list length has a word of its own for the forward substep (p2g empties it) and
+// The list length has a word of its own for the forward substep (g2p empties it) and
 // for the adjoint (k_restore does): with a pipelined adjoint the next
 // substep's list begins before this one's last kernel ends.
 int* list_counter(const LaunchCtx& L, bool adjoint) { return reinterpret_cast<int*>(L.blockbuf) + (adjoint ? 1 : 0); }
@@ -101,7 +101,7 @@ cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const d
   {
     constexpr int bs = kParticleThreads<S>;
     const unsigned pb = blocks_for(c.n_particles, bs);
-    const PoseTableArgs pt{L.n_tools, pose_f, pose_f1, L.poses_t, counter};
+    const PoseTableArgs pt{L.n_tools, pose_f, pose_f1, L.poses_t};
     // FP32: the CTAs-per-SM variant the tuning selects
     const int v = sizeof(S) == 4 ? L.tune.p2g_ctas : 0;
 #define MPM_P2G(KERNEL) \
@@ -129,7 +129,7 @@ cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const d
     const unsigned pb = blocks_for(c.n_particles, bs);
     const int v = sizeof(T) == 4 ? L.tune.g2p_ctas : 0;
 #define MPM_G2P(KERNEL) \
-  MPM_LAUNCH_PDL(L, MPM_K_G2P, KERNEL, pb, bs, c, st0, st1, L.pscene, gout, (const int*)L.active, (const int*)counter, gin, keep, keep_slot)
+  MPM_LAUNCH_PDL(L, MPM_K_G2P, KERNEL, pb, bs, c, st0, st1, L.pscene, gout, counter, keep, keep_slot)
     if constexpr (sizeof(T) == 4) {
       if (v == 10)
         MPM_G2P((k_g2p<T, 10>));

@@ -20,15 +20,15 @@
 // and flags the blocks that particle stencils touch, k_list_blocks turns the flags
 // into a device-side list and clears them, grid_op and grid_op.grad run over that
 // list with grid-stride loops (no host round trip; capturable in a CUDA graph), and
-// a kernel after the p2g grid's last reader zeroes its listed blocks (g2p forward,
-// grid_op.grad itself in the adjoint).  So no pass over the particles only marks
-// blocks and none only clears the grid.  One substep of 64 scenes (1.1M particles,
-// 32 us of compulsory traffic): with the marking in g2p and a compaction that also
-// clears, p2g 82, grid_op 14, g2p 48, clear 8 us; now 85, 14, 39 and 7.  The zeroing
-// is in g2p because that kernel waits for latency and has bandwidth to spare (+2 us);
-// in grid_op, which is bound by bandwidth, it cost 12.  Nodes outside the list hold
-// no mass, so grid_op leaves them at zero exactly as the dense reference does; g2p
-// and p2g.grad only read nodes inside the list.
+// the p2g grid's last reader zeroes its listed blocks (grid_op forward, grid_op.grad
+// in the adjoint).  So no pass over the particles only marks blocks and none only
+// clears the grid.  One substep of 64 scenes (1.1M particles, 32 us of compulsory
+// traffic): with the marking in g2p and a compaction that also clears, p2g 82,
+// grid_op 14, g2p 48, clear 8 us; now 85, 14, 37 and 7.  Both kernels store the zeros
+// last: next to the load of the same node they cost grid_op 12 us and grid_op.grad
+// 12 (34 against 22).  Nodes outside the list hold no mass, so grid_op leaves them at
+// zero exactly as the dense reference does; g2p and p2g.grad only read nodes inside
+// the list.
 #pragma once
 #include "../../include/mpm_gb300.h"
 #include "mpm_math.cuh"
@@ -772,7 +772,6 @@ struct PoseTableArgs {
   int n_tools;
   const double *pose_f, *pose_f1;
   void* poses;  // T[n_tools * 16]
-  int* counter;  // the list's length, emptied by the forward p2g
 };
 template <typename T>
 MPM_DI void pose_table_fill(const PoseTableArgs& a, int64_t i, int64_t stride) {
@@ -907,7 +906,6 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
   } else {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     pose_table_fill<T>(pt, i, (int64_t)gridDim.x * blockDim.x);
-    if (i == 0) *pt.counter = 0;
     p2g_chunk<T, S>(c, st, st_out, pscene, order, grid, flags, i);
   }
 }
@@ -1045,7 +1043,8 @@ MPM_DI double node_rcp(double m) { return rcp64(m); }
 // kernel returns at once.  FP32: at least 16 CTAs per SM (64 registers, a small
 // spill): with the grid-stride width of 16 CTAs per SM all of them are
 // resident at once (measured 9.8 -> 9.2 us on 32 scenes against 80 registers).
-// Adjoint (zero_b given): the block of zero_b (the velocity adjoint) is zeroed.
+// The block's nodes of grid_in are zeroed at the end; in the adjoint (zero_b given),
+// where grid_op.grad still reads grid_in, those of zero_b (the velocity adjoint).
 template <typename T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<T> c, const int* __restrict__ active,
                                                 const int* __restrict__ n_active, Node<T>* __restrict__ grid_in,
@@ -1066,7 +1065,6 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<
     const SceneToolView<T> sh(tools_t, poses_t, tool_off, scene);
     const int64_t idx = gb * 64 + threadIdx.x;
     Node<T> in = grid_in[idx];
-    if (zero_b) zero_b[idx] = zero;
     Node<T>* stored = start >= 0 ? reinterpret_cast<Node<T>*>(store.blocks) + ((start + b) << 7) : nullptr;
     if (stored) {
       stored[threadIdx.x] = in;
@@ -1086,6 +1084,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 1) k_grid_op(Consts<
     }
     grid_out[idx] = out;
     if (stored) stored[64 + threadIdx.x] = out;
+    (zero_b ? zero_b : grid_in)[idx] = zero;
   }
 }
 
@@ -1166,16 +1165,14 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
   store_row(st_out, c.ld, p, 6, 9, nC);
   return true;
 }
-// Ends the substep's block bookkeeping: the listed blocks of the p2g grid are zeroed,
-// and one thread books what grid_op put into the grid store (store_slot >= 0).  The
-// next p2g empties the list.
+// One thread ends the substep's block bookkeeping: it books what grid_op put into the
+// grid store (store_slot >= 0) and empties the list.
 // At least MB CTAs of 128 threads per SM (MpmTuning.g2p_ctas; 0 = 8 in FP32:
 // at most 64 registers)
 template <typename T, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k_g2p(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
                                              const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
-                                             const int* __restrict__ active, const int* __restrict__ counter,
-                                             Node<T>* __restrict__ grid_in, MpmGridStore store, int store_slot) {
+                                             int* __restrict__ counter, MpmGridStore store, int store_slot) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < c.n_particles;
   const int scene = valid ? __ldcg(pscene + p) : 0;  // issued with x
@@ -1183,10 +1180,10 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
   if (valid) g2p_particle(c, st, st_out, p, scene, grid, xn);
   pdl_wait();  // grid_op reads the counter (and lanes without a stencil have not waited)
   pdl_trigger();
-  const int na = *counter;
-  if (store_slot >= 0 && blockIdx.x == 0 && threadIdx.x == 0) store_book(store, store_slot, na);
-  for (int64_t i = p; i < (int64_t)na * 64; i += (int64_t)gridDim.x * blockDim.x)
-    grid_in[(int64_t)active[i >> 6] * 64 + (i & 63)] = Node<T>{T(0), T(0), T(0), T(0)};
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (store_slot >= 0) store_book(store, store_slot, *counter);
+    *counter = 0;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1415,6 +1412,9 @@ MPM_DI T warp_reduce_scatter16(T (&v)[16], int& k) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// When saved points at a slot start >= 0 (the grid store holds the substep), the p2g
+// grid's nodes are read from the store and grid_in, which was not restored, stays
+// zero; else grid_in's listed blocks are zeroed here, by their last reader.
 // At least MB CTAs of 64 threads per SM (MpmTuning.grid_op_adj_ctas; 0 = 6:
 // at most 168 registers)
 template <typename T, int MB = 0>
@@ -1424,18 +1424,21 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
                                                     const Node<T>* __restrict__ g_grid, Node<T>* __restrict__ g_in,
                                                     const Tool<T>* __restrict__ tools_t,
                                                     const T* __restrict__ poses_t, const int* __restrict__ tool_off,
+                                                    const void* __restrict__ kept, const int64_t* __restrict__ saved,
                                                     double* __restrict__ g_pose_f, double* __restrict__ g_pose_f1) {
   pdl_wait();     // g_grid is g2p.grad's output
   pdl_trigger();  // p2g.grad recomputes its particles' stress meanwhile
   const int na = *n_active;
+  const int64_t start = saved ? *saved : -1;
   for (int b = blockIdx.x; b < na; b += gridDim.x) {
     const int64_t gb = active[b];
     int I[3];
     const int scene = block_node(c, gb, threadIdx.x, I);
     const SceneToolView<T> sh(tools_t, poses_t, tool_off, scene);
     const int64_t idx = gb * 64 + threadIdx.x;
-    Node<T> in = grid_in[idx];
-    grid_in[idx] = Node<T>{T(0), T(0), T(0), T(0)};  // its last reader
+    const Node<T>* from =
+        start >= 0 ? reinterpret_cast<const Node<T>*>(kept) + ((start + b) << 7) + threadIdx.x : grid_in + idx;
+    const Node<T> in = *from;
     Node<T> go = g_grid[idx];
     const bool active_node = in.w > T(1e-12) && (go.x != T(0) || go.y != T(0) || go.z != T(0));
     const T p[3] = {T(I[0]) * c.dx, T(I[1]) * c.dx, T(I[2]) * c.dx};
@@ -1478,6 +1481,7 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
       res.w = -(g[0] * in.x + g[1] * in.y + g[2] * in.z) * inv * inv;
     }
     g_in[idx] = res;
+    if (start < 0) grid_in[idx] = Node<T>{T(0), T(0), T(0), T(0)};
   }
 }
 
@@ -1632,13 +1636,14 @@ __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) 
 // start of an adjoint substep
 // ---------------------------------------------------------------------------
 // Converts the substep's tool poses, and when the grid store's slot holds the
-// substep, restores the active list, its length, grid a (p2g) and grid a_out
-// (grid_op output) and zeroes the same blocks of grid b (the velocity adjoint).
+// substep, restores the active list, its length and grid a_out (grid_op output) and
+// zeroes the same blocks of grid b (the velocity adjoint); grid_op.grad, the one
+// reader of the p2g grid, takes that from the store (an iteration of 64 scenes,
+// 1.1M particles: 35.9 -> 34.7 ms, restoring it too cost 10 us a substep).
 // Otherwise it empties the list, for the p2g that follows.  Grid-stride.
 template <typename T>
 __global__ void __launch_bounds__(256) k_restore(int* __restrict__ counter, MpmGridStore store, int slot,
-                                                 int* __restrict__ active, Node<T>* __restrict__ a,
-                                                 Node<T>* __restrict__ a_out, Node<T>* __restrict__ b,
+                                                 int* __restrict__ active, Node<T>* __restrict__ a_out, Node<T>* __restrict__ b,
                                                  PoseTableArgs pt) {
   pdl_wait();
   pdl_trigger();
@@ -1653,7 +1658,6 @@ __global__ void __launch_bounds__(256) k_restore(int* __restrict__ counter, MpmG
     const int blk = store.block_ids[start + (i >> 6)];
     if ((i & 63) == 0) active[i >> 6] = blk;
     const Node<T>* sb = src + ((start + (i >> 6)) << 7) + (i & 63);
-    a[(int64_t)blk * 64 + (i & 63)] = sb[0];
     a_out[(int64_t)blk * 64 + (i & 63)] = sb[64];
     b[(int64_t)blk * 64 + (i & 63)] = z;
   }
