@@ -11,8 +11,10 @@
 //                         Primitive.get_collision_idx / collision_projection
 //                         (primive_base.py:135-150) and Box._project (primitives.py:370-372)
 //
-// One warp per scene: lane t runs the kinematics of the scene's tool t, then
-// the warp evaluates each collision pair's 600 surface points together.  The
+// One warp per scene.  A scene without collision pairs and rolling pins: eight lanes
+// per tool, one per component of its pose (ToolLane).  Any other: lane t runs the
+// kinematics of the scene's tool t, then the warp evaluates each collision pair's 600
+// surface points together.  The
 // adjoint follows the reference's autodiff: apply_collision_projection.grad and
 // set_surface_points.grad run before forward_kinematics.grad of the substep,
 // read the poses of frame f+1 as stored after the projection, and take the
@@ -309,6 +311,204 @@ MPM_DI void project_frame_vjp(const MpmToolDesc* __restrict__ tools, int t0, int
   __syncwarp();
 }
 
+// ---------------------------------------------------------------------------
+// Eight lanes per tool.  The substeps of an action are one chain per tool, and a warp
+// issues an FP64 operation every 64 cycles whatever the number of its lanes, so the
+// chain's length in operations is its time: a lane per tool takes some 45 a substep
+// forward and 100 backward, a lane per component 14 and 30.  The pose stays in
+// registers from one substep to the next, and the adjoint's loads are issued one
+// substep ahead (19 substeps: forward 45 -> 25 us, adjoint 118 -> 53; 50 substeps of
+// 64 scenes: 116 -> 59 and 316 -> 126).
+// Lane k of a tool holds pose component k < 3: position, 3: gap, 4 + c: quaternion c.
+// A product with the action's quaternion w is, for component c,
+//   o_c = sum_j m[j] r_{c^j}   and its adjoint   gr_c = sum_j n[j] go_{c^j},
+// m[j], n[j] = +-w[j], so the other components come from shuffles within four lanes.
+// ---------------------------------------------------------------------------
+struct ToolLane {
+  int t, k;          // tool and component
+  bool mine;         // the tool exists
+  int kind;          // bounds: 0 none, 1 position, 2 gap, 3 gap from below
+  double lo, hi;
+  bool right;        // the rotation is applied on the right
+  MPM_DI int pose_at() const { return k < 3 ? k : k == 3 ? 7 : k - 1; }
+  MPM_DI int vel_at() const { return k < 3 ? k : k == 3 ? 6 : k == 4 ? 7 : k - 2; }
+};
+MPM_DI ToolLane tool_lane(const MpmToolDesc* __restrict__ tools, int t0, int nt, int first) {
+  const int lane = threadIdx.x & 31, i = first + (lane >> 3);
+  ToolLane L;
+  L.k = lane & 7;
+  L.mine = i < nt;
+  L.t = t0 + (L.mine ? i : 0);
+  const MpmToolDesc& d = tools[L.t];
+  const int type = d.type;
+  L.right = right_rotation(type);
+  L.kind = 0;
+  L.lo = -INFINITY;
+  L.hi = INFINITY;
+  if (L.k < 3) {
+    L.kind = 1;
+    L.lo = d.lower[L.k];
+    L.hi = d.upper[L.k];
+  } else if (L.k == 3 && has_gap_vel(type)) {
+    L.kind = type == TOOL_CHOPSTICKS ? 3 : 2;
+    L.lo = d.min_gap;
+    if (L.kind == 2) L.hi = d.max_gap;
+  }
+  return L;
+}
+// clamp_pos and the gap's bounds: the value a is kept (pass) or replaced by a bound
+MPM_DI double bounded(const ToolLane& L, double a, bool& pass) {
+  const bool pos = L.kind == 1;
+  const double x = pos ? L.hi : L.lo, y = pos ? L.lo : L.hi;
+  const bool c1 = (pos ? a : x) < (pos ? x : a);
+  const double r = c1 ? a : x;
+  const bool c2 = (pos ? y : r) < (pos ? r : y);
+  pass = c1 && (c2 || L.kind == 3);
+  return c2 ? r : y;
+}
+// the velocity of component vel_at() (action_velocity)
+MPM_DI double lane_velocity(const ToolLane& L, const MpmToolDesc& d, const double* a, int n_sub) {
+  const int v = L.vel_at();
+  const bool on = d.action_dim > 0 && (v < 3 || (v < 6 && d.action_dim > 3) || (v == 6 && has_gap_vel(d.type)));
+  return on ? a[v] * d.action_scale[v] / n_sub : 0.0;
+}
+MPM_DI double flip(double a, bool minus) { return minus ? -a : a; }
+// m (and n) of this lane's component for the action's quaternion of velocity w
+// (lanes 5..7 of the tool hold it)
+MPM_DI void lane_rotation(const ToolLane& L, double v, double* w, double* m, double* n) {
+  const int base = threadIdx.x & 24;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) w[j] = __shfl_sync(0xffffffffu, v, base + 5 + j);
+  double q[4];
+  w2quat(w, q);
+  const int c = L.k & 3;
+  const bool R = L.right;
+  // bit c: the sign of m[j], n[j] is minus (left; right flips components 1..3 against 1..3)
+  m[0] = n[0] = q[0];
+  m[1] = flip(q[1], c == 0 || (c == 2 && !R) || (c == 3 && R));
+  m[2] = flip(q[2], c == 0 || (c == 3 && !R) || (c == 1 && R));
+  m[3] = flip(q[3], c == 0 || (c == 1 && !R) || (c == 2 && R));
+  n[1] = flip(q[1], c == 1 || (c == 3 && !R) || (c == 2 && R));
+  n[2] = flip(q[2], c == 2 || (c == 1 && !R) || (c == 3 && R));
+  n[3] = flip(q[3], c == 3 || (c == 2 && !R) || (c == 1 && R));
+}
+MPM_DI double quad_sum(double a) {
+  a += __shfl_xor_sync(0xffffffffu, a, 1);
+  return a + __shfl_xor_sync(0xffffffffu, a, 2);
+}
+// sum_j m[j] r_{c^j}
+MPM_DI double quad_product(const double* m, double r) {
+  double o = m[0] * r;
+#pragma unroll
+  for (int j = 1; j < 4; ++j) o += m[j] * __shfl_xor_sync(0xffffffffu, r, j);
+  return o;
+}
+
+MPM_DI void lanes_action(const MpmToolDesc* __restrict__ tools, int t0, int nt, int n_tools,
+                         const double* __restrict__ action, double* __restrict__ vel, double* pose, int n_sub) {
+  for (int first = 0; first < nt; first += 4) {
+    const ToolLane L = tool_lane(tools, t0, nt, first);
+    const double v = L.mine ? lane_velocity(L, tools[L.t], action + 8 * L.t, n_sub) : 0.0;
+    double w[3], m[4], n[4];
+    lane_rotation(L, v, w, m, n);
+    const double dv = L.k == 3 ? -v : v;
+    double* at = pose + (int64_t)L.t * 8 + L.pose_at();
+    double* vat = vel + (int64_t)L.t * 8 + L.vel_at();
+    const int64_t row = (int64_t)n_tools * 8;
+    double p = L.mine ? *at : 0.0;
+    for (int s = 0; s < n_sub; ++s) {
+      const double o = quad_product(m, p);
+      const double q = o * inv_len(quad_sum(o * o));
+      bool pass;
+      const double a = bounded(L, p + dv, pass);
+      p = L.k > 3 ? q : L.kind ? a : p;
+      at += row;
+      if (L.mine) {
+        *vat = v;
+        *at = p;
+      }
+      vat += row;
+    }
+  }
+}
+
+MPM_DI void lanes_action_bwd(const MpmToolDesc* __restrict__ tools, int t0, int nt, int n_tools,
+                             const double* __restrict__ vel, const double* __restrict__ pose, double* g_pose,
+                             double* __restrict__ g_action, int n_sub) {
+  const int base = threadIdx.x & 24;
+  const int64_t row = (int64_t)n_tools * 8;
+  for (int first = 0; first < nt; first += 4) {
+    const ToolLane L = tool_lane(tools, t0, nt, first);
+    const int c = L.k & 3;
+    const bool R = L.right;
+    const bool minus[4] = {c != 0, (c == 3 && !R) || (c == 2 && R), (c == 1 && !R) || (c == 3 && R),
+                           (c == 2 && !R) || (c == 1 && R)};
+    const double* pat = pose + (int64_t)L.t * 8 + L.pose_at();
+    const double* vat = vel + (int64_t)L.t * 8 + L.vel_at();
+    double* gat = g_pose + (int64_t)L.t * 8 + L.pose_at();
+    const auto load = [&](const double* a, int s) { return L.mine && s >= 0 ? a[s * row] : 0.0; };
+    double g = load(gat, n_sub);  // adjoint of frame s + 1
+    double p = load(pat, n_sub - 1), v = load(vat, n_sub - 1), held = load(gat, n_sub - 1);
+    // w2quat and its adjoint once per run of substeps with the same angular velocity
+    double v_run = v, gv = 0.0, gw = 0.0, w[3], m[4], n[4];
+    lane_rotation(L, v, w, m, n);
+    const auto end_run = [&]() {
+      double gq[4], gaa[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) gq[j] = __shfl_sync(0xffffffffu, gw, base + 4 + j);
+      w2quat_vjp(w, gq, gaa);
+      if (L.k > 4) gv += L.k == 5 ? gaa[0] : L.k == 6 ? gaa[1] : gaa[2];
+      gw = 0.0;
+    };
+    for (int s = n_sub - 1; s >= 0; --s) {
+      const double p_next = load(pat, s - 1), v_next = load(vat, s - 1), held_next = load(gat, s - 1);
+      if (__any_sync(0xffffffffu, L.k > 4 && __double_as_longlong(v) != __double_as_longlong(v_run))) {
+        end_run();  // of every tool in the warp: a run may be summed in parts
+        lane_rotation(L, v, w, m, n);
+        v_run = v;
+      }
+      const double o = quad_product(m, p);
+      const double iL = inv_len(quad_sum(o * o));
+      const double on = quad_sum(o * g) * iL * iL;
+      const double go = (g - o * on) * iL;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double r = __shfl_xor_sync(0xffffffffu, p, j);  // r_{c^j}
+        gw += __shfl_sync(0xffffffffu, go, base + 4 + j) * flip(r, minus[j]);
+      }
+      const double gr = quad_product(n, go);
+      bool pass;
+      bounded(L, L.k == 3 ? p - v : p + v, pass);
+      double g0 = gr;
+      if (L.k < 4) {
+        g0 = L.kind == 0 || pass ? g : 0.0;
+        if (L.kind && pass) gv += L.k == 3 ? -g : g;
+      }
+      // frame s gets this step's contribution by an atomic add: frame 0 of the action is
+      // also the last frame of the action before, whose MPM adjoint may be adding pose
+      // gradients to it at the same time
+      if (L.mine && g0 != 0.0) atomicAdd(gat + s * row, g0);
+      g = held + g0;
+      p = p_next;
+      v = v_next;
+      held = held_next;
+    }
+    end_run();
+    if (L.mine) {
+      // set_velocity.grad: v = a * scale / n_sub for every substep of the action
+      const MpmToolDesc& d = tools[L.t];
+      const int i = L.vel_at();
+      const bool on = d.action_dim > 0 && (i < 3 || (i < 6 && d.action_dim > 3) || (i == 6 && has_gap_vel(d.type)));
+      if (on) g_action[8 * L.t + i] += gv * d.action_scale[i] / n_sub;
+    }
+  }
+}
+// no lane needs the whole pose of a tool
+MPM_DI bool by_component(const MpmToolDesc* __restrict__ tools, int t0, int nt, int np) {
+  const int lane = threadIdx.x & 31;
+  return np == 0 && !__any_sync(0xffffffffu, lane < nt && rolling_pin(tools[t0 + lane].type));
+}
+
 __global__ void k_tools_action(const MpmToolDesc* __restrict__ tools, const int* __restrict__ tool_off,
                                const int* __restrict__ pair_off, int n_scenes, int n_tools, int n_pairs,
                                const double* __restrict__ coll_pts, const double* __restrict__ action,
@@ -318,6 +518,10 @@ __global__ void k_tools_action(const MpmToolDesc* __restrict__ tools, const int*
   const int lane = threadIdx.x & 31;
   const int t0 = tool_off[scene], nt = tool_off[scene + 1] - t0;
   const int np = pair_off[scene + 1] - pair_off[scene];
+  if (by_component(tools, t0, nt, np)) {
+    lanes_action(tools, t0, nt, n_tools, action, vel, pose, n_sub);
+    return;
+  }
   const bool mine = lane < nt;
   MpmToolDesc d;
   double vv[8], wq[4] = {1, 0, 0, 0};
@@ -349,6 +553,10 @@ __global__ void k_tools_action_bwd(const MpmToolDesc* __restrict__ tools, const 
   const int lane = threadIdx.x & 31;
   const int t0 = tool_off[scene], nt = tool_off[scene + 1] - t0;
   const int np = pair_off[scene + 1] - pair_off[scene];
+  if (by_component(tools, t0, nt, np)) {
+    lanes_action_bwd(tools, t0, nt, n_tools, vel, pose, g_pose, g_action, n_sub);
+    return;
+  }
   const bool mine = lane < nt;
   const int t = t0 + lane;
   MpmToolDesc d;
