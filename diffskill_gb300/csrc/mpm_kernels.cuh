@@ -381,13 +381,6 @@ MPM_DI T sel3(T a0, T a1, T a2, int i) {
   return i == 0 ? a0 : (i == 1 ? a1 : a2);
 }
 template <typename T>
-MPM_DI void add3(T& a0, T& a1, T& a2, int i, T v) {
-  a0 += i == 0 ? v : T(0);
-  a1 += i == 1 ? v : T(0);
-  a2 += i == 2 ? v : T(0);
-}
-
-template <typename T>
 MPM_DI long long cell_key(const Consts<T>& c, int scene, const Stencil<T>& s) {
   return (long long)scene * c.G + ((long long)s.base[0] * c.n_grid + s.base[1]) * c.n_grid + s.base[2];
 }

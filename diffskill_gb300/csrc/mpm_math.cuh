@@ -20,10 +20,6 @@ MPM_DI double msqrt(double x) { return sqrt(x); }
 // exp and log of the return map (log of singular values near 1, exp of the
 // projected strains): the accurate library functions.  __logf's error near 1
 // is absolute (about 2^-21), i.e. hundreds of ulp of a strain of 1e-3.
-MPM_DI float mexp(float x) { return expf(x); }
-MPM_DI double mexp(double x) { return exp(x); }
-MPM_DI float mlog(float x) { return logf(x); }
-MPM_DI double mlog(double x) { return log(x); }
 // log(1 + x) and exp(x) - 1 for the FP32 strains (x = s - 1 of a singular
 // value, or a projected log-strain), accurate to the result's own precision:
 // for |x| < 1/64 by their Taylor series (truncation below 3e-12 and 2e-13
@@ -103,19 +99,6 @@ template <typename T>
 MPM_DI T det3(const T* A) {
   return A[0] * (A[4] * A[8] - A[5] * A[7]) - A[1] * (A[3] * A[8] - A[5] * A[6]) +
          A[2] * (A[3] * A[7] - A[4] * A[6]);
-}
-// cofactor matrix = d det / d A
-template <typename T>
-MPM_DI void cof3(const T* A, T* Cf) {
-  Cf[0] = A[4] * A[8] - A[5] * A[7];
-  Cf[1] = A[5] * A[6] - A[3] * A[8];
-  Cf[2] = A[3] * A[7] - A[4] * A[6];
-  Cf[3] = A[2] * A[7] - A[1] * A[8];
-  Cf[4] = A[0] * A[8] - A[2] * A[6];
-  Cf[5] = A[1] * A[6] - A[0] * A[7];
-  Cf[6] = A[1] * A[5] - A[2] * A[4];
-  Cf[7] = A[2] * A[3] - A[0] * A[5];
-  Cf[8] = A[0] * A[4] - A[1] * A[3];
 }
 
 // FP64 arithmetic from FP32 starting values.  GB300 issues one FP64
