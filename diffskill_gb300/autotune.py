@@ -54,8 +54,8 @@ FP32_ONLY = ("p2g_ctas", "g2p_adj_ctas", "p2g_adj_ctas", "g2p_ctas", "grid_op_ad
 @dataclass
 class Tuning:
     p2g_ctas: int = 7
-    g2p_adj_ctas: int = 6
-    p2g_adj_ctas: int = 5
+    g2p_adj_ctas: int = 8
+    p2g_adj_ctas: int = 4
     grid_ctas_per_sm: int = 16
     g2p_ctas: int = 8
     grid_op_adj_ctas: int = 6
