@@ -213,12 +213,18 @@ MPM_DI WarpRows warp_rows(long long key, bool ok) {
 // run three times per substep and diverged over the row groups: 2,850 instructions
 // per warp in p2g and 2,288 in g2p.grad, now 2,225 and 1,760 (1.1M particles: p2g 128
 // to 81 us, g2p.grad 136 to 86).
+constexpr int kStagedGroups = 7;
 struct RowStage {
-  float4 q0[32];       // u.x, u.y, G00, G10
-  float4 q1[32];       // G01, G11, G02, G12
-  float4 q2[32];       // u.z, G20, G21, G22
-  float wyz[32][9];
-  float wx[32][4];
+  union {
+    struct {
+      float4 q0[32];  // u.x, u.y, G00, G10
+      float4 q1[32];  // G01, G11, G02, G12
+      float4 q2[32];  // u.z, G20, G21, G22
+      float wyz[32][9];
+      float wx[32][4];
+    };
+    float4 nodes[kStagedGroups][27];  // g2p.grad, before: the nodes that a group gathers
+  };
   Node<float>* base[32];  // grid of the row's scene
   int off[32][12];        // ax[3], ay[3], az[3] of the row's stencil
 };
@@ -232,8 +238,7 @@ MPM_DI float2 fma2(float2 a, float2 b, float2 c) {
   return f2_of(d);
 }
 // row r of the stage: the lane's particle (u, G row-major)
-MPM_DI void row_put(RowStage& sb, int r, const float* u, const float* G, const Stencil<float>& s, const StencilAddr& A,
-                    Node<float>* grid) {
+MPM_DI void row_put(RowStage& sb, int r, const float* u, const float* G, const Stencil<float>& s) {
   sb.q0[r] = make_float4(u[0], u[1], G[0], G[3]);
   sb.q1[r] = make_float4(G[1], G[4], G[2], G[5]);
   sb.q2[r] = make_float4(u[2], G[6], G[7], G[8]);
@@ -242,6 +247,8 @@ MPM_DI void row_put(RowStage& sb, int r, const float* u, const float* G, const S
 #pragma unroll
     for (int oz = 0; oz < 3; ++oz) sb.wyz[r][oy * 3 + oz] = s.w[oy][1] * s.w[oz][2];
   *reinterpret_cast<float4*>(sb.wx[r]) = make_float4(s.w[0][0], s.w[1][0], s.w[2][0], 0.f);
+}
+MPM_DI void row_addresses(RowStage& sb, int r, const StencilAddr& A, Node<float>* grid) {
   sb.base[r] = grid;
   int4* off = reinterpret_cast<int4*>(sb.off[r]);
   off[0] = make_int4(A.ax[0], A.ax[1], A.ax[2], A.ay[0]);
@@ -843,7 +850,8 @@ MPM_DI void p2g_chunk(const Consts<T>& c, const T* __restrict__ st, T* __restric
   flag_blocks(c, ok && rows.first, s.base, scene, flags);
   if constexpr (sizeof(T) == 4) {
     __syncwarp();  // a strided caller's previous chunk has been read
-    row_put(*sb, rows.row, pm, affine, s, A, g);
+    row_addresses(*sb, rows.row, A, g);
+    row_put(*sb, rows.row, pm, affine, s);
     __syncwarp();
     row_scatter<true>(*sb, rows.tails, rows.emit, c.p_mass);
   } else {
@@ -1186,11 +1194,11 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) 
 // g_grid
 // st1 (frame f+1, may be null): its v rows are the g2p output, so the clamp
 // mask needs no second gather of the grid.
-// FP32: 8 CTAs of 128 threads per SM by default (64 registers, 48 B of spill): it
-// waits on its gathers (1.1M particles: 5, 6, 7, 8 CTAs 95.6, 90.8, 89.3, 86.3 us);
+// FP32: 8 CTAs of 128 threads per SM by default (64 registers, 60 B of spill): it
+// waits on its gathers (1.1M particles: 5, 6, 7, 8 CTAs 94.1, 88.3, 83.7, 83.4 us);
 // MB > 0: MB CTAs per SM (MpmTuning.g2p_adj_ctas)
 template <typename T, int MB = 0>
-__global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ st1,
+__global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 8)) k_g2p_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ st1,
                                                  const T* __restrict__ g1, T* __restrict__ g0,
                                                  const int* __restrict__ pscene, const int* __restrict__ order,
                                                  bool add, const Node<T>* __restrict__ grid,
@@ -1280,10 +1288,15 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_ad
     ux[i] = gnv[i] - (gC[3 * i] * s.fx[0] + gC[3 * i + 1] * s.fx[1] + gC[3 * i + 2] * s.fx[2]);
   }
   // weight adjoints h(o) = gv(o) . u(o), summed axis by axis against the weights
-  // and their derivatives; the 27 gathers of the grid velocity come in one
-  // unrolled loop before the scatter, which then touches no global memory but
-  // its atomics
-  if (ok) {
+  // and their derivatives; the gathers of the grid velocity come before the scatter,
+  // which then touches no global memory but its atomics.  FP32: the L1's wavefronts
+  // bound the gathers (76 % of their peak; 27 loads of 16 B per lane from some 12
+  // lines each), and the lanes of one cell read the same nodes, so 27 lanes fetch a
+  // cell's nodes once into the row stage and the lanes read them there: 1.1M
+  // particles 85.4 -> 83.4 us, 0.8M 64.7 -> 61.5, 30,000 19.6 -> 16.4.  A warp of more
+  // cells than the stage holds gathers for itself (a loop over the cells, one copy of
+  // the arithmetic, kept more registers live: 89.7 us)
+  const auto gather = [&](auto&& node) {
     T dw[3][3];
     stencil_derivatives(s, dw);
     T sx = T(0), sy = T(0), sz = T(0);
@@ -1298,7 +1311,7 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_ad
         T l0 = T(0), lz = T(0);
 #pragma unroll
         for (int oz = 0; oz < 3; ++oz) {
-          const Node<T> n = g[A.at(ox, oy, oz)];
+          const Node<T> n = node(ox, oy, oz);
           const T gv[3] = {n.x, n.y, n.z};
           const T h = dot3(gv, vz);
           l0 += s.w[oz][2] * h;
@@ -1321,9 +1334,50 @@ __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : 8) k_g2p_ad
     gfx[0] += sx;
     gfx[1] += sy;
     gfx[2] += sz;
+  };
+  if constexpr (sizeof(T) == 4) {
+    row_addresses(*sb, rows.row, A, gg);
+    __syncwarp();
+    if (__popc(rows.emit) <= kStagedGroups) {  // the same for the whole warp
+      const int lane = threadIdx.x & 31, node = lane < 27 ? lane : 26;
+      const int ox = node / 9, oy = node / 3 % 3, oz = node % 3;
+      unsigned m = rows.emit;
+      for (int b = 0; b < kStagedGroups && m; b += 4) {
+        float4 v[4];
+        unsigned left = m;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {  // four loads in flight
+          if (left) {
+            const int r = __ffs(left) - 1;
+            left &= left - 1u;
+            v[k] = *reinterpret_cast<const float4*>(grid + (sb->base[r] - g_grid) +
+                                                    (sb->off[r][ox] + sb->off[r][3 + oy] + sb->off[r][6 + oz]));
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (m) {
+            m &= m - 1u;
+            if (lane < 27) sb->nodes[b + k][lane] = v[k];
+          }
+        }
+      }
+      __syncwarp();
+      const float4* mine = sb->nodes[ok ? __popc(rows.emit & ((1u << rows.row) - 1u)) : 0];
+      if (ok)
+        gather([&](int ax, int ay, int az) {
+          const float4 v = mine[9 * ax + 3 * ay + az];
+          return Node<T>{v.x, v.y, v.z, v.w};
+        });
+      __syncwarp();
+    } else if (ok) {
+      gather([&](int ax, int ay, int az) { return g[A.at(ax, ay, az)]; });
+    }
+  } else if (ok) {
+    gather([&](int ax, int ay, int az) { return g[A.at(ax, ay, az)]; });
   }
   if constexpr (sizeof(T) == 4) {
-    row_put(*sb, rows.row, ux, gC, s, A, gg);
+    row_put(*sb, rows.row, ux, gC, s);
     __syncwarp();
     row_scatter<false>(*sb, rows.tails, rows.emit, 0.f);
   } else {

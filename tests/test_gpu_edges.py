@@ -138,3 +138,27 @@ def test_forward_of_extreme_deformations(gpu_lib, prec, tol):
     got = s1[:, :sc.n_particles].double().cpu().numpy().T
     for k, sl in GROUPS.items():
         assert rel_err(got[:, sl], ref[:, sl]) < tol, k
+
+
+# one cell per warp, as many as g2p.grad stages, one more, and a cell per lane
+@pytest.mark.parametrize("cells", [1, 4, 7, 8, 32])
+def test_adjoint_by_cells_per_warp(gpu_lib, cells):
+    """FP32, at the tolerance of the substep's adjoint test; a ragged last warp."""
+    n, sc = 101, small_scene(n=101, tools=[], precision="fp32")
+    rng, dx = np.random.default_rng(cells), sc.sim.dx
+    cell = np.arange(n) % cells
+    corner = np.stack([cell % 4, cell // 4 % 4, cell // 16], -1) * 2 + 24
+    x = (corner + 0.5 + rng.uniform(0.05, 0.95, (n, 3))) * dx
+    st = perturbed_state(x.astype(np.float32).astype(np.float64), seed=4)
+    eng, o = MpmEngine(sc.sim, [[]], [n]), Oracle(sc.sim, [])
+    g1 = rng.normal(size=st.shape)
+    zero = np.zeros((1, 8))
+    ref = o.substep_bwd(zero, zero, st, g1, np.zeros((1, 8)), np.zeros((1, 8)))
+    pose = torch.zeros((4, 1, 8), dtype=torch.float64, device=eng.device)
+    s0, s1, gg1, gg0 = _soa(eng, st), eng.new_state(), _soa(eng, g1), eng.new_state()
+    eng.substep(s0, s1, pose[0], pose[1])
+    eng.substep_bwd(s0, gg1, gg0, pose[0], pose[1], pose[2], pose[3], st1=s1)
+    torch.cuda.synchronize()
+    got = gg0[:, :n].double().cpu().numpy().T
+    for k, sl in GROUPS.items():
+        assert rel_err(got[:, sl], ref[:, sl]) < 2e-4, k
