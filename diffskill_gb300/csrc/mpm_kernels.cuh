@@ -1102,23 +1102,10 @@ MPM_DI void line_sums(const Stencil<T>& s, const Node<T>& n0, const Node<T>& n1,
   }
 }
 
-// g2p of particle p (mpm_simulator.py:265-284): writes rows 0..14 of st_out
-// and xn; returns false (the state copied unchanged) for a particle whose
-// stencil left the grid
-template <typename T>
-MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __restrict__ st_out, int64_t p, int scene,
-                         const Node<T>* __restrict__ grid, T* xn) {
-  T x[3];
-  load_row_cg(st, c.ld, p, 0, 3, x);
-  Stencil<T> s;
-  if (!make_stencil(c, x, s)) {  // flagged by k_p2g; the particle keeps its state
-#pragma unroll
-    for (int k = 0; k < 15; ++k) st_out[(int64_t)k * c.ld + p] = __ldcg(st + (int64_t)k * c.ld + p);
-    return false;
-  }
-  const Node<T>* g = grid + (int64_t)scene * c.G;
-  const StencilAddr A = stencil_addr(c, s);
-  pdl_wait();  // the grid is grid_op's output
+// sums of g2p over the stencil's nodes, node(ox, oy, oz); writes rows 0..14 and xn
+template <typename T, typename F>
+MPM_DI void g2p_sums(const Consts<T>& c, T* __restrict__ st_out, int64_t p, const T* x, const Stencil<T>& s, F&& node,
+                     T* xn) {
   // C = k4 sum_o wgt v(o) (o - fx)^T = k4 (m1 - nv fx^T) with m1 = sum_o wgt v(o) o^T,
   // summed axis by axis (line_sums): per component 24 operations on each of the 9
   // lines along z and 12 on each plane, where a sum over nodes took 12 per node
@@ -1131,7 +1118,7 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
     T p0[3] = {T(0), T(0), T(0)}, py[3] = {T(0), T(0), T(0)}, pz[3] = {T(0), T(0), T(0)};
 #pragma unroll
     for (int oy = 0; oy < 3; ++oy) {
-      const Node<T> n0 = g[A.at(ox, oy, 0)], n1 = g[A.at(ox, oy, 1)], n2 = g[A.at(ox, oy, 2)];
+      const Node<T> n0 = node(ox, oy, 0), n1 = node(ox, oy, 1), n2 = node(ox, oy, 2);
       T l0[3], l1[3];
       line_sums(s, n0, n1, n2, l0, l1);
       const T wy = s.w[oy][1];
@@ -1164,21 +1151,111 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
   store_row(st_out, c.ld, p, 0, 3, xn);
   store_row(st_out, c.ld, p, 3, 3, nv);
   store_row(st_out, c.ld, p, 6, 9, nC);
+}
+
+// g2p of particle p (mpm_simulator.py:265-284): writes rows 0..14 of st_out
+// and xn; returns false (the state copied unchanged) for a particle whose
+// stencil left the grid
+template <typename T>
+MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __restrict__ st_out, int64_t p, int scene,
+                         const Node<T>* __restrict__ grid, T* xn) {
+  T x[3];
+  load_row_cg(st, c.ld, p, 0, 3, x);
+  Stencil<T> s;
+  if (!make_stencil(c, x, s)) {  // flagged by k_p2g; the particle keeps its state
+#pragma unroll
+    for (int k = 0; k < 15; ++k) st_out[(int64_t)k * c.ld + p] = __ldcg(st + (int64_t)k * c.ld + p);
+    return false;
+  }
+  const Node<T>* g = grid + (int64_t)scene * c.G;
+  const StencilAddr A = stencil_addr(c, s);
+  pdl_wait();  // the grid is grid_op's output
+  g2p_sums(c, st_out, p, x, s, [&](int ox, int oy, int oz) { return g[A.at(ox, oy, oz)]; }, xn);
   return true;
+}
+// FP32, one gather of the nodes per cell of a warp, as in g2p.grad: the lanes of a cell
+// find each other by __match_any_sync, 27 lanes fetch the cell's nodes, all read them
+// from shared memory.  For launches of more than one wave, where the L1's wavefronts
+// bound the gathers (1.1M particles 36.6 -> 34.3 us, 0.8M 28.6 -> 26.6); smaller ones
+// wait for one warp's chain, which the grouping makes longer (30,000 particles in the
+// caller's order 8.3 -> 9.6 us), so they gather lane by lane.
+struct GatherStage {
+  float4 nodes[kStagedGroups][27];
+  const Node<float>* base[kStagedGroups];
+  int off[kStagedGroups][9];
+};
+MPM_DI void g2p_warp(const Consts<float>& c, const float* __restrict__ st, float* __restrict__ st_out, int64_t p, bool valid,
+                     int scene, const Node<float>* __restrict__ grid, GatherStage& sb) {
+  float x[3] = {0.f, 0.f, 0.f}, xn[3];
+  if (valid) load_row_cg(st, c.ld, p, 0, 3, x);
+  Stencil<float> s;
+  zero_stencil(s);
+  const bool ok = valid && make_stencil(c, x, s);
+  if (valid && !ok) {
+#pragma unroll
+    for (int k = 0; k < 15; ++k) st_out[(int64_t)k * c.ld + p] = __ldcg(st + (int64_t)k * c.ld + p);
+  }
+  const Node<float>* g = grid + (int64_t)scene * c.G;
+  if (!ok) zero_stencil(s);
+  const StencilAddr A = stencil_addr(c, s);
+  const int lane = threadIdx.x & 31;
+  const unsigned peers = __match_any_sync(0xffffffffu, ok ? cell_key(c, scene, s) : -1 - (long long)lane);
+  const int first = __ffs(peers) - 1;
+  const unsigned leaders = __ballot_sync(0xffffffffu, ok && lane == first);
+  const int ng = __popc(leaders);
+  pdl_wait();
+  if (ng <= kStagedGroups) {
+    const int mine = __popc(leaders & ((1u << first) - 1u));
+    if (ok && lane == first) {
+      sb.base[mine] = g;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        sb.off[mine][k] = A.ax[k];
+        sb.off[mine][3 + k] = A.ay[k];
+        sb.off[mine][6 + k] = A.az[k];
+      }
+    }
+    __syncwarp();
+    const int node = lane < 27 ? lane : 26, ox = node / 9, oy = node / 3 % 3, oz = node % 3;
+    for (int b = 0; b < ng; b += 4) {
+      float4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (b + k < ng)
+          v[k] = *reinterpret_cast<const float4*>(sb.base[b + k] +
+                                                  (sb.off[b + k][ox] + sb.off[b + k][3 + oy] + sb.off[b + k][6 + oz]));
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (b + k < ng && lane < 27) sb.nodes[b + k][lane] = v[k];
+    }
+    __syncwarp();
+    if (ok)
+      g2p_sums(c, st_out, p, x, s, [&](int ax, int ay, int az) {
+        const float4 v = sb.nodes[mine][9 * ax + 3 * ay + az];
+        return Node<float>{v.x, v.y, v.z, v.w};
+      }, xn);
+  } else if (ok) {
+    g2p_sums(c, st_out, p, x, s, [&](int ox, int oy, int oz) { return g[A.at(ox, oy, oz)]; }, xn);
+  }
 }
 // One thread ends the substep's block bookkeeping: it books what grid_op put into the
 // grid store (store_slot >= 0) and empties the list.
 // At least MB CTAs of 128 threads per SM (MpmTuning.g2p_ctas; 0 = 8 in FP32:
 // at most 64 registers)
-template <typename T, int MB = 0>
+template <typename T, int MB = 0, bool Shared = false>
 __global__ void __launch_bounds__(kParticleThreads<T>, MB > 0 ? MB : (sizeof(T) == 4 ? 8 : 1)) k_g2p(Consts<T> c, const T* __restrict__ st, T* __restrict__ st_out,
                                              const int* __restrict__ pscene, const Node<T>* __restrict__ grid,
                                              int* __restrict__ counter, MpmGridStore store, int store_slot) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < c.n_particles;
   const int scene = valid ? __ldcg(pscene + p) : 0;  // issued with x
-  T xn[3];
-  if (valid) g2p_particle(c, st, st_out, p, scene, grid, xn);
+  if constexpr (Shared) {
+    __shared__ GatherStage stage[kParticleThreads<T> / 32];
+    g2p_warp(c, st, st_out, p, valid, scene, grid, stage[threadIdx.x >> 5]);
+  } else {
+    T xn[3];
+    if (valid) g2p_particle(c, st, st_out, p, scene, grid, xn);
+  }
   pdl_wait();  // grid_op reads the counter (and lanes without a stencil have not waited)
   pdl_trigger();
   if (blockIdx.x == 0 && threadIdx.x == 0) {

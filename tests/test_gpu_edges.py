@@ -162,3 +162,33 @@ def test_adjoint_by_cells_per_warp(gpu_lib, cells):
     got = gg0[:, :n].double().cpu().numpy().T
     for k, sl in GROUPS.items():
         assert rel_err(got[:, sl], ref[:, sl]) < 2e-4, k
+
+
+@pytest.mark.parametrize("sort", [True, False])
+def test_g2p_shared_gathers_equal_lane_gathers(gpu_lib, sort):
+    """More particles than a wave of CTAs holds (8 x 128 per SM), a ragged last warp and one
+    particle outside the grid: the default shape shares its gathers within a cell, 10 CTAs
+    per SM gather lane by lane.  Unsorted, most warps hold more cells than fit.  The two
+    runs' grids differ in the order of their FP32 sums (1e-7; 1e-6 relative in C)."""
+    from diffskill_gb300 import autotune
+
+    n = 8 * 128 * torch.cuda.get_device_properties(0).multi_processor_count + 77
+    sc = small_scene(n=64, tools=[], precision="fp32")
+    eng = MpmEngine(sc.sim, [[]], [n])
+    rng = np.random.default_rng(1)
+    st0 = _soa(eng, perturbed_state(rng.uniform(0.3, 0.5, (n, 3)), seed=1))
+    st0[0, 5] = 7.0
+    if sort:
+        by_cell, perm = eng.new_state(), torch.empty(n, dtype=torch.int32, device=eng.device)
+        eng.sort_frame(st0, by_cell, perm)
+        st0 = by_cell
+    pose = torch.zeros((1, 8), dtype=torch.float64, device=eng.device)
+    outs = []
+    for ctas in (8, 10):
+        autotune.apply(eng, autotune.Tuning(g2p_ctas=ctas))
+        st1 = eng.new_state()
+        eng.substep(st0, st1, pose, pose)
+        outs.append(st1[:, :n].double())
+    torch.cuda.synchronize()
+    for sl in GROUPS.values():
+        assert float((outs[0][sl] - outs[1][sl]).abs().max()) <= 1e-5 * float(outs[1][sl].abs().max())
