@@ -9,6 +9,7 @@
 #include <string>
 #include <vector>
 
+#include "mpm_done.h"
 #include "mpm_launch.h"
 #include "mpm_math.cuh"
 #include "mpm_tools.cuh"
@@ -42,8 +43,8 @@ struct MpmHandle {
   void* d_tools_t = nullptr;  // tools in the compute precision (converted by mpm_set_tools)
   void* d_poses_t = nullptr;  // poses of the current substep in the compute precision
   mpm::SortScratch sort;      // particle re-sort (mpm_sort_frame)
-  int* d_order = nullptr;     // particles by cell for the substeps of mpm_substeps_fwd / _bwd
-  bool ordered = false;       // d_order holds a permutation
+  int* d_order = nullptr;     // particles by cell for the substeps of mpm_substeps_fwd / _bwd; always a permutation
+  mpm::Done ordered;          // d_order was sorted
   // pipelined adjoint (mpm_set_pipelined_adjoint): the grid preparation of an
   // adjoint substep runs on pipe_side beside the previous substep's p2g.grad
   bool pipelined = false;
@@ -129,6 +130,16 @@ mpm::LaunchCtx ctx(MpmHandle* h, void* stream) {
   L.prof = &h->prof;
   L.tune = h->tune;
   return L;
+}
+// the capture that work submitted to the stream is recorded in (0: none, it runs)
+unsigned long long capture_of(void* stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &st, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return st == cudaStreamCaptureStatusActive ? id : 0;
 }
 int check_device(MpmHandle* h) {
   int dev = -1;
@@ -227,6 +238,8 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
   // the p2g grid and the block flags start at zero; every substep leaves them so
   ok = ok && cudaMemset(h->d_blockbuf, 0, bbytes) == cudaSuccess;
   ok = ok && cudaMemset(h->grid[0], 0, gbytes) == cudaSuccess;
+  // the order of runs is a permutation before any sort has run
+  ok = ok && mpm::launch_identity_order(p.n_particles, h->d_order, nullptr) == cudaSuccess;
   // the pipelined adjoint's internal stream and events (created here, outside any stream capture)
   ok = ok && cudaStreamCreateWithFlags(&h->pipe_side, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&h->pipe_grid_done, cudaEventDisableTiming) == cudaSuccess;
@@ -637,7 +650,8 @@ int check_sortable(MpmHandle* h, const char* fn) {
 // 30,000 624 / 821 and 541 / 787, 100,000 1,670 / 1,439 and 869 / 1,269; FP64 8,000
 // 1,717 / 3,435 and 1,702 / 3,430, 16,000 2,089 / 3,624 and 1,867 / 3,566.  An
 // adjoint run takes the order of the last forward run: any permutation is right,
-// and a particle seldom changes its cell within an action.
+// and a particle seldom changes its cell within an action.  It sorts for itself when
+// no run has, or only one in another capture, which may never be replayed.
 static bool run_ordered(const MpmHandle* h, int32_t n) {
   const size_t bytes = (size_t)24 * (size_t)h->p.ld * real_size(h->p.precision);
   const int64_t least = h->p.precision == MPM_PREC_FP64 ? 12000 : 20000;
@@ -650,7 +664,7 @@ static int sort_run(MpmHandle* h, const void* frame, void* stream) {
                             ? mpm::launch_sort_order<double>(L, (const double*)frame, h->d_order, h->sort)
                             : mpm::launch_sort_order<float>(L, (const float*)frame, h->d_order, h->sort);
   if (e != cudaSuccess) return cuda_fail(h, e, "particle order");
-  h->ordered = true;
+  h->ordered.mark(capture_of(stream));
   return MPM_OK;
 }
 
@@ -697,7 +711,7 @@ int mpm_substeps_bwd(MpmHandle* h, const void* frames, void* g_frames, const dou
   const size_t frame = (size_t)24 * (size_t)h->p.ld * real_size(h->p.precision);
   const size_t pose = (size_t)8 * (size_t)(h->n_tools > 0 ? h->n_tools : 1);
   const int* order = run_ordered(h, n) ? h->d_order : nullptr;
-  if (order && !h->ordered) MPM_TRY(sort_run(h, frames, stream));
+  if (order && !h->ordered.holds(capture_of(stream))) MPM_TRY(sort_run(h, frames, stream));
   // no forward substep in between: each one's grid preparation runs beside the
   // p2g.grad of the one before (mpm_set_pipelined_adjoint)
   const bool pipelined = h->pipelined;

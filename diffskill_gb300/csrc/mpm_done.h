@@ -1,0 +1,22 @@
+// Whether work that later calls of a handle rely on has been done.
+#pragma once
+
+namespace mpm {
+
+// Work submitted to a stream is done for every later call.  Work recorded in a stream
+// capture is done for the calls of the same capture only: the graph may be discarded,
+// or replayed at any later time.  Captures are told apart by CUDA's capture id (0: no
+// capture).
+struct Done {
+  bool run = false;
+  unsigned long long recorded = 0;
+  bool holds(unsigned long long capture) const { return run || (capture != 0 && capture == recorded); }
+  void mark(unsigned long long capture) {
+    if (capture != 0)
+      recorded = capture;
+    else
+      run = true;
+  }
+};
+
+}  // namespace mpm

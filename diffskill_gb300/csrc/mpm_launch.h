@@ -116,6 +116,8 @@ cudaError_t launch_sort_frame(const LaunchCtx& L, const T* src, T* dst, int32_t*
 // the permutation of launch_sort_frame alone
 template <typename T>
 cudaError_t launch_sort_order(const LaunchCtx& L, const T* src, int32_t* perm, const SortScratch& s);
+// order[i] = i
+cudaError_t launch_identity_order(int64_t n, int* order, cudaStream_t s);
 template <typename T>
 cudaError_t launch_unsort_frame(const LaunchCtx& L, const T* src, T* dst, const int32_t* perm);
 

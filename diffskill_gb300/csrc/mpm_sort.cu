@@ -244,6 +244,15 @@ cudaError_t launch_sort_order(const LaunchCtx& L, const T* src, int32_t* perm, c
   return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256) k_identity_order(int64_t n, int* __restrict__ order) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) order[i] = (int)i;
+}
+cudaError_t launch_identity_order(int64_t n, int* order, cudaStream_t s) {
+  if (n > 0) k_identity_order<<<blocks_of(n, 256), 256, 0, s>>>(n, order);
+  return cudaGetLastError();
+}
+
 template <typename T>
 cudaError_t launch_sort_frame(const LaunchCtx& L, const T* src, T* dst, int32_t* perm, const SortScratch& s) {
   const MpmParams& p = *L.p;

@@ -1,0 +1,39 @@
+"""Host-side rules of the native library that need no GPU: compiled from its headers."""
+from __future__ import annotations
+
+import os
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+DONE = r"""
+#include "mpm_done.h"
+#define CHECK(x) if (!(x)) return __LINE__
+int main() {
+  mpm::Done d;
+  CHECK(!d.holds(0) && !d.holds(7));
+  d.mark(7);  // recorded in capture 7, which may never run
+  CHECK(d.holds(7) && !d.holds(0) && !d.holds(8));
+  d.mark(8);
+  CHECK(d.holds(8) && !d.holds(7) && !d.holds(0));
+  d.mark(0);  // ran: for every later call, in a capture or not
+  CHECK(d.holds(0) && d.holds(8) && d.holds(9));
+  d.mark(9);
+  CHECK(d.holds(0) && d.holds(10));
+  return 0;
+}
+"""
+
+
+def _run(tmp_path, source):
+    """0, or the line of the first check that fails."""
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text(source)
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-I", os.path.join(ROOT, "diffskill_gb300", "csrc"), str(src), "-o",
+                    str(exe)], check=True)
+    return subprocess.run([str(exe)]).returncode
+
+
+def test_recorded_work_is_done_for_its_own_capture_only(tmp_path):
+    """What a capture only recorded must not count as done for a call outside it."""
+    assert _run(tmp_path, DONE) == 0
