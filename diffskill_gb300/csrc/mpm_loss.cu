@@ -349,7 +349,10 @@ MPM_DI unsigned cluster_size() {
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
+// (.aligned: the warp's threads execute it together, so those that come from a branch
+// meet first)
 MPM_DI void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

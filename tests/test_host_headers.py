@@ -1,7 +1,9 @@
 """Host-side rules of the native library that need no GPU: compiled from its headers."""
 from __future__ import annotations
 
+import glob
 import os
+import re
 import subprocess
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -37,3 +39,17 @@ def _run(tmp_path, source):
 def test_recorded_work_is_done_for_its_own_capture_only(tmp_path):
     """What a capture only recorded must not count as done for a call outside it."""
     assert _run(tmp_path, DONE) == 0
+
+
+def test_aligned_cluster_barriers_follow_a_warp_barrier():
+    """barrier.cluster.*.aligned is undefined unless all threads of the warp execute it
+    together, and nothing but a warp barrier brings them together after a branch: each
+    arrive has one directly before it (the wait follows the arrive)."""
+    arrives = 0
+    for path in glob.glob(os.path.join(ROOT, "diffskill_gb300", "csrc", "*.cu*")):
+        code = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"barrier\.cluster\.arrive[.a-z]*\.aligned", code):
+            arrives += 1
+            before = code[:code.rfind("asm", 0, m.start())].rstrip()
+            assert before.endswith("__syncwarp();"), path
+    assert arrives
