@@ -27,7 +27,7 @@ struct MpmHandle {
   MpmToolDesc* d_tools = nullptr;
   int n_tools = 0;
   MpmTuning tune = {0, 0, 0, 0, 0, 0};  // mpm_set_tuning
-  bool dirty = false;  // a launch failed inside a substep: grid a and the block flags may not be zero
+  mpm::Restored zero;  // grid a and the block flags are zero
   std::vector<MpmToolDesc> h_tools;
   unsigned int* d_status = nullptr;
   int* d_flags = nullptr;  // convergence flags and counters of mpm_target_sdf
@@ -238,6 +238,7 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
   // the p2g grid and the block flags start at zero; every substep leaves them so
   ok = ok && cudaMemset(h->d_blockbuf, 0, bbytes) == cudaSuccess;
   ok = ok && cudaMemset(h->grid[0], 0, gbytes) == cudaSuccess;
+  h->zero.now.mark(0);
   // the order of runs is a permutation before any sort has run
   ok = ok && mpm::launch_identity_order(p.n_particles, h->d_order, nullptr) == cudaSuccess;
   // the pipelined adjoint's internal stream and events (created here, outside any stream capture)
@@ -433,21 +434,22 @@ static int check_store(MpmHandle* h, const MpmGridStore* store, int32_t slot) {
 }
 
 // Between substeps grid a and the block flags are zero; a substep that failed on the
-// way left them unknown, so the next one clears them.
+// way left them unknown, so the next one clears them (and, where that one was only
+// recorded in a capture, so does the next one outside it).
 static int substep_begin(MpmHandle* h, void* stream) {
-  if (h->dirty) {
+  const unsigned long long capture = h->zero.now.run ? 0 : capture_of(stream);
+  if (!h->zero.begin(capture)) {
     cudaError_t e = cudaMemsetAsync(h->grid[0], 0, (size_t)h->p.n_scenes * h->G * 4 * real_size(h->p.precision),
                                     (cudaStream_t)stream);
     if (e == cudaSuccess)
       e = cudaMemsetAsync(h->d_blockbuf, 0, mpm::blockbuf_bytes(h->p.n_scenes, h->p.n_grid), (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(h, e, "clearing the grid");
   }
-  h->dirty = true;
   return MPM_OK;
 }
-static int substep_done(MpmHandle* h, cudaError_t e, const char* what) {
+static int substep_done(MpmHandle* h, cudaError_t e, const char* what, void* stream) {
   if (e != cudaSuccess) return cuda_fail(h, e, what);
-  h->dirty = false;
+  h->zero.end(h->zero.before.run ? 0 : capture_of(stream));
   return MPM_OK;
 }
 
@@ -480,7 +482,7 @@ static int substep_fwd_impl(MpmHandle* h, const void* state_f, void* state_f1, c
       e = mpm::launch_substep_fwd<double, double>(L, (const double*)state_f, (double*)state_f1, pose_f, pose_f1,
                                                   store, slot);
   }
-  return substep_done(h, e, "mpm_substep_fwd");
+  return substep_done(h, e, "mpm_substep_fwd", stream);
 }
 
 static int substep_bwd_impl(MpmHandle* h, const void* state_f, const void* state_f1, const void* g_state_f1,
@@ -551,7 +553,7 @@ static int substep_bwd_impl(MpmHandle* h, const void* state_f, const void* state
     h->pipe_pending = e == cudaSuccess;
     h->pipe_stream = stream;
   }
-  return substep_done(h, e, "mpm_substep_bwd");
+  return substep_done(h, e, "mpm_substep_bwd", stream);
 }
 
 int mpm_set_pipelined_adjoint(MpmHandle* h, int32_t on) {

@@ -19,4 +19,20 @@ struct Done {
   }
 };
 
+// A state that each call needs and leaves behind it (the p2g grid and the block flags
+// are zero).  begin() says whether the state holds for a call in this capture, else the
+// call makes it first; until end() it is unknown, as it stays after a call that failed.
+struct Restored {
+  Done now, before;
+  bool begin(unsigned long long capture) {
+    before = now;
+    now = Done{};
+    return before.holds(capture);
+  }
+  void end(unsigned long long capture) {
+    now = before;
+    now.mark(capture);
+  }
+};
+
 }  // namespace mpm

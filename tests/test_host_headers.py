@@ -27,6 +27,35 @@ int main() {
 """
 
 
+RESTORED = r"""
+#include "mpm_done.h"
+#define CHECK(x) if (!(x)) return __LINE__
+int main() {
+  mpm::Restored z;
+  z.now.mark(0);  // as a handle is created
+  CHECK(z.begin(0));
+  z.end(0);
+  CHECK(z.begin(5));  // a capture of a state that holds restores nothing
+  z.end(5);
+  CHECK(z.begin(0));  // and this call fails: no end()
+  CHECK(!z.begin(6));  // restored in capture 6
+  z.end(6);
+  CHECK(z.begin(6));  // once per capture
+  z.end(6);
+  CHECK(!z.begin(7));  // not in another
+  z.end(7);
+  CHECK(!z.begin(0));  // and not outside
+  z.end(0);
+  CHECK(z.begin(0));
+  z.end(0);
+  CHECK(z.begin(8));
+  z.end(8);
+  CHECK(z.begin(0));
+  return 0;
+}
+"""
+
+
 def _run(tmp_path, source):
     """0, or the line of the first check that fails."""
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
@@ -39,6 +68,10 @@ def _run(tmp_path, source):
 def test_recorded_work_is_done_for_its_own_capture_only(tmp_path):
     """What a capture only recorded must not count as done for a call outside it."""
     assert _run(tmp_path, DONE) == 0
+
+
+def test_a_failed_call_is_followed_by_a_clearing_one_in_each_capture_and_outside(tmp_path):
+    assert _run(tmp_path, RESTORED) == 0
 
 
 def test_aligned_cluster_barriers_follow_a_warp_barrier():
