@@ -43,6 +43,8 @@ struct MpmHandle {
   void* d_tools_t = nullptr;  // tools in the compute precision (converted by mpm_set_tools)
   void* d_poses_t = nullptr;  // poses of the current substep in the compute precision
   mpm::SortScratch sort;      // particle re-sort (mpm_sort_frame)
+  std::mutex pool_mu;
+  cudaMemPool_t pool = nullptr;  // scratch of single calls, ordered by their streams
   int* d_order = nullptr;     // particles by cell for the substeps of mpm_substeps_fwd / _bwd; always a permutation
   mpm::Done ordered;          // d_order was sorted
   // pipelined adjoint (mpm_set_pipelined_adjoint): the grid preparation of an
@@ -140,6 +142,35 @@ unsigned long long capture_of(void* stream) {
     return 0;
   }
   return st == cudaStreamCaptureStatusActive ? id : 0;
+}
+// Scratch of one call, to be given back by cudaFreeAsync on the same stream (nullptr
+// when there is no memory): calls on several streams have their own.  It comes from a
+// pool of the handle, which keeps up to 32 MiB (2 us for both calls; the device's
+// default pool returns everything at each synchronisation), and in a capture from the
+// graph's memory.
+unsigned char* call_scratch(MpmHandle* h, size_t bytes, cudaStream_t stream) {
+  void* ptr = nullptr;
+  cudaError_t e;
+  if (capture_of(stream) != 0) {
+    e = cudaMallocAsync(&ptr, bytes, stream);
+  } else {
+    std::lock_guard<std::mutex> lk(h->pool_mu);
+    e = cudaSuccess;
+    if (!h->pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = h->device;
+      e = cudaMemPoolCreate(&h->pool, &props);
+      if (e != cudaSuccess) h->pool = nullptr;
+      unsigned long long keep = 32ull << 20;
+      if (e == cudaSuccess) e = cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ptr, bytes, h->pool, stream);
+  }
+  if (e == cudaSuccess) return (unsigned char*)ptr;
+  cudaGetLastError();
+  return nullptr;
 }
 int check_device(MpmHandle* h) {
   int dev = -1;
@@ -274,6 +305,7 @@ int mpm_destroy(MpmHandle* h) {
   cudaFree(h->d_coll_pts);
   cudaFree(h->d_tools_t);
   cudaFree(h->d_poses_t);
+  if (h->pool) cudaMemPoolDestroy(h->pool);
   if (h->pipe_side) cudaStreamDestroy(h->pipe_side);
   if (h->pipe_grid_done) cudaEventDestroy(h->pipe_grid_done);
   if (h->pipe_prep_done) cudaEventDestroy(h->pipe_prep_done);
@@ -983,11 +1015,16 @@ int mpm_render_trace(MpmHandle* h, const MpmRenderVolume* vol, const MpmRenderVi
   MPM_TRY(check_aligned(h, color, "color"));
   MPM_TRY(check_aligned(h, image, "image", true));
   mpm::LaunchCtx L = ctx(h, stream);
+  unsigned char* empty = view->show_particles ? call_scratch(h, mpm::render_bricks(*vol), L.stream) : nullptr;
   cudaError_t e = h->p.precision == MPM_PREC_FP64
-                      ? mpm::launch_render_trace<double>(L, *vol, *view, t0, nt, pose, tool_color, depth, normal,
-                                                         color, image)
-                      : mpm::launch_render_trace<float>(L, *vol, *view, t0, nt, pose, tool_color, depth, normal,
-                                                        color, image);
+                      ? mpm::launch_render_trace<double>(L, *vol, *view, t0, nt, pose, tool_color, empty, depth,
+                                                         normal, color, image)
+                      : mpm::launch_render_trace<float>(L, *vol, *view, t0, nt, pose, tool_color, empty, depth,
+                                                        normal, color, image);
+  if (empty) {
+    const cudaError_t freed = cudaFreeAsync(empty, L.stream);
+    if (e == cudaSuccess) e = freed;
+  }
   return e == cudaSuccess ? MPM_OK : cuda_fail(h, e, "mpm_render_trace");
 }
 

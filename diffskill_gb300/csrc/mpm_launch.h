@@ -167,10 +167,12 @@ cudaError_t launch_tool_distance_bwd(const LaunchCtx& L, const int* col_off, con
 template <typename T>
 cudaError_t launch_render_bake(const LaunchCtx& L, const T* st, int64_t p0, int64_t n, const unsigned int* colors,
                                const MpmRenderVolume& v);
+// empty: scratch of render_bricks(v) bytes, or null (the march then loads every sample)
+size_t render_bricks(const MpmRenderVolume& v);
 template <typename T>
 cudaError_t launch_render_trace(const LaunchCtx& L, const MpmRenderVolume& v, const MpmRenderView& view, int t0,
-                                int nt, const double* pose, const float* tool_color, float* depth, float* normal,
-                                float* color, float* image);
+                                int nt, const double* pose, const float* tool_color, unsigned char* empty,
+                                float* depth, float* normal, float* color, float* image);
 // tool kinematics of one action with collision projection (mpm_kinematics.cu)
 cudaError_t launch_tools_action(const LaunchCtx& L, int n_tools, const int* pair_off, int n_pairs,
                                 const double* coll_pts, const double* action, double* vel, double* pose, double* coll,

@@ -223,8 +223,9 @@ MPM_DI V3 mapply_pos(const float* M, V3 p) {
 }
 
 // empty[brick]: every SDF voxel that a sample in the brick's 8^3 cells reads is
-// exactly 1 (nothing within five voxels); nb = bricks per axis
+// exactly 1 (nothing within five voxels), read if Bricks; nb = bricks per axis
 constexpr int BRICK = 8;
+template <bool Bricks>
 struct Volume {
   const float* sdf;
   const float* color;
@@ -259,12 +260,14 @@ MPM_DI void sample_tex(const float* tex, int nc, const int* res, const float* q,
   }
 }
 // pos normalised to the volume box; inside iff every coordinate is in [0, 1]
-MPM_DI bool vol_coord(const Volume& V, V3 pos, float* q) {
+template <bool B>
+MPM_DI bool vol_coord(const Volume<B>& V, V3 pos, float* q) {
   for (int c = 0; c < 3; ++c) q[c] = (comp(pos, c) - V.b0[c]) / (V.b1[c] - V.b0[c]);
   const float mn = fminf(fminf(q[0], q[1]), q[2]), mx = fmaxf(fmaxf(q[0], q[1]), q[2]);
   return mn >= 0.0f && mx <= 1.0f;
 }
-MPM_DI float sample_sdf(const Volume& V, V3 pos) {
+template <bool B>
+MPM_DI float sample_sdf(const Volume<B>& V, V3 pos) {
   float q[3], s = 0.0f;
   if (vol_coord(V, pos, q)) {
     // in an empty brick sample_tex's interpolation of eight ones, without its loads
@@ -275,7 +278,7 @@ MPM_DI float sample_sdf(const Volume& V, V3 pos) {
       b[c] = ((int)t < V.res[c] - 1) ? (int)t : V.res[c] - 1;
       fx[c] = t - (float)b[c];
     }
-    if (V.empty[((b[0] / BRICK) * V.nb[1] + b[1] / BRICK) * V.nb[2] + b[2] / BRICK]) {
+    if (B && V.empty[((b[0] / BRICK) * V.nb[1] + b[1] / BRICK) * V.nb[2] + b[2] / BRICK]) {
       const float c00 = (1 - fx[0]) + fx[0];
       const float c0 = c00 * (1 - fx[1]) + c00 * fx[1];
       s = c0 * (1 - fx[2]) + c0 * fx[2];
@@ -286,13 +289,15 @@ MPM_DI float sample_sdf(const Volume& V, V3 pos) {
   }
   return s;
 }
-MPM_DI V3 sample_color(const Volume& V, V3 pos) {
+template <bool B>
+MPM_DI V3 sample_color(const Volume<B>& V, V3 pos) {
   float q[3], c[3] = {0.0f, 0.0f, 0.0f};
   if (vol_coord(V, pos, q)) sample_tex(V.color, 3, V.res, q, c);
   return v3(c[0], c[1], c[2]);
 }
 // central differences with d = 1e-3, normalised (particle_sdf.py:306-315)
-MPM_DI V3 sample_normal(const Volume& V, V3 p) {
+template <bool B>
+MPM_DI V3 sample_normal(const Volume<B>& V, V3 p) {
   const float d = 1e-3f;
   float n[3];
   for (int i = 0; i < 3; ++i) {
@@ -390,7 +395,7 @@ MPM_DI TT ray_tool_sdf(const RayTool<TT>& r, const TT* p) {  // tool_sdf
   return ray_shape_sdf(r, r.at[0], r.pose.gap, p);
 }
 
-template <typename TT>
+template <typename TT, bool Bricks>
 __global__ void __launch_bounds__(128)
     k_rb_trace(const float* __restrict__ vsdf, const float* __restrict__ vcolor, const float* __restrict__ bbox,
                int r0, int r1, int r2, float threshold, Camera cam, int resx, int resy, float biasx, float biasy,
@@ -411,7 +416,7 @@ __global__ void __launch_bounds__(128)
   const int64_t pix = (int64_t)px * resy + py;
   const float* V2W = cam.m;
   const float* W2V = cam.m + 16;
-  Volume V;
+  Volume<Bricks> V;
   V.sdf = vsdf;
   V.color = vcolor;
   V.empty = empty;
@@ -538,24 +543,27 @@ cudaError_t launch_render_bake(const LaunchCtx& L, const T* st, int64_t p0, int6
   return cudaGetLastError();
 }
 
+inline int bricks(int res) { return (res + BRICK - 1) / BRICK; }
+size_t render_bricks(const MpmRenderVolume& v) {
+  return (size_t)bricks(v.res[0]) * bricks(v.res[1]) * bricks(v.res[2]);
+}
+
 template <typename T>
 cudaError_t launch_render_trace(const LaunchCtx& L, const MpmRenderVolume& v, const MpmRenderView& view, int t0,
-                                int nt, const double* pose, const float* tool_color, float* depth, float* normal,
-                                float* color, float* image) {
+                                int nt, const double* pose, const float* tool_color, unsigned char* empty,
+                                float* depth, float* normal, float* color, float* image) {
   Camera cam;
   for (int k = 0; k < 16; ++k) {
     cam.m[k] = view.v2w[k];
     cam.m[16 + k] = view.w2v[k];
   }
   const unsigned ntiles = (unsigned)(((view.res[0] + 15) / 16) * (int64_t)((view.res[1] + 7) / 8));
-  // which bricks of the volume are empty: kept in vol.packed, which only a bake
-  // reads (traces of the same volume write the same bytes)
-  unsigned char* empty = reinterpret_cast<unsigned char*>(v.packed);
-  const int nb[3] = {(v.res[0] + BRICK - 1) / BRICK, (v.res[1] + BRICK - 1) / BRICK, (v.res[2] + BRICK - 1) / BRICK};
-  if (view.show_particles)
-    MPM_LAUNCH(L, MPM_K_OTHER, k_rb_bricks, nblk((int64_t)nb[0] * nb[1] * nb[2] * 32, 256), 256, v.sdf, v.res[0],
-               v.res[1], v.res[2], nb[0], nb[1], nb[2], empty);
-  MPM_LAUNCH(L, MPM_K_OTHER, k_rb_trace<T>, ntiles, 128, v.sdf, v.color, v.bbox, v.res[0], v.res[1],
+  if (empty)
+    MPM_LAUNCH(L, MPM_K_OTHER, k_rb_bricks, nblk((int64_t)render_bricks(v) * 32, 256), 256, v.sdf, v.res[0], v.res[1],
+               v.res[2], bricks(v.res[0]), bricks(v.res[1]), bricks(v.res[2]), empty);
+  // two kernels: a test of the pointer at each sample took 1 % of a trace
+  const auto trace = empty ? k_rb_trace<T, true> : k_rb_trace<T, false>;
+  MPM_LAUNCH(L, MPM_K_OTHER, trace, ntiles, 128, v.sdf, v.color, v.bbox, v.res[0], v.res[1],
              v.res[2], view.sdf_threshold, cam, view.res[0], view.res[1], view.bias[0], view.bias[1], L.tools, t0,
              nt, pose, tool_color, view.show_particles, (const unsigned char*)empty, depth, normal, color, image);
   return cudaGetLastError();
@@ -565,7 +573,8 @@ cudaError_t launch_render_trace(const LaunchCtx& L, const MpmRenderVolume& v, co
   template cudaError_t launch_render_bake<T>(const LaunchCtx&, const T*, int64_t, int64_t, const unsigned int*,    \
                                              const MpmRenderVolume&);                                              \
   template cudaError_t launch_render_trace<T>(const LaunchCtx&, const MpmRenderVolume&, const MpmRenderView&, int, \
-                                              int, const double*, const float*, float*, float*, float*, float*);
+                                              int, const double*, const float*, unsigned char*, float*, float*, float*,     \
+                                              float*);
 MPM_INST_RENDER(float)
 MPM_INST_RENDER(double)
 

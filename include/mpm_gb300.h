@@ -358,8 +358,7 @@ typedef struct MpmRenderVolume {
   int32_t res[3];              /* voxels per axis (default 168^3) */
   int32_t bake_size;           /* splat radius in voxels (default 6) */
   double dx;                   /* voxel size (default 1/150) */
-  unsigned long long* packed;  /* uint64[res] scratch of both calls: (quantised distance << 24) | rgb while baking,
-                                  empty-brick flags while tracing */
+  unsigned long long* packed;  /* uint64[res] scratch of a bake: (quantised distance << 24) | rgb */
   float* sdf;                  /* float[res] baked SDF, smoothed twice */
   float* sdf_copy;             /* float[res] scratch */
   float* color;                /* float[res][3] */
