@@ -382,11 +382,6 @@ MPM_DI void zero_stencil(Stencil<T>& s) {
     for (int k = 0; k < 3; ++k) s.w[k][d] = T(0);
   }
 }
-// a[i] for a runtime i in 0..2 without local memory
-template <typename T>
-MPM_DI T sel3(T a0, T a1, T a2, int i) {
-  return i == 0 ? a0 : (i == 1 ? a1 : a2);
-}
 template <typename T>
 MPM_DI long long cell_key(const Consts<T>& c, int scene, const Stencil<T>& s) {
   return (long long)scene * c.G + ((long long)s.base[0] * c.n_grid + s.base[1]) * c.n_grid + s.base[2];

@@ -54,6 +54,11 @@ MPM_DI bool finite(T x) {
   return isfinite(x);
 }
 
+// a[i] for a runtime i in 0..2 without local memory
+template <typename T>
+MPM_DI T sel3(T a0, T a1, T a2, int i) {
+  return i == 0 ? a0 : (i == 1 ? a1 : a2);
+}
 template <typename T>
 MPM_DI T dot3(const T* a, const T* b) {
   return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];

@@ -5,8 +5,8 @@
 // sorted by eigenvalue, then U from Gram-Schmidt on B = A V.  Output follows
 // the convention of ti.svd used by plb/engine/mpm_simulator.py:127-129:
 // A = U diag(s) V^T, det U = det V = +1, s0 >= s1 >= |s2|, s2 may be negative.
-// FP32 takes the shifted form (svd3_shifted), FP64 an FP32 decomposition that
-// is refined in FP64 (svd3_left64).
+// FP32 takes the rotations of A A^T - I (svd3_left32), FP64 an FP32 decomposition
+// that is refined in FP64 (svd3_left64).
 //
 // Backward: backward_svd of plb/engine/mpm_simulator.py:137-156 with the
 // +-1e-6 clamp of clamp() (184-192) on s_j^2 - s_i^2.
@@ -196,117 +196,92 @@ MPM_DI void svd3(const T* A, T* U, T* s, T* V) {
   }
 }
 
-// FP32 SVD of A = I + D given the displacement D = A - I (not A itself), so
-// that the strain information (of size |D|, typically 1e-4 .. 1e-2) keeps
-// FP32's relative precision instead of the absolute precision of numbers
-// near 1.  The same cyclic Jacobi rotations as svd3 act on the shifted
-// symmetric matrix M = A^T A - I = D + D^T + D^T D (same eigenvectors V,
-// eigenvalues s^2 - 1), converged relative to M itself.  Returns U, V, s and
-// sm1 = s - 1 (from (s^2 - 1) / (1 + s), exact as s -> 1).  Same conventions
-// as svd3: det U = det V = +1, s0 >= s1 >= |s2|, s2 may be negative.
-// convergence of the shifted sweeps: off-diagonal^2 <= kShiftedTol * diagonal^2 of M
-constexpr float kShiftedTol = 1e-14f;
-MPM_DI void svd3_shifted(const float* D, float* U, float* s, float* sm1, float* V) {
-  float M[9];
+// The rest of an SVD from the left, for any matrix: U's columns are eigenvectors of
+// A A^T with eigenvalues ev (any common offset), B = A^T U.  Orders the columns by
+// eigenvalue, keeping det U = 1, and takes V from Gram-Schmidt on B's columns, longest
+// first, so that the short singular vectors are as exact as the long ones.  Returns
+// |b0|, v1 . b1 and v2 . b2 in n (the singular values, the last one signed).
+template <typename T>
+MPM_DI void left_gram_schmidt(T* U, T* ev, T* B, T* n, T* V) {
+  const auto order = [&](int a, int b) {
+    if (ev[a] < ev[b]) {
+      const T t = ev[a];
+      ev[a] = ev[b];
+      ev[b] = t;
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+      for (int k = 0; k < 3; ++k) {  // a swap, and one column negated: det U is kept
+        const T u = U[k * 3 + a], w = B[k * 3 + a];
+        U[k * 3 + a] = U[k * 3 + b];
+        B[k * 3 + a] = B[k * 3 + b];
+        U[k * 3 + b] = -u;
+        B[k * 3 + b] = -w;
+      }
+    }
+  };
+  order(0, 1);
+  order(0, 2);
+  order(1, 2);
+  const T b0[3] = {B[0], B[3], B[6]}, b1[3] = {B[1], B[4], B[7]}, b2[3] = {B[2], B[5], B[8]};
+  T v0[3] = {T(1), T(0), T(0)}, v1[3], v2[3];
+  n[0] = T(0);
+  const T d0 = dot3(b0, b0);
+  if (d0 != T(0)) {  // (NaN too)
+    const T inv = inv_len(d0);
+    n[0] = d0 * inv;
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      M[i * 3 + j] = D[i * 3 + j] + D[j * 3 + i] + (D[i] * D[j] + D[3 + i] * D[3 + j] + D[6 + i] * D[6 + j]);
-  float a00 = M[0], a11 = M[4], a22 = M[8], a01 = M[1], a02 = M[2], a12 = M[5];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) V[k] = (k % 4 == 0) ? 1.f : 0.f;
-  for (int sweep = 0; sweep < SvdIters<float>::max_sweeps; ++sweep) {
-    const float off = a01 * a01 + a02 * a02 + a12 * a12;
-    const float dg = a00 * a00 + a11 * a11 + a22 * a22;
-    // relative to M; the absolute floor stops sweeps on rounding noise (rigid rotations, M ~ 0)
-    if (off <= kShiftedTol * dg + 1e-30f) break;
-    jacobi_rot(a00, a11, a01, a02, a12, V, 0, 1);
-    jacobi_rot(a00, a22, a02, a01, a12, V, 0, 2);
-    jacobi_rot(a11, a22, a12, a01, a02, V, 1, 2);
+    for (int k = 0; k < 3; ++k) v0[k] = b0[k] * inv;
   }
-  float ev[3] = {a00, a11, a22};
-  bool flip = false;
-  if (ev[0] < ev[1]) { swap_cols(V, ev, 0, 1); flip = !flip; }
-  if (ev[0] < ev[2]) { swap_cols(V, ev, 0, 2); flip = !flip; }
-  if (ev[1] < ev[2]) { swap_cols(V, ev, 1, 2); flip = !flip; }
-  if (flip) {
+  const T pr = dot3(v0, b1);
+  T r[3] = {b1[0] - pr * v0[0], b1[1] - pr * v0[1], b1[2] - pr * v0[2]};
+  T d1 = dot3(r, r);
+  if (d1 == T(0)) {  // A of rank <= 1: any unit vector orthogonal to v0
+    int m = (mabs(v0[0]) < mabs(v0[1])) ? 0 : 1;
+    if (mabs(v0[2]) < mabs(sel3(v0[0], v0[1], v0[2], m))) m = 2;
+    const T pe = sel3(v0[0], v0[1], v0[2], m);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) V[k * 3 + 2] = -V[k * 3 + 2];
+    for (int k = 0; k < 3; ++k) r[k] = (k == m ? T(1) : T(0)) - pe * v0[k];
+    d1 = dot3(r, r);
   }
-  // B = A V = V + D V, U by Gram-Schmidt as in svd3
-  float B[9];
-  mm(D, V, B);
+  const T inv = inv_len(d1);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) B[k] += V[k];
-  float b0[3] = {B[0], B[3], B[6]}, b1[3] = {B[1], B[4], B[7]}, b2[3] = {B[2], B[5], B[8]};
-  float u0[3], u1[3], u2[3];
-  const float d0 = dot3(b0, b0);
-  if (d0 > 0.f) {
-    const float inv = inv_len(d0);
+  for (int k = 0; k < 3; ++k) v1[k] = r[k] * inv;
+  cross3(v0, v1, v2);
+  n[1] = dot3(v1, b1);
+  n[2] = dot3(v2, b2);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) u0[k] = b0[k] * inv;
-  } else {
-    u0[0] = 1.f; u0[1] = 0.f; u0[2] = 0.f;
-  }
-  const float pr = dot3(u0, b1);
-  float r1[3] = {b1[0] - pr * u0[0], b1[1] - pr * u0[1], b1[2] - pr * u0[2]};
-  const float d1 = dot3(r1, r1);
-  if (d1 > 0.f) {
-    const float inv = inv_len(d1);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) u1[k] = r1[k] * inv;
-  } else {
-    int m = (fabsf(u0[0]) < fabsf(u0[1])) ? 0 : 1;
-    if (fabsf(u0[2]) < fabsf(u0[m])) m = 2;
-    float e[3] = {0.f, 0.f, 0.f};
-    e[m] = 1.f;
-    const float pe = dot3(u0, e);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) r1[k] = e[k] - pe * u0[k];
-    const float inv = 1.f / sqrtf(dot3(r1, r1));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) u1[k] = r1[k] * inv;
-  }
-  cross3(u0, u1, u2);
-  // s_i - 1 = (s_i^2 - 1) / (1 + s_i), s_i^2 - 1 the eigenvalue of M; the sign
-  // of s2 (an inverted element) from u2 . b2 as in svd3
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float q = fmaxf(1.f + ev[i], 0.f);
-    const float r = sqrtf(q);
-    sm1[i] = ev[i] / (1.f + r);
-    s[i] = r;
-  }
-  if (dot3(u2, b2) < 0.f) {
-    s[2] = -s[2];
-    sm1[2] = s[2] - 1.f;
-  }
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    U[r * 3 + 0] = u0[r];
-    U[r * 3 + 1] = u1[r];
-    U[r * 3 + 2] = u2[r];
+  for (int k = 0; k < 3; ++k) {
+    V[k * 3] = v0[k];
+    V[k * 3 + 1] = v1[k];
+    V[k * 3 + 2] = v2[k];
   }
 }
 
-// The plain shifted SVD, out of line: for the few matrices that svd3_left32
-// leaves to it.
-__device__ __noinline__ inline void svd3_plain32(const float* D, float* U, float* s, float* sm1, float* V) {
-  svd3_shifted(D, U, s, sm1, V);
-}
-// FP32 SVD of A = I + D = U diag(s) V^T from the left: the Jacobi rotations of
-// svd3_shifted on A A^T - I = D + D^T + D D^T give U and s^2 - 1 at once, so the
-// forward pass, which needs no V, has neither svd3_shifted's product A V nor its
-// Gram-Schmidt, and V = A^T U diag(1/s) takes their place in the adjoint.  The
-// values are in no particular order (nothing depends on it).  A rotation scales
-// its two columns by sqrt(c^2 + s^2) = 1 + O(1e-7), so each column is normalised
-// once at the end by 3/2 - |u|^2 / 2.  detA = det(I + D).  Returns true (plain) for an inverted or
-// nearly singular matrix (s < 0.2): then U, s, sm1, V come from svd3_shifted
-// and is = 0.  V is written when plain or WithV; is = 1/s.
+// convergence of the shifted sweeps: off-diagonal^2 <= kShiftedTol * diagonal^2
+constexpr float kShiftedTol = 1e-14f;
+// FP32 SVD of A = I + D = U diag(s) V^T from the left, given the displacement D = A - I
+// (not A itself), so that the strain information (of size |D|, typically 1e-4 .. 1e-2)
+// keeps FP32's relative precision instead of the absolute precision of numbers near
+// 1: Jacobi rotations on A A^T - I = D + D^T + D D^T, converged relative to that
+// matrix, give U and s^2 - 1, and s - 1 = (s^2 - 1) / (1 + s) is exact as s -> 1.  The
+// forward pass, which needs no V, then has neither a product A V nor a Gram-Schmidt,
+// and V = A^T U diag(1/s) takes their place in the adjoint.  The values are in no
+// particular order (nothing depends on it).  A rotation scales its two columns by
+// sqrt(c^2 + s^2) = 1 + O(1e-7), so each column is normalised once at the end by
+// 3/2 - |u|^2 / 2.  detA = det(I + D).  V is written when WithV; is = 1/s.
+//
+// U carries a rounding error of 1e-7, and A^T U / s that error times the ratio of A's
+// longest to its shortest axis.  So an inverted or strongly deformed matrix,
+// |A A^T - I|^2 (Frobenius) of kLeftNorm2 or more, takes V from Gram-Schmidt: then
+// true (plain) is returned, V is written, is = 0, and s[2] may be negative.  Median
+// relative error, without and with it, of newF at a smallest s of 0.2 .. 0.25: 3.4e-7,
+// 2.0e-7; at 0.5 .. 0.7: 1.0e-7, 8.9e-8; of the gradient of C at a largest s of
+// 3 .. 10: 1.8e-6, 6.0e-7 (an SVD by Gram-Schmidt throughout: 2.2e-7, 9.2e-8 and
+// 6.7e-7).  Below kLeftNorm2 the two agree to 3 %; dough, which yields at strains near
+// 0.01, is far below it.
+constexpr float kLeftNorm2 = 0.5f;
 template <bool WithV>
 MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* sm1, float* is, float* V) {
-  float ev[3];
+  float ev[3], norm2;
   {
     float a00 = 2.f * D[0] + dot3(D, D), a11 = 2.f * D[4] + dot3(D + 3, D + 3), a22 = 2.f * D[8] + dot3(D + 6, D + 6);
     float a01 = D[1] + D[3] + dot3(D, D + 3), a02 = D[2] + D[6] + dot3(D, D + 6), a12 = D[5] + D[7] + dot3(D + 3, D + 6);
@@ -324,6 +299,7 @@ MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* s
     ev[0] = a00;
     ev[1] = a11;
     ev[2] = a22;
+    norm2 = a00 * a00 + a11 * a11 + a22 * a22;
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -332,23 +308,22 @@ MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* s
     U[3 + k] *= f;
     U[6 + k] *= f;
   }
-  const bool plain = !(fminf(fminf(ev[0], ev[1]), ev[2]) > -0.96f && detA > 0.f);
-  if (plain) {
-    float Dl[9], Ul[9], sl[3], ml[3], Vl[9];
+  if (!(norm2 < kLeftNorm2 && detA > 0.f)) {
+    float B[9], n[3];
+    mTm(D, U, B);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) Dl[k] = D[k];
-    svd3_plain32(Dl, Ul, sl, ml, Vl);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      U[k] = Ul[k];
-      V[k] = Vl[k];
-    }
+    for (int k = 0; k < 9; ++k) B[k] += U[k];
+    left_gram_schmidt(U, ev, B, n, V);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      s[k] = sl[k];
-      sm1[k] = ml[k];
-      is[k] = 0.f;
+      s[k] = sqrtf(fmaxf(1.f + ev[k], 0.f));
+      sm1[k] = ev[k] / (1.f + s[k]);  // (s^2 - 1) / (s + 1)
     }
+    if (n[2] < 0.f) {
+      s[2] = -s[2];
+      sm1[2] = s[2] - 1.f;
+    }
+    is[0] = is[1] = is[2] = 0.f;
     return true;
   }
 #pragma unroll
@@ -401,7 +376,7 @@ __device__ __noinline__ inline void svd3_plain64(const double* A, double* U, dou
 // An FP64 Jacobi rotation costs about 68 FP64 instructions, and svd3 takes
 // four to five sweeps of three: about 900 of the 1,245 FP64 instructions that
 // p2g spent on a particle.  Here the sweeps run in FP32 on the shifted matrix
-// A A^T - I (relative to the strain, as svd3_shifted), and FP64 only refines:
+// A A^T - I (relative to the strain, as svd3_left32), and FP64 only refines:
 // - U is orthonormalised by Gram-Schmidt (a unit vector's norm is 1 + O(1e-6),
 //   so 1/|u| is a two-term series);
 // - S = U^T A A^T U is then diagonal but for E of about 1e-6 of the strain;
