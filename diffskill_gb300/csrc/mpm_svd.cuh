@@ -1,12 +1,12 @@
 // 3x3 SVD and its clamped backward on the device.
 //
-// Forward: cyclic Jacobi eigen-decomposition of A^T A with symmetric Schur
-// rotations (Golub & Van Loan, "Matrix Computations", Sec. 8.5.2), columns
-// sorted by eigenvalue, then U from Gram-Schmidt on B = A V.  Output follows
-// the convention of ti.svd used by plb/engine/mpm_simulator.py:127-129:
-// A = U diag(s) V^T, det U = det V = +1, s0 >= s1 >= |s2|, s2 may be negative.
-// FP32 takes the rotations of A A^T - I (svd3_left32), FP64 an FP32 decomposition
-// that is refined in FP64 (svd3_left64).
+// Forward: A = U diag(s) V^T with det U = det V = +1 and the sign of det A on the last
+// value, as ti.svd (plb/engine/mpm_simulator.py:127-129), from the left: a cyclic Jacobi
+// eigen-decomposition of A A^T with symmetric Schur rotations (Golub & Van Loan,
+// "Matrix Computations", Sec. 8.5.2) gives U and s^2, then V = A^T U / s.  The values
+// come in no particular order (nothing depends on it) but where V is taken by
+// Gram-Schmidt: s0 >= s1 >= |s2| there.  FP32 rotates A A^T - I (svd3_left32), FP64
+// refines an FP32 decomposition (svd3_left64).
 //
 // Backward: backward_svd of plb/engine/mpm_simulator.py:137-156 with the
 // +-1e-6 clamp of clamp() (184-192) on s_j^2 - s_i^2.
@@ -111,91 +111,6 @@ MPM_DI void jacobi_rot(T& app, T& aqq, T& apq, T& arp, T& arq, T* V, int p, int 
   }
 }
 
-template <typename T>
-MPM_DI void swap_cols(T* V, T* ev, int a, int b) {
-  T t = ev[a];
-  ev[a] = ev[b];
-  ev[b] = t;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    T x = V[k * 3 + a];
-    V[k * 3 + a] = V[k * 3 + b];
-    V[k * 3 + b] = x;
-  }
-}
-
-template <typename T>
-MPM_DI void svd3(const T* A, T* U, T* s, T* V) {
-  T S[9];
-  mTm(A, A, S);
-  T a00 = S[0], a11 = S[4], a22 = S[8], a01 = S[1], a02 = S[2], a12 = S[5];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) V[k] = (k % 4 == 0) ? T(1) : T(0);
-  for (int sweep = 0; sweep < SvdIters<T>::max_sweeps; ++sweep) {
-    T off = a01 * a01 + a02 * a02 + a12 * a12;
-    T dg = a00 * a00 + a11 * a11 + a22 * a22;
-    if (off <= SvdIters<T>::tol * dg) break;
-    jacobi_rot(a00, a11, a01, a02, a12, V, 0, 1);  // r = 2: (s_20, s_21)
-    jacobi_rot(a00, a22, a02, a01, a12, V, 0, 2);  // r = 1: (s_10, s_12)
-    jacobi_rot(a11, a22, a12, a01, a02, V, 1, 2);  // r = 0: (s_01, s_02)
-  }
-  // descending eigenvalues; each swap flips det V
-  T ev[3] = {a00, a11, a22};
-  bool flip = false;
-  if (ev[0] < ev[1]) { swap_cols(V, ev, 0, 1); flip = !flip; }
-  if (ev[0] < ev[2]) { swap_cols(V, ev, 0, 2); flip = !flip; }
-  if (ev[1] < ev[2]) { swap_cols(V, ev, 1, 2); flip = !flip; }
-  if (flip) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) V[k * 3 + 2] = -V[k * 3 + 2];
-  }
-  T B[9];
-  mm(A, V, B);
-  T b0[3] = {B[0], B[3], B[6]}, b1[3] = {B[1], B[4], B[7]}, b2[3] = {B[2], B[5], B[8]};
-  T u0[3], u1[3], u2[3];
-  // column norms from one reciprocal square root each: |b| = b.b / sqrt(b.b)
-  T d0 = dot3(b0, b0);
-  T n0 = T(0);
-  if (d0 > T(0)) {
-    T inv = inv_len(d0);
-    n0 = d0 * inv;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) u0[k] = b0[k] * inv;
-  } else {
-    u0[0] = T(1); u0[1] = T(0); u0[2] = T(0);
-  }
-  T pr = dot3(u0, b1);
-  T r1[3] = {b1[0] - pr * u0[0], b1[1] - pr * u0[1], b1[2] - pr * u0[2]};
-  T d1 = dot3(r1, r1);
-  if (d1 > T(0)) {
-    T inv = inv_len(d1);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) u1[k] = r1[k] * inv;
-  } else {
-    // any unit vector orthogonal to u0 (A of rank <= 1)
-    int m = (mabs(u0[0]) < mabs(u0[1])) ? 0 : 1;
-    if (mabs(u0[2]) < mabs(u0[m])) m = 2;
-    T e[3] = {T(0), T(0), T(0)};
-    e[m] = T(1);
-    T pe = dot3(u0, e);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) r1[k] = e[k] - pe * u0[k];
-    T inv = T(1) / msqrt(dot3(r1, r1));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) u1[k] = r1[k] * inv;
-  }
-  cross3(u0, u1, u2);
-  s[0] = n0;
-  s[1] = dot3(u1, b1);
-  s[2] = dot3(u2, b2);
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    U[r * 3 + 0] = u0[r];
-    U[r * 3 + 1] = u1[r];
-    U[r * 3 + 2] = u2[r];
-  }
-}
-
 // The rest of an SVD from the left, for any matrix: U's columns are eigenvectors of
 // A A^T with eigenvalues ev (any common offset), B = A^T U.  Orders the columns by
 // eigenvalue, keeping det U = 1, and takes V from Gram-Schmidt on B's columns, longest
@@ -231,8 +146,13 @@ MPM_DI void left_gram_schmidt(T* U, T* ev, T* B, T* n, T* V) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) v0[k] = b0[k] * inv;
   }
-  const T pr = dot3(v0, b1);
-  T r[3] = {b1[0] - pr * v0[0], b1[1] - pr * v0[1], b1[2] - pr * v0[2]};
+  T r[3] = {b1[0], b1[1], b1[2]};
+#pragma unroll
+  for (int pass = 0; pass < 2; ++pass) {  // twice: b1 may be nothing but its part along v0
+    const T pr = dot3(v0, r);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r[k] -= pr * v0[k];
+  }
   T d1 = dot3(r, r);
   if (d1 == T(0)) {  // A of rank <= 1: any unit vector orthogonal to v0
     int m = (mabs(v0[0]) < mabs(v0[1])) ? 0 : 1;
@@ -343,11 +263,11 @@ MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* s
   return false;
 }
 
-// Two parts of svd3_left64 that few particles reach, out of line so that the
-// kernels do not carry their registers: Jacobi sweeps in FP64 on a matrix whose
-// eigenvalues nearly coincide (S = s00, s11, s22, s01, s02, s12 and U, both
-// updated), and the plain SVD of a matrix that is inverted, nearly singular or
-// not finite.
+// Two parts of svd3_left64 that few particles reach, out of line so that the kernels do
+// not carry their registers (inline, the second one made the adjoint of 37,001 FP64
+// particles 3 % slower): Jacobi sweeps in FP64 on a matrix whose eigenvalues nearly
+// coincide (S = s00, s11, s22, s01, s02, s12 and U, both updated), and V by
+// Gram-Schmidt.
 __device__ __noinline__ inline void jacobi64_finish(double* S, double* U) {
   double a00 = S[0], a11 = S[1], a22 = S[2], a01 = S[3], a02 = S[4], a12 = S[5];
   for (int sweep = 0; sweep < SvdIters<double>::max_sweeps; ++sweep) {
@@ -362,32 +282,37 @@ __device__ __noinline__ inline void jacobi64_finish(double* S, double* U) {
   S[1] = a11;
   S[2] = a22;
 }
-__device__ __noinline__ inline void svd3_plain64(const double* A, double* U, double* s, double* V) {
-  svd3(A, U, s, V);
+__device__ __noinline__ inline void left_gram_schmidt64(const double* A, double* U, double* S, double* s, double* V) {
+  double B[9];
+  mTm(A, U, B);
+  left_gram_schmidt(U, S, B, s, V);
 }
 
 // FP64 SVD A = U diag(s) V^T from the left: U and s^2 are the eigenvectors and
-// eigenvalues of A A^T, V = A^T U diag(1/s).  Unlike svd3 the values are in no
-// particular order (nothing here depends on it), unless `plain` is returned:
-// then the matrix was inverted, nearly singular (s < 0.2) or not finite, and
-// U, s, V and `is` come from svd3, s[2] perhaps negative.  V is written when
-// plain or WithV; is = 1/s (plain: 0 for s at or below the return map's 0.05).
+// eigenvalues of A A^T, V = A^T U diag(1/s), the values in no particular order, unless
+// `plain` is returned: then the matrix was inverted, strongly deformed (an s below 0.2
+// or above 3) or not finite, V comes from Gram-Schmidt, and s[2] is perhaps negative.
+// V is written when plain or WithV; is = 1/s (plain: 0 for s at or below the return
+// map's 0.05).
 //
-// An FP64 Jacobi rotation costs about 68 FP64 instructions, and svd3 takes
-// four to five sweeps of three: about 900 of the 1,245 FP64 instructions that
-// p2g spent on a particle.  Here the sweeps run in FP32 on the shifted matrix
+// An FP64 Jacobi rotation costs about 68 FP64 instructions, and four to five sweeps
+// of three were about 900 of the 1,245 FP64 instructions that p2g spent on a
+// particle.  Here the sweeps run in FP32 on the shifted matrix
 // A A^T - I (relative to the strain, as svd3_left32), and FP64 only refines:
 // - U is orthonormalised by Gram-Schmidt (a unit vector's norm is 1 + O(1e-6),
 //   so 1/|u| is a two-term series);
-// - S = U^T A A^T U is then diagonal but for E of about 1e-6 of the strain;
+// - S = U^T A A^T U is then diagonal but for E of at most 1e-6 of the strain;
 //   Q = exp(X) with the antisymmetric X = X1 + X2 of second-order perturbation
 //   theory, X1_pq = E_pq / (S_qq - S_pp), X2_pq = 1/2 [E, X1]_pq / (S_qq - S_pp),
-//   diagonalises it to E X^2, far below FP64's rounding of S for |X| <= 2e-4;
-// - a pair with a larger X (eigenvalues nearly equal, but not within rounding)
-//   takes FP64 sweeps instead (jacobi64_finish).
-// About 180 FP64 instructions.  p2g of 0.76M particles (FP32 state, FP64 SVD):
-// 1469 -> 547 us; its
-// adjoint: 2096 -> 1087 us.
+//   diagonalises it to E X^2;
+// - where that is above FP64's rounding of S, or X above 2e-4 (eigenvalues nearly
+//   equal, but not within rounding), FP64 sweeps finish it instead (jacobi64_finish):
+//   under one matrix in 20,000 at strains up to 0.3, one in 250 at singular values of
+//   0.2 .. 3.  With |X| <= 2e-4 alone E X^2 reached 600 times the rounding: newF, worst
+//   of 20,000 at 0.2 .. 3, 2.0e-14, now 2.8e-15, by FP64 sweeps 4.3e-15; with
+//   |X| <= 2e-5 alone, as exact, 1 % of an iteration went into sweeps.
+// About 180 FP64 instructions, and 100 more for a plain matrix.  p2g of 0.76M particles
+// (FP32 state, FP64 SVD): 1469 -> 494 us; its adjoint: 2096 -> 997 us.
 template <bool WithV>
 MPM_DI bool svd3_left64(const double* A, double* U, double* s, double* is, double* V) {
   double S[6];  // 00, 11, 22, 01, 02, 12
@@ -467,6 +392,9 @@ MPM_DI bool svd3_left64(const double* A, double* U, double* s, double* is, doubl
     x[q] = fma(fma(-x[q], gap, E), r, x[q]);
     x32[q] = e32[q] * r32[q];
   }
+  const float me = fmaxf(fmaxf(fabsf(e32[0]), fabsf(e32[1])), fabsf(e32[2]));
+  const float mx = fmaxf(fmaxf(fabsf(x32[0]), fabsf(x32[1])), fabsf(x32[2]));
+  far = far || !(me * mx * mx <= round);
   if (far) {
     double Sl[6], Ul[9];
 #pragma unroll
@@ -501,13 +429,16 @@ MPM_DI bool svd3_left64(const double* A, double* U, double* s, double* is, doubl
 #pragma unroll
     for (int k = 0; k < 9; ++k) U[k] = T1[k];
   }
-  const bool plain = !(S[0] > 0.04 && S[1] > 0.04 && S[2] > 0.04 && S[0] < 1e6 && S[1] < 1e6 && S[2] < 1e6 &&
-                       det3(A) > 0.0);
-  if (plain) {
-    double Al[9], Ul[9], sl[3], Vl[9];
+  if (!(S[0] > 0.04 && S[1] > 0.04 && S[2] > 0.04 && S[0] < 9.0 && S[1] < 9.0 && S[2] < 9.0 && det3(A) > 0.0)) {
+    double Al[9], Ul[9], Sl[3], sl[3], Vl[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) Al[k] = A[k];
-    svd3_plain64(Al, Ul, sl, Vl);
+    for (int k = 0; k < 9; ++k) {
+      Al[k] = A[k];
+      Ul[k] = U[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) Sl[k] = S[k];
+    left_gram_schmidt64(Al, Ul, Sl, sl, Vl);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       U[k] = Ul[k];

@@ -9,6 +9,16 @@ template <typename T, typename F>
 void each(long n, const T* A, T* U, T* s, T* V, int* plain, F&& svd) {
   for (long i = 0; i < n; ++i) plain[i] = svd(A + 9 * i, U + 9 * i, s + 3 * i, V + 9 * i);
 }
+// Jacobi sweeps on the symmetric m00, m11, m22, m01, m02, m12
+template <typename T>
+void sweeps(T* m, T* u) {
+  for (int k = 0; k < 9; ++k) u[k] = k % 4 == 0;
+  for (int sweep = 0; sweep < 12; ++sweep) {
+    mpm::jacobi_rot(m[0], m[1], m[3], m[4], m[5], u, 0, 1);
+    mpm::jacobi_rot(m[0], m[2], m[4], m[3], m[5], u, 0, 2);
+    mpm::jacobi_rot(m[1], m[2], m[5], m[3], m[4], u, 1, 2);
+  }
+}
 }  // namespace
 
 extern "C" {
@@ -22,25 +32,36 @@ void left32(long n, const float* D, float* U, float* s, float* V, int* plain) {
     return (int)mpm::svd3_left32<true>(d, det, u, sv, sm1, is, v);
   });
 }
-// of I + D with V by Gram-Schmidt, whatever the deformation
+void left64(long n, const double* A, double* U, double* s, double* V, int* plain) {
+  each(n, A, U, s, V, plain, [](const double* a, double* u, double* sv, double* v) {
+    double is[3];
+    return (int)mpm::svd3_left64<true>(a, u, sv, is, v);
+  });
+}
+// V by Gram-Schmidt, whatever the deformation: of I + D, and of A
 void by_gram_schmidt32(long n, const float* D, float* U, float* s, float* V, int* plain) {
   each(n, D, U, s, V, plain, [](const float* d, float* u, float* sv, float* v) {
-    float m[6], ev[3], B[9], norms[3];
+    float m[6], B[9], norms[3];
     for (int i = 0; i < 3; ++i) m[i] = 2.f * d[4 * i] + mpm::dot3(d + 3 * i, d + 3 * i);
     m[3] = d[1] + d[3] + mpm::dot3(d, d + 3);
     m[4] = d[2] + d[6] + mpm::dot3(d, d + 6);
     m[5] = d[5] + d[7] + mpm::dot3(d + 3, d + 6);
-    for (int k = 0; k < 9; ++k) u[k] = k % 4 == 0;
-    for (int sweep = 0; sweep < 8; ++sweep) {
-      mpm::jacobi_rot(m[0], m[1], m[3], m[4], m[5], u, 0, 1);
-      mpm::jacobi_rot(m[0], m[2], m[4], m[3], m[5], u, 0, 2);
-      mpm::jacobi_rot(m[1], m[2], m[5], m[3], m[4], u, 1, 2);
-    }
-    for (int k = 0; k < 3; ++k) ev[k] = m[k];
+    sweeps(m, u);
     mpm::mTm(d, u, B);
     for (int k = 0; k < 9; ++k) B[k] += u[k];
-    mpm::left_gram_schmidt(u, ev, B, norms, v);
-    for (int k = 0; k < 3; ++k) sv[k] = norms[2] < 0.f && k == 2 ? -sqrtf(1.f + ev[k]) : sqrtf(1.f + ev[k]);
+    mpm::left_gram_schmidt(u, m, B, norms, v);
+    for (int k = 0; k < 3; ++k) sv[k] = norms[2] < 0.f && k == 2 ? -sqrtf(1.f + m[k]) : sqrtf(1.f + m[k]);
+    return 1;
+  });
+}
+void by_gram_schmidt64(long n, const double* A, double* U, double* s, double* V, int* plain) {
+  each(n, A, U, s, V, plain, [](const double* a, double* u, double* sv, double* v) {
+    double m[6] = {mpm::dot3(a, a),     mpm::dot3(a + 3, a + 3), mpm::dot3(a + 6, a + 6),
+                   mpm::dot3(a, a + 3), mpm::dot3(a, a + 6),     mpm::dot3(a + 3, a + 6)};
+    double B[9];
+    sweeps(m, u);
+    mpm::mTm(a, u, B);
+    mpm::left_gram_schmidt(u, m, B, sv, v);
     return 1;
   });
 }
