@@ -568,7 +568,7 @@ MPM_DI void p2g_particle_f64(const MatConsts<double>& m, const double* C, const 
 #pragma unroll
   for (int i = 0; i < 3; ++i) P.ehat[i] = eps[i] - mean;
   const double n2 = dot3(P.ehat, P.ehat) + 1e-8;
-  P.inrm = rsqrt64(n2);
+  P.inrm = rsqrt64_mid(n2);  // (a sum of squared logarithms)
   P.nrm = n2 * P.inrm;
   P.dg = P.nrm - m.ysm;
   P.yield = P.dg > 0.0;
@@ -1029,7 +1029,7 @@ MPM_DI void store_book(const MpmGridStore& st, int slot, int n) {
 
 // 1 / m of a node with mass (m > 1e-12)
 MPM_DI float node_rcp(float m) { return 1.f / m; }
-MPM_DI double node_rcp(double m) { return rcp64(m); }
+MPM_DI double node_rcp(double m) { return rcp64_normal(m); }
 
 // grid_op over the active blocks: one 64-thread CTA per block, grid-stride.
 // store_slot >= 0: list block b of grid_in and of grid_out are also copied to

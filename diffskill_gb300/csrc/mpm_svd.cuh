@@ -45,12 +45,11 @@ MPM_DI void rot_tc(float theta, float& t, float& c) {
   c = rsqrtf(fmaf(t, t, 1.0f));
 }
 
-// a / b; FP32 by the approximate reciprocal (|b| < 2^126 here), FP64 by rcp64
-// (1e-30 < |b| < 1e30).  Used for the return map, for the Jacobi angle
-// (angle_div: FP64 divides as such there), and for the SVD backward's 1 / (s_j^2 - s_i^2), whose divisor
-// is clamped to |b| >= 1e-6.  The substep kernels are built with -ftz=true, so
+// a / b; FP32 by the approximate reciprocal (|b| < 2^126 here), FP64 by rcp64_normal.
+// Used for the return map, for the Jacobi angle (angle_div: FP64 divides as such there),
+// and for the SVD backward's 1 / (s_j^2 - s_i^2), whose divisor is clamped to |b| >= 1e-6.  The substep kernels are built with -ftz=true, so
 // a subnormal s_pq compares equal to 0 and is never a divisor.
-MPM_DI double fast_div(double a, double b) { return a * rcp64(b); }
+MPM_DI double fast_div(double a, double b) { return a * rcp64_normal(b); }
 MPM_DI float fast_div(float a, float b) { return __fdividef(a, b); }
 MPM_DI double angle_div(double a, double b) { return a / b; }  // any quotient
 MPM_DI float angle_div(float a, float b) { return __fdividef(a, b); }
@@ -60,7 +59,7 @@ MPM_DI float angle_div(float a, float b) { return __fdividef(a, b); }
 // (|z| < 1/15: truncation below 3e-18 of the result)
 MPM_DI double log_strain64(double s, double sm1) {
   if (fabs(sm1) < 0.125) {
-    const double z = 2.0 * sm1 * rcp64(s + 1.0);  // 2 z
+    const double z = 2.0 * sm1 * rcp64_mid(s + 1.0);  // 2 z
     const double w = 0.25 * z * z;
     const double p = fma(w, fma(w, fma(w, fma(w, fma(w, 1.0 / 13.0, 1.0 / 11.0), 1.0 / 9.0), 1.0 / 7.0), 1.0 / 5.0),
                          1.0 / 3.0);
@@ -453,7 +452,7 @@ MPM_DI bool svd3_left64(const double* A, double* U, double* s, double* is, doubl
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    is[k] = rsqrt64(S[k]);
+    is[k] = rsqrt64_mid(S[k]);
     s[k] = S[k] * is[k];
   }
   if constexpr (WithV) {

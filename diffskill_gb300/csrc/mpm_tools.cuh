@@ -424,7 +424,7 @@ MPM_DI void local_sdf_grad(const Tool<T>& t, const T* q, T gap, T g, T* gq, T* g
   if (capsule_shape(t.type)) {
     T p2[3], dp;
     capsule_p2(t, q, p2, &dp);
-    T iL = quot(g, len14(p2));
+    T iL = quot_normal(g, len14(p2));
     gq[0] += p2[0] * iL;
     gq[1] += p2[1] * iL * dp;
     gq[2] += p2[2] * iL;
@@ -557,7 +557,7 @@ MPM_DI void shape_sdf_vjp(const Tool<T>& t, const T* pos, const T* rot, T gap, c
                           T* grot, T* ggap) {
   if (t.type == TOOL_SPHERE) {
     const T d[3] = {p[0] - pos[0], p[1] - pos[1], p[2] - pos[2]};
-    T c = quot(g, len14(d));
+    T c = quot_normal(g, len14(d));
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       if (gp) gp[k] += c * d[k];
@@ -624,7 +624,7 @@ MPM_DI void collider_v(const T* pos0, const T* rot0, const T* pos1, const T* rot
   T rel[3], nw[3];
   inv_trans(p, pos0, rot0, rel);
   qrot(rot1, rel, nw);
-  T idt = quot(T(1), dt);
+  T idt = quot_normal(T(1), dt);
 #pragma unroll
   for (int k = 0; k < 3; ++k) cv[k] = (nw[k] + pos1[k] - p[k]) * idt;
 }
@@ -633,7 +633,7 @@ MPM_DI void collider_v_vjp(const T* pos0, const T* rot0, const T* pos1, const T*
                            T* gpos0, T* grot0, T* gpos1, T* grot1) {
   T rel[3];
   inv_trans(p, pos0, rot0, rel);
-  T idt = quot(T(1), dt);
+  T idt = quot_normal(T(1), dt);
   const T gnw[3] = {g[0] * idt, g[1] * idt, g[2] * idt};
 #pragma unroll
   for (int k = 0; k < 3; ++k) gpos1[k] += gnw[k];
@@ -678,8 +678,8 @@ MPM_DI bool out_of_range(const Tool<T>& t, const T* pos, const T* rot, T gap, co
     }
     const float margin = 1e-4f + 1e-5f * (fabsf(d[0]) + fabsf(d[1]) + fabsf(d[2]));
     const float dist = shape_sdf(f, origin, r, cut_f32(gap), d) - margin;
-    const float soft = cut_f32(t.softness);
-    return dist > 0.f && (soft <= 0.f || dist * soft > 3.f);
+    // (no influence where softness <= 0: a sign or a zero high word)
+    return dist > 0.f && (__double2hiint(t.softness) <= 0 || dist * cut_f32(t.softness) > 3.f);
   } else {
     return false;
   }
@@ -712,7 +712,7 @@ MPM_DI bool collide_fwd(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, 
   T flag = (nc < T(0) && moving(vt)) ? T(1) : T(0);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    T vtf = quot(vt[k], vtn) * m;
+    T vtf = quot_normal(vt[k], vtn) * m;
     T vt2 = vtf * flag + vt[k] * (T(1) - flag);
     vout[k] = cv[k] + iv[k] * (T(1) - infl) + vt2 * infl;
   }
@@ -751,7 +751,7 @@ MPM_DI void collide_vjp(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, 
   T g_cv[3], g_iv[3], g_vt[3], g_vtf[3], g_infl = T(0);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    T vtf = quot(vt[k], vtn) * m;
+    T vtf = quot_normal(vt[k], vtn) * m;
     T vt2 = vtf * flag + vt[k] * (T(1) - flag);
     g_cv[k] = gout[k];
     g_iv[k] = gout[k] * (T(1) - infl);
@@ -760,15 +760,15 @@ MPM_DI void collide_vjp(const Tool<T>& t, const T* pos0, const T* rot0, T gap0, 
     g_vt[k] = gout[k] * infl * (T(1) - flag);
   }
   T gvtf_vt = dot3(g_vtf, vt);
-  T g_vtn = quot(-gvtf_vt * m, vtn * vtn);
-  T g_m = quot(gvtf_vt, vtn);
+  T g_vtn = quot_normal(-gvtf_vt * m, vtn * vtn);
+  T g_m = quot_normal(gvtf_vt, vtn);
   T g_nc = T(0);
   if (!(a < T(0))) {
     g_vtn += g_m;
     g_nc += g_m * t.friction;
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) g_vt[k] += quot(g_vtf[k] * m, vtn) + quot(g_vtn * vt[k], vtn);
+  for (int k = 0; k < 3; ++k) g_vt[k] += quot_normal(g_vtf[k] * m, vtn) + quot_normal(g_vtn * vt[k], vtn);
   T g_D[3] = {T(0), T(0), T(0)};
 #pragma unroll
   for (int k = 0; k < 3; ++k) g_iv[k] += g_vt[k];

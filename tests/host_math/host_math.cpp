@@ -1,7 +1,7 @@
 // Device math of mpm_math.cuh and mpm_svd.cuh, compiled for the host and called on arrays.
 #include "cuda_runtime.h"
 
-#include "mpm_svd.cuh"
+#include "math_calls.h"
 
 namespace {
 // U, s, V and 1/s of n matrices, and whether the plain form was taken
@@ -22,6 +22,10 @@ void sweeps(T* m, T* u) {
 }  // namespace
 
 extern "C" {
+int scalar(int what, int n, const double* x, double* y) {
+  for (int i = 0; i < n; ++i) y[i] = calls::call(what, x[i]);
+  return 0;
+}
 // of I + D
 void left32(long n, const float* D, float* U, float* s, float* V, int* plain) {
   each(n, D, U, s, V, plain, [](const float* d, float* u, float* sv, float* v) {

@@ -12,11 +12,14 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "diffskill_gb300", "csrc")
 
 
+INCLUDE = ["-I", os.path.join(HERE, "host_math"), "-I", CSRC]
+
+
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("host_math") / "host_math.so")
     subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fPIC", "-shared", "-Wno-unknown-pragmas",
-                    "-I", os.path.join(HERE, "host_math"), "-I", CSRC, os.path.join(HERE, "host_math", "host_math.cpp"),
+                    *INCLUDE, os.path.join(HERE, "host_math", "host_math.cpp"),
                     "-o", out], check=True)
     return ctypes.CDLL(out)
 
@@ -114,3 +117,108 @@ def test_left_svd_of_inverted_and_singular_matrices(lib, name, ulp):
     for W in (U, V):
         assert np.abs(np.linalg.det(W.astype(np.float64)) - 1).max() < 30 * ulp
     assert np.abs(np.sort(got, 1) - np.sort(s, 1)).max() < 2 * tol
+
+
+RCP, RSQRT, SQRT, LOG, EXPM1, CUT, WIDEN, EXACT, ROUND, QUOT, RCP_MID, RSQRT_MID = range(12)
+TINY, HUGE = 2.0 ** -1022, 2.0 ** 1023
+FTINY = 2.0 ** -126
+
+
+def _ftz(x):
+    """x in FP32 as a conversion under -ftz gives it: rounded to 24 bits, and what is then
+    below the normal range a zero of its sign."""
+    with np.errstate(over="ignore", invalid="ignore"):
+        x = np.asarray(x, np.float64)
+        small = (x * 2.0 ** 64).astype(np.float32).astype(np.float64) * 2.0 ** -64
+        y = np.where(abs(x) < 2.0 ** -60, small, x.astype(np.float32))
+    return np.where(abs(y) < FTINY, np.copysign(0.0, y), y).astype(np.float32)
+
+
+def _range(rng, lo, hi, n=20000):
+    """n values of both signs, their logarithms spread over [lo, hi]; and the two ends."""
+    x = np.exp2(rng.uniform(np.log2(lo), np.log2(hi), n)) * rng.choice([-1.0, 1.0], n)
+    return np.concatenate([x, [lo, -lo, hi, -hi]])
+
+
+def check_scalar_helpers(call):
+    """``call(which, x)``: the helpers against numpy over the ranges they state."""
+    rng = np.random.default_rng(6)
+    inf, nan = np.inf, np.nan
+
+    def near(got, want, ulps):
+        assert (abs(got - want) <= ulps * 2.0 ** -52 * abs(want)).all()
+
+    def same(got, want):
+        assert np.array_equal(np.asarray(got, np.float64).view(np.int64),
+                              np.asarray(want, np.float64).view(np.int64))
+
+    # half an ulp of the last rounding, the rounding of e and its cube: below 1.5 ulp
+    x = np.concatenate([_range(rng, TINY, 2.0 ** 1021), 2.0 ** np.arange(-40, 40.0), np.linspace(1, 4, 2001)])
+    near(call(RCP, x), 1 / x, 1.5)
+    near(call(QUOT, x), 3 / x, 2.5)
+    near(call(RSQRT, abs(x)), 1 / np.sqrt(abs(x)), 1.5)
+    near(call(SQRT, abs(x)), np.sqrt(abs(x)), 2.5)
+    x = np.concatenate([_range(rng, FTINY, 2.0 ** 125), np.linspace(1, 4, 2001)])
+    near(call(RCP_MID, x), 1 / x, 1.5)
+    near(call(RSQRT_MID, abs(x)), 1 / np.sqrt(abs(x)), 1.5)
+    same(call(RCP, np.array([0.0, -0.0, inf, -inf])), [inf, -inf, 0.0, -0.0])
+    same(call(RCP, np.array([HUGE, -HUGE, 1e-310])), [0.0, -0.0, inf])
+    same(call(RSQRT, np.array([0.0, 1e-310, inf])), [inf, inf, 0.0])
+    same(call(SQRT, np.array([inf])), [inf])
+    for f in (RCP, RSQRT, SQRT):
+        assert np.isnan(call(f, np.array([nan, -nan]))).all()
+    assert np.isnan(call(RSQRT, np.array([-1.0, -inf]))).all()
+    # the series and, from 1/8, the library's functions: some four roundings
+    x = np.concatenate([_range(rng, 1e-12, 0.25), [0.125, -0.125, 0.0]])
+    s = 1.0 + x
+    near(call(LOG, x), np.log1p(s - 1.0), 4)
+    near(call(EXPM1, x), np.expm1(x), 4)
+    # conversions: exact, or to nearest even
+    x = np.concatenate([_range(rng, FTINY, 2.0 ** 127), [0.0, -0.0]])
+    same(call(CUT, x), (x.view(np.int64) & ~0x1fffffff).view(np.float64))
+    same(call(CUT, np.array([inf, -inf, nan, 2.0 ** 128, FTINY / 2])), [0.0, -0.0, 0.0, 0.0, 0.0])
+    f = _ftz(x)
+    same(call(WIDEN, f.astype(np.float64)), f)
+    f = np.concatenate([f, np.float32([inf, -inf, FTINY / 2, -FTINY / 2])])
+    same(call(EXACT, f.astype(np.float64)), _ftz(f))
+    assert np.isnan(call(EXACT, np.array([nan]))).all() and np.isnan(call(ROUND, np.array([nan, -nan]))).all()
+    one, ulp = np.array([1.0, 1.0 + 2.0 ** -23, 1.5]), 2.0 ** -23
+    ties = np.concatenate([one + ulp / 2, one + ulp / 2 + 2.0 ** -52, one + ulp / 2 - 2.0 ** -52, one + ulp / 4])
+    edge = np.array([2.0 ** 128, 2.0 ** 128 * (1 - 2.0 ** -25), 2.0 ** 128 * (1 - 2.0 ** -24), 3e38, 1e39, inf,
+                     FTINY * (1 - 2.0 ** -30), FTINY * (1 - 2.0 ** -24), FTINY / 2, 1e-60])
+    x = np.concatenate([_range(rng, 1e-50, 1e45), ties, -ties, edge, -edge, [0.0, -0.0]])
+    same(call(ROUND, x), _ftz(x))
+
+
+def test_scalar_helpers_on_the_host(lib):
+    """Over all of FP64's range, its ends, rounding ties, infinities and NaN."""
+    def call(which, x):
+        x = np.ascontiguousarray(x, np.float64)
+        y = np.zeros_like(x)
+        assert lib.scalar(which, len(x), _ptr(x), _ptr(y)) == 0
+        return y
+
+    check_scalar_helpers(call)
+
+
+@pytest.mark.gpu
+def test_scalar_helpers_on_the_device(tmp_path):
+    """The same with the device's own approximations of 1/x and 1/sqrt(x), compiled with
+    the substep's flags."""
+    import torch
+
+    from diffskill_gb300 import build
+
+    out = str(tmp_path / "device_math.so")
+    subprocess.run([build.nvcc(), *build.ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", *build._FAST32,
+                    "-I", CSRC, "-o", out, os.path.join(HERE, "host_math", "device_math.cu"), "-lcudart"], check=True)
+    dev = ctypes.CDLL(out)
+
+    def call(which, x):
+        a = torch.as_tensor(np.ascontiguousarray(x, np.float64), device="cuda")
+        y = torch.zeros_like(a)
+        torch.cuda.synchronize()
+        assert dev.scalar(which, a.numel(), ctypes.c_void_p(a.data_ptr()), ctypes.c_void_p(y.data_ptr())) == 0
+        return y.cpu().numpy()
+
+    check_scalar_helpers(call)
