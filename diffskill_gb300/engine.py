@@ -392,9 +392,10 @@ class GridStore:
         # per stored block: the p2g grid block, then the grid_op output block
         self.blocks = torch.empty((max(self.capacity, 1), 2, 64, 4), dtype=eng.dtype, device=dev)
         self.block_ids = torch.empty(max(self.capacity, 1), dtype=torch.int32, device=dev)
-        self.slot_start = torch.full((n_slots,), -1, dtype=torch.int64, device=dev)
-        self.slot_count = torch.empty(n_slots, dtype=torch.int32, device=dev)  # read where slot_start >= 0
-        self.bump = torch.zeros(1, dtype=torch.int64, device=dev)
+        words = torch.empty(1 + n_slots + (n_slots + 1) // 2, dtype=torch.int64, device=dev)
+        self.bump, self.slot_start = words[:1], words[1:1 + n_slots]
+        self.slot_count = words[1 + n_slots:].view(torch.int32)[:n_slots]  # read where slot_start >= 0
+        self.reset()
         st = _lib.MpmGridStore()
         st.blocks = self.blocks.data_ptr()
         st.block_ids = self.block_ids.data_ptr()

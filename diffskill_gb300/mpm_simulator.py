@@ -96,24 +96,30 @@ class MPMSimulator:
         self.grid_m_t = torch.zeros((1, eng.G), dtype=eng.dtype, device=eng.device)
         self.grid_m_grad_t = torch.zeros_like(self.grid_m_t)
         # which entries of a tool's pose are its state, and where the flat action's
-        # entries sit in an action's [T, 8] row
-        state = torch.zeros((T, 8), dtype=torch.bool)
-        for i, p in enumerate(self.primitives):
-            state[i, :p.state_dim] = True
-        self._state_mask = state.to(eng.device)
+        # entries sit in an action's [T, 8] row (one copy to the device for both)
         dims = self.primitives.action_dims
-        self._act_index = torch.tensor([8 * i + k for i in range(eng.T) for k in range(dims[i + 1] - dims[i])],
-                                       dtype=torch.long, device=eng.device)
+        state = [0] * (8 * T)
+        for i, p in enumerate(self.primitives):
+            state[8 * i:8 * i + p.state_dim] = [1] * p.state_dim
+        index = [8 * i + k for i in range(eng.T) for k in range(dims[i + 1] - dims[i])]
+        both = torch.tensor(state + index, dtype=torch.long).to(eng.device)
+        self._state_mask = both[:8 * T].reshape(T, 8) != 0
+        self._act_index = both[8 * T:]
         # the grids of each substep, for its adjoint: slot s belongs to substep(s) as it
         # last ran, and is emptied whenever frame s or the poses of frames s, s + 1 change
-        free, _ = torch.cuda.mem_get_info(eng.device)
         block = 2 * 64 * 4 * (8 if eng.dtype == torch.float64 else 4) + 4
         # a particle touches at most 8 of the grid's blocks; 512 and one per 64 particles
         # hold a dough several times over (30,000 particles in a 64^3 grid touch 108,
         # 100,000 in a 128^3 grid 400).  All blocks of a 64^3 grid, 436 MB for 25 FP64
         # substeps, took 0.4 ms to allocate; a substep that does not fit is recomputed
         worst = M * min((eng.n_grid // 4) ** 3, 8 * max(eng.P, 1), 512 + eng.P // 64)
-        self._store = GridStore(eng, M, min(worst, min(1 << 30, free // 16) // block))
+        most = 1 << 28
+        if worst * block > most:  # (asking for the free memory takes 18 us)
+            most = max(most, min(1 << 30, torch.cuda.mem_get_info(eng.device)[0] // 16))
+        try:
+            self._store = GridStore(eng, M, min(worst, most // block))
+        except torch.cuda.OutOfMemoryError:
+            self._store = GridStore(eng, M, 0)  # every adjoint substep recomputes its grids
         self.cur = 0
 
     def _t64(self, a) -> torch.Tensor:
@@ -242,8 +248,11 @@ class MPMSimulator:
             s = np.asarray(s, dtype=np.float64).reshape(-1)
             new[i, :len(s)] = s
             given[i, :len(s)] = True
-        both = self._t64(np.stack([new, given]))
-        self._pose[f].copy_(torch.where(both[1] != 0, both[0], self._pose[f]))
+        if given.all():
+            self._pose[f].copy_(torch.from_numpy(new))
+        else:
+            both = self._t64(np.stack([new, given]))
+            self._pose[f].copy_(torch.where(both[1] != 0, both[0], self._pose[f]))
         self._store.reset() if f == 0 else self._store.forget(f - 1, f)
 
     def reset(self, x) -> None:
