@@ -418,6 +418,16 @@ class GridStore:
         if first <= last:
             self.slot_start[first:last + 1].fill_(-1)
 
+    def drop(self, first: int) -> None:
+        """Empty slots ``first`` and up, and give the space behind the slots below them
+        back (device-side; capturable)."""
+        if first <= 0:
+            return self.reset()
+        start = self.slot_start[:first]
+        ends = torch.where(start >= 0, start + self.slot_count[:first], 0)
+        self.bump.copy_(ends.max())
+        self.slot_start[first:].fill_(-1)
+
     def bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (self.blocks, self.block_ids, self.slot_start,
                                                            self.slot_count, self.bump))
@@ -543,6 +553,16 @@ class Horizon:
         need = (max(len(self.boundaries), 1), max(self.eng.P, 1))
         if self.perms is None or self.perms.shape[0] < need[0]:
             self.perms = torch.zeros(need, dtype=torch.int32, device=self.eng.device)
+
+    def drop(self, first: int) -> None:
+        """Empty slots ``first`` and up, and give the space behind the slots below them
+        back (device-side; capturable)."""
+        if first <= 0:
+            return self.reset()
+        start = self.slot_start[:first]
+        ends = torch.where(start >= 0, start + self.slot_count[:first], 0)
+        self.bump.copy_(ends.max())
+        self.slot_start[first:].fill_(-1)
 
     def bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in

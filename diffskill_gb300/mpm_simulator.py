@@ -120,6 +120,7 @@ class MPMSimulator:
             self._store = GridStore(eng, M, min(worst, most // block))
         except torch.cuda.OutOfMemoryError:
             self._store = GridStore(eng, M, 0)  # every adjoint substep recomputes its grids
+        self._booked = self._again = 0  # slots from _booked up are empty; substeps run again
         self.cur = 0
 
     def _t64(self, a) -> torch.Tensor:
@@ -134,7 +135,7 @@ class MPMSimulator:
             eng.softness = softness
             from . import _lib
             _lib.check(eng.lib.mpm_set_tools(eng.h, eng._descs, eng.T), eng.h, "mpm_set_tools")
-            self._store.reset()
+            self._forget_all()
 
     # ------------------------------------------------------------- tools
     def _set_action(self, s: int, action: np.ndarray, only: Optional[int] = None) -> None:
@@ -172,7 +173,20 @@ class MPMSimulator:
         """Substeps first .. first + n - 1 in order."""
         if not 0 <= first <= first + n < self.max_steps:
             raise IndexError(f"substeps {first} .. {first + n - 1} run past max_steps={self.max_steps}")
+        if first < self._booked:
+            # run again: its grids take new space.  Once that is as many substeps as there
+            # are, what the later slots hold is given back (30 us; the store has room for
+            # several times as many)
+            self._again += n
+            if self._again >= self.max_steps:
+                self._again = 0
+                self._store.drop(first)
+        self._booked = max(self._booked, first + n)
         self._eng.substeps(self._frames[first], self._pose[first], n, self._store, first)
+
+    def _forget_all(self) -> None:
+        self._store.reset()
+        self._booked = self._again = 0
 
     def substep_grad(self, s: int) -> None:
         """``substep_grad`` (mpm_simulator.py:325-345): frame-(s+1) adjoint -> frame s (accumulated)."""
@@ -199,7 +213,7 @@ class MPMSimulator:
     def copyframe(self, source: int, target: int) -> None:
         self._frames[target].copy_(self._frames[source])
         self._pose[target].copy_(self._pose[source])
-        self._store.reset()
+        self._forget_all()
 
     # ----------------------------------------------------------------- io
     def _rows(self, f: int, r0: int, r1: int) -> np.ndarray:
@@ -253,7 +267,7 @@ class MPMSimulator:
         else:
             both = self._t64(np.stack([new, given]))
             self._pose[f].copy_(torch.where(both[1] != 0, both[0], self._pose[f]))
-        self._store.reset() if f == 0 else self._store.forget(f - 1, f)
+        self._forget_all() if f == 0 else self._store.forget(f - 1, f)
 
     def reset(self, x) -> None:
         """``reset`` (402-413): x given, v = 0, F = I, C = 0 at frame 0."""
@@ -261,7 +275,7 @@ class MPMSimulator:
         if self._eng is None or x.shape[0] != self.n_particles[None]:
             self.initialize(x.shape[0])
         self._frames[0].copy_(self._eng.init_state([x]))
-        self._store.reset()
+        self._forget_all()
         self.cur = 0
 
     def get_m(self) -> np.ndarray:
