@@ -36,7 +36,7 @@ CANDIDATES: Dict[str, Sequence[int]] = {
     "g2p_adj_ctas": (8, 5, 6, 7),
     "p2g_adj_ctas": (4, 5, 6),
     "grid_ctas_per_sm": (16, 8, 32),
-    "g2p_ctas": (8, 10, 12),
+    "g2p_ctas": (8, 10, 12),  # (10 and 12 gather lane by lane; 8 by cell in large sorted batches)
     "grid_op_adj_ctas": (6, 12, 16),
 }
 # the profiler kinds (diffskill_gb300._lib.KERNEL_KINDS) whose times decide each field

@@ -47,6 +47,7 @@ struct MpmHandle {
   cudaMemPool_t pool = nullptr;  // scratch of single calls, ordered by their streams
   int* d_order = nullptr;     // particles by cell for the substeps of mpm_substeps_fwd / _bwd; always a permutation
   mpm::Done ordered;          // d_order was sorted
+  bool sorts = false;         // mpm_sort_frame was called: the frames are sorted by cell now and then
   // pipelined adjoint (mpm_set_pipelined_adjoint): the grid preparation of an
   // adjoint substep runs on pipe_side beside the previous substep's p2g.grad
   bool pipelined = false;
@@ -131,6 +132,7 @@ mpm::LaunchCtx ctx(MpmHandle* h, void* stream) {
   L.launches = &h->launches;
   L.prof = &h->prof;
   L.tune = h->tune;
+  L.sorted = h->sorts;
   return L;
 }
 // the capture that work submitted to the stream is recorded in (0: none, it runs)
@@ -682,7 +684,9 @@ int check_sortable(MpmHandle* h, const char* fn) {
 // particles and a few substeps have to earn.  19 substeps forward / adjoint in the
 // caller's order and by cell, us: FP32 16,000 particles 480 / 665 and 497 / 686,
 // 30,000 624 / 821 and 541 / 787, 100,000 1,670 / 1,439 and 869 / 1,269; FP64 8,000
-// 1,717 / 3,435 and 1,702 / 3,430, 16,000 2,089 / 3,624 and 1,867 / 3,566.  An
+// 1,717 / 3,435 and 1,702 / 3,430, 16,000 2,089 / 3,624 and 1,867 / 3,566.  FP32 state with
+// the FP64 SVD: 8,000 649 / 2,186 and 673 / 2,193, 20,000 760 / 2,327 and 772 / 2,302,
+// 30,000 925 / 2,707 and 895 / 2,532, 100,000 2,202 / 5,850 and 2,226 / 5,578.  An
 // adjoint run takes the order of the last forward run: any permutation is right,
 // and a particle seldom changes its cell within an action.  It sorts for itself when
 // no run has, or only one in another capture, which may never be replayed.
@@ -790,6 +794,7 @@ int mpm_sort_frame(MpmHandle* h, const void* src, void* dst, int32_t* perm, void
                       ? mpm::launch_sort_frame<double>(L, (const double*)src, (double*)dst, perm, h->sort)
                       : mpm::launch_sort_frame<float>(L, (const float*)src, (float*)dst, perm, h->sort);
   if (e != cudaSuccess) return cuda_fail(h, e, "mpm_sort_frame");
+  h->sorts = true;
   return MPM_OK;
 }
 

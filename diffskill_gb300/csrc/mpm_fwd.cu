@@ -135,8 +135,8 @@ cudaError_t launch_substep_fwd(const LaunchCtx& L, const T* st0, T* st1, const d
         MPM_G2P((k_g2p<T, 10>));
       else if (v == 12)
         MPM_G2P((k_g2p<T, 12>));
-      else if (!L.order && c.n_particles > (int64_t)8 * bs * L.sm_count)
-        // more than a wave of CTAs, particles sorted by cell (measured at the kernel)
+      else if (L.sorted && !L.order && c.n_particles > (int64_t)8 * bs * L.sm_count)
+        // more than a wave of CTAs, of a caller that re-sorts its frames (measured at the kernel)
         MPM_G2P((k_g2p<T, 0, true>));
       else
         MPM_G2P(k_g2p<T>);

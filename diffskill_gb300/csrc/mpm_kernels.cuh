@@ -1171,9 +1171,12 @@ MPM_DI bool g2p_particle(const Consts<T>& c, const T* __restrict__ st, T* __rest
 // FP32, one gather of the nodes per cell of a warp, as in g2p.grad: the lanes of a cell
 // find each other by __match_any_sync, 27 lanes fetch the cell's nodes, all read them
 // from shared memory.  For launches of more than one wave, where the L1's wavefronts
-// bound the gathers (1.1M particles 36.6 -> 34.3 us, 0.8M 28.6 -> 26.6); smaller ones
-// wait for one warp's chain, which the grouping makes longer (30,000 particles in the
-// caller's order 8.3 -> 9.6 us), so they gather lane by lane.
+// bound the gathers (1.1M particles of one scene by cell 34.6 -> 30.6 us, 200,000 11.9
+// -> 11.1); smaller ones wait for one warp's chain, which the grouping makes longer
+// (30,000 particles in the caller's order 8.3 -> 9.6 us), so they gather lane by lane.
+// So do the frames of callers that never sort them: their warps hold more cells than fit
+// and gather lane by lane here too, from an L1 that the stages have halved (unsorted
+// 400,000 particles 30.5 us without the stages and 38.5 with them, 1.1M 65 and 85).
 struct GatherStage {
   float4 nodes[kStagedGroups][27];
   const Node<float>* base[kStagedGroups];

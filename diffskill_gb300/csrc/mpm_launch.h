@@ -50,6 +50,7 @@ struct LaunchCtx {
   int64_t* launches;           // launch counter
   Profiler* prof;              // may be null
   MpmTuning tune = {0, 0, 0, 0, 0, 0};  // launch shapes (mpm_set_tuning); 0 = default
+  bool sorted = false;         // the caller re-sorts its frames by cell (has called mpm_sort_frame)
   const int* order = nullptr;  // [n_particles] particle of each thread of the scattering kernels; null: thread i, particle i
   bool add = false;            // the adjoint adds to the gradient frame it writes
 };
