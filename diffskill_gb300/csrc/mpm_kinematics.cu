@@ -12,7 +12,8 @@
 //                         (primive_base.py:135-150) and Box._project (primitives.py:370-372)
 //
 // One warp per scene.  A scene without collision pairs and rolling pins: eight lanes
-// per tool, one per component of its pose (ToolLane).  Any other: lane t runs the
+// per tool, one per component of its pose (ToolLane; of more than four tools only in
+// actions of more than 12 substeps).  Any other: lane t runs the
 // kinematics of the scene's tool t, then the warp evaluates each collision pair's 600
 // surface points together.  The
 // adjoint follows the reference's autodiff: apply_collision_projection.grad and
@@ -503,10 +504,14 @@ MPM_DI void lanes_action_bwd(const MpmToolDesc* __restrict__ tools, int t0, int 
     }
   }
 }
-// no lane needs the whole pose of a tool
-MPM_DI bool by_component(const MpmToolDesc* __restrict__ tools, int t0, int nt, int np) {
+// No lane needs the whole pose of a tool, and the warp's four tools at a time are worth
+// it: more than four take two turns of the start and end of a chain, which only more
+// than a dozen substeps earn (5 tools by component and by tool, forward / adjoint, us: 4
+// substeps 20.5 / 43.0 and 18.5 / 32.8, 12 32.8 / 71.7 and 32.8 / 69.7, 19 43.0 / 94.3 and
+// 43.0 / 102.5; up to four tools, 1 substep 10.2 / 18.5 and 14.3 / 20.5).
+MPM_DI bool by_component(const MpmToolDesc* __restrict__ tools, int t0, int nt, int np, int n_sub) {
   const int lane = threadIdx.x & 31;
-  return np == 0 && !__any_sync(0xffffffffu, lane < nt && rolling_pin(tools[t0 + lane].type));
+  return np == 0 && (nt <= 4 || n_sub > 12) && !__any_sync(0xffffffffu, lane < nt && rolling_pin(tools[t0 + lane].type));
 }
 
 __global__ void k_tools_action(const MpmToolDesc* __restrict__ tools, const int* __restrict__ tool_off,
@@ -518,7 +523,7 @@ __global__ void k_tools_action(const MpmToolDesc* __restrict__ tools, const int*
   const int lane = threadIdx.x & 31;
   const int t0 = tool_off[scene], nt = tool_off[scene + 1] - t0;
   const int np = pair_off[scene + 1] - pair_off[scene];
-  if (by_component(tools, t0, nt, np)) {
+  if (by_component(tools, t0, nt, np, n_sub)) {
     lanes_action(tools, t0, nt, n_tools, action, vel, pose, n_sub);
     return;
   }
@@ -553,7 +558,7 @@ __global__ void k_tools_action_bwd(const MpmToolDesc* __restrict__ tools, const 
   const int lane = threadIdx.x & 31;
   const int t0 = tool_off[scene], nt = tool_off[scene + 1] - t0;
   const int np = pair_off[scene + 1] - pair_off[scene];
-  if (by_component(tools, t0, nt, np)) {
+  if (by_component(tools, t0, nt, np, n_sub)) {
     lanes_action_bwd(tools, t0, nt, n_tools, vel, pose, g_pose, g_action, n_sub);
     return;
   }

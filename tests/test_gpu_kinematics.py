@@ -45,3 +45,9 @@ def test_eight_lanes_per_tool_match_oracle(gpu_lib, n_tools, n_sub):
         eng.tools_action_bwd(v, p, g, ga)
         assert rel_err(g.cpu().numpy(), g_ref) < 1e-11
         assert rel_err(ga.cpu().numpy()[:, :7], ga_ref) < 1e-11
+
+
+# on both sides of where more than four tools take a lane per component
+@pytest.mark.parametrize("n_sub", [12, 13])
+def test_five_tools_at_the_line_between_the_two_forms(gpu_lib, n_sub):
+    test_eight_lanes_per_tool_match_oracle(gpu_lib, 5, n_sub)
