@@ -245,23 +245,41 @@ class MPMSimulator:
         n = len(state[0])
         if self._eng is None or n != self.n_particles[None]:
             self.initialize(n)
-        # the rows are transposed and rounded to the frame's type on the device
-        for rows, a in ((slice(0, 3), state[0]), (slice(3, 6), state[1]), (slice(15, 24), state[2]),
-                        (slice(6, 15), state[3])):
-            self._frames[f, rows, :n].copy_(self._t64(a).reshape(n, -1).t())
-        self._set_poses(f, {i: s for i, s in enumerate(state[4:4 + self.n_primitive])})
+        # everything is checked before the first write: a state that is refused changes no
+        # frame.  The rows are transposed and rounded to the frame's type on the device.
+        def rows(a):  # [n, 3], or what broadcasts to it
+            t = self._t64(np.asarray(a, dtype=np.float64).T)
+            while t.dim() > 2 and t.shape[0] == 1:
+                t = t[0]
+            return t.expand(3, n)
+
+        frame = self._frames[f, :, :n]
+        parts = [(frame[0:3], rows(state[0])), (frame[3:6], rows(state[1])),
+                 (frame[15:24], self._t64(state[2]).reshape(n, 9).t()),
+                 (frame[6:15], self._t64(state[3]).reshape(n, 9).t())]
+        poses = self._pose_rows(dict(enumerate(state[4:4 + self.n_primitive])))
+        for part, a in parts:
+            part.copy_(a)
+        self._write_poses(f, *poses)
 
     def set_primitive_state(self, f: int, state) -> None:
-        self._set_poses(f, {i: s for i, s in enumerate(state[4:4 + self.n_primitive])})
+        self._set_poses(f, dict(enumerate(state[4:4 + self.n_primitive])))
 
     def _set_poses(self, f: int, states: dict) -> None:
         """Leading pose entries of the tools ``states`` at frame ``f``."""
+        self._write_poses(f, *self._pose_rows(states))
+
+    def _pose_rows(self, states: dict):
+        """The tools' poses with the entries of ``states``, and which entries these are."""
         new = np.full((max(self.n_primitive, 1), 8), np.nan)
         given = np.zeros(new.shape, dtype=bool)
         for i, s in states.items():
             s = np.asarray(s, dtype=np.float64).reshape(-1)
             new[i, :len(s)] = s
             given[i, :len(s)] = True
+        return new, given
+
+    def _write_poses(self, f: int, new: np.ndarray, given: np.ndarray) -> None:
         if given.all():
             self._pose[f].copy_(torch.from_numpy(new))
         else:

@@ -104,3 +104,31 @@ def test_running_from_a_later_frame_again_keeps_the_store(gpu_lib):
         # and a loop's; another action touches a few blocks more
         assert int(sim._store.bump) <= 1.3 * used * (F + sim.max_steps + 2 * SUB + 2) / F
     _check(sc, sim, range(F))
+
+
+# shapes of a state's parts that would only fit after a reshape or a broadcast, another
+# number of particles, a tool's state that is too long
+REFUSED = {
+    "x [n, 1, 3]": (0, lambda a: a[:, None, :]),
+    "v [3, n]": (1, lambda a: a.T),
+    "v flat": (1, lambda a: a.reshape(-1)),
+    "F [n, 1]": (2, lambda a: a[:, 0, :1]),
+    "C [n, 1]": (3, lambda a: a[:, 0, :1]),
+    "F of fewer particles": (2, lambda a: a[1:]),
+    "a tool of nine entries": (4, lambda a: np.zeros(9)),
+}
+
+
+@pytest.mark.parametrize("what", REFUSED)
+def test_a_state_of_the_wrong_shape_is_refused_and_changes_nothing(gpu_lib, what):
+    sc, env, acts = _env()
+    sim = env.simulator
+    _forward(sim, acts)
+    frames, pose = sim._frames.clone(), sim._pose.clone()
+    part, change = REFUSED[what]
+    st = _state(sim, 4, 0.004)
+    st[part] = change(st[part])
+    with pytest.raises((RuntimeError, ValueError)):
+        sim.set_state(4, st)
+    assert torch.equal(sim._frames, frames) and torch.equal(sim._pose, pose)
+    _check(sc, sim, range(F))
