@@ -285,7 +285,8 @@ class MPMSimulator:
         else:
             both = self._t64(np.stack([new, given]))
             self._pose[f].copy_(torch.where(both[1] != 0, both[0], self._pose[f]))
-        self._forget_all() if f == 0 else self._store.forget(f - 1, f)
+        # (counted from the end, f is another frame and another row of poses: forget all)
+        self._forget_all() if f <= 0 else self._store.forget(f - 1, f)
 
     def reset(self, x) -> None:
         """``reset`` (402-413): x given, v = 0, F = I, C = 0 at frame 0."""

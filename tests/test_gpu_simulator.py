@@ -57,6 +57,12 @@ def _state(sim, f, shift):
     return st
 
 
+# frames counted from the end are frames, and rows of poses, of their own
+MUTATE_FROM_THE_END = {
+    "set_state": lambda sim: sim.set_state(-6, _state(sim, -6, 0.004)),
+    "set_primitive_state": lambda sim: sim.set_primitive_state(-7, _state(sim, -7, 0.004)),
+    "a tool's position": lambda sim: sim.primitives[0].set_state(-5, sim._pose[-5, 0, :3].cpu().numpy() + 0.003),
+}
 MUTATE = {
     "set_state at 0": lambda sim, acts: sim.set_state(0, _state(sim, 0, 0.004)),
     "set_state at 4": lambda sim, acts: sim.set_state(4, _state(sim, 4, 0.004)),
@@ -82,6 +88,14 @@ def test_gradients_after_a_change_without_a_new_forward(gpu_lib, what):
     assert sim._store.stored_slots() == F
     MUTATE[what](sim, acts)
     _check(sc, sim, range(F))
+
+
+@pytest.mark.parametrize("what", MUTATE_FROM_THE_END)
+def test_gradients_after_a_change_counted_from_the_end(gpu_lib, what):
+    sc, env, acts = _env()
+    _forward(env.simulator, acts)
+    MUTATE_FROM_THE_END[what](env.simulator)
+    _check(sc, env.simulator, range(F))
 
 
 def test_running_from_a_later_frame_again_keeps_the_store(gpu_lib):
