@@ -43,8 +43,11 @@ struct MpmHandle {
   void* d_tools_t = nullptr;  // tools in the compute precision (converted by mpm_set_tools)
   void* d_poses_t = nullptr;  // poses of the current substep in the compute precision
   mpm::SortScratch sort;      // particle re-sort (mpm_sort_frame)
-  std::mutex pool_mu;
-  cudaMemPool_t pool = nullptr;  // scratch of single calls, ordered by their streams
+  // scratch of single calls, ordered by their streams (call_scratch)
+  std::mutex scratch_mu;
+  unsigned char* d_scratch = nullptr;   // for the calls of one stream
+  unsigned long long scratch_stream = 0;  // its id (0: none yet)
+  cudaMemPool_t pool = nullptr;         // for the others
   int* d_order = nullptr;     // particles by cell for the substeps of mpm_substeps_fwd / _bwd; always a permutation
   mpm::Done ordered;          // d_order was sorted
   bool sorts = false;         // mpm_sort_frame was called: the frames are sorted by cell now and then
@@ -145,18 +148,30 @@ unsigned long long capture_of(void* stream) {
   }
   return st == cudaStreamCaptureStatusActive ? id : 0;
 }
-// Scratch of one call, to be given back by cudaFreeAsync on the same stream (nullptr
-// when there is no memory): calls on several streams have their own.  It comes from a
-// pool of the handle, which keeps up to 32 MiB (2 us for both calls; the device's
-// default pool returns everything at each synchronisation), and in a capture from the
-// graph's memory.
+// Scratch of one call, to be given back by return_scratch on the same stream (nullptr
+// when there is no memory).  The calls of the stream that asks first share d_scratch, which
+// costs nothing (a first trace of a small image took 0.54 ms from the pool, whose creation
+// is most of the difference, and takes 0.45); the caller holds scratch_mu until its work is
+// submitted, so that two threads' calls do not mix.  Calls on other streams have memory of
+// their own, from a pool of the handle that keeps up to 32 MiB (2 us for both calls; the
+// device's default pool returns everything at each synchronisation), and calls in a
+// capture from the graph's memory.
+constexpr size_t kOwnScratch = 64 << 10;
 unsigned char* call_scratch(MpmHandle* h, size_t bytes, cudaStream_t stream) {
   void* ptr = nullptr;
   cudaError_t e;
   if (capture_of(stream) != 0) {
     e = cudaMallocAsync(&ptr, bytes, stream);
   } else {
-    std::lock_guard<std::mutex> lk(h->pool_mu);
+    unsigned long long id = 0;  // (unique in the process, so no later stream has it)
+    if (bytes <= kOwnScratch && cudaStreamGetId(stream, &id) != cudaSuccess) {
+      cudaGetLastError();
+      id = 0;
+    }
+    if (id != 0) {
+      if (h->scratch_stream == 0) h->scratch_stream = id;
+      if (h->scratch_stream == id) return h->d_scratch;
+    }
     e = cudaSuccess;
     if (!h->pool) {
       cudaMemPoolProps props = {};
@@ -173,6 +188,9 @@ unsigned char* call_scratch(MpmHandle* h, size_t bytes, cudaStream_t stream) {
   if (e == cudaSuccess) return (unsigned char*)ptr;
   cudaGetLastError();
   return nullptr;
+}
+cudaError_t return_scratch(MpmHandle* h, unsigned char* ptr, cudaStream_t stream) {
+  return ptr && ptr != h->d_scratch ? cudaFreeAsync(ptr, stream) : cudaSuccess;
 }
 int check_device(MpmHandle* h) {
   int dev = -1;
@@ -262,6 +280,7 @@ int mpm_create(const MpmParams* params, const int64_t* scene_offsets, MpmHandle*
   part(&h->sort.keys_b, np * sizeof(uint32_t));
   part(&h->sort.vals_b, np * sizeof(int32_t));
   part(&h->d_order, np * sizeof(int));
+  part(&h->d_scratch, kOwnScratch);
   part(&h->sort.hist, mpm::sort_hist_words(p.n_particles) * sizeof(uint32_t));
   bool ok = cudaMalloc(&h->arena, at) == cudaSuccess;
   for (auto& q : parts) *q.first = ok ? h->arena + q.second : nullptr;
@@ -1020,16 +1039,15 @@ int mpm_render_trace(MpmHandle* h, const MpmRenderVolume* vol, const MpmRenderVi
   MPM_TRY(check_aligned(h, color, "color"));
   MPM_TRY(check_aligned(h, image, "image", true));
   mpm::LaunchCtx L = ctx(h, stream);
+  std::lock_guard<std::mutex> lk(h->scratch_mu);
   unsigned char* empty = view->show_particles ? call_scratch(h, mpm::render_bricks(*vol), L.stream) : nullptr;
   cudaError_t e = h->p.precision == MPM_PREC_FP64
                       ? mpm::launch_render_trace<double>(L, *vol, *view, t0, nt, pose, tool_color, empty, depth,
                                                          normal, color, image)
                       : mpm::launch_render_trace<float>(L, *vol, *view, t0, nt, pose, tool_color, empty, depth,
                                                         normal, color, image);
-  if (empty) {
-    const cudaError_t freed = cudaFreeAsync(empty, L.stream);
-    if (e == cudaSuccess) e = freed;
-  }
+  const cudaError_t freed = return_scratch(h, empty, L.stream);
+  if (e == cudaSuccess) e = freed;
   return e == cudaSuccess ? MPM_OK : cuda_fail(h, e, "mpm_render_trace");
 }
 

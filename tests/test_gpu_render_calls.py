@@ -62,6 +62,29 @@ def test_traces_of_two_volumes_on_two_streams(gpu_lib):
                 assert torch.equal(o[k], ref[i][k]), k
 
 
+def test_traces_beside_the_stream_that_traced_first(gpu_lib):
+    """The handle's own scratch belongs to the stream of its first trace: traces on another
+    stream at the same time, and on a third after it, have theirs."""
+    a, b, sa, sb = _two_renderers()
+    first, second, third = (torch.cuda.Stream() for _ in range(3))
+    a.set_particles(sa)
+    b.set_particles(sb)
+    torch.cuda.synchronize()
+    outs = {id(a): [], id(b): []}
+    for _ in range(8):
+        for r, stream in ((a, first), (b, second), (b, first), (a, third)):
+            with torch.cuda.stream(stream):
+                outs[id(r)].append(r.trace())
+    torch.cuda.synchronize()
+    for r in (a, b):
+        ref = r.trace()
+        torch.cuda.synchronize()
+        for o in outs[id(r)]:
+            for k in KEYS:
+                assert torch.equal(o[k], ref[k]), k
+    assert not torch.equal(outs[id(a)][0]["depth"], outs[id(b)][0]["depth"])
+
+
 def test_captured_trace(gpu_lib):
     """The first trace of a handle, recorded in a graph and replayed twice."""
     a, _, st, _ = _two_renderers()
