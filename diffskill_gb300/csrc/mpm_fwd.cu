@@ -36,10 +36,7 @@ Consts<T> make_consts(const LaunchCtx& L) {
     using S = std::decay_t<decltype(m.dt)>;
     const double mu2 = 2.0 * double(c.mu);
     m.dt = S(c.dt);
-    m.lam = S(c.lam);
-    m.ks = S(c.ks);
     m.p_mass = S(c.p_mass);
-    m.mu2 = S(mu2);
     m.mu2ks = S(mu2 * double(c.ks));
     m.lamks = S(double(c.lam) * double(c.ks));
     m.ysm = S(double(c.yield_stress) / mu2);

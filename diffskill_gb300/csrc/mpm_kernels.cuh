@@ -47,9 +47,9 @@ struct alignas(4 * sizeof(T)) Node {
 // products that every thread would otherwise form (on the FP64 pipe, in FP64)
 template <typename S>
 struct MatConsts {
-  S dt, lam, ks, p_mass;
-  S mu2, mu2ks, lamks;  // 2 mu, 2 mu ks, lam ks
-  S ysm;                // yield_stress / (2 mu)
+  S dt, p_mass;
+  S mu2ks, lamks;  // 2 mu ks, lam ks
+  S ysm;           // yield_stress / (2 mu)
 };
 
 template <typename T>
@@ -417,7 +417,7 @@ struct P2G {
   S U[9], s[3], V[9];
   S is[3];   // 1 / s (0: the SVD was plain, see svd3_left32 and svd3_left64)
   S sm1[3];  // s - 1 (FP32: from the shifted SVD, exact as s -> 1)
-  S sigc[3], ehat[3], nrm, inrm, dg, k, e[3];  // inrm = 1 / nrm (FP64 only)
+  S ehat[3], nrm, inrm, dg, k, e[3];  // inrm = 1 / nrm (FP64 only)
   bool yield;
   S J;
   S em1[3];  // singular values of newF minus 1 (e - 1 when yielding, else s - 1)
@@ -463,9 +463,7 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
   float eps[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const bool above = 0.05f < P.s[i];
-    P.sigc[i] = above ? P.s[i] : 0.05f;
-    eps[i] = above ? log1p_strain(P.sm1[i]) : logf(0.05f);
+    eps[i] = 0.05f < P.s[i] ? log1p_strain(P.sm1[i]) : logf(0.05f);
   }
   const float esum = eps[0] + eps[1] + eps[2];
   const float mean = third(esum);
@@ -495,7 +493,7 @@ MPM_DI void p2g_particle_f32(const MatConsts<float>& m, const float* C, const fl
     }
   }
   // the return map keeps the volume, unless a singular value sits at the 0.05
-  // floor (then J = prod sigc)
+  // floor (then J is the product of the clamped values)
   if (P.yield && !(0.05f < P.s[0] && 0.05f < P.s[1] && 0.05f < P.s[2])) Jm1 = expm1f(esum);
   P.J = 1.f + Jm1;
   // (newF - R) newF^T = U diag(e - 1) V^T V diag(e) U^T = U diag((e - 1) e) U^T
@@ -675,7 +673,7 @@ MPM_DI void return_map_sigma_grad(const P2G<S>& P, const S* MN, S* gs) {
     if constexpr (sizeof(S) == 8)
       gs[i] = (S(0.05) < P.s[i]) ? g_eps[i] * P.is[i] : S(0);
     else
-      gs[i] = (S(0.05) < P.s[i]) ? fast_div(g_eps[i], P.sigc[i]) : S(0);
+      gs[i] = (S(0.05) < P.s[i]) ? fast_div(g_eps[i], P.s[i]) : S(0);
   }
 }
 
