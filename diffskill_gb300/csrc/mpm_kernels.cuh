@@ -24,7 +24,7 @@
 // in the adjoint).  So no pass over the particles only marks blocks and none only
 // clears the grid.  One substep of 64 scenes (1.1M particles, 32 us of compulsory
 // traffic): with the marking in g2p and a compaction that also clears, p2g 82,
-// grid_op 14, g2p 48, clear 8 us; now 85, 14, 37 and 7.  Both kernels store the zeros
+// grid_op 14, g2p 48, clear 8 us; now 85, 14, 37 (34 with the gathers by cell) and 7.  Both kernels store the zeros
 // last: next to the load of the same node they cost grid_op 12 us and grid_op.grad
 // 12 (34 against 22).  Nodes outside the list hold no mass, so grid_op leaves them at
 // zero exactly as the dense reference does; g2p and p2g.grad only read nodes inside
@@ -1608,9 +1608,9 @@ __global__ void __launch_bounds__(64, MB > 0 ? MB : (sizeof(T) == 4 ? 6 : 1)) k_
 // p2g.grad + svd_grad + compute_F_tmp.grad: gathers g_in; reads the partial
 // x gradient left in g0 by k_g2p_adj and writes all 24 rows of g0 (add: adds to
 // rows 3..23; k_g2p_adj already added rows 0..2 to theirs).
-// FP32: 4 CTAs of 128 threads per SM by default (128 registers, 48 B of spill;
-// 1.1M particles: 4, 5, 6 CTAs 112.7, 118.8, 130.0 us, the latter spilling 160
-// and 430 B); MB > 0: MB CTAs per SM (MpmTuning.p2g_adj_ctas)
+// FP32: 4 CTAs of 128 threads per SM by default (128 registers, 88 B of spill stores and
+// 108 of loads; 1.1M particles: 4, 5, 6 CTAs 112.7, 118.8, 130.0 us, the latter spilling
+// 444 / 572 and 632 / 744 B); MB > 0: MB CTAs per SM (MpmTuning.p2g_adj_ctas)
 template <typename T, typename S, int MB = 0>
 __global__ void __launch_bounds__(kParticleThreads<S>, MB > 0 ? MB : (sizeof(S) == 4 ? 4 : 8)) k_p2g_adj(Consts<T> c, const T* __restrict__ st, const T* __restrict__ g1,
                                                  T* __restrict__ g0, const int* __restrict__ pscene, bool add,

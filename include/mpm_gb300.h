@@ -7,8 +7,13 @@
  * plb/engine/primitive/primive_base.py.  Host code (Python, ctypes) keeps the
  * reference's API and owns all state buffers; this library receives raw
  * device pointers and sizes, launches on the caller's CUDA stream, and never
- * frees caller memory.  The only memory it owns is the per-handle grid
- * scratch allocated by mpm_create and freed by mpm_destroy.
+ * frees caller memory.  The memory it owns is each handle's: grids and scratch
+ * allocated by mpm_create, and a pool of at most 32 MiB once traces run on a
+ * second stream (mpm_render_trace); mpm_destroy frees both.
+ *
+ * A handle serves one substep, adjoint or sort at a time.  Such calls must not
+ * overlap on the GPU: between substeps the p2g grid and its block flags are
+ * zero, and overlapping calls leave values there that later substeps add to.
  *
  * Layouts (all device pointers, "real" = float or double per precision):
  *   particle state of one frame: real[24][ld], component-major (SoA):
