@@ -185,8 +185,11 @@ constexpr float kShiftedTol = 1e-14f;
 // forward pass, which needs no V, then has neither a product A V nor a Gram-Schmidt,
 // and V = A^T U diag(1/s) takes their place in the adjoint.  The values are in no
 // particular order (nothing depends on it).  A rotation scales its two columns by
-// sqrt(c^2 + s^2) = 1 + O(1e-7), so each column is normalised once at the end by
-// 3/2 - |u|^2 / 2.  detA = det(I + D).  V is written when WithV; is = 1/s.
+// sqrt(c^2 + s^2) = 1 + O(1e-7), so each column is normalised once at the end
+// (unit_column).  So is each column of V, whose length has the error of the approximate
+// is, mostly of one sign: the adjoint takes an elastic particle's gradient of F through
+// U (U^T g V) V^T in every substep, and 3e-8 each time made the action gradients of 5,000
+// substeps 1e-4 to 2e-4 too small.  detA = det(I + D).  V is written when WithV; is = 1/s.
 //
 // U carries a rounding error of 1e-7, and A^T U / s that error times the ratio of A's
 // longest to its shortest axis.  So an inverted or strongly deformed matrix,
@@ -198,6 +201,15 @@ constexpr float kShiftedTol = 1e-14f;
 // 6.7e-7).  Below kLeftNorm2 the two agree to 3 %; dough, which yields at strains near
 // 0.01, is far below it.
 constexpr float kLeftNorm2 = 0.5f;
+// the column u of a 3x3 matrix, of length 1 + O(1e-7), normalised: u + u (1 - |u|^2) / 2.
+// (The factor 3/2 - |u|^2 / 2 itself, rounded above and below 1 to different spacings,
+// leaves columns 1e-8 short on average.)
+MPM_DI void unit_column(float* u) {
+  const float e = 0.5f * fmaf(-u[6], u[6], fmaf(-u[3], u[3], fmaf(-u[0], u[0], 1.f)));
+  u[0] = fmaf(u[0], e, u[0]);
+  u[3] = fmaf(u[3], e, u[3]);
+  u[6] = fmaf(u[6], e, u[6]);
+}
 template <bool WithV>
 MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* sm1, float* is, float* V) {
   float ev[3], norm2;
@@ -221,12 +233,7 @@ MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* s
     norm2 = a00 * a00 + a11 * a11 + a22 * a22;
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float f = 1.5f - 0.5f * (U[k] * U[k] + U[3 + k] * U[3 + k] + U[6 + k] * U[6 + k]);
-    U[k] *= f;
-    U[3 + k] *= f;
-    U[6 + k] *= f;
-  }
+  for (int k = 0; k < 3; ++k) unit_column(U + k);
   if (!(norm2 < kLeftNorm2 && detA > 0.f)) {
     float B[9], n[3];
     mTm(D, U, B);
@@ -258,6 +265,8 @@ MPM_DI bool svd3_left32(const float* D, float detA, float* U, float* s, float* s
     for (int r = 0; r < 3; ++r)
 #pragma unroll
       for (int k = 0; k < 3; ++k) V[r * 3 + k] = (V[r * 3 + k] + U[r * 3 + k]) * is[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) unit_column(V + k);
   }
   return false;
 }
