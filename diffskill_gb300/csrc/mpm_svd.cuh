@@ -188,8 +188,8 @@ constexpr float kShiftedTol = 1e-14f;
 // sqrt(c^2 + s^2) = 1 + O(1e-7), so each column is normalised once at the end
 // (unit_column).  So is each column of V, whose length has the error of the approximate
 // is, mostly of one sign: the adjoint takes an elastic particle's gradient of F through
-// U (U^T g V) V^T in every substep, and 3e-8 each time made the action gradients of 5,000
-// substeps 1e-4 to 2e-4 too small.  detA = det(I + D).  V is written when WithV; is = 1/s.
+// U (U^T g V) V^T in every substep, and 2e-8 to 7e-8 each time made the action gradients
+// of 5,000 substeps 1e-4 to 2e-4 too small.  detA = det(I + D).  V is written when WithV; is = 1/s.
 //
 // U carries a rounding error of 1e-7, and A^T U / s that error times the ratio of A's
 // longest to its shortest axis.  So an inverted or strongly deformed matrix,
